@@ -90,6 +90,98 @@ __device__ __forceinline__ void block_sum(double (&v)[NV]) {
   __syncthreads();
 }
 
+// Per-step scalars of the device-resident Lanczos recurrence.  st layout:
+//   st[0..1] raw sum conj(Q)(HQ) from hv   st[2] acc   st[3] s (scale of Q)
+//   st[4] sweep coefficient alpha*s       st[5] |w|^2 from the sweep
+// phase 0 (after hv, step k):    alpha_k = s^2 Re(raw); coef = alpha_k * s
+// phase 1 (after sweep, step k): beta_k = sqrt(|w|^2); acc = -beta_k * s; s = 1/beta_k
+__device__ __forceinline__ void lanczos_scalar_update(int phase, int k, double *st, double *alpha, double *beta) {
+  if (phase == 0) {
+    const double s = st[3];
+    const double a = s * s * st[0];
+    alpha[k] = a;
+    st[4] = a * s;
+  } else {
+    const double b = sqrt(st[5]);
+    beta[k] = b;
+    st[2] = -b * st[3];
+    st[3] = 1.0 / b;
+  }
+}
+
+// Where a launch's sum goes: `nrec` records of partial sums at `part`, this launch's blocks
+// writing records [rec0, rec0 + gridDim.x) (the records before them come from an earlier
+// launch on the same stream); phase < 0: no scalar update.
+struct SumOut {
+  double *part;
+  int rec0, nrec;
+  unsigned *done;
+  double *out;
+  int phase;
+  LanczosTail lt;
+};
+
+inline SumOut sum_out(double *part, int rec0, int nrec, unsigned *done, double *out, int phase = -1,
+                      const LanczosTail *lt = nullptr) {
+  return SumOut{part, rec0, nrec, done, out, lt ? phase : -1, lt ? *lt : LanczosTail{0, nullptr, nullptr, nullptr}};
+}
+
+// Sum over all records by the block that finishes last (atomicInc wraps `done` back to zero for
+// the next launch), in record order, so the result does not depend on which block that is.  A
+// one-block launch for this sum took 5 us after every H*v, sweep and dot (its start, then the
+// latency of ~1200 records); here the last block's part is ~1.5 us and the launch is gone.
+// write(v): stores the sums (thread 0 of the last block).
+template <int NV, typename Write>
+__device__ __forceinline__ void grid_sum(double (&v)[NV], const SumOut &s, Write write) {
+  __shared__ int s_last;
+  block_sum<NV>(v);
+  if (threadIdx.x == 0) {
+    double *p = s.part + (size_t)(s.rec0 + blockIdx.x) * NV;
+#pragma unroll
+    for (int k = 0; k < NV; k++) p[k] = v[k];
+    __threadfence();
+    s_last = atomicInc(s.done, gridDim.x - 1) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+#pragma unroll
+  for (int k = 0; k < NV; k++) v[k] = 0.0;
+  for (int i = threadIdx.x; i < s.nrec; i += blockDim.x)
+#pragma unroll
+    for (int k = 0; k < NV; k++) v[k] += __ldcg(s.part + (size_t)i * NV + k);
+  block_sum<NV>(v);
+  if (threadIdx.x == 0) {
+    write(v);
+    if (s.phase >= 0) lanczos_scalar_update(s.phase, s.lt.k, s.lt.st, s.lt.alpha, s.lt.beta);
+  }
+}
+template <int NV>
+__device__ __forceinline__ void grid_sum(double (&v)[NV], const SumOut &s) {
+  grid_sum<NV>(v, s, [&](const double(&w)[NV]) {
+#pragma unroll
+    for (int k = 0; k < NV; k++) s.out[k] = w[k];
+  });
+}
+
+// Launches a kernel that begins with cudaGridDependencySynchronize: its CTAs may take their places
+// while the kernel before it on the stream drains, so the launch itself (1-2 us, as long as the
+// work of a small sector's vector kernel) is not waited for.
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // Sums `n` partial records of NV doubles (stride NV) into out[0..NV).  One block.
 template <int NV>
 __global__ void finalize_partials_kernel(const double *__restrict__ part, int n, double *__restrict__ out) {

@@ -440,10 +440,9 @@ int lanczos_run(Sector *s, VecType vt, const double *h_init, const LanczosOption
   }
   void *pp = P.p, *qq = Q.p;
   auto do_step = [&](int k) -> int {
-    RET(hv_native(s, vt, qq, pp, st + 2, st + 0));
-    RET(lanczos_scalars(s, 0, k, st, (double *)AL.p, (double *)BE.p));
-    RET(vec_lanczos_sweep(s, vt, st + 4, pp, qq, st + 5));
-    RET(lanczos_scalars(s, 1, k, st, (double *)AL.p, (double *)BE.p));
+    const LanczosTail lt{k, st, (double *)AL.p, (double *)BE.p};
+    RET(hv_native(s, vt, qq, pp, st + 2, st + 0, true, &lt));
+    RET(vec_lanczos_sweep(s, vt, st + 4, pp, qq, st + 5, &lt));
     std::swap(pp, qq);
     return 0;
   };

@@ -23,6 +23,8 @@ struct RowBlockPlan;
 // Real or complex double scalar for host/device code.
 struct cplx { double x, y; };
 
+constexpr int kHvBlockMax = 8;  // vectors of one block product
+
 enum VecType : int { kReal64 = 0, kComplex128 = 1 };
 
 // Upper-half entry of the split-term plan: source row = row + delta (grand-canonical
@@ -36,12 +38,20 @@ struct HiEnt {
 // lower-half terms, per upper half the applicable upper-half terms, the rest generic.
 // Device pointers; lo_ptr == nullptr means no plan (every term generic).
 struct SplitPlan {
-  uint32_t *lo_ptr = nullptr, *lo_ent = nullptr, *hi_ptr = nullptr;
+  uint32_t *lo_ptr = nullptr, *lo_ent = nullptr, *hi_ptr = nullptr;  // lo_ptr: entries of each lower half
+  uint32_t lo_stride = 0;  // lo_ent[slot * lo_stride + lower half]
   HiEnt *hi_ent = nullptr;
   double *coef = nullptr;
   BitTerm *gen = nullptr;  // terms left to the generic path
   int ngen = 0;
   int64_t n_lo_ent = 0, n_hi_ent = 0;
+};
+
+// Scalar bookkeeping of one Lanczos step, done by the launch that produces its sum: the H*v
+// (phase 0) and the sweep (phase 1) of step k (lanczos_scalar_update, device_util.cuh).
+struct LanczosTail {
+  int k;
+  double *st, *alpha, *beta;
 };
 
 struct Sector {
@@ -67,6 +77,8 @@ struct Sector {
   int ndterms = 0;
   double *d_red = nullptr;         // reduction partials
   double *d_scal = nullptr;        // small device scalars (dot results)
+  unsigned *d_done = nullptr;      // kHvBlockMax counters of finished blocks (grid_sum), zero between launches;
+                                   // in the last d_scal slots
   int red_blocks = 0;
   int num_sms = 0;
   // Optional specialised plan (canonical Hubbard).  When present, the drivers keep
@@ -91,6 +103,15 @@ int split_plan_for_terms(Sector *s, const std::vector<BitTerm> &T, SplitPlan *pl
                          std::vector<int> *gen_out, std::string *err);
 void split_plan_free(SplitPlan *p);
 
+// A canonical sector's blocks: the rows sharing upper half ib are [row0, row0 + n), their lower
+// halves low[low0, low0 + n).  Blocks whose lower halves are the same, in the same order, share
+// them in `low` (a class); a lower half is in at most one class.
+struct SectorBlock {
+  uint32_t ib, row0, low0, n;
+};
+int sector_blocks(const Sector *s, std::vector<SectorBlock> *out, std::vector<uint32_t> *low, std::string *err);
+constexpr int kBlockPiece = 512;  // rows of a block taken by one warp
+
 // specialise = false skips the specialised kernel plans (the batched engine uses the
 // general row kernel only).
 int sector_build(const Model &m, int device, Sector **out, std::string *err, bool specialise = true);
@@ -101,7 +122,8 @@ void sector_free(Sector *s);
 // v0 = acc * v0 + s * (H v1) with (acc, s) = d_coef[0..1] read on the device, and the raw
 // sum_r conj(v1[r]) (H v1)[r] written to d_out[0..1] (re, im).  HPhi's mltply
 // (src/mltply.c:56-132) is acc = s = 1, prdct = d_out.  acc == 0 never reads v0.
-int hv_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out);
+int hv_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
+              const LanczosTail *lt = nullptr);
 
 // Native vector order: HPhi order unless a specialised plan defines its own (then an
 // exact per-block permutation of it).  hv_native runs the fastest kernel on native
@@ -111,12 +133,11 @@ bool has_native_order(const Sector *s);
 // hv_block_applies): v0_b = acc_b * v0_b + scale_b * H v1_b with (acc_b, scale_b) at
 // d_coef + b * cstride and <v1_b|H v1_b> at d_out + b * ostride; d_part holds
 // 2 * nb * red_blocks doubles.
-constexpr int kHvBlockMax = 8;
 bool hv_block_applies(const Sector *s, VecType vt);
 int hv_block_native(Sector *s, VecType vt, int nb, int64_t stride, const void *d_v1, void *d_v0,
                     const double *d_coef, int cstride, double *d_out, int ostride, double *d_part);
 int hv_native(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
-              bool acc_read = true);
+              bool acc_read = true, const LanczosTail *lt = nullptr);
 int to_native(Sector *s, VecType vt, const void *d_hphi, void *d_native);
 int from_native(Sector *s, VecType vt, const void *d_native, void *d_hphi);
 // hv_native with caller-provided scratch: d_part receives the per-block partial sums
@@ -139,12 +160,13 @@ int vec_axpby(Sector *s, VecType vt, double a, const void *d_x, double b, void *
 int vec_scale(Sector *s, VecType vt, double a, void *d_x);
 // Lanczos sweep: p = p - alpha*sq*q in place and d_out[0] = |p|^2 (one pass).
 int vec_lanczos_sweep(Sector *s, VecType vt, const double *d_alpha_scale, void *d_p, const void *d_q,
-                      double *d_out);
+                      double *d_out, const LanczosTail *lt = nullptr);
 // Diagonal observables of a vector: d_out[0] = sum |v|^2 n_up n_dn over sites (doublon),
 // d_out[1] = sum |v|^2 * Sz, d_out[2] = sum |v|^2 * N.
 int vec_diag_observables(Sector *s, VecType vt, const void *d_v, double *d_out);
 
-// Device-side Lanczos scalar update (see vecops.cu); st is a device array of >= 6 doubles.
+// Device-side Lanczos scalar update as a launch of its own (lanczos_scalar_update); st is a
+// device array of >= 6 doubles.
 int lanczos_scalars(Sector *s, int phase, int k, double *st, double *alpha, double *beta);
 // p = p - a_sq*q; vg += c_over_b * p  (eigenvector replay)
 int vec_replay_sweep(Sector *s, VecType vt, double a_sq, double c_over_b, void *p, const void *q, void *vg);

@@ -26,12 +26,14 @@ namespace {
 constexpr int kHvThreads = 256;
 constexpr int kSmemTermMax = 1024;  // 48 KiB of BitTerm
 
+// Eight blocks per SM for real vectors (32 registers): the grid is 8 blocks per SM, and at 40
+// registers a second wave took the 24-site chain's H*v from 146 to 187 us.
 template <typename T, bool GC, bool SMEM>
-__global__ void __launch_bounds__(kHvThreads) hv_general_kernel(
+__global__ void __launch_bounds__(kHvThreads, sizeof(T) == 8 ? 8 : 4) hv_general_kernel(
     int64_t dim, const uint64_t *__restrict__ list_1, const uint32_t *__restrict__ l21,
     const uint32_t *__restrict__ l22, int lo_bits, uint64_t lo_mask, SplitView split,
     const BitTerm *__restrict__ gterms, int nterms, const double *__restrict__ diag, const T *__restrict__ v1,
-    T *__restrict__ v0, const double *__restrict__ coef, double *__restrict__ part) {
+    T *__restrict__ v0, const double *__restrict__ coef, SumOut so) {
   const double acc = coef[0], scale = coef[1];
   extern __shared__ BitTerm sterms[];
   const BitTerm *terms = gterms;
@@ -68,15 +70,11 @@ __global__ void __launch_bounds__(kHvThreads) hv_general_kernel(
     y = VT<T>::scale(scale, y);
     v0[r] = (acc == 0.0) ? y : VT<T>::add(VT<T>::scale(acc, v0[r]), y);
   }
-  block_sum<2>(pr);
-  if (threadIdx.x == 0) {
-    part[2 * blockIdx.x] = pr[0];
-    part[2 * blockIdx.x + 1] = pr[1];
-  }
+  grid_sum<2>(pr, so);
 }
 
 template <typename T, bool GC>
-void launch_general(Sector *s, const T *v1, T *v0, const double *coef) {
+void launch_general(Sector *s, const T *v1, T *v0, const double *coef, const SumOut &so) {
   const int grid = s->red_blocks;
   const uint64_t lo_mask = s->ihfbit - 1;
   const SplitView sv = split_view(s->split);
@@ -84,11 +82,11 @@ void launch_general(Sector *s, const T *v1, T *v0, const double *coef) {
     const size_t smem = sizeof(BitTerm) * (size_t)s->split.ngen;
     hv_general_kernel<T, GC, true><<<grid, kHvThreads, smem, s->stream>>>(
         s->dim, s->d_list_1, s->d_list_2_1, s->d_list_2_2, s->lo_bits, lo_mask, sv, s->split.gen, s->split.ngen,
-        s->d_diag, v1, v0, coef, s->d_red);
+        s->d_diag, v1, v0, coef, so);
   } else {
     hv_general_kernel<T, GC, false><<<grid, kHvThreads, 0, s->stream>>>(
         s->dim, s->d_list_1, s->d_list_2_1, s->d_list_2_2, s->lo_bits, lo_mask, sv, s->split.gen, s->split.ngen,
-        s->d_diag, v1, v0, coef, s->d_red);
+        s->d_diag, v1, v0, coef, so);
   }
 }
 
@@ -152,9 +150,10 @@ __global__ void __launch_bounds__(kHvThreads) hv_block_kernel(
       const uint32_t ia = (uint32_t)(c & lo_mask);
       const uint64_t ib = c >> lo_bits;
       const int64_t base = GC ? (int64_t)(c & ~lo_mask) : (int64_t)__ldg(l22 + ib) - 3;
-      const uint32_t l0 = __ldg(split.lo_ptr + ia), l1 = __ldg(split.lo_ptr + ia + 1);
-      for (uint32_t e = l0; e < l1; e++) {
-        const uint32_t v = __ldg(split.lo_ent + e);
+      const uint32_t nl = __ldg(split.lo_ptr + ia);
+      const uint32_t *le = split.lo_ent + ia;
+      for (uint32_t e = 0; e < nl; e++, le += split.lo_stride) {
+        const uint32_t v = __ldg(le);
         const uint32_t tgt = v & ((1u << kSplitTargetBits) - 1u);
         const uint32_t k = v >> kSplitTargetBits;
         const int64_t j = GC ? (base | (int64_t)tgt) : base + (int64_t)tgt;
@@ -286,20 +285,24 @@ int hv_block_native(Sector *s, VecType vt, int nb, int64_t stride, const void *d
   return 0;
 }
 
-int hv_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out) {
+int hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
+                      double *d_part, const LanczosTail *lt) {
   if (vt == kReal64 && s->model.complex_terms) {
     set_error("H has complex coefficients: real vectors are not allowed");
     return -1;
   }
-  if (rb_applies(s, vt)) return rb_hv_launch(s, vt, d_v1, d_v0, d_coef, d_out);
-  if (vt == kReal64) {
-    if (s->gc) launch_general<double, true>(s, (const double *)d_v1, (double *)d_v0, d_coef);
-    else launch_general<double, false>(s, (const double *)d_v1, (double *)d_v0, d_coef);
-  } else {
-    if (s->gc) launch_general<cplx, true>(s, (const cplx *)d_v1, (cplx *)d_v0, d_coef);
-    else launch_general<cplx, false>(s, (const cplx *)d_v1, (cplx *)d_v0, d_coef);
+  if (rb_applies(s, vt)) {
+    if (rb_hv_launch_scratch(s, vt, d_v1, d_v0, d_coef, d_out, d_part) != 0) return -1;
+    return lt ? lanczos_scalars(s, 0, lt->k, lt->st, lt->alpha, lt->beta) : 0;
   }
-  finalize_partials_kernel<2><<<1, 256, 0, s->stream>>>(s->d_red, s->red_blocks, d_out);
+  const SumOut so = sum_out(d_part, 0, s->red_blocks, s->d_done, d_out, 0, lt);
+  if (vt == kReal64) {
+    if (s->gc) launch_general<double, true>(s, (const double *)d_v1, (double *)d_v0, d_coef, so);
+    else launch_general<double, false>(s, (const double *)d_v1, (double *)d_v0, d_coef, so);
+  } else {
+    if (s->gc) launch_general<cplx, true>(s, (const cplx *)d_v1, (cplx *)d_v0, d_coef, so);
+    else launch_general<cplx, false>(s, (const cplx *)d_v1, (cplx *)d_v0, d_coef, so);
+  }
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error(std::string("hv launch failed: ") + cudaGetErrorString(e));
@@ -308,44 +311,13 @@ int hv_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double 
   return 0;
 }
 
-int hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
-                      double *d_part) {
-  if (vt == kReal64 && s->model.complex_terms) {
-    set_error("H has complex coefficients: real vectors are not allowed");
-    return -1;
+int hv_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
+              const LanczosTail *lt) {
+  if (rb_applies(s, vt)) {
+    if (rb_hv_launch(s, vt, d_v1, d_v0, d_coef, d_out) != 0) return -1;
+    return lt ? lanczos_scalars(s, 0, lt->k, lt->st, lt->alpha, lt->beta) : 0;
   }
-  if (rb_applies(s, vt)) return rb_hv_launch_scratch(s, vt, d_v1, d_v0, d_coef, d_out, d_part);
-  const int grid = s->red_blocks;
-  const uint64_t lo_mask = s->ihfbit - 1;
-  const bool smem_terms = s->split.ngen <= kSmemTermMax;
-  const size_t smem = smem_terms ? sizeof(BitTerm) * (size_t)s->split.ngen : 0;
-  const SplitView sv = split_view(s->split);
-#define HPHI_GENERAL_LAUNCH(T, GC)                                                                              \
-  do {                                                                                                          \
-    if (smem_terms)                                                                                             \
-      hv_general_kernel<T, GC, true><<<grid, kHvThreads, smem, s->stream>>>(                                    \
-          s->dim, s->d_list_1, s->d_list_2_1, s->d_list_2_2, s->lo_bits, lo_mask, sv, s->split.gen,             \
-          s->split.ngen, s->d_diag, (const T *)d_v1, (T *)d_v0, d_coef, d_part);                               \
-    else                                                                                                        \
-      hv_general_kernel<T, GC, false><<<grid, kHvThreads, 0, s->stream>>>(                                      \
-          s->dim, s->d_list_1, s->d_list_2_1, s->d_list_2_2, s->lo_bits, lo_mask, sv, s->split.gen,             \
-          s->split.ngen, s->d_diag, (const T *)d_v1, (T *)d_v0, d_coef, d_part);                               \
-  } while (0)
-  if (vt == kReal64) {
-    if (s->gc) HPHI_GENERAL_LAUNCH(double, true);
-    else HPHI_GENERAL_LAUNCH(double, false);
-  } else {
-    if (s->gc) HPHI_GENERAL_LAUNCH(cplx, true);
-    else HPHI_GENERAL_LAUNCH(cplx, false);
-  }
-#undef HPHI_GENERAL_LAUNCH
-  finalize_partials_kernel<2><<<1, 256, 0, s->stream>>>(d_part, grid, d_out);
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    set_error(std::string("hv launch failed: ") + cudaGetErrorString(e));
-    return -1;
-  }
-  return 0;
+  return hv_launch_scratch(s, vt, d_v1, d_v0, d_coef, d_out, s->d_red, lt);
 }
 
 size_t hv_scratch_doubles(const Sector *s, VecType vt) {
@@ -359,16 +331,19 @@ int hv_native_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const
                       double *d_part, int *d_counter) {
   if (s->prod) return prod_hv_launch_scratch(s, vt, d_v1, d_v0, d_coef, d_out, d_part, d_counter);
   if (s->hub) return hub_hv_launch_scratch(s, vt, d_v1, d_v0, d_coef, d_out, d_part, d_counter);
-  return hv_launch_scratch(s, vt, d_v1, d_v0, d_coef, d_out, d_part);
+  return hv_launch_scratch(s, vt, d_v1, d_v0, d_coef, d_out, d_part, nullptr);
 }
 
 bool has_native_order(const Sector *s) { return s->hub != nullptr || s->prod != nullptr; }
 
 int hv_native(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
-              bool acc_read) {
-  if (s->prod) return prod_hv_launch(s, vt, d_v1, d_v0, d_coef, d_out);
-  if (s->hub) return hub_hv_launch(s, vt, d_v1, d_v0, d_coef, d_out, acc_read);
-  return hv_launch(s, vt, d_v1, d_v0, d_coef, d_out);
+              bool acc_read, const LanczosTail *lt) {
+  if (s->prod) return prod_hv_launch(s, vt, d_v1, d_v0, d_coef, d_out, lt);
+  if (s->hub) {
+    if (hub_hv_launch(s, vt, d_v1, d_v0, d_coef, d_out, acc_read) != 0) return -1;
+    return lt ? lanczos_scalars(s, 0, lt->k, lt->st, lt->alpha, lt->beta) : 0;
+  }
+  return hv_launch(s, vt, d_v1, d_v0, d_coef, d_out, lt);
 }
 
 int to_native(Sector *s, VecType vt, const void *in, void *out) {

@@ -18,29 +18,22 @@
 // (down hops) alone:
 //   (H v)[u, d] = D(u, d) v[u, d] + sum_{down hops} c(d) v[u, d'] + sum_{up hops} c(u) v[u', d].
 //
-// Kernel: persistent CTAs take whole rows u from an atomic dispenser.  The row v1[u, :]
-// (C(N, Ndown) elements) is staged in shared memory; down hops are gathers inside it driven
-// by an ELL table ell_dn[slot][d] (source rank, coefficient index), read coalesced across
-// the lanes that own consecutive d; up hops of the row (the same for every d) are staged in
-// shared memory and applied as coalesced reads of the source rows v1[u', :]; the diagonal is
-// rebuilt from per-species tables plus U * popcount(u & d) (or read when it has other
-// cross-species terms).  Each row's <v1|H v1> contribution is reduced in the CTA and summed
-// over rows in a fixed order afterwards, so results do not depend on scheduling.
+// Two passes: a row pass (diagonal + down hops: every row is a gather inside itself) and a column
+// pass (up hops: whole source rows), for real and complex vectors and any coefficients that fall
+// into at most kMaxGroups values up to sign.  The row pass stages rows in shared memory (a complex
+// row as its two planes) and reads them through an edge-coloured gather table per coefficient:
+// within each slot of a warp, the 16 lanes of a half-warp hit 16 different shared-memory bank
+// pairs, so every 8-byte gather takes the minimum two wavefronts; entries are 16-bit word indices
+// with the hop's sign in bit 15, eight per lane in one 16-byte load, and empty slots point at zero
+// words placed one per bank.  The column pass walks the matrix in column chunks (all rows of chunk
+// 0, then chunk 1, ...) so the source rows of the chunk being processed stay in L2 while every row
+// gathers its ~N/2 up-hop sources.  Both passes take their work by static striding and keep
+// per-CTA partial sums of <v1|H v1>; the last CTA of the column pass adds them up in order.
 //
-// Two-pass form (real vectors, down hops of one magnitude |t|; the default there).  H v is
-// split into a row pass (diagonal + down hops: every row is a gather inside itself) and a
-// column pass (up hops: whole source rows).  The row pass stages two rows per CTA in shared
-// memory and reads them through an edge-coloured gather table: within each slot of a warp,
-// the 16 lanes of a half-warp hit 16 different shared-memory bank pairs, so every 8-byte
-// gather takes the minimum two wavefronts; entries are 16-bit word indices with the hop's
-// sign in bit 15, eight per lane in one 16-byte load issued a column block ahead, and empty
-// slots point at zero words placed one per bank.  The column pass walks
-// the matrix in column chunks (all rows of chunk 0, then chunk 1, ...) so the source rows of
-// the chunk being processed stay in L2 while every row gathers its ~N/2 up-hop sources; a
-// warp takes one row and 128 columns, its lanes hold the row's packed hop entries and
-// broadcast them by shuffles, and every source row is read as two 512-byte warp loads.
-// Both passes take their work by static striding (no dispenser) and keep per-CTA partial
-// sums of <v1|H v1>, so the result is reproducible.
+// One pass (no down hops, more coefficients than groups, or HPHI_B200_PROD=single): persistent
+// CTAs take whole rows u from an atomic dispenser; down hops are gathers inside the staged row
+// driven by an ELL table ell_dn[slot][d] (source rank, coefficient index), up hops coalesced reads
+// of the source rows; each row's <v1|H v1> is reduced in the CTA and summed over rows afterwards.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -224,85 +217,89 @@ __global__ void __launch_bounds__(kProdThreads, 2) prod_hv_kernel(ProdArgs a, co
   retire(counter);
 }
 
-constexpr int kDownThreads = 1024;            // row pass: one CTA per SM, two rows at a time
-constexpr int kRow2Bytes = 103168;            // shared-memory offset of the second row (>= (12870 + 16) * 8)
-constexpr int kUpThreads = 128;               // column pass
-constexpr int kUpBatch = 8;                   // source loads in flight per thread
-constexpr int kUpMinBlocks = 12;               // CTAs per SM (40 registers)
-constexpr int kUpChunk = 2 * kUpThreads;      // columns per column-pass task (two per thread)
-
-struct TwoPassArgs {
-  int npad;                    // Dc rounded up to a multiple of 32
-  int groups;                  // slot groups of 8 stored per warp (max over warps)
-  const uint4 *gat;            // [npad / 32][groups][32 lanes] 8 entries: word | sign << 15
-  const uint8_t *wslots;       // [npad / 32] slots of each warp's 32 columns
-  double t_dn;                 // magnitude of every down hop
-  double t_up;                 // magnitude of every up hop (up_uniform)
-  int up_uniform;              // usrc carries the sign in bit 31 and ucf is unused
-  const int *usrc;             // [Uc][wu] up-hop source rank
-  const double *ucf;           // [Uc][wu] up-hop coefficient
-  const uint8_t *nus;          // [Uc] up hops of each row
-  const uint32_t *usrc16;      // [Uc][wu2] two up hops per word: rank | sign << 15 (16 bits each)
-  int wu2;                     // words per row of usrc16 (0: no packed table)
-};
-
 __device__ __forceinline__ double flip_sign(double x, uint32_t sg) {
   return __hiloint2double(__double2hiint(x) ^ (int)sg, __double2loint(x));
 }
 
-// Row pass: v0[u, :] = acc * v0[u, :] + scale * (D + down hops) v1[u, :] for two rows at a time;
-// part[blockIdx] = sum over the CTA's rows of v1 . (D + down) v1.  The two rows are staged
-// by bulk asynchronous copies completing on an mbarrier (per-thread cp.async when the rows
-// are not 16-byte aligned); a bounded wait that gives up makes the CTA's partial sum NaN.
-// Gathers: each 16-bit table entry (word | sign << 15) serves both rows.
-__global__ void __launch_bounds__(kDownThreads, 1) prod_down_kernel(ProdArgs a, TwoPassArgs b,
-                                                                   const double *__restrict__ v1,
-                                                                   double *__restrict__ v0,
-                                                                   const double *__restrict__ coef,
-                                                                   double *__restrict__ part) {
-  extern __shared__ __align__(128) double rows[];  // row 0 at 0, row 1 at kRow2Bytes; each Dc + 16 words
+constexpr int kMaxGroups = 8;     // coefficients of one species, up to sign (two-pass kernels)
+constexpr int kUpThreads = 256;   // column pass: 8 warps per CTA
+constexpr int kUpMinBlocks = 3;   // CTAs per SM (at most 85 registers)
+constexpr int kUpChunk = 128;     // doubles of a row per warp task (4 per lane)
+constexpr int kUpBatch = 4;       // up hops per batch: 64 bytes per lane and hop pair in flight
+
+// Hops of one species are grouped by coefficient up to sign; the row pass walks one gather
+// table per group and multiplies each group's signed sum once, so no coefficient is looked up
+// per element.
+struct TwoPassArgs {
+  int npad;                    // Dc rounded up to a multiple of 32
+  int ng;                      // groups of down hops
+  const uint4 *gat;            // per warp of 32 columns its groups' sets of 8 slots: [32 lanes] 8 entries word | sign << 15
+  const uint4 *whead;          // per warp: first set, slots of groups 0-3 and 4-7 (8 bits each)
+  const double2 *cf_dn;        // [ng] coefficients
+  const uint8_t *nus;          // [Uc] up hops of each row
+  int wu2;                     // words per row of up_ent
+  const uint32_t *up_ent;      // [Uc][wu2] one group: two hops per word, rank | sign << 15 (16 bits each);
+                               // several: one hop per word, rank | (2 * group + sign) << 16
+  const double2 *cf_up;        // [up groups] coefficients
+  int ngu;
+};
+
+// Row pass shapes by row length: P planes of STRIDE words (a row and 16 zero words) per CTA.
+// A plane is a real row or the real or imaginary part of a complex one; every table entry is
+// decoded once for all P planes.  Long rows leave room for two planes and one CTA per SM;
+// shorter ones take four planes and as many CTAs as shared memory holds, which hides the
+// staging of one CTA behind the gathers of the others.
+template <int STRIDE> struct RowShape;
+template <> struct RowShape<12896> { static constexpr int P = 2, threads = 1024, ctas = 1; };  // Dc <= 12,880 (N = 16)
+template <> struct RowShape<6560> { static constexpr int P = 2, threads = 512, ctas = 2; };    // 6,435 (N = 15)
+template <> struct RowShape<3456> { static constexpr int P = 4, threads = 512, ctas = 2; };    // 3,432 (N = 14)
+template <> struct RowShape<1744> { static constexpr int P = 4, threads = 256, ctas = 4; };    // 1,716 (N = 13)
+template <> struct RowShape<960> { static constexpr int P = 4, threads = 256, ctas = 4; };     // 924 (N = 12)
+
+// Row pass: v0[u, :] = acc * v0[u, :] + scale * (D + down hops) v1[u, :] for the rows of P
+// planes at a time; part[blockIdx] = sum over the CTA's rows of conj(v1) (D + down) v1.  Real
+// rows are staged by bulk asynchronous copies completing on an mbarrier (per-thread cp.async
+// when they are not 16-byte aligned), complex ones are split into their parts on the way; a
+// bounded wait that gives up makes the CTA's partial sum NaN.  Bound by the L1 data pipe: each
+// element reads ~20 operands of 8 bytes from shared memory.
+// ONSITE: the cross-species diagonal is u0 * popcount(u & d) (cross_mode 0).
+template <int STRIDE, bool CPLX, bool ONSITE>
+__global__ void __launch_bounds__(RowShape<STRIDE>::threads, RowShape<STRIDE>::ctas)
+prod_row_kernel(ProdArgs a, TwoPassArgs b, const double *__restrict__ v1, double *__restrict__ v0,
+                const double *__restrict__ coef, double *__restrict__ part) {
+  constexpr int P = RowShape<STRIDE>::P, NT = RowShape<STRIDE>::threads;
+  constexpr int R = CPLX ? P / 2 : P;   // rows per task
+  constexpr int W = CPLX ? 2 : 1;       // planes per row
+  extern __shared__ __align__(128) double planes[];
   __shared__ uint64_t bar;
-  double *row1 = rows + kRow2Bytes / 8;
   const double acc = coef[0], scale = coef[1];
-  const int Dc = a.Dc, Uc = a.Uc;
-  const int tid = threadIdx.x;
-  double pr = 0.0;
-  // rows arrive by bulk copies when they start on 16-byte boundaries and are whole 16-byte units
-  const bool bulk = (Dc % 2 == 0) && ((uintptr_t)v1 % 16 == 0);
-  const uint32_t sm0 = smem_u32(rows), sm1 = sm0 + kRow2Bytes;
+  const int Dc = a.Dc, Uc = a.Uc, tid = threadIdx.x, lane = tid & 31;
+  __shared__ double2 s_c[kMaxGroups];
+  if (tid < b.ng) s_c[tid] = b.cf_dn[tid];
+  double pr = 0.0, pi = 0.0;
+  const bool bulk = !CPLX && (Dc % 2 == 0) && ((uintptr_t)v1 % 16 == 0);
   if (tid == 0) mbar_init(&bar, 1);
   mbar_fence_init();
-  if (tid < 16) {  // zero words after each row (one per bank pair), never overwritten by the copies
-    rows[Dc + tid] = 0.0;
-    row1[Dc + tid] = 0.0;
-  }
+  for (int k = tid; k < 16 * P; k += NT)  // zero words after each plane (one per bank pair), never overwritten
+    planes[(k >> 4) * STRIDE + Dc + (k & 15)] = 0.0;
   uint32_t phase = 0;
   bool ok = true;
-  for (int u0 = 2 * blockIdx.x; u0 < Uc; u0 += 2 * gridDim.x) {
-    const bool two = u0 + 1 < Uc;
-    __syncthreads();  // the previous rows are no longer read
-    const double *s0 = v1 + (int64_t)u0 * Dc;
-    const double *s1 = two ? s0 + Dc : s0;
+  for (int u0 = R * blockIdx.x; u0 < Uc; u0 += R * gridDim.x) {
+    const int nr = min(R, Uc - u0);  // rows past the last one repeat it and are not stored
+    __syncthreads();                 // the previous planes are no longer read
     if (bulk) {
       if (tid == 0) {
-        mbar_arrive_expect_tx(&bar, (uint32_t)(2 * Dc * 8));
-        bulk_g2s(rows, s0, (uint32_t)(Dc * 8), &bar);
-        bulk_g2s(row1, s1, (uint32_t)(Dc * 8), &bar);
+        mbar_arrive_expect_tx(&bar, (uint32_t)(R * Dc * 8));
+#pragma unroll
+        for (int q = 0; q < R; q++)
+          bulk_g2s(planes + q * STRIDE, v1 + (int64_t)(u0 + min(q, nr - 1)) * Dc, (uint32_t)(Dc * 8), &bar);
       }
-    } else {
-      for (int i = tid; i < Dc; i += kDownThreads) {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sm0 + 8 * i), "l"(s0 + i) : "memory");
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sm1 + 8 * i), "l"(s1 + i) : "memory");
+      // the next rows toward L2 while these are processed (a hint, no completion)
+      const int un = u0 + R * gridDim.x;
+      if (tid < R && un + tid < Uc) {
+        const double *pf = v1 + (int64_t)(un + tid) * Dc;
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(pf), "r"((uint32_t)(Dc * 8)) : "memory");
       }
-      asm volatile("cp.async.commit_group;\n" ::: "memory");
-    }
-    // the next pair's rows toward L2 while this pair is processed (a hint, no completion)
-    const int un = u0 + 2 * gridDim.x;
-    if (bulk && tid < 2 && un + tid < Uc) {
-      const double *pf = v1 + (int64_t)(un + tid) * Dc;
-      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(pf), "r"((uint32_t)(Dc * 8)) : "memory");
-    }
-    if (bulk) {
       const bool got = mbar_wait(&bar, phase);
       phase ^= 1;
       if (__syncthreads_or(!got)) {
@@ -310,280 +307,309 @@ __global__ void __launch_bounds__(kDownThreads, 1) prod_down_kernel(ProdArgs a, 
         mbar_wait(&bar, phase ^ 1);  // copies still in flight land before the CTA leaves (bounded)
         break;
       }
+    } else if (CPLX) {
+#pragma unroll
+      for (int q = 0; q < R; q++) {
+        const double2 *s = reinterpret_cast<const double2 *>(v1) + (int64_t)(u0 + min(q, nr - 1)) * Dc;
+#pragma unroll 4
+        for (int i = tid; i < Dc; i += NT) {
+          const double2 z = __ldg(s + i);
+          planes[(2 * q) * STRIDE + i] = z.x;
+          planes[(2 * q + 1) * STRIDE + i] = z.y;
+        }
+      }
+      __syncthreads();
     } else {
+#pragma unroll
+      for (int q = 0; q < R; q++) {
+        const double *s = v1 + (int64_t)(u0 + min(q, nr - 1)) * Dc;
+        const uint32_t dst = smem_u32(planes + q * STRIDE);
+        for (int i = tid; i < Dc; i += NT)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst + 8 * i), "l"(s + i) : "memory");
+      }
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
       asm volatile("cp.async.wait_all;\n" ::: "memory");
       __syncthreads();
     }
-    const int ua1 = two ? u0 + 1 : u0;
-    const uint32_t uc0 = a.unrank_up[u0], uc1 = a.unrank_up[ua1];
-    const double du0 = a.du[u0], du1 = a.du[ua1];
-    const int lane = tid & 31;
-    const double tdn = b.t_dn;
-    const char *rb = reinterpret_cast<const char *>(rows);
-    for (int p = tid; p < b.npad; p += kDownThreads) {
-      const int w = p >> 5, ns = b.wslots[w];  // the same for the warp's 32 columns
-      const uint4 *gp = b.gat + ((int64_t)w * b.groups) * 32 + lane;
-      // per-column diagonal parts and the old v0, loaded before the gathers
+    uint32_t uc[R];
+    double du[R];
+#pragma unroll
+    for (int q = 0; q < R; q++) {
+      uc[q] = a.unrank_up[u0 + min(q, nr - 1)];
+      du[q] = a.du[u0 + min(q, nr - 1)];
+    }
+    const char *rb = reinterpret_cast<const char *>(planes);
+    for (int p = tid; p < b.npad; p += NT) {
+      // per-column diagonal parts, the old v0 and the first set of slots, loaded before the gathers
       const int pc = (p < Dc) ? p : Dc - 1;
-      const double ddp = (a.cross_mode == 2) ? 0.0 : __ldg(a.dd + pc);
+      const uint4 head = __ldg(b.whead + (p >> 5));  // the same for the warp's 32 columns
+      const uint4 *gp = b.gat + (int64_t)head.x * 32 + lane;
+      uint4 e = __ldg(gp);
+      const double ddp = (!ONSITE && a.cross_mode == 2) ? 0.0 : __ldg(a.dd + pc);
       const uint32_t cdp = __ldg(a.unrank_dn + pc);
-      double *o0 = v0 + (int64_t)u0 * Dc + pc;
-      const double y0old = (acc != 0.0) ? __ldcs(o0) : 0.0;
-      const double y1old = (acc != 0.0 && two) ? __ldcs(o0 + Dc) : 0.0;
-      double g0 = 0.0, g1 = 0.0;
-      // two 16-bit entries: word index (15 bits) | sign << 15; the sign is applied by flipping
-      // the sign bit of the gathered value; every slot at or beyond the warp's count holds a
-      // zero word, so only whole entry pairs are skipped
-      auto gather2 = [&](uint32_t r) {
-        const uint32_t o0 = (r << 3) & 0x3FFF8u, o1 = (r >> 13) & 0x3FFF8u;
-        const uint32_t s0 = r << 16;  // sign of the low entry at bit 31 (the high entry's is there already)
-        const double *x0 = reinterpret_cast<const double *>(rb + o0);
-        const double *x1 = reinterpret_cast<const double *>(rb + o1);
-        g0 += flip_sign(x0[0], s0 & 0x80000000u);
-        g1 += flip_sign(x0[kRow2Bytes / 8], s0 & 0x80000000u);
-        g0 += flip_sign(x1[0], r & 0x80000000u);
-        g1 += flip_sign(x1[kRow2Bytes / 8], r & 0x80000000u);
-      };
-      for (int g = 0; 8 * g < ns; g++) {
-        const uint4 e = __ldg(gp + g * 32);
-        gather2(e.x);
-        if (8 * g + 2 < ns) gather2(e.y);
-        if (8 * g + 4 < ns) gather2(e.z);
-        if (8 * g + 6 < ns) gather2(e.w);
+      double *o = v0 + ((int64_t)u0 * Dc + pc) * W;
+      double y[P], old[P];
+#pragma unroll
+      for (int q = 0; q < P; q++) y[q] = old[q] = 0.0;
+      if (acc != 0.0) {
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          if constexpr (CPLX) {
+            const double2 z = __ldcs(reinterpret_cast<const double2 *>(o + (int64_t)min(r, nr - 1) * Dc * W));
+            old[2 * r] = z.x;
+            old[2 * r + 1] = z.y;
+          } else {
+            old[r] = __ldcs(o + (int64_t)min(r, nr - 1) * Dc * W);
+          }
+        }
+      }
+      // two 16-bit entries: word index (15 bits) | sign << 15, the sign as a factor +-1; slots at
+      // or beyond the warp's count hold a zero word, so only whole half sets are skipped
+      for (int g = 0; g < b.ng; g++) {
+        const int ns = (int)(((g < 4 ? head.y : head.z) >> (8 * (g & 3))) & 255u);
+        double s[P];
+#pragma unroll
+        for (int q = 0; q < P; q++) s[q] = 0.0;
+        auto gather2 = [&](uint32_t r) {
+          const double *x0 = reinterpret_cast<const double *>(rb + ((r << 3) & 0x3FFF8u));
+          const double *x1 = reinterpret_cast<const double *>(rb + ((r >> 13) & 0x3FFF8u));
+          const double f0 = __hiloint2double((int)(((r << 16) & 0x80000000u) | 0x3FF00000u), 0);
+          const double f1 = __hiloint2double((int)((r & 0x80000000u) | 0x3FF00000u), 0);
+#pragma unroll
+          for (int q = 0; q < P; q++) s[q] = fma(f0, x0[q * STRIDE], s[q]);
+#pragma unroll
+          for (int q = 0; q < P; q++) s[q] = fma(f1, x1[q * STRIDE], s[q]);
+        };
+        for (int k = 0; k < ns; k += 8) {
+          const uint4 c = e;
+          gp += 32;
+          e = __ldg(gp);  // the next set (of the next group; one set past the last is allocated)
+          gather2(c.x);
+          gather2(c.y);
+          if (k + 4 < ns) {
+            gather2(c.z);
+            gather2(c.w);
+          }
+        }
+        const double2 c = s_c[g];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          if constexpr (CPLX) {
+            y[2 * r] += c.x * s[2 * r] - c.y * s[2 * r + 1];
+            y[2 * r + 1] += c.x * s[2 * r + 1] + c.y * s[2 * r];
+          } else {
+            y[r] = fma(c.x, s[r], y[r]);
+          }
+        }
       }
       if (p < Dc) {
-        auto diag = [&](int ua, uint32_t uc, double du) -> double {
-          if (a.cross_mode == 2) return __ldg(a.dfull + (int64_t)ua * Dc + p);
-          double D = du + ddp;
-          const uint32_t ud = uc & cdp;
-          if (a.cross_mode == 0) D += a.u0 * (double)__popc(ud);
-          else for (uint32_t m = ud; m; m &= m - 1) D += __ldg(a.usite + (__ffs(m) - 1));
-          return D;
-        };
-        const double x0 = rows[p], y0 = diag(u0, uc0, du0) * x0 + tdn * g0;
-        __stcs(o0, (acc == 0.0) ? scale * y0 : acc * y0old + scale * y0);
-        pr += x0 * y0;
-        if (two) {
-          const double x1 = row1[p], y1 = diag(ua1, uc1, du1) * x1 + tdn * g1;
-          __stcs(o0 + Dc, (acc == 0.0) ? scale * y1 : acc * y1old + scale * y1);
-          pr += x1 * y1;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          if (r >= nr) break;
+          double D;
+          const uint32_t ud = uc[r] & cdp;
+          if (ONSITE) {
+            // popcount as a double without a conversion: 2^52 + k, less 2^52
+            D = fma(a.u0, __hiloint2double(0x43300000, __popc(ud)) - 4503599627370496.0, du[r] + ddp);
+          } else if (a.cross_mode == 2) {
+            D = __ldg(a.dfull + (int64_t)(u0 + r) * Dc + p);
+          } else {
+            D = du[r] + ddp;
+            for (uint32_t m = ud; m; m &= m - 1) D += __ldg(a.usite + (__ffs(m) - 1));
+          }
+          double *orow = o + r * (int64_t)Dc * W;
+          if constexpr (CPLX) {
+            const double xr = planes[(2 * r) * STRIDE + p], xi = planes[(2 * r + 1) * STRIDE + p];
+            const double yr = D * xr + y[2 * r], yi = D * xi + y[2 * r + 1];
+            __stcs(reinterpret_cast<double2 *>(orow),
+                   acc == 0.0 ? make_double2(scale * yr, scale * yi)
+                              : make_double2(acc * old[2 * r] + scale * yr, acc * old[2 * r + 1] + scale * yi));
+            pr += xr * yr + xi * yi;
+            pi += xr * yi - xi * yr;
+          } else {
+            const double x = planes[r * STRIDE + p], yy = D * x + y[r];
+            __stcs(orow, (acc == 0.0) ? scale * yy : acc * old[r] + scale * yy);
+            pr += x * yy;
+          }
         }
       }
     }
   }
-  double v[2] = {ok ? pr : __longlong_as_double(0x7FF8000000000000ll), 0.0};
+  const double nan = __longlong_as_double(0x7FF8000000000000ll);
+  double v[2] = {ok ? pr : nan, ok ? pi : nan};
   block_sum<2>(v);
   if (tid == 0) {
     part[2 * blockIdx.x] = v[0];
-    part[2 * blockIdx.x + 1] = 0.0;
+    part[2 * blockIdx.x + 1] = v[1];
   }
 }
 
-// Column pass: v0[u, chunk] += scale * sum_up c * v1[u', chunk], chunk-major tasks by static
-// striding; part[blockIdx] = sum of v1 . (up hops) v1 over the CTA's tasks.  VEC2: Dc is even,
-// so a thread's two columns are one aligned 16-byte load.
-template <bool VEC2, bool UNIFORM>
-__global__ void __launch_bounds__(kUpThreads, kUpMinBlocks) prod_up_kernel(ProdArgs a, TwoPassArgs b, const double *__restrict__ v1,
-                                                             double *__restrict__ v0, const double *__restrict__ coef,
-                                                             double *__restrict__ part) {
-  __shared__ int s_src[kMaxUpWidth];
-  __shared__ double s_cf[UNIFORM ? 1 : kMaxUpWidth];
-  const double scale = coef[1];
-  const int Dc = a.Dc, Uc = a.Uc, wu = a.wu;
-  const int nchunk = (Dc + kUpChunk - 1) / kUpChunk;
-  const int64_t ntask = (int64_t)nchunk * Uc;
-  double pr = 0.0;
-  for (int64_t task = blockIdx.x; task < ntask; task += gridDim.x) {
-    const int c = (int)(task / Uc), u = (int)(task - (int64_t)c * Uc);
-    const int nu = b.nus[u];
-    __syncthreads();
-    for (int k = threadIdx.x; k < nu; k += kUpThreads) {
-      s_src[k] = b.usrc[(int64_t)u * wu + k];
-      if (!UNIFORM) s_cf[k] = b.ucf[(int64_t)u * wu + k];
-    }
-    __syncthreads();
-    const int d = c * kUpChunk + 2 * (int)threadIdx.x;
-    if (d >= Dc) continue;
-    const bool pair = VEC2 || d + 1 < Dc;
-    double h0 = 0.0, h1 = 0.0;
-    int k = 0;
-    for (; k + kUpBatch <= nu; k += kUpBatch) {
-      double w0[kUpBatch], w1[kUpBatch];
-#pragma unroll
-      for (int q = 0; q < kUpBatch; q++) {
-        const double *sp = v1 + (int64_t)(s_src[k + q] & 0x7FFFFFFF) * Dc + d;
-        if (VEC2) {
-          const double2 sv = __ldg(reinterpret_cast<const double2 *>(sp));
-          w0[q] = sv.x; w1[q] = sv.y;
-        } else {
-          w0[q] = __ldg(sp);
-          w1[q] = pair ? __ldg(sp + 1) : 0.0;
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < kUpBatch; q++) {
-        if (UNIFORM) {
-          const uint32_t sg = (uint32_t)s_src[k + q] & 0x80000000u;
-          h0 += flip_sign(w0[q], sg);
-          h1 += flip_sign(w1[q], sg);
-        } else {
-          h0 += s_cf[k + q] * w0[q];
-          h1 += s_cf[k + q] * w1[q];
-        }
-      }
-    }
-    for (; k < nu; k++) {
-      const double *sp = v1 + (int64_t)(s_src[k] & 0x7FFFFFFF) * Dc + d;
-      if (UNIFORM) {
-        const uint32_t sg = (uint32_t)s_src[k] & 0x80000000u;
-        h0 += flip_sign(__ldg(sp), sg);
-        if (pair) h1 += flip_sign(__ldg(sp + 1), sg);
-      } else {
-        h0 += s_cf[k] * __ldg(sp);
-        if (pair) h1 += s_cf[k] * __ldg(sp + 1);
-      }
-    }
-    if (UNIFORM) {
-      h0 *= b.t_up;
-      h1 *= b.t_up;
-    }
-    const double *xp = v1 + (int64_t)u * Dc + d;
-    double *yp = v0 + (int64_t)u * Dc + d;
-    double x0, x1 = 0.0, y0, y1 = 0.0;
-    // v0 is streamed (read and written once): evict-first, so it does not push the chunk of
-    // v1 that the following rows gather from out of L2
-    if (VEC2) {
-      const double2 xv = __ldg(reinterpret_cast<const double2 *>(xp));
-      const double2 yv = __ldcs(reinterpret_cast<const double2 *>(yp));
-      x0 = xv.x; x1 = xv.y; y0 = yv.x; y1 = yv.y;
-    } else {
-      x0 = __ldg(xp);
-      y0 = __ldcs(yp);
-      if (pair) { x1 = __ldg(xp + 1); y1 = __ldcs(yp + 1); }
-    }
-    pr += x0 * h0 + x1 * h1;
-    if (VEC2) {
-      __stcs(reinterpret_cast<double2 *>(yp), make_double2(y0 + scale * h0, y1 + scale * h1));
-    } else {
-      __stcs(yp, y0 + scale * h0);
-      if (pair) __stcs(yp + 1, y1 + scale * h1);
-    }
-  }
-  double v[2] = {pr, 0.0};
-  block_sum<2>(v);
-  if (threadIdx.x == 0) {
-    part[2 * blockIdx.x] = v[0];
-    part[2 * blockIdx.x + 1] = 0.0;
-  }
-}
+// Column pass: v0[u, chunk] += scale * sum_up c * v1[u', chunk].  A task is one row u and 128
+// doubles of it (128 real columns or 64 complex ones); V doubles per load: lane l reads doubles
+// 2l, 2l + 1 and 64 + 2l, 65 + 2l as two 16-byte loads (V = 2), or l, l + 32, ... one by one
+// where a row may start on an odd double (V = 1).  Tasks run chunk-major (every row of chunk 0,
+// then chunk 1, ...) by static striding over the warps of a grid that is resident at once, so
+// the 1 KB pieces of v1 the rows gather stay in L2.  Each lane holds hop entries of the row and
+// the warp broadcasts them by shuffles (no shared memory, no CTA barrier).  MULTI: several up
+// coefficients, each entry naming its own (read from shared memory at one address per warp);
+// else one real coefficient and signs.  The sum includes the row pass's records.  Bound by the
+// L1 data pipe: ~17 operands of 8 bytes per double.
+// TAYLOR: every finished element y of v0 also goes into a Taylor sum, sum += c * y (complex
+// vectors), which saves the sum's own pass over y.
+struct TaylorSum {
+  double2 *sum;
+  double2 c;
+};
 
-constexpr int kUpWThreads = 256;     // column pass, warp tasks: 8 warps per CTA
-constexpr int kUpWMinBlocks = 3;     // CTAs per SM (at most 85 registers)
-constexpr int kUpWChunk = 128;       // columns per warp task (4 per lane, two 16-byte loads)
-constexpr int kUpWBatch = 4;         // up hops per batch: 8 loads of 16 bytes in flight per lane
-
-// Column pass with warp tasks (uniform up hops, Dc even, 16-byte aligned vectors, Uc <= 32768,
-// at most 64 up hops per row): v0[u, chunk] += scale * t_up * sum_up sign * v1[u', chunk].  A
-// task is one row u and 128 columns (lane l: columns 2l, 2l + 1 and 64 + 2l, 65 + 2l, so each
-// load instruction of the warp reads 512 contiguous bytes); tasks run chunk-major (every row of chunk 0, then chunk
-// 1, ...) by static striding over the warps of a grid that is resident at once, so the 1 KB
-// pieces of v1 the rows gather stay in L2.  Each lane holds two 16-bit hop entries of the row
-// and the warp broadcasts them by shuffles (no shared memory, no CTA barrier).
-// part[blockIdx] = sum over the CTA's tasks of v1 . (up hops) v1.
-__global__ void __launch_bounds__(kUpWThreads, kUpWMinBlocks) prod_up_warp_kernel(ProdArgs a, TwoPassArgs b,
-                                                                                 const double *__restrict__ v1,
-                                                                                 double *__restrict__ v0,
-                                                                                 const double *__restrict__ coef,
-                                                                                 double *__restrict__ part) {
+template <int V, bool CPLX, bool MULTI, bool TAYLOR>
+__global__ void __launch_bounds__(kUpThreads, kUpMinBlocks) prod_col_kernel(ProdArgs a, TwoPassArgs b,
+                                                                          const double *__restrict__ v1,
+                                                                          double *__restrict__ v0,
+                                                                          const double *__restrict__ coef, SumOut so,
+                                                                          TaylorSum ts) {
+  static_assert(V == 2 || !CPLX, "complex rows are whole 16-byte units");
+  constexpr int NL = 4 / V;  // loads per lane and source row
+  __shared__ double2 s_cf[2 * kMaxGroups];
   const int lane = threadIdx.x & 31;
-  const int warp = (int)((blockIdx.x * (unsigned)kUpWThreads + threadIdx.x) >> 5);
-  const int nwarps = (int)(gridDim.x * (unsigned)kUpWThreads) >> 5;
-  const int Dc = a.Dc, Uc = a.Uc;
-  const int nchunk = (Dc + kUpWChunk - 1) / kUpWChunk;
+  const int warp = (int)((blockIdx.x * (unsigned)kUpThreads + threadIdx.x) >> 5);
+  const int nwarps = (int)(gridDim.x * (unsigned)kUpThreads) >> 5;
+  const int ncol = a.Dc * (CPLX ? 2 : 1), Uc = a.Uc;
+  const int nchunk = (ncol + kUpChunk - 1) / kUpChunk;
   const int64_t ntask = (int64_t)nchunk * Uc;
-  const double tup = b.t_up, st = coef[1] * b.t_up;
-  double pr = 0.0;
+  if (MULTI) {
+    if (threadIdx.x < 2 * b.ngu) {
+      const double2 c = b.cf_up[threadIdx.x >> 1];
+      s_cf[threadIdx.x] = (threadIdx.x & 1) ? make_double2(-c.x, -c.y) : c;
+    }
+    __syncthreads();
+  }
+  const double scale = coef[1], tup = (MULTI || b.ngu == 0) ? 1.0 : b.cf_up[0].x;
+  double pr = 0.0, pi = 0.0;
   // the row's hop count and packed entries of the next task are loaded one task ahead
   int64_t task = warp;
   int nu_n = 0;
-  uint32_t my_n = 0u;
+  uint32_t my_n = 0u, my2_n = 0u;
   auto fetch = [&](int64_t t) {
     if (t < ntask) {
       const int un = (int)(t % Uc);
       nu_n = b.nus[un];
-      my_n = (2 * lane < nu_n) ? __ldg(b.usrc16 + (int64_t)un * b.wu2 + lane) : 0u;
+      const uint32_t *e = b.up_ent + (int64_t)un * b.wu2;
+      my_n = ((MULTI ? 1 : 2) * lane < nu_n) ? __ldg(e + lane) : 0u;
+      if (MULTI) my2_n = (lane + 32 < nu_n) ? __ldg(e + lane + 32) : 0u;
     }
   };
   fetch(task);
-  const uint64_t rowb = (uint64_t)Dc * sizeof(double);
+  const uint64_t rowb = (uint64_t)ncol * sizeof(double);
   for (; task < ntask; task += nwarps) {
     const int c = (int)(task / Uc), u = (int)(task - (int64_t)c * Uc);
     const int nu = nu_n;
-    const uint32_t my = my_n;
+    const uint32_t my = my_n, my2 = my2_n;
     fetch(task + nwarps);
-    const int d = c * kUpWChunk + 2 * lane;     // columns d, d + 1 and d + 64, d + 65
-    const bool ok0 = d < Dc, ok1 = d + 64 < Dc;  // Dc is even: pairs are whole
-    // lanes past the last column read a valid pair (column 0) and discard what they summed
-    const char *base0 = reinterpret_cast<const char *>(v1 + (ok0 ? d : 0));
-    const char *base1 = reinterpret_cast<const char *>(v1 + (ok1 ? d + 64 : 0));
-    double h0 = 0.0, h1 = 0.0, h2 = 0.0, h3 = 0.0;
-    auto hop = [&](uint32_t e, double2 &w0, double2 &w1) {
-      const uint64_t off = (uint64_t)(e & 0x7FFFu) * rowb;
-      w0 = __ldg(reinterpret_cast<const double2 *>(base0 + off));
-      w1 = __ldg(reinterpret_cast<const double2 *>(base1 + off));
+    const int d = c * kUpChunk + V * lane;
+    const char *base[NL];
+    bool ok[NL];
+#pragma unroll
+    for (int j = 0; j < NL; j++) {
+      ok[j] = d + j * 32 * V < ncol;  // V = 2: ncol is even, pairs are whole
+      // lanes past the last column read column 0 and discard what they summed
+      base[j] = reinterpret_cast<const char *>(v1 + (ok[j] ? d + j * 32 * V : 0));
+    }
+    double h[4] = {0.0, 0.0, 0.0, 0.0};
+    auto load = [&](uint32_t rank, double (&x)[4]) {
+      const uint64_t off = (uint64_t)rank * rowb;
+#pragma unroll
+      for (int j = 0; j < NL; j++) {
+        if constexpr (V == 2) {
+          const double2 z = __ldg(reinterpret_cast<const double2 *>(base[j] + off));
+          x[2 * j] = z.x;
+          x[2 * j + 1] = z.y;
+        } else {
+          x[j] = __ldg(reinterpret_cast<const double *>(base[j] + off));
+        }
+      }
     };
-    auto add = [&](uint32_t e, const double2 &w0, const double2 &w1) {
-      const uint32_t sg = (e & 0x8000u) << 16;
-      h0 += flip_sign(w0.x, sg);
-      h1 += flip_sign(w0.y, sg);
-      h2 += flip_sign(w1.x, sg);
-      h3 += flip_sign(w1.y, sg);
+    auto entry = [&](int k) -> uint32_t {
+      if constexpr (MULTI) return __shfl_sync(0xFFFFFFFFu, k < 32 ? my : my2, k & 31);
+      const uint32_t word = __shfl_sync(0xFFFFFFFFu, my, (k >> 1) & 31);
+      return (k & 1) ? (word >> 16) : (word & 0xFFFFu);
+    };
+    auto rank_of = [&](uint32_t e) { return MULTI ? (e & 0xFFFFu) : (e & 0x7FFFu); };
+    auto add = [&](uint32_t e, const double (&x)[4]) {
+      if constexpr (MULTI) {
+        const double2 cc = s_cf[e >> 16];
+        if constexpr (CPLX) {
+#pragma unroll
+          for (int j = 0; j < 4; j += 2) {
+            h[j] = fma(cc.x, x[j], fma(-cc.y, x[j + 1], h[j]));
+            h[j + 1] = fma(cc.x, x[j + 1], fma(cc.y, x[j], h[j + 1]));
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; j++) h[j] = fma(cc.x, x[j], h[j]);
+        }
+      } else {
+        const uint32_t sg = (e & 0x8000u) << 16;
+#pragma unroll
+        for (int j = 0; j < 4; j++) h[j] += flip_sign(x[j], sg);
+      }
     };
     int k = 0;
-    for (; k + kUpWBatch <= nu; k += kUpWBatch) {
-      double2 w0[kUpWBatch], w1[kUpWBatch];
-      uint32_t e[kUpWBatch];
+    for (; k + kUpBatch <= nu; k += kUpBatch) {
+      double x[kUpBatch][4];
+      uint32_t e[kUpBatch];
+      if constexpr (MULTI) {
 #pragma unroll
-      for (int q = 0; q < kUpWBatch; q += 2) {
-        const uint32_t word = __shfl_sync(0xFFFFFFFFu, my, ((k + q) >> 1) & 31);
-        e[q] = word & 0xFFFFu;
-        e[q + 1] = word >> 16;
+        for (int q = 0; q < kUpBatch; q++) e[q] = entry(k + q);
+      } else {
+#pragma unroll
+        for (int q = 0; q < kUpBatch; q += 2) {
+          const uint32_t word = __shfl_sync(0xFFFFFFFFu, my, ((k + q) >> 1) & 31);
+          e[q] = word & 0xFFFFu;
+          e[q + 1] = word >> 16;
+        }
       }
 #pragma unroll
-      for (int q = 0; q < kUpWBatch; q++) hop(e[q], w0[q], w1[q]);
+      for (int q = 0; q < kUpBatch; q++) load(rank_of(e[q]), x[q]);
 #pragma unroll
-      for (int q = 0; q < kUpWBatch; q++) add(e[q], w0[q], w1[q]);
+      for (int q = 0; q < kUpBatch; q++) add(e[q], x[q]);
     }
     for (; k < nu; k++) {
-      const uint32_t word = __shfl_sync(0xFFFFFFFFu, my, (k >> 1) & 31);
-      const uint32_t e = (k & 1) ? (word >> 16) : (word & 0xFFFFu);
-      double2 w0, w1;
-      hop(e, w0, w1);
-      add(e, w0, w1);
+      const uint32_t e = entry(k);
+      double x[4];
+      load(rank_of(e), x);
+      add(e, x);
     }
-    const double *xp = v1 + (int64_t)u * Dc + d;
-    double *yp = v0 + (int64_t)u * Dc + d;
+    const double *xp = v1 + (int64_t)u * ncol + d;
+    double *yp = v0 + (int64_t)u * ncol + d;
     // v0 is streamed (read and written once): evict-first, so it does not push the chunk of
     // v1 that the following rows gather from out of L2
-    if (ok0) {
-      const double2 xv = __ldg(reinterpret_cast<const double2 *>(xp));
-      const double2 yv = __ldcs(reinterpret_cast<const double2 *>(yp));
-      pr += tup * (xv.x * h0 + xv.y * h1);
-      __stcs(reinterpret_cast<double2 *>(yp), make_double2(yv.x + st * h0, yv.y + st * h1));
-    }
-    if (ok1) {
-      const double2 xv = __ldg(reinterpret_cast<const double2 *>(xp + 64));
-      const double2 yv = __ldcs(reinterpret_cast<const double2 *>(yp + 64));
-      pr += tup * (xv.x * h2 + xv.y * h3);
-      __stcs(reinterpret_cast<double2 *>(yp + 64), make_double2(yv.x + st * h2, yv.y + st * h3));
+#pragma unroll
+    for (int j = 0; j < NL; j++) {
+      if (!ok[j]) continue;
+      if constexpr (V == 2) {
+        const double h0 = tup * h[2 * j], h1 = tup * h[2 * j + 1];
+        const double2 xv = __ldg(reinterpret_cast<const double2 *>(xp + 64 * j));
+        const double2 yv = __ldcs(reinterpret_cast<const double2 *>(yp + 64 * j));
+        pr += xv.x * h0 + xv.y * h1;
+        if (CPLX) pi += xv.x * h1 - xv.y * h0;
+        const double2 yn = make_double2(yv.x + scale * h0, yv.y + scale * h1);
+        __stcs(reinterpret_cast<double2 *>(yp + 64 * j), yn);
+        if constexpr (TAYLOR) {
+          double2 *tp = ts.sum + (((int64_t)u * ncol + d) >> 1) + 32 * j;
+          double2 t = __ldcs(tp);
+          t.x += ts.c.x * yn.x - ts.c.y * yn.y;
+          t.y += ts.c.x * yn.y + ts.c.y * yn.x;
+          __stcs(tp, t);
+        }
+      } else {
+        const double h0 = tup * h[j];
+        pr += __ldg(xp + 32 * j) * h0;
+        __stcs(yp + 32 * j, __ldcs(yp + 32 * j) + scale * h0);
+      }
     }
   }
-  double v[2] = {pr, 0.0};
-  block_sum<2>(v);
-  if (threadIdx.x == 0) {
-    part[2 * blockIdx.x] = v[0];
-    part[2 * blockIdx.x + 1] = 0.0;
-  }
+  double v[2] = {pr, pi};
+  grid_sum<2>(v, so);
 }
 
 __device__ __forceinline__ uint32_t compress_species(uint64_t c, int s, int N) {
@@ -592,64 +618,133 @@ __device__ __forceinline__ uint32_t compress_species(uint64_t c, int s, int N) {
   return x;
 }
 
-// sigma(c) of the species-first basis: (-1)^#{(down at i, up at j) : i < j}.
-__device__ __forceinline__ int species_parity(uint64_t c, int N) {
-  int cnt = 0, downs = 0;
-  for (int i = 0; i < N; i++) {
-    if ((c >> (2 * i)) & 1ull) cnt += downs;
-    downs += (int)((c >> (2 * i + 1)) & 1ull);
-  }
-  return cnt & 1;
-}
-
-// HPhi order <-> native order, per row r of HPhi's list_1; SIGN applies sigma (vectors),
-// without it the values are moved as they are (functions of the configuration).
-template <typename T, bool TO_NATIVE, bool SIGN>
-__global__ void prod_permute_kernel(int64_t dim, int N, int Dc, const uint64_t *__restrict__ list_1,
-                                    const uint16_t *__restrict__ rank, const uint16_t *__restrict__ pos_dn,
-                                    const T *__restrict__ in, T *__restrict__ out) {
+// A function of the configuration in HPhi's row order (the diagonal) to native order.
+__global__ void prod_permute_diag_kernel(int64_t dim, int N, int Dc, const uint64_t *__restrict__ list_1,
+                                         const uint16_t *__restrict__ rank, const uint16_t *__restrict__ pos_dn,
+                                         const double *__restrict__ in, double *__restrict__ out) {
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < dim; r += (int64_t)gridDim.x * blockDim.x) {
     const uint64_t c = list_1[r];
     const int64_t pos = (int64_t)rank[compress_species(c, 0, N)] * Dc + pos_dn[compress_species(c, 1, N)];
-    const double sg = (SIGN && species_parity(c, N)) ? -1.0 : 1.0;
-    if (TO_NATIVE) out[pos] = VT<T>::scale(sg, in[r]);
-    else out[r] = VT<T>::scale(sg, in[pos]);
+    out[pos] = in[r];
   }
 }
 
-// HPhi order -> native order as a gather over the native positions: position (up rank ua, down
-// position da) holds the configuration c with the up spins of unrank_up[ua] on the even bits
-// and the down spins of unrank_dn[da] on the odd bits, whose HPhi row is
-// list_2_1[c & lo_mask] + list_2_2[c >> lo_bits] - 3.  Writes are coalesced and only the reads
-// scattered, where the row-ordered form above scatters its writes.
-__device__ __forceinline__ uint64_t spread_even_bits(uint64_t x) {  // bit i -> bit 2i, x < 2^32
-  x &= 0xFFFFFFFFull;
-  x = (x | (x << 16)) & 0x0000FFFF0000FFFFull;
-  x = (x | (x << 8)) & 0x00FF00FF00FF00FFull;
-  x = (x | (x << 4)) & 0x0F0F0F0F0F0F0F0Full;
-  x = (x | (x << 2)) & 0x3333333333333333ull;
-  x = (x | (x << 1)) & 0x5555555555555555ull;
-  return x;
+// Sign sigma(c) from the two species' words: (-1)^#{down at i, up at j : i < j}; bit j of the
+// running xor of d, shifted up by one, is the parity of the downs below j.
+__device__ __forceinline__ uint32_t species_parity16(uint32_t u, uint32_t d) {
+  d ^= d << 1;
+  d ^= d << 2;
+  d ^= d << 4;
+  d ^= d << 8;
+  return (uint32_t)__popc(u & (d << 1)) & 1u;
+}
+__device__ __forceinline__ uint32_t compress_even(uint32_t x) {  // bit 2i -> bit i
+  x &= 0x55555555u;
+  x = (x | (x >> 1)) & 0x33333333u;
+  x = (x | (x >> 2)) & 0x0F0F0F0Fu;
+  x = (x | (x >> 4)) & 0x00FF00FFu;
+  return (x | (x >> 8)) & 0xFFFFu;
+}
+__host__ __device__ __forceinline__ uint32_t spread_even(uint32_t x) {  // bit i -> bit 2i, x < 2^16
+  x = (x | (x << 8)) & 0x00FF00FFu;
+  x = (x | (x << 4)) & 0x0F0F0F0Fu;
+  x = (x | (x << 2)) & 0x33333333u;
+  return (x | (x << 1)) & 0x55555555u;
+}
+template <typename T> __device__ __forceinline__ T signed_v(const T &x, uint32_t par);
+template <> __device__ __forceinline__ double signed_v<double>(const double &x, uint32_t par) { return par ? -x : x; }
+template <> __device__ __forceinline__ cplx signed_v<cplx>(const cplx &x, uint32_t par) {
+  return par ? cplx{-x.x, -x.y} : x;
 }
 
+// The two orders' permutations are bound by the L2 sectors of their scattered side (32 bytes
+// moved for each 8- or 16-byte element), so both run in an order in which every sector's other
+// elements are wanted soon: all rows of one group of up configurations that share their upper
+// sites (7 MB of the 4x4 half-filled sector), then the next group.  The row's words come from
+// a few bit steps instead of one step per site.  4x4 lattice with 6 + 6 electrons, real:
+// to native 693 -> 318, from native 1083 -> 368 us.
+
+constexpr int kPermThreads = 256;
+constexpr int kPermBatch = 4;    // elements in flight per thread
+
+// HPhi order -> native: a CTA per up configuration u.  HPhi's row of (u, d) is
+// list_2_1[lower half] + list_2_2[upper half] - 3; with u fixed each term depends on the downs
+// of one half only, so the two lookups become 2^(downs of the half) entries in shared memory.
 template <typename T>
-__global__ void prod_to_native_gather_kernel(int64_t n, int N, int Dc, const uint16_t *__restrict__ unrank_up,
-                                             const uint16_t *__restrict__ unrank_dn, const uint32_t *__restrict__ l21,
-                                             const uint32_t *__restrict__ l22, int lo_bits, uint64_t lo_mask,
-                                             const T *__restrict__ in, T *__restrict__ out) {
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t ua = p / Dc;
-    const int64_t da = p - ua * Dc;
-    const uint64_t c = spread_even_bits(__ldg(unrank_up + ua)) | (spread_even_bits(__ldg(unrank_dn + da)) << 1);
-    const int64_t r = (int64_t)__ldg(l21 + (c & lo_mask)) + (int64_t)__ldg(l22 + (c >> lo_bits)) - 3;
-    const double sg = species_parity(c, N) ? -1.0 : 1.0;
-    out[p] = VT<T>::scale(sg, in[r]);
+__global__ void __launch_bounds__(kPermThreads) prod_to_native_kernel(int N, int Uc, int Dc,
+                                                                      const uint16_t *__restrict__ unrank_up,
+                                                                      const uint16_t *__restrict__ unrank_dn,
+                                                                      const uint32_t *__restrict__ l21,
+                                                                      const uint32_t *__restrict__ l22,
+                                                                      const T *__restrict__ in, T *__restrict__ out) {
+  __shared__ uint32_t s_lo[256], s_hi[256];  // at most 8 downs of each half (N <= 16)
+  const int nlo = N / 2, nhi = N - nlo;      // HPhi's lower half: N bits, (N + 1) / 2 ups and N / 2 downs
+  const uint32_t mask = (uint32_t)((1ull << N) - 1);
+  for (int ua = blockIdx.x; ua < Uc; ua += gridDim.x) {
+    const uint32_t u = unrank_up[ua], cu = spread_even(u);
+    __syncthreads();  // the previous row's tables are no longer read
+    if (threadIdx.x < (1u << nlo)) s_lo[threadIdx.x] = __ldg(l21 + ((cu | (spread_even(threadIdx.x) << 1)) & mask));
+    if (threadIdx.x < (1u << nhi)) {
+      const uint64_t c = (uint64_t)cu | ((uint64_t)spread_even((uint32_t)threadIdx.x << nlo) << 1);
+      s_hi[threadIdx.x] = __ldg(l22 + (c >> N)) - 3u;
+    }
+    __syncthreads();
+    T *o = out + (int64_t)ua * Dc;
+    for (int d0 = threadIdx.x; d0 < Dc; d0 += kPermBatch * kPermThreads) {
+      T v[kPermBatch];
+      uint32_t d[kPermBatch];
+#pragma unroll
+      for (int q = 0; q < kPermBatch; q++) {
+        const int p = d0 + q * kPermThreads;
+        d[q] = __ldg(unrank_dn + (p < Dc ? p : d0));
+      }
+#pragma unroll
+      for (int q = 0; q < kPermBatch; q++) v[q] = ldg_v<T>(in + (s_lo[d[q] & ((1u << nlo) - 1)] + s_hi[d[q] >> nlo]));
+#pragma unroll
+      for (int q = 0; q < kPermBatch; q++) {
+        const int p = d0 + q * kPermThreads;
+        if (p < Dc) o[p] = signed_v<T>(v[q], species_parity16(u, d[q]));
+      }
+    }
+  }
+}
+
+// Native -> HPhi order, a warp per piece of an HPhi block; pieces run by upper ups, then upper downs.
+template <typename T>
+__global__ void __launch_bounds__(kPermThreads) prod_from_native_kernel(int N, int Dc, const SectorBlock *__restrict__ tasks,
+                                                                        int ntask, const uint32_t *__restrict__ low,
+                                                                        const uint16_t *__restrict__ rank,
+                                                                        const uint16_t *__restrict__ pos_dn,
+                                                                        const T *__restrict__ in, T *__restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  const int nwarps = (int)(gridDim.x * kPermThreads) >> 5;
+  for (int t = (int)(blockIdx.x * kPermThreads + threadIdx.x) >> 5; t < ntask; t += nwarps) {
+    const uint4 w = __ldg(reinterpret_cast<const uint4 *>(tasks) + t);
+    const uint64_t hi = (uint64_t)w.x << N;
+    const int n = (int)w.w;
+    for (int a0 = lane; a0 < n; a0 += 32 * kPermBatch) {
+      T v[kPermBatch];
+      uint32_t par[kPermBatch];
+#pragma unroll
+      for (int q = 0; q < kPermBatch; q++) {
+        const int a = a0 + 32 * q;
+        const uint32_t c32 = (uint32_t)hi | __ldg(low + w.z + (a < n ? a : a0));  // 2 N <= 32 bits
+        const uint32_t u = compress_even(c32), d = compress_even(c32 >> 1);
+        par[q] = species_parity16(u, d);
+        v[q] = ldg_v<T>(in + ((int64_t)__ldg(rank + u) * Dc + __ldg(pos_dn + d)));
+      }
+#pragma unroll
+      for (int q = 0; q < kPermBatch; q++) {
+        const int a = a0 + 32 * q;
+        if (a < n) out[(int64_t)w.y + a] = signed_v<T>(v[q], par[q]);
+      }
+    }
   }
 }
 
 // Diagonal observables in native order (expec_energy_flct_Hubbard, src/expec_energy_flct.c:259-330).
 template <typename T>
-__global__ void prod_obs_kernel(ProdArgs a, const T *__restrict__ v, double *__restrict__ part) {
+__global__ void prod_obs_kernel(ProdArgs a, const T *__restrict__ v, SumOut so) {
   double o[6] = {0, 0, 0, 0, 0, 0};
   const int64_t n = (int64_t)a.Uc * a.Dc;
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
@@ -660,9 +755,7 @@ __global__ void prod_obs_kernel(ProdArgs a, const T *__restrict__ v, double *__r
     const double D = (double)__popc(u & d), Nn = (double)(up + dn), Sz = 0.5 * (double)(up - dn);
     o[0] += w * D; o[1] += w * D * D; o[2] += w * Nn; o[3] += w * Nn * Nn; o[4] += w * Sz; o[5] += w * Sz * Sz;
   }
-  block_sum<6>(o);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 6; k++) part[6 * blockIdx.x + k] = o[k];
+  grid_sum<6>(o, so);
 }
 
 uint64_t binom_p(int n, int k) {
@@ -687,13 +780,18 @@ struct ProdPlan {
   std::vector<void *> allocs;
   int grid = 0;
   size_t smem[2] = {0, 0};  // real, complex
-  double *part = nullptr;   // partial sums: 2 * max(Uc, grid_dn + grid_up)
+  double *part = nullptr;   // partial sums: 2 * max(Uc, grid_row + grid_col)
   int *counter = nullptr;
-  bool two_pass = false;    // real vectors take the two-pass kernels
+  bool two_pass = false;    // the two-pass kernels apply
+  bool uniform = false;     // down hops of one magnitude, no complex hop
   TwoPassArgs tp{};
-  int grid_dn = 0, grid_up = 0;  // grid_up: records reserved for the column pass (either kernel)
-  int grid_upw = 0;              // grid of prod_up_warp_kernel (0: not applicable)
-  size_t smem_dn = 0;
+  int stride = 0;           // row pass shape (RowShape)
+  bool multi_up = false;    // several up coefficients, or a complex one
+  int grid_row[2] = {0, 0}, grid_col = 0;
+  std::vector<uint16_t> rank, pos_dn, unrank_up, unrank_dn;  // host copies of the position tables
+  const SectorBlock *perm = nullptr;  // pieces of HPhi's blocks for prod_from_native_kernel
+  const uint32_t *perm_low = nullptr;  // the blocks' lower halves
+  int nperm = 0;
 };
 
 void prod_plan_free(ProdPlan *p) {
@@ -776,13 +874,16 @@ void build_gather(const std::vector<std::vector<uint32_t>> &rows_dn, const std::
   const int nwarp = npad / 32;
   auto zero_word = [&](int bank) { return (uint32_t)(Dc + (((bank - Dc) % 16) + 16) % 16); };
   std::vector<std::vector<uint32_t>> lane_slots(npad);  // per column: entry of each slot of its half
+  std::vector<int> el, eb, L, B, colr, path;
+  std::vector<uint32_t> ev;
   wslots->assign(nwarp, 0);
   *nslots = 0;
   for (int w = 0; w < nwarp; w++) {
     int wmax = 0;
     for (int hw = 0; hw < 2; hw++) {
-      std::vector<int> el, eb;
-      std::vector<uint32_t> ev;
+      el.clear();
+      eb.clear();
+      ev.clear();
       for (int l = 0; l < 16; l++) {
         const int col = 32 * w + 16 * hw + l;
         if (col >= Dc) continue;
@@ -798,7 +899,9 @@ void build_gather(const std::vector<std::vector<uint32_t>> &rows_dn, const std::
       for (size_t i = 0; i < el.size(); i++) { ldeg[el[i]]++; bdeg[eb[i]]++; }
       int D = 0;
       for (int i = 0; i < 16; i++) D = std::max(D, std::max(ldeg[i], bdeg[i]));
-      std::vector<int> L(16 * std::max(D, 1), -1), B(16 * std::max(D, 1), -1), colr(el.size(), -1);
+      L.assign(16 * std::max(D, 1), -1);
+      B.assign(16 * std::max(D, 1), -1);
+      colr.assign(el.size(), -1);
       for (size_t i = 0; i < el.size(); i++) {
         const int l = el[i], bk = eb[i];
         int a = 0, c = 0;
@@ -806,7 +909,7 @@ void build_gather(const std::vector<std::vector<uint32_t>> &rows_dn, const std::
         while (B[bk * D + c] >= 0) c++;
         if (B[bk * D + a] >= 0) {
           // alternating a/c path from bank bk; swapping it frees a at bk
-          std::vector<int> path;
+          path.clear();
           int node = bk, want = a;
           bool at_bank = true;
           for (;;) {
@@ -827,13 +930,12 @@ void build_gather(const std::vector<std::vector<uint32_t>> &rows_dn, const std::
       }
       for (int l = 0; l < 16; l++) lane_slots[32 * w + 16 * hw + l].assign(D, 0u);
       for (int c = 0; c < D; c++) {
-        std::vector<int> free_banks;
-        for (int bk = 0; bk < 16; bk++)
-          if (B[bk * D + c] < 0) free_banks.push_back(bk);
-        size_t f = 0;
+        int f = 0;  // next bank pair that the slot may leave free
         for (int l = 0; l < 16; l++) {
           const int ed = L[l * D + c];
-          lane_slots[32 * w + 16 * hw + l][c] = (ed >= 0) ? ev[ed] : zero_word(free_banks[f++]) * 8u;
+          if (ed < 0)
+            while (B[f * D + c] >= 0) f++;
+          lane_slots[32 * w + 16 * hw + l][c] = (ed >= 0) ? ev[ed] : zero_word(f++) * 8u;
         }
       }
       wmax = std::max(wmax, D);
@@ -868,7 +970,10 @@ void build_gather(const std::vector<std::vector<uint32_t>> &rows_dn, const std::
 // load) (the edge colouring of build_gather), so positions decide both.  Start from the
 // configurations sorted by hop count (equal lane degrees in a half-warp), then swap positions
 // (within a half-warp: a bank change; across half-warps: only between equal hop counts) when
-// that does not raise the summed slot counts of the half-warps it touches.  rows[r]: sources
+// that does not raise the summed slot counts of the half-warps it touches.  A proposal moves a
+// source in the fullest bank pair of a half-warp that its bank pairs, not its lanes, hold up:
+// 40 per configuration reach the slot counts (within 1.5%) that 200 drawn blindly do, in a
+// quarter of the time (7 of 14 sites 180 -> 44 ms, 6 of 16 sites 820 -> 173 ms).  rows[r]: sources
 // of configuration r (ELL entries, source in the low 16 bits).  Returns the position of each
 // configuration; deterministic (fixed seed).
 std::vector<int> balance_positions(const std::vector<std::vector<uint32_t>> &rows) {
@@ -880,49 +985,66 @@ std::vector<int> balance_positions(const std::vector<std::vector<uint32_t>> &row
   for (int p = 0; p < n; p++) pos[order[p]] = p;
   const int ng = (n + G - 1) / G;
   if (n < 4 * G) return pos;
-  std::vector<std::vector<int>> src(n), rdr(n);
-  for (int r = 0; r < n; r++)
+  // sources and readers of each configuration, back to back
+  std::vector<int> src, rdr, s0(n + 1, 0), r0(n + 2, 0);
+  for (int r = 0; r < n; r++) {
     for (uint32_t e : rows[r]) {
-      const int q = (int)(e & 0xFFFFu);
-      src[r].push_back(q);
-      rdr[q].push_back(r);
+      src.push_back((int)(e & 0xFFFFu));
+      r0[(e & 0xFFFFu) + 2]++;
     }
+    s0[r + 1] = (int)src.size();
+  }
+  for (int r = 0; r < n; r++) r0[r + 2] += r0[r + 1];
+  rdr.resize(src.size());
+  for (int r = 0; r < n; r++)
+    for (int k = s0[r]; k < s0[r + 1]; k++) rdr[r0[src[k] + 1]++] = r;
   std::vector<int> at(order);  // configuration at each position
-  std::vector<int> load((size_t)ng * G, 0), lmax(ng, 0), D(ng, 0);
+  std::vector<uint16_t> load((size_t)ng * G, 0), lmax(ng, 0), D(ng, 0);
   for (int r = 0; r < n; r++) {
     const int g = pos[r] / G;
-    lmax[g] = std::max(lmax[g], (int)src[r].size());
-    for (int q : src[r]) load[(size_t)g * G + pos[q] % G]++;
+    lmax[g] = std::max(lmax[g], (uint16_t)(s0[r + 1] - s0[r]));
+    for (int k = s0[r]; k < s0[r + 1]; k++) load[(size_t)g * G + pos[src[k]] % G]++;
   }
   auto eval = [&](int g) {
-    int m = lmax[g];
+    uint16_t m = lmax[g];
     for (int k = 0; k < G; k++) m = std::max(m, load[(size_t)g * G + k]);
     return m;
   };
   for (int g = 0; g < ng; g++) D[g] = eval(g);
   uint64_t rng = 0x9E3779B97F4A7C15ull;
   auto next = [&]() { rng ^= rng << 13; rng ^= rng >> 7; rng ^= rng << 17; return rng; };
-  std::vector<int> touched;
+  std::vector<int> touched, nd;
   std::vector<char> mark(ng, 0);
   auto touch = [&](int g) { if (!mark[g]) { mark[g] = 1; touched.push_back(g); } };
   // adds (sgn = 1) or removes (-1) a configuration's edges: its reads (in its own half-warp)
   // and the reads of it; edges to `other` are left to the other configuration's call
   auto contrib = [&](int r, int p, int sgn, int other) {
     const int g = p / G, bk = p % G;
-    for (int q : src[r])
-      if (q != other) load[(size_t)g * G + pos[q] % G] += sgn;
-    for (int rr : rdr[r])
-      if (rr != other) { const int gg = pos[rr] / G; load[(size_t)gg * G + bk] += sgn; touch(gg); }
+    for (int k = s0[r]; k < s0[r + 1]; k++)
+      if (src[k] != other) load[(size_t)g * G + pos[src[k]] % G] += sgn;
+    for (int k = r0[r]; k < r0[r + 1]; k++)
+      if (rdr[k] != other) { const int gg = pos[rdr[k]] / G; load[(size_t)gg * G + bk] += sgn; touch(gg); }
     touch(g);
   };
-  const int64_t iters = std::min<int64_t>(200 * (int64_t)n, 4000000);
+  const int64_t iters = std::min<int64_t>(40 * (int64_t)n, 800000);
   for (int64_t it = 0; it < iters; it++) {
-    const int p1 = (int)(next() % n);
-    int p2;
-    if (next() & 1) p2 = (p1 / G) * G + (int)(next() % G);
-    else p2 = (int)(next() % n);
-    if (p2 >= n || p2 == p1 || src[at[p1]].size() != src[at[p2]].size()) continue;
+    const int gh = (int)(((next() >> 32) * (uint64_t)ng) >> 32);
+    if (D[gh] == lmax[gh]) continue;
+    const uint16_t *ld = &load[(size_t)gh * G];
+    const int hot = (int)(std::max_element(ld, ld + G) - ld);
+    const uint64_t rnd = next();
+    int p1 = -1;
+    for (int l = 0; l < G && p1 < 0; l++) {
+      const int p = gh * G + (((int)(rnd & 15) + l) & 15);
+      if (p >= n) continue;
+      for (int k = s0[at[p]]; k < s0[at[p] + 1]; k++)
+        if (pos[src[k]] % G == hot) { p1 = pos[src[k]]; break; }
+    }
+    if (p1 < 0) continue;
+    const int p2 = ((rnd >> 8) & 1) ? (p1 / G) * G + (int)((rnd >> 16) % G) : (int)((rnd >> 32) % (uint64_t)n);
+    if (p2 >= n || p2 == p1) continue;
     const int a = at[p1], b = at[p2];
+    if (s0[a + 1] - s0[a] != s0[b + 1] - s0[b]) continue;
     touched.clear();
     contrib(a, p1, -1, -1);
     contrib(b, p2, -1, a);
@@ -930,7 +1052,7 @@ std::vector<int> balance_positions(const std::vector<std::vector<uint32_t>> &row
     contrib(a, p2, +1, -1);
     contrib(b, p1, +1, a);
     long before = 0, after = 0;
-    std::vector<int> nd(touched.size());
+    nd.resize(touched.size());
     for (size_t i = 0; i < touched.size(); i++) {
       before += D[touched[i]];
       nd[i] = eval(touched[i]);
@@ -960,6 +1082,198 @@ void build_gather_table(const std::vector<std::vector<uint32_t>> &rows, int n, s
   build_gather(rows, unit, n, (n + 31) / 32 * 32, gat, wslots, &nslots, groups);
 }
 
+// The species (0 up, 1 down) and hop of a term that moves one electron; false for any other.
+static bool species_hop(const BitTerm &t, SpeciesHop *h, int *species) {
+  if (__builtin_popcountll(t.flip) != 2 || t.cm != t.flip) return false;
+  const int p = __builtin_ctzll(t.flip), q = 63 - __builtin_clzll(t.flip);
+  if ((p & 1) != (q & 1)) return false;
+  if (t.cv != (1ull << p) && t.cv != (1ull << q)) return false;
+  const int created = __builtin_ctzll(t.cv), annihilated = (created == p) ? q : p;
+  const double sg = (__builtin_popcountll(t.cv & t.sm) & 1) ? -1.0 : 1.0;
+  *h = SpeciesHop{created >> 1, annihilated >> 1, sg * t.re, sg * t.im};
+  *species = p & 1;
+  return true;
+}
+
+// Groups hops by coefficient up to sign: at time index k hop h has the coefficient
+// gsign[h] * cf[k * groups + gid[h]] (static H: one index).  seq[k][h]: coefficients; hops share
+// a group when their whole sequences agree up to one sign.
+struct HopGroups {
+  int n = 0;
+  std::vector<int> gid, gsign;
+  std::vector<double2> cf;
+};
+static bool coef_groups(const std::vector<std::vector<double2>> &seq, HopGroups *G) {
+  const size_t nk = seq.size(), nh = seq[0].size();
+  std::vector<size_t> rep;
+  for (size_t h = 0; h < nh; h++) {
+    int sign = 0;
+    size_t g = 0;
+    for (; g < rep.size() && sign == 0; g++)
+      for (int sg : {1, -1}) {
+        bool same = true;
+        for (size_t k = 0; k < nk && same; k++)
+          same = seq[k][h].x == sg * seq[k][rep[g]].x && seq[k][h].y == sg * seq[k][rep[g]].y;
+        if (same) { sign = sg; break; }
+      }
+    if (sign == 0) {
+      if (rep.size() == (size_t)kMaxGroups) return false;
+      rep.push_back(h);
+      sign = 1;
+      g = rep.size();
+    }
+    G->gid.push_back((int)g - 1);
+    G->gsign.push_back(sign);
+  }
+  G->n = (int)rep.size();
+  for (size_t k = 0; k < nk; k++)
+    for (size_t r : rep) G->cf.push_back(seq[k][r]);
+  return true;
+}
+static std::vector<std::vector<double2>> static_seq(const std::vector<SpeciesHop> &hops) {
+  std::vector<std::vector<double2>> q(1);
+  for (const SpeciesHop &h : hops) q[0].push_back(make_double2(h.re, h.im));
+  return q;
+}
+
+template <typename F>
+static void with_row_kernel(int stride, bool cplx_v, bool onsite, F f) {
+#define HPHI_ROW(S)                                                                                                     \
+  case S:                                                                                                               \
+    if (onsite) cplx_v ? f(prod_row_kernel<S, true, true>, RowShape<S>{}) : f(prod_row_kernel<S, false, true>, RowShape<S>{});  \
+    else cplx_v ? f(prod_row_kernel<S, true, false>, RowShape<S>{}) : f(prod_row_kernel<S, false, false>, RowShape<S>{});       \
+    break;
+  switch (stride) {
+    HPHI_ROW(960) HPHI_ROW(1744) HPHI_ROW(3456) HPHI_ROW(6560) HPHI_ROW(12896)
+  }
+#undef HPHI_ROW
+}
+
+// Tables and launch shapes of the two-pass kernels.  rows_*: per configuration its hops as
+// source | (2 * hop + sign) << 16.
+static int two_pass_build(Sector *s, ProdPlan *p, const std::vector<std::vector<uint32_t>> &rows_dn,
+                          const std::vector<std::vector<uint32_t>> &rows_up, const HopGroups (&G)[2], std::string *err) {
+  const int Uc = p->args.Uc, Dc = p->args.Dc;
+  TwoPassArgs &b = p->tp;
+  b.npad = (Dc + 31) / 32 * 32;
+  b.ng = G[1].n;
+  const int nw = b.npad / 32;
+  std::vector<std::vector<uint32_t>> tabs(b.ng);
+  std::vector<std::vector<uint8_t>> slots(b.ng);
+  std::vector<int> gsets(b.ng);
+  for (int g = 0; g < b.ng; g++) {
+    std::vector<std::vector<uint32_t>> rows(Dc);
+    for (int r = 0; r < Dc; r++)
+      for (uint32_t e : rows_dn[r]) {
+        const uint32_t h = (e >> 16) >> 1, sign = (e >> 16) & 1u;
+        if (G[1].gid[h] == g) rows[r].push_back((e & 0xFFFFu) | ((sign ^ (G[1].gsign[h] < 0 ? 1u : 0u)) << 16));
+      }
+    build_gather_table(rows, Dc, &tabs[g], &slots[g], &gsets[g]);
+  }
+  std::vector<uint4> gat, whead(nw);
+  for (int w = 0; w < nw; w++) {
+    uint64_t cnt = 0;
+    whead[w].x = (uint32_t)(gat.size() / 32);
+    for (int g = 0; g < b.ng; g++) {
+      cnt |= (uint64_t)slots[g][w] << (8 * g);
+      const uint32_t *t = &tabs[g][(size_t)w * gsets[g] * 128];
+      for (int i = 0; i < (slots[g][w] + 7) / 8 * 32; i++) gat.push_back(make_uint4(t[4 * i], t[4 * i + 1], t[4 * i + 2], t[4 * i + 3]));
+    }
+    whead[w].y = (uint32_t)cnt;
+    whead[w].z = (uint32_t)(cnt >> 32);
+    whead[w].w = 0;
+  }
+  gat.resize(gat.size() + 32, make_uint4(0, 0, 0, 0));  // read ahead, never used
+  b.ngu = G[0].n;
+  p->multi_up = b.ngu > 1 || Uc > 32768;
+  for (const double2 &c : G[0].cf) p->multi_up = p->multi_up || c.y != 0.0;
+  size_t wu = 1;
+  std::vector<uint8_t> nus(Uc, 0);
+  for (int r = 0; r < Uc; r++) {
+    nus[r] = (uint8_t)rows_up[r].size();
+    wu = std::max(wu, rows_up[r].size());
+  }
+  b.wu2 = p->multi_up ? (int)wu : (int)(wu + 1) / 2;
+  std::vector<uint32_t> ent((size_t)Uc * b.wu2, 0u);
+  for (int r = 0; r < Uc; r++)
+    for (size_t k = 0; k < rows_up[r].size(); k++) {
+      const uint32_t e = rows_up[r][k], h = (e >> 16) >> 1, src = e & 0xFFFFu;
+      const uint32_t sign = ((e >> 16) & 1u) ^ (G[0].gsign[h] < 0 ? 1u : 0u);
+      uint32_t *row = &ent[(size_t)r * b.wu2];
+      if (p->multi_up) row[k] = src | ((2u * (uint32_t)G[0].gid[h] + sign) << 16);
+      else row[k / 2] |= (src | (sign << 15)) << (16 * (k % 2));
+    }
+  if (upload(p, gat, &b.gat, err) || upload(p, whead, &b.whead, err) || upload(p, G[1].cf, &b.cf_dn, err) ||
+      upload(p, nus, &b.nus, err) || upload(p, ent, &b.up_ent, err) || upload(p, G[0].cf, &b.cf_up, err))
+    return -1;
+  for (int st : {960, 1744, 3456, 6560, 12896})
+    if (Dc + 16 <= st) {
+      p->stride = st;
+      break;
+    }
+  for (int cv = 0; cv < 2; cv++) {
+    int rc = 0;
+    with_row_kernel(p->stride, cv == 1, p->args.cross_mode == 0, [&](auto kernel, auto shape) {
+      using S = decltype(shape);
+      const size_t smem = sizeof(double) * (size_t)S::P * p->stride;
+      int per_sm = 0;
+      if (raise_smem_limit((const void *)kernel, smem) != cudaSuccess ||
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, S::threads, smem) != cudaSuccess || per_sm < 1)
+        rc = -1;
+      const int rows = cv ? S::P / 2 : S::P;
+      p->grid_row[cv] = std::max(1, std::min((Uc + rows - 1) / rows, per_sm * s->num_sms));
+    });
+    if (rc != 0) {
+      *err = "product plan: row pass does not fit";
+      return -1;
+    }
+  }
+  int col = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&col, prod_col_kernel<2, true, true, false>, kUpThreads, 0);
+  const int64_t ntask = (int64_t)Uc * ((2 * Dc + kUpChunk - 1) / kUpChunk);
+  p->grid_col = (int)std::max<int64_t>(1, std::min<int64_t>(std::max(1, col) * s->num_sms, (ntask + 7) / 8));
+  p->two_pass = true;
+  p->uniform = b.ng == 1;
+  for (const HopGroups &g : G)
+    for (const double2 &c : g.cf) p->uniform = p->uniform && c.y == 0.0;
+  const int nrec = std::max(p->grid_row[0], p->grid_row[1]) + p->grid_col;
+  if (nrec > Uc || !p->part) {
+    if (p->part) p->allocs.erase(std::find(p->allocs.begin(), p->allocs.end(), (void *)p->part));
+    cudaFree(p->part);
+    p->part = nullptr;
+    if (cudaMalloc(&p->part, sizeof(double) * 2 * (size_t)nrec) != cudaSuccess) {
+      *err = "product plan: device allocation failed";
+      return -1;
+    }
+    p->allocs.push_back(p->part);
+  }
+  return 0;
+}
+
+// Pieces of HPhi's blocks, by upper ups, then upper downs.
+static int perm_tasks_build(Sector *s, ProdPlan *p, std::string *err) {
+  std::vector<SectorBlock> blk, tasks;
+  std::vector<uint32_t> low;
+  if (sector_blocks(s, &blk, &low, err) != 0) return -1;
+  // the upper half's even bits are ups when N (the lower half's bits) is even, else downs
+  const uint32_t up_bits = (p->args.N % 2 == 0) ? 0x5555u : 0xAAAAu;
+  std::vector<std::pair<uint32_t, uint32_t>> order;  // (upper ups and downs, block)
+  for (size_t b = 0; b < blk.size(); b++) {
+    uint32_t up = 0, dn = 0;
+    for (int i = 0; i < 16; i++)
+      if ((blk[b].ib >> i) & 1u) ((up_bits >> i) & 1u ? up : dn) |= 1u << (i / 2);
+    order.push_back({(up << 8) | dn, (uint32_t)b});
+  }
+  std::sort(order.begin(), order.end());
+  for (const auto &o : order) {
+    const SectorBlock &b = blk[o.second];
+    for (uint32_t a = 0; a < b.n; a += kBlockPiece)
+      tasks.push_back(SectorBlock{b.ib, b.row0 + a, b.low0 + a, std::min<uint32_t>(kBlockPiece, b.n - a)});
+  }
+  p->nperm = (int)tasks.size();
+  return upload(p, tasks, &p->perm, err) || upload(p, low, &p->perm_low, err) ? -1 : 0;
+}
+
 int prod_plan_build(Sector *s, std::string *err) {
   const Model &m = s->model;
   s->prod = nullptr;
@@ -967,13 +1281,10 @@ int prod_plan_build(Sector *s, std::string *err) {
   const int N = m.nsite;
   std::vector<SpeciesHop> hops[2];
   for (const BitTerm &t : m.offdiag) {
-    if (__builtin_popcountll(t.flip) != 2 || t.cm != t.flip) return 0;
-    const int p = __builtin_ctzll(t.flip), q = 63 - __builtin_clzll(t.flip);
-    if ((p & 1) != (q & 1)) return 0;
-    if (t.cv != (1ull << p) && t.cv != (1ull << q)) return 0;
-    const int created = __builtin_ctzll(t.cv), annihilated = (created == p) ? q : p;
-    const double sg = (__builtin_popcountll(t.cv & t.sm) & 1) ? -1.0 : 1.0;
-    hops[p & 1].push_back(SpeciesHop{created >> 1, annihilated >> 1, sg * t.re, sg * t.im});
+    SpeciesHop h;
+    int sp;
+    if (!species_hop(t, &h, &sp)) return 0;
+    hops[sp].push_back(h);
   }
   if (hops[0].size() > 16000 || hops[1].size() > 16000) return 0;
   const int Uc = (int)binom_p(N, m.nup), Dc = (int)binom_p(N, m.ndown);
@@ -995,17 +1306,14 @@ int prod_plan_build(Sector *s, std::string *err) {
   int wd = 0, wu = 0;
   build_ell(hops[1], unrank_dn, rank, &rows_dn, &wd);
   build_ell(hops[0], unrank_up, rank, &rows_up, &wu);
-  // Two-pass kernels (real vectors): every down hop of one magnitude, real up hops, the
-  // second staged row at its fixed offset.  HPHI_B200_PROD=single keeps the one-pass kernel.
+  // Two-pass kernels: few enough coefficients per species (up to sign), the planes of a row in
+  // shared memory.  HPHI_B200_PROD=single keeps the one-pass kernel.
+  HopGroups G[2];
   bool two_pass_ok;
-  double tmag;
   {
     const char *pe = getenv("HPHI_B200_PROD");
-    two_pass_ok = !(pe && std::string(pe) == "single") && !hops[1].empty() &&
-                  (size_t)(Dc + 16) * 8 <= (size_t)kRow2Bytes && wd <= 255;
-    tmag = hops[1].empty() ? 0.0 : std::fabs(hops[1][0].re);
-    for (const SpeciesHop &h : hops[1]) two_pass_ok = two_pass_ok && h.im == 0.0 && std::fabs(h.re) == tmag && tmag > 0.0;
-    for (const SpeciesHop &h : hops[0]) two_pass_ok = two_pass_ok && h.im == 0.0;
+    two_pass_ok = !(pe && std::string(pe) == "single") && !hops[1].empty() && Dc + 16 <= 12896 && wd <= 255 &&
+                  wu <= 64 && coef_groups(static_seq(hops[1]), &G[1]) && coef_groups(static_seq(hops[0]), &G[0]);
   }
   // Down configurations take the positions balanced for the row pass's gather table
   // (balance_positions); HPHI_B200_BALANCE=0 keeps rank order.  Up configurations keep
@@ -1118,8 +1426,7 @@ int prod_plan_build(Sector *s, std::string *err) {
     }
     p->allocs.push_back(q);
     const unsigned nb = (unsigned)std::min<int64_t>((s->dim + 255) / 256, (int64_t)s->num_sms * 16);
-    prod_permute_kernel<double, true, false><<<nb, 256, 0, s->stream>>>(s->dim, N, Dc, s->d_list_1, a.rank, a.pos_dn,
-                                                                        s->d_diag, (double *)q);
+    prod_permute_diag_kernel<<<nb, 256, 0, s->stream>>>(s->dim, N, Dc, s->d_list_1, a.rank, a.pos_dn, s->d_diag, (double *)q);
     if (cudaStreamSynchronize(s->stream) != cudaSuccess) {
       *err = "product plan: diagonal permutation failed";
       return fail();
@@ -1147,130 +1454,71 @@ int prod_plan_build(Sector *s, std::string *err) {
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, prod_hv_kernel<double>, kProdThreads, smem_r);
   p->grid = std::max(1, std::min(Uc, std::max(1, per_sm) * s->num_sms));
-  {
-    if (two_pass_ok) {
-      TwoPassArgs &b = p->tp;
-      b.npad = (Dc + 31) / 32 * 32;
-      b.t_dn = tmag;
-      std::vector<uint32_t> gat;
-      std::vector<uint8_t> wslots;
-      int nslots = 0;
-      build_gather(rows_dn, hops[1], Dc, b.npad, &gat, &wslots, &nslots, &b.groups);
-      std::vector<uint4> gat4(gat.size() / 4);
-      for (size_t i = 0; i < gat4.size(); i++) gat4[i] = make_uint4(gat[4 * i], gat[4 * i + 1], gat[4 * i + 2], gat[4 * i + 3]);
-      b.t_up = hops[0].empty() ? 0.0 : std::fabs(hops[0][0].re);
-      b.up_uniform = b.t_up > 0.0 ? 1 : 0;
-      for (const SpeciesHop &h : hops[0]) b.up_uniform = b.up_uniform && std::fabs(h.re) == b.t_up;
-      const int wuu = std::max(wu, 1);
-      std::vector<int> usrc((size_t)Uc * wuu, 0);
-      std::vector<double> ucf((size_t)Uc * wuu, 0.0);
-      std::vector<uint8_t> nus(Uc, 0);
-      for (int r = 0; r < Uc; r++) {
-        for (size_t k = 0; k < rows_up[r].size(); k++) {
-          const uint32_t e = rows_up[r][k], h = (e >> 16) >> 1, sign = (e >> 16) & 1u;
-          const double cf = sign ? -hops[0][h].re : hops[0][h].re;
-          usrc[(size_t)r * wuu + k] = (int)(e & 0xFFFFu) | ((b.up_uniform && cf < 0) ? (int)0x80000000 : 0);
-          ucf[(size_t)r * wuu + k] = cf;
-        }
-        nus[r] = (uint8_t)rows_up[r].size();
-      }
-      // packed up-hop table of the warp-task column pass (uniform hops, ranks below 2^15)
-      std::vector<uint32_t> usrc16;
-      b.wu2 = 0;
-      if (b.up_uniform && Uc <= 32768 && wu <= 64) {
-        b.wu2 = std::max(1, (wu + 1) / 2);
-        usrc16.assign((size_t)Uc * b.wu2, 0u);
-        for (int r = 0; r < Uc; r++)
-          for (int k = 0; k < (int)nus[r]; k++) {
-            const uint32_t e = (uint32_t)usrc[(size_t)r * wuu + k];
-            const uint32_t e16 = (e & 0x7FFFu) | ((e >> 31) << 15);
-            usrc16[(size_t)r * b.wu2 + k / 2] |= (k % 2) ? (e16 << 16) : e16;
-          }
-      }
-      if (upload(p, gat4, &b.gat, err) || upload(p, wslots, &b.wslots, err) || upload(p, usrc, &b.usrc, err) ||
-          upload(p, ucf, &b.ucf, err) || upload(p, nus, &b.nus, err) || upload(p, usrc16, &b.usrc16, err))
-        return fail();
-      p->smem_dn = (size_t)kRow2Bytes + (size_t)(Dc + 16) * 8;
-      if (raise_smem_limit((const void *)prod_down_kernel, p->smem_dn) != cudaSuccess) {
-        *err = "product plan: shared-memory attribute rejected (row pass)";
-        return fail();
-      }
-      int up_per_sm = 0, upw_per_sm = 0;
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&up_per_sm, prod_up_kernel<true, true>, kUpThreads, 0);
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&upw_per_sm, prod_up_warp_kernel, kUpWThreads, 0);
-      p->grid_dn = std::max(1, std::min((Uc + 1) / 2, s->num_sms));
-      p->grid_upw = (b.wu2 > 0) ? std::max(1, upw_per_sm) * s->num_sms : 0;
-      {
-        const char *ue = getenv("HPHI_B200_UPPASS");
-        if (ue && std::string(ue) == "block") p->grid_upw = 0;
-      }
-      p->grid_up = std::max(std::max(1, std::max(1, up_per_sm) * s->num_sms), p->grid_upw);
-      p->two_pass = true;
-      if (2 * (p->grid_dn + p->grid_up) > 2 * Uc) {
-        cudaFree(p->part);
-        p->allocs.erase(std::find(p->allocs.begin(), p->allocs.end(), (void *)p->part));
-        p->part = nullptr;
-        if (cudaMalloc(&p->part, sizeof(double) * 2 * (size_t)(p->grid_dn + p->grid_up)) != cudaSuccess) {
-          *err = "product plan: device allocation failed";
-          return fail();
-        }
-        p->allocs.push_back(p->part);
-      }
-    }
-  }
+  if (two_pass_ok && two_pass_build(s, p, rows_dn, rows_up, G, err) != 0) return fail();
+  p->rank.swap(rank);
+  p->pos_dn.swap(pos_dn);
+  p->unrank_up.swap(unrank_up);
+  p->unrank_dn.swap(unrank_dn);
+  if (perm_tasks_build(s, p, err) != 0) return fail();
   s->prod = p;
   return 0;
 }
 
-bool prod_two_pass(const Sector *s) { return s->prod && s->prod->two_pass; }
+// The kernel number that hphi_info reports: 3 for hops of one real magnitude per species.
+bool prod_two_pass(const Sector *s) { return s->prod && s->prod->two_pass && s->prod->uniform; }
 
 size_t prod_scratch_doubles(const Sector *s, VecType vt) {
   const ProdPlan *p = s->prod;
-  // the two-pass kernels (real vectors) keep one partial sum per CTA of each pass; the
-  // one-pass kernel one per row
-  if (vt == kReal64 && p->two_pass) return 2 * (size_t)(p->grid_dn + p->grid_up);
-  return 2 * (size_t)p->args.Uc;
+  // the two-pass kernels keep one partial sum per CTA of each pass, the one-pass kernel one per
+  // row; callers with a fixed scratch (hphi_mltply_device_noalloc) are told of the latter for every
+  // input but real vectors under uniform hops, so the sectors they refuse stay the same
+  const size_t two = p->two_pass ? 2 * (size_t)(p->grid_row[vt == kReal64 ? 0 : 1] + p->grid_col) : 0;
+  if (p->two_pass && p->uniform && vt == kReal64) return two;
+  return std::max(two, 2 * (size_t)p->args.Uc);
 }
 
 namespace {
-// Row pass then column pass; partial sums at d_part (grid_dn + grid_up records of 2).
-void two_pass_launch(Sector *s, const double *v1, double *v0, const double *d_coef, double *d_out, double *d_part) {
-  ProdPlan *p = s->prod;
-  prod_down_kernel<<<p->grid_dn, kDownThreads, p->smem_dn, s->stream>>>(p->args, p->tp, v1, v0, d_coef, d_part);
-  const bool vec2 = (p->args.Dc % 2 == 0) && ((((uintptr_t)v1) | ((uintptr_t)v0)) % 16 == 0);
-  double *pu = d_part + 2 * p->grid_dn;
-  if (vec2 && p->grid_upw > 0) {
-    prod_up_warp_kernel<<<p->grid_upw, kUpWThreads, 0, s->stream>>>(p->args, p->tp, v1, v0, d_coef, pu);
-    finalize_partials_kernel<2><<<1, 256, 0, s->stream>>>(d_part, p->grid_dn + p->grid_upw, d_out);
-    return;
+// Row pass then column pass; partial sums at d_part (grid_row + grid_col records of 2).
+void two_pass_launch(Sector *s, const ProdPlan *p, bool cv, const double *v1, double *v0, const double *d_coef,
+                     double *d_out, double *d_part, const LanczosTail *lt, const TaylorSum &ts = TaylorSum{}) {
+  const int gr = p->grid_row[cv], gc = p->grid_col;
+  with_row_kernel(p->stride, cv, p->args.cross_mode == 0, [&](auto kernel, auto shape) {
+    using S = decltype(shape);
+    kernel<<<gr, S::threads, sizeof(double) * (size_t)S::P * p->stride, s->stream>>>(p->args, p->tp, v1, v0, d_coef, d_part);
+  });
+  const SumOut so = sum_out(d_part, gr, gr + gc, s->d_done, d_out, 0, lt);
+  // 16-byte loads where every row starts on a 16-byte boundary
+  const bool v2 = cv || ((p->args.Dc % 2 == 0) && ((((uintptr_t)v1) | ((uintptr_t)v0)) % 16 == 0));
+#define HPHI_COL_T(V, C, M, T) \
+  prod_col_kernel<V, C, M, T><<<gc, kUpThreads, 0, s->stream>>>(p->args, p->tp, v1, v0, d_coef, so, ts)
+#define HPHI_COL(V, C, M) HPHI_COL_T(V, C, M, false)
+  if (cv && ts.sum) {
+    if (p->multi_up) HPHI_COL_T(2, true, true, true);
+    else HPHI_COL_T(2, true, false, true);
+  } else if (cv) {
+    if (p->multi_up) HPHI_COL(2, true, true);
+    else HPHI_COL(2, true, false);
+  } else if (v2) {
+    if (p->multi_up) HPHI_COL(2, false, true);
+    else HPHI_COL(2, false, false);
+  } else {
+    if (p->multi_up) HPHI_COL(1, false, true);
+    else HPHI_COL(1, false, false);
   }
-  const int g = p->grid_up;
-  if (vec2 && p->tp.up_uniform)
-    prod_up_kernel<true, true><<<g, kUpThreads, 0, s->stream>>>(p->args, p->tp, v1, v0, d_coef, pu);
-  else if (vec2)
-    prod_up_kernel<true, false><<<g, kUpThreads, 0, s->stream>>>(p->args, p->tp, v1, v0, d_coef, pu);
-  else if (p->tp.up_uniform)
-    prod_up_kernel<false, true><<<g, kUpThreads, 0, s->stream>>>(p->args, p->tp, v1, v0, d_coef, pu);
-  else
-    prod_up_kernel<false, false><<<g, kUpThreads, 0, s->stream>>>(p->args, p->tp, v1, v0, d_coef, pu);
-  finalize_partials_kernel<2><<<1, 256, 0, s->stream>>>(d_part, p->grid_dn + p->grid_up, d_out);
+#undef HPHI_COL
+#undef HPHI_COL_T
 }
-}  // namespace
 
-int prod_hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
-                           double *d_part, int *d_counter) {
+int prod_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out, double *d_part,
+                int *d_counter, const LanczosTail *lt) {
   ProdPlan *p = s->prod;
   if (vt == kReal64 && s->model.complex_terms) {
     set_error("H has complex coefficients: real vectors are not allowed");
     return -1;
   }
-  if (vt == kReal64 && p->two_pass) {
-    two_pass_launch(s, (const double *)d_v1, (double *)d_v0, d_coef, d_out, d_part);
+  if (p->two_pass) {
+    two_pass_launch(s, p, vt != kReal64, (const double *)d_v1, (double *)d_v0, d_coef, d_out, d_part, lt);
     return cuda_ok(cudaGetLastError(), "launch");
-  }
-  if (cudaMemsetAsync(d_counter, 0, 2 * sizeof(int), s->stream) != cudaSuccess) {
-    set_error("product kernel: clearing the row counter failed");
-    return -1;
   }
   if (vt == kReal64)
     prod_hv_kernel<double><<<p->grid, kProdThreads, p->smem[0], s->stream>>>(
@@ -1279,59 +1527,102 @@ int prod_hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, 
     prod_hv_kernel<cplx><<<p->grid, kProdThreads, p->smem[1], s->stream>>>(p->args, (const cplx *)d_v1,
                                                                            (cplx *)d_v0, d_coef, d_part, d_counter);
   finalize_partials_kernel<2><<<1, 256, 0, s->stream>>>(d_part, p->args.Uc, d_out);
-  return cuda_ok(cudaGetLastError(), "launch");
+  if (cuda_ok(cudaGetLastError(), "launch") != 0) return -1;
+  return lt ? lanczos_scalars(s, 0, lt->k, lt->st, lt->alpha, lt->beta) : 0;
 }
+}  // namespace
 
-int prod_hv_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out) {
-  ProdPlan *p = s->prod;
-  if (vt == kReal64 && s->model.complex_terms) {
-    set_error("H has complex coefficients: real vectors are not allowed");
+int prod_hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
+                           double *d_part, int *d_counter) {
+  if (!s->prod->two_pass && cudaMemsetAsync(d_counter, 0, 2 * sizeof(int), s->stream) != cudaSuccess) {
+    set_error("product kernel: clearing the row counter failed");
     return -1;
   }
-  if (vt == kReal64 && p->two_pass) {
-    two_pass_launch(s, (const double *)d_v1, (double *)d_v0, d_coef, d_out, p->part);
-    return cuda_ok(cudaGetLastError(), "launch");
+  return prod_launch(s, vt, d_v1, d_v0, d_coef, d_out, d_part, d_counter, nullptr);
+}
+
+int prod_hv_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
+                   const LanczosTail *lt) {
+  return prod_launch(s, vt, d_v1, d_v0, d_coef, d_out, s->prod->part, s->prod->counter, lt);
+}
+
+// Time evolution: H(t) = the static terms plus those of a time index.  The plan holds the hops
+// of all indices once and a coefficient per group and index; its positions and diagonal are the
+// static plan's, so vectors, permutations and observables are those of s->prod.  *out stays
+// null where the two-pass kernels do not apply (terms other than hops, more coefficient groups
+// than kMaxGroups).
+int prod_te_plan_build(Sector *s, const std::vector<BitTerm> &terms, const std::vector<std::vector<double2>> &coefs,
+                       ProdPlan **out, std::string *err) {
+  *out = nullptr;
+  const ProdPlan *base = s->prod;
+  if (!base || coefs.empty() || base->args.Dc + 16 > 12896) return 0;
+  std::vector<SpeciesHop> hops[2];
+  std::vector<std::vector<double2>> seq[2];
+  for (auto &q : seq) q.resize(coefs.size());
+  for (size_t t = 0; t < terms.size(); t++) {
+    SpeciesHop h;
+    int sp;
+    BitTerm unit = terms[t];  // the term's sign alone
+    unit.re = 1.0;
+    unit.im = 0.0;
+    if (!species_hop(unit, &h, &sp)) return 0;
+    hops[sp].push_back(h);
+    for (size_t k = 0; k < coefs.size(); k++)
+      seq[sp][k].push_back(make_double2(h.re * coefs[k][t].x, h.re * coefs[k][t].y));
   }
-  if (vt == kReal64)
-    prod_hv_kernel<double><<<p->grid, kProdThreads, p->smem[0], s->stream>>>(
-        p->args, (const double *)d_v1, (double *)d_v0, d_coef, p->part, p->counter);
-  else
-    prod_hv_kernel<cplx><<<p->grid, kProdThreads, p->smem[1], s->stream>>>(p->args, (const cplx *)d_v1,
-                                                                           (cplx *)d_v0, d_coef, p->part, p->counter);
-  finalize_partials_kernel<2><<<1, 256, 0, s->stream>>>(p->part, p->args.Uc, d_out);
+  if (hops[1].empty() || hops[0].size() > 16000 || hops[1].size() > 16000) return 0;
+  HopGroups G[2];
+  if (!coef_groups(seq[0], &G[0]) || !coef_groups(seq[1], &G[1])) return 0;
+  std::vector<std::vector<uint32_t>> rows_dn, rows_up;
+  int wd = 0, wu = 0;
+  build_ell(hops[1], base->unrank_dn, base->pos_dn, &rows_dn, &wd);
+  build_ell(hops[0], base->unrank_up, base->rank, &rows_up, &wu);
+  if (wd > 255 || wu > 64) return 0;
+  ProdPlan *p = new ProdPlan();
+  p->args = base->args;
+  if (two_pass_build(s, p, rows_dn, rows_up, G, err) != 0) {
+    prod_plan_free(p);
+    return -1;
+  }
+  *out = p;
+  return 0;
+}
+
+int prod_te_launch(Sector *s, const ProdPlan *te, int index, const void *d_v1, void *d_v0, const double *d_coef,
+                   double *d_out, void *d_sum, double c_re, double c_im) {
+  ProdPlan p;  // the tables of this index's coefficients
+  p.args = te->args;
+  p.tp = te->tp;
+  p.tp.cf_dn += (size_t)index * te->tp.ng;
+  p.tp.cf_up += (size_t)index * te->tp.ngu;
+  p.stride = te->stride;
+  p.multi_up = te->multi_up;
+  p.grid_row[1] = te->grid_row[1];
+  p.grid_col = te->grid_col;
+  two_pass_launch(s, &p, true, (const double *)d_v1, (double *)d_v0, d_coef, d_out, te->part, nullptr,
+                  TaylorSum{(double2 *)d_sum, make_double2(c_re, c_im)});
   return cuda_ok(cudaGetLastError(), "launch");
 }
 
 int prod_permute(Sector *s, VecType vt, const void *in, void *out, bool to_native) {
-  ProdPlan *p = s->prod;
-  const unsigned nb = (unsigned)std::min<int64_t>((s->dim + 255) / 256, (int64_t)s->num_sms * 16);
-  const int N = p->args.N, Dc = p->args.Dc;
-  if (to_native && s->d_list_2_1 && s->d_list_2_2) {
-    const uint64_t lo_mask = s->ihfbit - 1;
+  const ProdPlan *p = s->prod;
+  const ProdArgs &a = p->args;
+  if (to_native) {
+    const unsigned nb = (unsigned)std::min(a.Uc, s->num_sms * 8);
     if (vt == kReal64)
-      prod_to_native_gather_kernel<double><<<nb, 256, 0, s->stream>>>(
-          s->dim, N, Dc, p->args.unrank_up, p->args.unrank_dn, s->d_list_2_1, s->d_list_2_2, s->lo_bits, lo_mask,
-          (const double *)in, (double *)out);
+      prod_to_native_kernel<double><<<nb, kPermThreads, 0, s->stream>>>(
+          a.N, a.Uc, a.Dc, a.unrank_up, a.unrank_dn, s->d_list_2_1, s->d_list_2_2, (const double *)in, (double *)out);
     else
-      prod_to_native_gather_kernel<cplx><<<nb, 256, 0, s->stream>>>(
-          s->dim, N, Dc, p->args.unrank_up, p->args.unrank_dn, s->d_list_2_1, s->d_list_2_2, s->lo_bits, lo_mask,
-          (const cplx *)in, (cplx *)out);
-    return cuda_ok(cudaGetLastError(), "permute");
-  }
-  if (vt == kReal64) {
-    if (to_native)
-      prod_permute_kernel<double, true, true><<<nb, 256, 0, s->stream>>>(s->dim, N, Dc, s->d_list_1, p->args.rank, p->args.pos_dn,
-                                                                         (const double *)in, (double *)out);
-    else
-      prod_permute_kernel<double, false, true><<<nb, 256, 0, s->stream>>>(s->dim, N, Dc, s->d_list_1, p->args.rank, p->args.pos_dn,
-                                                                          (const double *)in, (double *)out);
+      prod_to_native_kernel<cplx><<<nb, kPermThreads, 0, s->stream>>>(
+          a.N, a.Uc, a.Dc, a.unrank_up, a.unrank_dn, s->d_list_2_1, s->d_list_2_2, (const cplx *)in, (cplx *)out);
   } else {
-    if (to_native)
-      prod_permute_kernel<cplx, true, true><<<nb, 256, 0, s->stream>>>(s->dim, N, Dc, s->d_list_1, p->args.rank, p->args.pos_dn,
-                                                                       (const cplx *)in, (cplx *)out);
+    const unsigned nb = (unsigned)std::min((p->nperm + 7) / 8, s->num_sms * 8);
+    if (vt == kReal64)
+      prod_from_native_kernel<double><<<nb, kPermThreads, 0, s->stream>>>(a.N, a.Dc, p->perm, p->nperm, p->perm_low, a.rank,
+                                                                          a.pos_dn, (const double *)in, (double *)out);
     else
-      prod_permute_kernel<cplx, false, true><<<nb, 256, 0, s->stream>>>(s->dim, N, Dc, s->d_list_1, p->args.rank, p->args.pos_dn,
-                                                                        (const cplx *)in, (cplx *)out);
+      prod_from_native_kernel<cplx><<<nb, kPermThreads, 0, s->stream>>>(a.N, a.Dc, p->perm, p->nperm, p->perm_low, a.rank,
+                                                                        a.pos_dn, (const cplx *)in, (cplx *)out);
   }
   return cuda_ok(cudaGetLastError(), "permute");
 }
@@ -1339,11 +1630,11 @@ int prod_permute(Sector *s, VecType vt, const void *in, void *out, bool to_nativ
 int prod_observables(Sector *s, VecType vt, const void *v, double *d_out) {
   ProdPlan *p = s->prod;
   const int nb = s->red_blocks;
+  const SumOut so = sum_out(s->d_red, 0, nb, s->d_done, d_out);
   if (vt == kReal64)
-    prod_obs_kernel<double><<<nb, 256, 0, s->stream>>>(p->args, (const double *)v, s->d_red);
+    prod_obs_kernel<double><<<nb, 256, 0, s->stream>>>(p->args, (const double *)v, so);
   else
-    prod_obs_kernel<cplx><<<nb, 256, 0, s->stream>>>(p->args, (const cplx *)v, s->d_red);
-  finalize_partials_kernel<6><<<1, 256, 0, s->stream>>>(s->d_red, nb, d_out);
+    prod_obs_kernel<cplx><<<nb, 256, 0, s->stream>>>(p->args, (const cplx *)v, so);
   return cuda_ok(cudaGetLastError(), "observables");
 }
 

@@ -107,9 +107,10 @@ __global__ void __launch_bounds__(kRowThreads) rb_row_kernel(RBArgs p, SplitView
       const uint64_t c = hi | ia;
       const T x = row[a];
       T y = VT<T>::scale(__ldg(diag + r), x);
-      const uint32_t e0 = __ldg(sv.lo_ptr + ia), e1 = __ldg(sv.lo_ptr + ia + 1);
-      for (uint32_t e = e0; e < e1; e++) {
-        const uint32_t v = __ldg(sv.lo_ent + e);
+      const uint32_t nl = __ldg(sv.lo_ptr + ia);
+      const uint32_t *le = sv.lo_ent + ia;
+      for (uint32_t e = 0; e < nl; e++, le += sv.lo_stride) {
+        const uint32_t v = __ldg(le);
         const int src = (int)(v & ((1u << kSplitTargetBits) - 1u)) - p.lo_base;
         const double2 w = __ldg(cf + (v >> kSplitTargetBits));
         y = VT<T>::add(y, VT<T>::cmul_re_im(w.x, w.y, row[src]));

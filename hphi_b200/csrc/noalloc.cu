@@ -16,9 +16,10 @@
 // stream before it returns (it reads <v1|H|v1> back to the host).  The first call on a
 // device looks up the array's device address (cudaGetSymbolAddress, which may load the
 // module); make that first call before any stream capture.  The partial sums it needs are
-// 2 per CTA of the two passes for real vectors on the product-layout Hubbard kernels
-// (a few thousand), 2 per row of the up-spin matrix for its complex one-pass kernel, 2 per
-// block otherwise; a sector that needs more than the array holds is refused.
+// 2 per CTA of the two passes for real vectors under hops of one magnitude on the
+// product-layout Hubbard kernels (a few thousand), 2 per row of the up-spin matrix for the
+// other vectors and hops there, 2 per block otherwise; a sector that needs more than the array
+// holds is refused.
 #include <cuda_runtime.h>
 
 #include <mutex>

@@ -217,18 +217,27 @@ int split_plan_for_terms(Sector *s, const std::vector<BitTerm> &T, SplitPlan *pl
     CK(cudaMemcpy(P.gen, gen.data(), sizeof(BitTerm) * gen.size(), cudaMemcpyHostToDevice));
   }
   if (!usable) return 0;
-  // coefficient table: index 2i / 2i+1 = +/- coefficient of the i-th tabulated term
+  // Coefficient table.  tab_out: index 2i / 2i + 1 = +/- the i-th tabulated term's, so that a caller
+  // can replace the values; else one place per value, so that a warp's lookups meet in few lines.
   std::vector<int> tab;
   for (int q : lo_t) tab.push_back(q);
   for (int q : hi_t) tab.push_back(q);
   if (tab_out) *tab_out = tab;
-  std::vector<double> coef(4 * tab.size() + 2, 0.0);
-  for (size_t i = 0; i < tab.size(); i++) {
-    coef[4 * i] = T[tab[i]].re;
-    coef[4 * i + 1] = T[tab[i]].im;
-    coef[4 * i + 2] = -T[tab[i]].re;
-    coef[4 * i + 3] = -T[tab[i]].im;
-  }
+  std::vector<double> coef;
+  std::vector<uint32_t> coef_at;  // [2 * tabulated term + sign]
+  std::map<std::pair<double, double>, uint32_t> seen;
+  for (int q : tab)
+    for (double sg : {1.0, -1.0}) {
+      const std::pair<double, double> v{sg * T[q].re, sg * T[q].im};
+      const uint32_t next = (uint32_t)(coef.size() / 2);
+      const uint32_t at = tab_out ? next : seen.emplace(v, next).first->second;
+      if (at == next) {
+        coef.push_back(v.first);
+        coef.push_back(v.second);
+      }
+      coef_at.push_back(at);
+    }
+  coef.resize(coef.size() + 2, 0.0);
   std::vector<uint32_t> l21, l22;
   if (!s->gc) {
     l21.resize(s->ihfbit);
@@ -237,26 +246,34 @@ int split_plan_for_terms(Sector *s, const std::vector<BitTerm> &T, SplitPlan *pl
     CK(cudaMemcpy(l22.data(), s->d_list_2_2, sizeof(uint32_t) * s->sdim, cudaMemcpyDeviceToHost));
   }
   const uint64_t nlo = s->ihfbit, nhi = s->sdim;
-  std::vector<uint32_t> lo_ptr(nlo + 1, 0), lo_ent;
-  for (uint64_t ia = 0; ia < nlo; ia++) {
-    lo_ptr[ia] = (uint32_t)lo_ent.size();
-    if (!s->gc && l21[ia] == 0) continue;
-    for (size_t i = 0; i < lo_t.size(); i++) {
-      const BitTerm &t = T[lo_t[i]];
-      if ((ia & t.cm) != t.cv) continue;
-      const uint64_t src = ia ^ t.flip;
-      const uint64_t val = s->gc ? src : l21[src];
-      if (!s->gc && val == 0) continue;
-      if (val >= (1ull << kSplitTargetBits)) {
-        *err = "split plan: lower-half value out of range";
-        return -1;
+  std::vector<uint32_t> lo_ptr(nlo, 0), lo_ent;
+  for (int pass = 0; pass < 2; pass++) {  // count, then fill slot by slot
+    uint32_t most = 0;
+    for (uint64_t ia = 0; ia < nlo; ia++) {
+      uint32_t n = 0;
+      if (!s->gc && l21[ia] == 0) continue;
+      for (size_t i = 0; i < lo_t.size(); i++) {
+        const BitTerm &t = T[lo_t[i]];
+        if ((ia & t.cm) != t.cv) continue;
+        const uint64_t src = ia ^ t.flip;
+        const uint64_t val = s->gc ? src : l21[src];
+        if (!s->gc && val == 0) continue;
+        if (val >= (1ull << kSplitTargetBits)) {
+          *err = "split plan: lower-half value out of range";
+          return -1;
+        }
+        if (pass == 1) {
+          const uint32_t k = coef_at[2 * i + (size_t)(__builtin_popcountll(ia & t.sm) & 1)];
+          lo_ent[(size_t)n * nlo + ia] = (uint32_t)val | (k << kSplitTargetBits);
+        }
+        n++;
       }
-      const uint32_t k = 2 * (uint32_t)i + (uint32_t)(__builtin_popcountll(ia & t.sm) & 1);
-      lo_ent.push_back((uint32_t)val | (k << kSplitTargetBits));
+      lo_ptr[ia] = n;
+      most = std::max(most, n);
     }
-    if (lo_ent.size() > 0xFFFFFFF0ull) { *err = "split plan: too many entries"; return -1; }
+    if (pass == 0) lo_ent.assign((size_t)most * nlo, 0u);
   }
-  lo_ptr[nlo] = (uint32_t)lo_ent.size();
+  P.lo_stride = (uint32_t)nlo;
   std::vector<uint32_t> hi_ptr(nhi + 1, 0);
   std::vector<HiEnt> hi_ent;
   for (uint64_t ib = 0; ib < nhi; ib++) {
@@ -274,7 +291,7 @@ int split_plan_for_terms(Sector *s, const std::vector<BitTerm> &T, SplitPlan *pl
         if (l22[src] == 0) continue;
         h.delta = (int64_t)l22[src] - (int64_t)l22[ib];
       }
-      h.k = 2 * (uint32_t)(lo_t.size() + i) + (uint32_t)(__builtin_popcountll(cfg & t.sm) & 1);
+      h.k = coef_at[2 * (lo_t.size() + i) + (size_t)(__builtin_popcountll(cfg & t.sm) & 1)];
       hi_ent.push_back(h);
     }
     if (hi_ent.size() > 0xFFFFFFF0ull) { *err = "split plan: too many entries"; return -1; }
@@ -337,6 +354,61 @@ int64_t sector_dim(const Model &m) {
   return (int64_t)binom_host(m.nsite, m.ne);
 }
 
+namespace {
+__global__ void first_lower_kernel(int n, const uint32_t *__restrict__ start, const uint64_t *__restrict__ list_1,
+                                   uint64_t lo_mask, uint32_t *__restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = (uint32_t)(list_1[start[i]] & lo_mask);
+}
+}  // namespace
+
+int sector_blocks(const Sector *s, std::vector<SectorBlock> *out, std::vector<uint32_t> *low, std::string *err) {
+  out->clear();
+  low->clear();
+  std::vector<uint32_t> l22(s->sdim), start, ibs;
+  CK(cudaMemcpy(l22.data(), s->d_list_2_2, sizeof(uint32_t) * l22.size(), cudaMemcpyDeviceToHost));
+  for (uint64_t ib = 0; ib < s->sdim; ib++)
+    if (l22[ib]) {
+      ibs.push_back((uint32_t)ib);
+      start.push_back(l22[ib] - 1u);
+    }
+  // a lower half belongs to one class (list_2_1 gives it one rank), so a block's first one names it
+  uint32_t *d = nullptr;
+  std::vector<uint32_t> first(start.size());
+  CK(cudaMalloc(&d, sizeof(uint32_t) * 2 * std::max<size_t>(1, start.size())));
+  cudaError_t e = cudaMemcpy(d, start.data(), sizeof(uint32_t) * start.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && !start.empty()) {
+    first_lower_kernel<<<(unsigned)((start.size() + 255) / 256), 256, 0, s->stream>>>(
+        (int)start.size(), d, s->d_list_1, s->ihfbit - 1, d + start.size());
+    e = cudaMemcpyAsync(first.data(), d + start.size(), sizeof(uint32_t) * start.size(), cudaMemcpyDeviceToHost, s->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+  }
+  cudaFree(d);
+  CK(e);
+  struct Class {
+    uint32_t n, low0;
+  };
+  std::map<uint32_t, Class> cls;  // by first lower half
+  std::vector<uint64_t> rows;
+  for (size_t b = 0; b < start.size(); b++) {
+    const int64_t end = b + 1 < start.size() ? (int64_t)start[b + 1] : s->dim;
+    const int64_t n = end - (int64_t)start[b];
+    auto it = cls.find(first[b]);
+    if (n > 0 && it == cls.end()) {
+      it = cls.emplace(first[b], Class{(uint32_t)n, (uint32_t)low->size()}).first;
+      rows.resize((size_t)n);
+      CK(cudaMemcpy(rows.data(), s->d_list_1 + start[b], sizeof(uint64_t) * (size_t)n, cudaMemcpyDeviceToHost));
+      for (uint64_t c : rows) low->push_back((uint32_t)(c & (s->ihfbit - 1)));
+    }
+    if (n <= 0 || it->second.n != (uint32_t)n) {
+      *err = "sector blocks: unexpected layout";
+      return -1;
+    }
+    out->push_back(SectorBlock{ibs[b], start[b], it->second.low0, (uint32_t)n});
+  }
+  return 0;
+}
+
 int sector_build(const Model &m, int device, Sector **out, std::string *err, bool specialise) {
   CK(cudaSetDevice(device));
   Sector *s = new Sector();
@@ -349,6 +421,8 @@ int sector_build(const Model &m, int device, Sector **out, std::string *err, boo
   s->red_blocks = nsm * 8;
   CK(cudaMalloc(&s->d_red, sizeof(double) * 8 * (size_t)s->red_blocks));
   CK(cudaMalloc(&s->d_scal, sizeof(double) * 64));
+  s->d_done = reinterpret_cast<unsigned *>(s->d_scal + 64 - kHvBlockMax);
+  CK(cudaMemsetAsync(s->d_done, 0, sizeof(unsigned) * kHvBlockMax, s->stream));
 
   const int nbits = m.nbits;
   s->gc = m.rows_are_configs();
@@ -592,6 +666,10 @@ int sector_build(const Model &m, int device, Sector **out, std::string *err, boo
     cudaFree(d_cnt); cudaFree(d_jb); cudaFree(d_total); cudaFree(d_need);
   }
 
+  // a block per 256 rows at most: the 1184-block grids of 8 per SM cost small sectors more in
+  // block starts and partial sums than in rows
+  s->red_blocks = (int)std::min<int64_t>(s->red_blocks, std::max<int64_t>(1, (s->dim + 255) / 256));
+
   // Terms.
   s->nterms = (int)m.offdiag.size();
   s->ndterms = (int)m.diag.size();
@@ -622,7 +700,8 @@ int sector_build(const Model &m, int device, Sector **out, std::string *err, boo
   // Row-block plan (spin sectors): from 2^24 rows up, where the vectors no longer stay in L2
   // and the general kernel's scattered gathers go to memory (below that the general kernel is
   // faster); HPHI_B200_KERNEL=rowblock builds it at any size.
-  if (specialise && kname != "general" && !s->prod && !s->hub && (kname == "rowblock" || s->dim >= (1ll << 24))) {
+  if (specialise && kname != "general" && !s->prod && !s->hub &&
+      (kname == "rowblock" || s->dim >= (1ll << 24))) {
     if (rb_plan_build(s, err) != 0) return -1;
   }
   *out = s;

@@ -24,15 +24,17 @@ namespace hphi {
 constexpr int kSplitTargetBits = 20;
 
 struct SplitView {
-  const uint32_t *lo_ptr;   // [2^lo_bits + 1] or nullptr (no plan)
-  const uint32_t *lo_ent;
+  const uint32_t *lo_ptr;   // [2^lo_bits] number of entries, or nullptr (no plan)
+  const uint32_t *lo_ent;   // slot by slot: the lanes of a warp have neighbouring lower halves, so
+  uint32_t lo_stride;       // their entries of one slot come from a few lines (lists one after
+                            // another put every lane on its own line)
   const uint32_t *hi_ptr;   // [2^hi_bits + 1]
   const HiEnt *hi_ent;
   const double *coef;       // (re, im) per coefficient index, sign included
 };
 
 __host__ inline SplitView split_view(const SplitPlan &p) {
-  return SplitView{p.lo_ptr, p.lo_ent, p.hi_ptr, p.hi_ent, p.coef};
+  return SplitView{p.lo_ptr, p.lo_ent, p.lo_stride, p.hi_ptr, p.hi_ent, p.coef};
 }
 
 // Adds the lower- and upper-half terms of row r (configuration c) to y.  load(j) returns
@@ -43,9 +45,10 @@ __device__ __forceinline__ A split_terms(const SplitView &P, uint64_t c, int64_t
   const uint32_t ia = (uint32_t)(c & lo_mask);
   const uint64_t ib = c >> lo_bits;
   const int64_t base = GC ? (int64_t)(c & ~lo_mask) : (int64_t)__ldg(l22 + ib) - 3;
-  const uint32_t l0 = __ldg(P.lo_ptr + ia), l1 = __ldg(P.lo_ptr + ia + 1);
-  for (uint32_t e = l0; e < l1; e++) {
-    const uint32_t v = __ldg(P.lo_ent + e);
+  const uint32_t nl = __ldg(P.lo_ptr + ia);
+  const uint32_t *le = P.lo_ent + ia;
+  for (uint32_t e = 0; e < nl; e++, le += P.lo_stride) {
+    const uint32_t v = __ldg(le);
     const uint32_t tgt = v & ((1u << kSplitTargetBits) - 1u);
     const uint32_t k = v >> kSplitTargetBits;
     const int64_t j = GC ? (base | (int64_t)tgt) : base + (int64_t)tgt;

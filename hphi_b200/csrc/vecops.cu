@@ -3,7 +3,8 @@
 // The reference does these as separate OpenMP loops over 1-based complex arrays
 // (recurrence sweep src/Lanczos_EigenValue.c:153-160, beta src/Lanczos_EigenValue.c:170-177,
 // TPQ Multiply src/Multiply.c:42-68).  Here every reduction writes one record per
-// block and a single block sums the records, so results do not depend on timing.
+// block and the block that finishes last sums the records in order (grid_sum), so results do
+// not depend on timing.
 #include <cuda_runtime.h>
 
 #include <string>
@@ -18,23 +19,21 @@ namespace {
 constexpr int kThreads = 256;
 
 template <typename T>
-__global__ void norm2_kernel(int64_t n, const T *__restrict__ x, double *__restrict__ part) {
+__global__ void norm2_kernel(int64_t n, const T *__restrict__ x, SumOut so) {
   double v[1] = {0.0};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     v[0] += VT<T>::abs2(x[i]);
-  block_sum<1>(v);
-  if (threadIdx.x == 0) part[blockIdx.x] = v[0];
+  grid_sum<1>(v, so);
 }
 
 template <typename T>
-__global__ void dot_kernel(int64_t n, const T *__restrict__ x, const T *__restrict__ y, double *__restrict__ part) {
+__global__ void dot_kernel(int64_t n, const T *__restrict__ x, const T *__restrict__ y, SumOut so) {
   double v[2] = {0.0, 0.0};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     v[0] += VT<T>::conj_mul_re(x[i], y[i]);
     v[1] += VT<T>::conj_mul_im(x[i], y[i]);
   }
-  block_sum<2>(v);
-  if (threadIdx.x == 0) { part[2 * blockIdx.x] = v[0]; part[2 * blockIdx.x + 1] = v[1]; }
+  grid_sum<2>(v, so);
 }
 
 template <typename T>
@@ -52,7 +51,9 @@ __global__ void scale_kernel(int64_t n, double a, T *__restrict__ x) {
 // p <- p - (alpha*sq) q and |p|^2, alpha*sq read from device memory.
 template <typename T>
 __global__ void lanczos_sweep_kernel(int64_t n, const double *__restrict__ coef, T *__restrict__ p,
-                                     const T *__restrict__ q, double *__restrict__ part) {
+                                     const T *__restrict__ q, SumOut so) {
+  cudaGridDependencySynchronize();  // launch_chained
+  cudaTriggerProgrammaticLaunchCompletion();
   const double c = coef[0];
   double v[1] = {0.0};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -60,8 +61,7 @@ __global__ void lanczos_sweep_kernel(int64_t n, const double *__restrict__ coef,
     p[i] = w;
     v[0] += VT<T>::abs2(w);
   }
-  block_sum<1>(v);
-  if (threadIdx.x == 0) part[blockIdx.x] = v[0];
+  grid_sum<1>(v, so);
 }
 
 // Occupation statistics of a configuration, as expec_energy_flct_Hubbard /
@@ -73,7 +73,7 @@ __global__ void lanczos_sweep_kernel(int64_t n, const double *__restrict__ coef,
 template <typename T>
 __global__ void diag_obs_kernel(int64_t n, int gc, int spin, int nsite, int site_bits, int sum2s,
                                 const uint64_t *__restrict__ list_1, const T *__restrict__ x,
-                                double *__restrict__ part) {
+                                SumOut so) {
   double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   const uint64_t even = 0x5555555555555555ull;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -101,10 +101,7 @@ __global__ void diag_obs_kernel(int64_t n, int gc, int spin, int nsite, int site
     v[2] += w * N; v[3] += w * N * N;
     v[4] += w * Sz; v[5] += w * Sz * Sz;
   }
-  block_sum<6>(v);
-  if (threadIdx.x == 0)
-#pragma unroll
-    for (int k = 0; k < 6; k++) part[6 * blockIdx.x + k] = v[k];
+  grid_sum<6>(v, so);
 }
 
 __global__ void real_from_c128_kernel(int64_t n, const cplx *__restrict__ src, double *__restrict__ dst) {
@@ -114,6 +111,10 @@ __global__ void real_from_c128_kernel(int64_t n, const cplx *__restrict__ src, d
 __global__ void c128_from_real_kernel(int64_t n, const double *__restrict__ src, cplx *__restrict__ dst) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     dst[i] = cplx{src[i], 0.0};
+}
+
+SumOut red_out(Sector *s, double *out, int phase = -1, const LanczosTail *lt = nullptr) {
+  return sum_out(s->d_red, 0, s->red_blocks, s->d_done, out, phase, lt);
 }
 
 int check_launch(const char *what) {
@@ -128,18 +129,16 @@ int check_launch(const char *what) {
 }  // namespace
 
 int vec_norm2(Sector *s, VecType vt, const void *x, double *out) {
-  if (vt == kReal64) norm2_kernel<double><<<s->red_blocks, kThreads, 0, s->stream>>>(s->dim, (const double *)x, s->d_red);
-  else norm2_kernel<cplx><<<s->red_blocks, kThreads, 0, s->stream>>>(s->dim, (const cplx *)x, s->d_red);
-  finalize_partials_kernel<1><<<1, 256, 0, s->stream>>>(s->d_red, s->red_blocks, out);
+  if (vt == kReal64) norm2_kernel<double><<<s->red_blocks, kThreads, 0, s->stream>>>(s->dim, (const double *)x, red_out(s, out));
+  else norm2_kernel<cplx><<<s->red_blocks, kThreads, 0, s->stream>>>(s->dim, (const cplx *)x, red_out(s, out));
   return check_launch("vec_norm2");
 }
 
 int vec_dot(Sector *s, VecType vt, const void *x, const void *y, double *out) {
   if (vt == kReal64)
-    dot_kernel<double><<<s->red_blocks, kThreads, 0, s->stream>>>(s->dim, (const double *)x, (const double *)y, s->d_red);
+    dot_kernel<double><<<s->red_blocks, kThreads, 0, s->stream>>>(s->dim, (const double *)x, (const double *)y, red_out(s, out));
   else
-    dot_kernel<cplx><<<s->red_blocks, kThreads, 0, s->stream>>>(s->dim, (const cplx *)x, (const cplx *)y, s->d_red);
-  finalize_partials_kernel<2><<<1, 256, 0, s->stream>>>(s->d_red, s->red_blocks, out);
+    dot_kernel<cplx><<<s->red_blocks, kThreads, 0, s->stream>>>(s->dim, (const cplx *)x, (const cplx *)y, red_out(s, out));
   return check_launch("vec_dot");
 }
 
@@ -157,14 +156,15 @@ int vec_scale(Sector *s, VecType vt, double a, void *x) {
   return check_launch("vec_scale");
 }
 
-int vec_lanczos_sweep(Sector *s, VecType vt, const double *coef, void *p, const void *q, double *out) {
+int vec_lanczos_sweep(Sector *s, VecType vt, const double *coef, void *p, const void *q, double *out,
+                      const LanczosTail *lt) {
+  const SumOut so = red_out(s, out, 1, lt);
   if (vt == kReal64)
-    lanczos_sweep_kernel<double><<<s->red_blocks, kThreads, 0, s->stream>>>(s->dim, coef, (double *)p,
-                                                                            (const double *)q, s->d_red);
+    launch_chained(lanczos_sweep_kernel<double>, s->red_blocks, kThreads, 0, s->stream, s->dim, coef, (double *)p,
+                   (const double *)q, so);
   else
-    lanczos_sweep_kernel<cplx><<<s->red_blocks, kThreads, 0, s->stream>>>(s->dim, coef, (cplx *)p, (const cplx *)q,
-                                                                          s->d_red);
-  finalize_partials_kernel<1><<<1, 256, 0, s->stream>>>(s->d_red, s->red_blocks, out);
+    launch_chained(lanczos_sweep_kernel<cplx>, s->red_blocks, kThreads, 0, s->stream, s->dim, coef, (cplx *)p,
+                   (const cplx *)q, so);
   return check_launch("vec_lanczos_sweep");
 }
 
@@ -176,11 +176,10 @@ int vec_diag_observables(Sector *s, VecType vt, const void *x, double *out) {
   for (int q = 0; q < m.nsite && m.general_spin; q++) sum2s += m.locspn[q];
   if (vt == kReal64)
     diag_obs_kernel<double><<<s->red_blocks, kThreads, 0, s->stream>>>(
-        s->dim, s->gc ? 1 : 0, spin, m.nsite, gbits, sum2s, s->d_list_1, (const double *)x, s->d_red);
+        s->dim, s->gc ? 1 : 0, spin, m.nsite, gbits, sum2s, s->d_list_1, (const double *)x, red_out(s, out));
   else
     diag_obs_kernel<cplx><<<s->red_blocks, kThreads, 0, s->stream>>>(
-        s->dim, s->gc ? 1 : 0, spin, m.nsite, gbits, sum2s, s->d_list_1, (const cplx *)x, s->d_red);
-  finalize_partials_kernel<6><<<1, 256, 0, s->stream>>>(s->d_red, s->red_blocks, out);
+        s->dim, s->gc ? 1 : 0, spin, m.nsite, gbits, sum2s, s->d_list_1, (const cplx *)x, red_out(s, out));
   return check_launch("vec_diag_observables");
 }
 
@@ -227,24 +226,8 @@ int vec_to_host_c128(Sector *s, VecType vt, const void *d, double *h) {
 namespace hphi {
 namespace {
 
-// Per-step scalar bookkeeping of the device-resident Lanczos recurrence.  st layout:
-//   st[0..1] raw sum conj(Q)(HQ) from hv   st[2] acc   st[3] s (scale of Q)
-//   st[4] sweep coefficient alpha*s       st[5] |w|^2 from the sweep
-// phase 0 (after hv, step k):    alpha_k = s^2 Re(raw); coef = alpha_k * s
-// phase 1 (after sweep, step k): beta_k = sqrt(|w|^2); acc = -beta_k * s; s = 1/beta_k
 __global__ void lanczos_scalars_kernel(int phase, int k, double *st, double *alpha, double *beta) {
-  if (threadIdx.x != 0) return;
-  if (phase == 0) {
-    const double s = st[3];
-    const double a = s * s * st[0];
-    alpha[k] = a;
-    st[4] = a * s;
-  } else {
-    const double b = sqrt(st[5]);
-    beta[k] = b;
-    st[2] = -b * st[3];
-    st[3] = 1.0 / b;
-  }
+  if (threadIdx.x == 0) lanczos_scalar_update(phase, k, st, alpha, beta);
 }
 
 // Eigenvector replay sweep (src/Lanczos_EigenVector.c:150-190): with the stored
@@ -263,15 +246,14 @@ __global__ void replay_sweep_kernel(int64_t n, double a_sq, double c_over_b, T *
 // w = (L*sv)*v - (sh/Ns)*h written into v, |w|^2 into part.
 template <typename T>
 __global__ void tpq_sweep_kernel(int64_t n, double cv, double ch, T *__restrict__ v, const T *__restrict__ h,
-                                 double *__restrict__ part) {
+                                 SumOut so) {
   double acc[1] = {0.0};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const T w = VT<T>::sub(VT<T>::scale(cv, v[i]), VT<T>::scale(ch, h[i]));
     v[i] = w;
     acc[0] += VT<T>::abs2(w);
   }
-  block_sum<1>(acc);
-  if (threadIdx.x == 0) part[blockIdx.x] = acc[0];
+  grid_sum<1>(acc, so);
 }
 
 // CG sweep of the eigenvector refinement (src/CG_EigenVector.c:143-185) with the shifted
@@ -279,7 +261,7 @@ __global__ void tpq_sweep_kernel(int64_t n, double cv, double ch, T *__restrict_
 template <typename T>
 __global__ void cg_sweep_kernel(int64_t n, double a, double shift, const T *__restrict__ p,
                                 const T *__restrict__ hp, T *__restrict__ x, T *__restrict__ r,
-                                double *__restrict__ part) {
+                                SumOut so) {
   double acc[1] = {0.0};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const T pi = p[i];
@@ -289,8 +271,7 @@ __global__ void cg_sweep_kernel(int64_t n, double a, double shift, const T *__re
     r[i] = w;
     acc[0] += VT<T>::abs2(w);
   }
-  block_sum<1>(acc);
-  if (threadIdx.x == 0) part[blockIdx.x] = acc[0];
+  grid_sum<1>(acc, so);
 }
 
 // Adds amp * start_value(seed, configuration, 0) to the real part of an HPhi-order vector
@@ -342,13 +323,13 @@ int vec_replay_sweep(Sector *s, VecType vt, double a_sq, double c_over_b, void *
 }
 
 int vec_tpq_sweep(Sector *s, VecType vt, double cv, double ch, void *v, const void *h, double *out) {
+  const SumOut so = sum_out(s->d_red, 0, s->red_blocks, s->d_done, out);
   if (vt == kReal64)
     tpq_sweep_kernel<double><<<s->red_blocks, kThreads, 0, s->stream>>>(s->dim, cv, ch, (double *)v,
-                                                                        (const double *)h, s->d_red);
+                                                                        (const double *)h, so);
   else
     tpq_sweep_kernel<cplx><<<s->red_blocks, kThreads, 0, s->stream>>>(s->dim, cv, ch, (cplx *)v, (const cplx *)h,
-                                                                      s->d_red);
-  finalize_partials_kernel<1><<<1, 256, 0, s->stream>>>(s->d_red, s->red_blocks, out);
+                                                                      so);
   return check_launch("vec_tpq_sweep");
 }
 
@@ -360,11 +341,10 @@ int vec_cg_sweep(Sector *s, VecType vt, double a, double shift, const void *p, c
                  double *out) {
   if (vt == kReal64)
     cg_sweep_kernel<double><<<s->red_blocks, kThreads, 0, s->stream>>>(
-        s->dim, a, shift, (const double *)p, (const double *)hp, (double *)x, (double *)r, s->d_red);
+        s->dim, a, shift, (const double *)p, (const double *)hp, (double *)x, (double *)r, red_out(s, out));
   else
     cg_sweep_kernel<cplx><<<s->red_blocks, kThreads, 0, s->stream>>>(s->dim, a, shift, (const cplx *)p,
-                                                                     (const cplx *)hp, (cplx *)x, (cplx *)r, s->d_red);
-  finalize_partials_kernel<1><<<1, 256, 0, s->stream>>>(s->d_red, s->red_blocks, out);
+                                                                     (const cplx *)hp, (cplx *)x, (cplx *)r, red_out(s, out));
   return check_launch("vec_cg_sweep");
 }
 

@@ -1,0 +1,107 @@
+"""Every H*v path against the general row kernel (HPHI_B200_KERNEL=general, itself pinned to the
+reference by test_gpu_parity) at the sizes where a path can go wrong: the shapes of the row, block
+and tile kernels and one below and above their limits, odd row lengths, one-row sectors,
+coefficient groups up to and past what a plan holds."""
+import os
+
+import numpy as np
+import pytest
+
+import hphi_b200
+from hphi_b200 import expert
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def _open(path, general=False):
+    saved = os.environ.get("HPHI_B200_KERNEL")
+    os.environ.pop("HPHI_B200_KERNEL", None)
+    if general:
+        os.environ["HPHI_B200_KERNEL"] = "general"
+    try:
+        return hphi_b200.Hamiltonian(path)
+    finally:
+        os.environ.pop("HPHI_B200_KERNEL", None)
+        if saved is not None:
+            os.environ["HPHI_B200_KERNEL"] = saved
+
+
+def _compare(m, tmp_path, vts=(hphi_b200.REAL64, hphi_b200.COMPLEX128)):
+    """v0 = acc v0 + scale H v1 and <v1|H|v1> in HPhi's order, both paths.  Bound: a row sums at most
+    ~200 products in another order, so |difference| <= 200 eps |H| |v| elementwise; 1e-13 of the
+    largest element leaves a margin for the sums' size."""
+    path = m.write(str(tmp_path))
+    Ha, Hg = _open(path), _open(path, general=True)
+    try:
+        for vt in vts:
+            dt = torch.float64 if vt == hphi_b200.REAL64 else torch.complex128
+            g = torch.Generator(device="cuda").manual_seed(7)
+            v1 = torch.randn(Ha.dim, dtype=dt, device="cuda", generator=g)
+            w = torch.randn(Ha.dim, dtype=dt, device="cuda", generator=g)
+            for acc, scale in ((0.0, 1.0), (0.5, -2.0)):
+                out, pr = [], []
+                for H in (Ha, Hg):
+                    v0 = w.clone() if acc else torch.full_like(w, float("nan"))
+                    torch.cuda.synchronize()
+                    pr.append(H.mltply_device(v0.data_ptr(), v1.data_ptr(), vt, acc=acc, scale=scale))
+                    out.append(v0)
+                big = out[1].abs().max().item()
+                assert (out[0] - out[1]).abs().max().item() <= 1e-13 * big
+                n = torch.linalg.vector_norm(v1).item() * torch.linalg.vector_norm(out[1]).item()
+                assert abs(pr[0] - pr[1]) <= 1e-13 * max(n, abs(pr[1]))
+        return Ha.info["kernel"]
+    finally:
+        Ha.close()
+        Hg.close()
+
+
+def _hubbard(N, nup, ndown, phases=0, anisotropic=0):
+    """Ring of N sites; `phases` hops carry their own phase, `anisotropic` their own amplitude."""
+    m = expert.hubbard(N, [], 1.0, 4.0, nup, ndown)
+    for k, (i, j) in enumerate(expert.chain_bonds(N)):
+        t = (1.0 + 0.05 * k if k < anisotropic else 1.0) * np.exp(1j * (0.1 * (k + 1) if k < phases else 0.0))
+        for s in (0, 1):
+            m.trans += [(i, s, j, s, t.real, t.imag), (j, s, i, s, t.real, -t.imag)]
+    return m
+
+
+PROD = {
+    # rows of 924, 1287 (odd), 1716, 3432, 5005 (odd) and 8008 elements: every row shape, both loads
+    "n12": lambda: _hubbard(12, 3, 6),
+    "n13": lambda: _hubbard(13, 2, 5),
+    "n13_6": lambda: _hubbard(13, 3, 6),
+    "n14": lambda: _hubbard(14, 2, 7),
+    "n15": lambda: _hubbard(15, 2, 6),
+    "n16": lambda: _hubbard(16, 2, 6),
+    "n7_odd": lambda: _hubbard(7, 3, 3),
+    "one_row": lambda: _hubbard(6, 6, 3),
+    "one_column": lambda: _hubbard(6, 3, 6),
+    "two_amplitudes": lambda: _hubbard(10, 5, 4, anisotropic=1),
+    "eight_amplitudes": lambda: _hubbard(10, 5, 4, anisotropic=8),
+    "ten_amplitudes": lambda: _hubbard(10, 5, 4, anisotropic=10),   # past the groups: the one-pass kernel
+}
+
+
+@pytest.mark.parametrize("name", list(PROD))
+def test_product_layout(name, tmp_path):
+    assert _compare(PROD[name](), tmp_path) in (2, 3)
+
+
+@pytest.mark.parametrize("phases", [1, 3, 10])
+def test_product_layout_complex_coefficients(phases, tmp_path):
+    _compare(_hubbard(10, 5, 4, phases=phases), tmp_path, vts=(hphi_b200.COMPLEX128,))
+
+
+@pytest.mark.parametrize("N, nup, ndown", [(1, 1, 0), (5, 2, 3), (8, 4, 4), (11, 5, 6), (12, 6, 6)])
+@pytest.mark.parametrize("vt", [hphi_b200.REAL64, hphi_b200.COMPLEX128])
+def test_native_order_round_trip(N, nup, ndown, vt, tmp_path):
+    """to_native then from_native is the identity, bit for bit (a permutation with signs)."""
+    m = expert.hubbard(N, expert.chain_bonds(N) if N > 1 else [], 1.0, 4.0, nup, ndown)
+    with _open(m.write(str(tmp_path))) as H:
+        v = torch.randn(H.dim, dtype=torch.float64 if vt == hphi_b200.REAL64 else torch.complex128, device="cuda")
+        a, b = torch.zeros_like(v), torch.zeros_like(v)
+        torch.cuda.synchronize()
+        H.to_native(v.data_ptr(), a.data_ptr(), vt)
+        H.from_native(a.data_ptr(), b.data_ptr(), vt)
+        assert torch.equal(v, b)
