@@ -54,6 +54,8 @@ struct LanczosTail {
   double *st, *alpha, *beta;
 };
 
+struct SectorBlock;
+
 struct Sector {
   Model model;
   int device = 0;
@@ -90,6 +92,9 @@ struct Sector {
   // rows that share an upper half (hv_rowblock.cu).
   RowBlockPlan *rb = nullptr;
   SplitPlan split;
+  SectorBlock *d_pieces = nullptr;  // sector_pieces
+  uint32_t *d_low = nullptr;
+  int npieces = 0, nlow = 0;
   // General spin: the device tables above are indexed by packed digit codes; HPhi's own
   // mixed-radix lists (src/sz.c:795-830, 1564-1590) are kept here for export.
   std::vector<uint64_t> gs_list_1, gs_list_2_1, gs_list_2_2;
@@ -110,7 +115,9 @@ struct SectorBlock {
   uint32_t ib, row0, low0, n;
 };
 int sector_blocks(const Sector *s, std::vector<SectorBlock> *out, std::vector<uint32_t> *low, std::string *err);
-constexpr int kBlockPiece = 512;  // rows of a block taken by one warp
+// The blocks in pieces of at most kBlockPiece rows and `low` on the device, made on first use.
+constexpr int kBlockPiece = 512;
+int sector_pieces(Sector *s, std::string *err);
 
 // specialise = false skips the specialised kernel plans (the batched engine uses the
 // general row kernel only).

@@ -409,6 +409,27 @@ int sector_blocks(const Sector *s, std::vector<SectorBlock> *out, std::vector<ui
   return 0;
 }
 
+int sector_pieces(Sector *s, std::string *err) {
+  if (s->d_pieces) return 0;
+  std::vector<SectorBlock> blk, pc;
+  std::vector<uint32_t> low;
+  if (sector_blocks(s, &blk, &low, err) != 0) return -1;
+  // class by class: neighbouring warps read the same per-class tables
+  std::stable_sort(blk.begin(), blk.end(), [](const SectorBlock &x, const SectorBlock &y) { return x.low0 < y.low0; });
+  for (const SectorBlock &b : blk)
+    for (uint32_t a = 0; a < b.n; a += kBlockPiece)
+      pc.push_back(SectorBlock{b.ib, b.row0 + a, b.low0 + a, std::min<uint32_t>(kBlockPiece, b.n - a)});
+  CK(cudaMalloc(&s->d_low, sizeof(uint32_t) * std::max<size_t>(1, low.size())));
+  CK(cudaMemcpy(s->d_low, low.data(), sizeof(uint32_t) * low.size(), cudaMemcpyHostToDevice));
+  SectorBlock *d = nullptr;
+  CK(cudaMalloc(&d, sizeof(SectorBlock) * std::max<size_t>(1, pc.size())));
+  s->d_pieces = d;
+  CK(cudaMemcpy(d, pc.data(), sizeof(SectorBlock) * pc.size(), cudaMemcpyHostToDevice));
+  s->npieces = (int)pc.size();
+  s->nlow = (int)low.size();
+  return 0;
+}
+
 int sector_build(const Model &m, int device, Sector **out, std::string *err, bool specialise) {
   CK(cudaSetDevice(device));
   Sector *s = new Sector();
@@ -715,7 +736,7 @@ void sector_free(Sector *s) {
   cudaFree(s->d_list_1); cudaFree(s->d_list_2_1); cudaFree(s->d_list_2_2); cudaFree(s->d_diag);
   cudaFree(s->d_terms); cudaFree(s->d_dterms); cudaFree(s->d_red); cudaFree(s->d_scal);
   cudaFree(s->split.lo_ptr); cudaFree(s->split.lo_ent); cudaFree(s->split.hi_ptr); cudaFree(s->split.hi_ent);
-  cudaFree(s->split.coef); cudaFree(s->split.gen);
+  cudaFree(s->split.coef); cudaFree(s->split.gen); cudaFree(s->d_pieces); cudaFree(s->d_low);
   hub_plan_free(s->hub);
   prod_plan_free(s->prod);
   rb_plan_free(s->rb);
