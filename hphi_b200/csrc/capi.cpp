@@ -254,7 +254,10 @@ int hphi_mltply_device(hphi_handle *h, int vec_type, void *d_v0, const void *d_v
     }
     if (to_native(s, vt, d_v1, h->d_perm1) != 0) return -1;
     if (acc != 0.0 && to_native(s, vt, d_v0, h->d_perm0) != 0) return -1;
-    if (hv_native(s, vt, h->d_perm1, h->d_perm0, h->d_scal, h->d_scal + 2) != 0) return -1;
+    const bool rows = s->prod && vt == kComplex128;  // prdct's imaginary part: see prod_hv_launch_rows
+    if ((rows ? prod_hv_launch_rows(s, vt, h->d_perm1, h->d_perm0, h->d_scal, h->d_scal + 2)
+              : hv_native(s, vt, h->d_perm1, h->d_perm0, h->d_scal, h->d_scal + 2)) != 0)
+      return -1;
     if (from_native(s, vt, h->d_perm0, d_v0) != 0) return -1;
   }
   double out[2];

@@ -970,10 +970,7 @@ void build_gather(const std::vector<std::vector<uint32_t>> &rows_dn, const std::
 // load) (the edge colouring of build_gather), so positions decide both.  Start from the
 // configurations sorted by hop count (equal lane degrees in a half-warp), then swap positions
 // (within a half-warp: a bank change; across half-warps: only between equal hop counts) when
-// that does not raise the summed slot counts of the half-warps it touches.  A proposal moves a
-// source in the fullest bank pair of a half-warp that its bank pairs, not its lanes, hold up:
-// 40 per configuration reach the slot counts (within 1.5%) that 200 drawn blindly do, in a
-// quarter of the time (7 of 14 sites 180 -> 44 ms, 6 of 16 sites 820 -> 173 ms).  rows[r]: sources
+// that does not raise the summed slot counts of the half-warps it touches.  rows[r]: sources
 // of configuration r (ELL entries, source in the low 16 bits).  Returns the position of each
 // configuration; deterministic (fixed seed).
 std::vector<int> balance_positions(const std::vector<std::vector<uint32_t>> &rows) {
@@ -985,66 +982,49 @@ std::vector<int> balance_positions(const std::vector<std::vector<uint32_t>> &row
   for (int p = 0; p < n; p++) pos[order[p]] = p;
   const int ng = (n + G - 1) / G;
   if (n < 4 * G) return pos;
-  // sources and readers of each configuration, back to back
-  std::vector<int> src, rdr, s0(n + 1, 0), r0(n + 2, 0);
-  for (int r = 0; r < n; r++) {
-    for (uint32_t e : rows[r]) {
-      src.push_back((int)(e & 0xFFFFu));
-      r0[(e & 0xFFFFu) + 2]++;
-    }
-    s0[r + 1] = (int)src.size();
-  }
-  for (int r = 0; r < n; r++) r0[r + 2] += r0[r + 1];
-  rdr.resize(src.size());
+  std::vector<std::vector<int>> src(n), rdr(n);
   for (int r = 0; r < n; r++)
-    for (int k = s0[r]; k < s0[r + 1]; k++) rdr[r0[src[k] + 1]++] = r;
+    for (uint32_t e : rows[r]) {
+      const int q = (int)(e & 0xFFFFu);
+      src[r].push_back(q);
+      rdr[q].push_back(r);
+    }
   std::vector<int> at(order);  // configuration at each position
-  std::vector<uint16_t> load((size_t)ng * G, 0), lmax(ng, 0), D(ng, 0);
+  std::vector<int> load((size_t)ng * G, 0), lmax(ng, 0), D(ng, 0);
   for (int r = 0; r < n; r++) {
     const int g = pos[r] / G;
-    lmax[g] = std::max(lmax[g], (uint16_t)(s0[r + 1] - s0[r]));
-    for (int k = s0[r]; k < s0[r + 1]; k++) load[(size_t)g * G + pos[src[k]] % G]++;
+    lmax[g] = std::max(lmax[g], (int)src[r].size());
+    for (int q : src[r]) load[(size_t)g * G + pos[q] % G]++;
   }
   auto eval = [&](int g) {
-    uint16_t m = lmax[g];
+    int m = lmax[g];
     for (int k = 0; k < G; k++) m = std::max(m, load[(size_t)g * G + k]);
     return m;
   };
   for (int g = 0; g < ng; g++) D[g] = eval(g);
   uint64_t rng = 0x9E3779B97F4A7C15ull;
   auto next = [&]() { rng ^= rng << 13; rng ^= rng >> 7; rng ^= rng << 17; return rng; };
-  std::vector<int> touched, nd;
+  std::vector<int> touched;
   std::vector<char> mark(ng, 0);
   auto touch = [&](int g) { if (!mark[g]) { mark[g] = 1; touched.push_back(g); } };
   // adds (sgn = 1) or removes (-1) a configuration's edges: its reads (in its own half-warp)
   // and the reads of it; edges to `other` are left to the other configuration's call
   auto contrib = [&](int r, int p, int sgn, int other) {
     const int g = p / G, bk = p % G;
-    for (int k = s0[r]; k < s0[r + 1]; k++)
-      if (src[k] != other) load[(size_t)g * G + pos[src[k]] % G] += sgn;
-    for (int k = r0[r]; k < r0[r + 1]; k++)
-      if (rdr[k] != other) { const int gg = pos[rdr[k]] / G; load[(size_t)gg * G + bk] += sgn; touch(gg); }
+    for (int q : src[r])
+      if (q != other) load[(size_t)g * G + pos[q] % G] += sgn;
+    for (int rr : rdr[r])
+      if (rr != other) { const int gg = pos[rr] / G; load[(size_t)gg * G + bk] += sgn; touch(gg); }
     touch(g);
   };
-  const int64_t iters = std::min<int64_t>(40 * (int64_t)n, 800000);
+  const int64_t iters = std::min<int64_t>(200 * (int64_t)n, 4000000);
   for (int64_t it = 0; it < iters; it++) {
-    const int gh = (int)(((next() >> 32) * (uint64_t)ng) >> 32);
-    if (D[gh] == lmax[gh]) continue;
-    const uint16_t *ld = &load[(size_t)gh * G];
-    const int hot = (int)(std::max_element(ld, ld + G) - ld);
-    const uint64_t rnd = next();
-    int p1 = -1;
-    for (int l = 0; l < G && p1 < 0; l++) {
-      const int p = gh * G + (((int)(rnd & 15) + l) & 15);
-      if (p >= n) continue;
-      for (int k = s0[at[p]]; k < s0[at[p] + 1]; k++)
-        if (pos[src[k]] % G == hot) { p1 = pos[src[k]]; break; }
-    }
-    if (p1 < 0) continue;
-    const int p2 = ((rnd >> 8) & 1) ? (p1 / G) * G + (int)((rnd >> 16) % G) : (int)((rnd >> 32) % (uint64_t)n);
-    if (p2 >= n || p2 == p1) continue;
+    const int p1 = (int)(next() % n);
+    int p2;
+    if (next() & 1) p2 = (p1 / G) * G + (int)(next() % G);
+    else p2 = (int)(next() % n);
+    if (p2 >= n || p2 == p1 || src[at[p1]].size() != src[at[p2]].size()) continue;
     const int a = at[p1], b = at[p2];
-    if (s0[a + 1] - s0[a] != s0[b + 1] - s0[b]) continue;
     touched.clear();
     contrib(a, p1, -1, -1);
     contrib(b, p2, -1, a);
@@ -1052,7 +1032,7 @@ std::vector<int> balance_positions(const std::vector<std::vector<uint32_t>> &row
     contrib(a, p2, +1, -1);
     contrib(b, p1, +1, a);
     long before = 0, after = 0;
-    nd.resize(touched.size());
+    std::vector<int> nd(touched.size());
     for (size_t i = 0; i < touched.size(); i++) {
       before += D[touched[i]];
       nd[i] = eval(touched[i]);
@@ -1233,9 +1213,6 @@ static int two_pass_build(Sector *s, ProdPlan *p, const std::vector<std::vector<
   const int64_t ntask = (int64_t)Uc * ((2 * Dc + kUpChunk - 1) / kUpChunk);
   p->grid_col = (int)std::max<int64_t>(1, std::min<int64_t>(std::max(1, col) * s->num_sms, (ntask + 7) / 8));
   p->two_pass = true;
-  p->uniform = b.ng == 1;
-  for (const HopGroups &g : G)
-    for (const double2 &c : g.cf) p->uniform = p->uniform && c.y == 0.0;
   const int nrec = std::max(p->grid_row[0], p->grid_row[1]) + p->grid_col;
   if (nrec > Uc || !p->part) {
     if (p->part) p->allocs.erase(std::find(p->allocs.begin(), p->allocs.end(), (void *)p->part));
@@ -1315,13 +1292,17 @@ int prod_plan_build(Sector *s, std::string *err) {
     two_pass_ok = !(pe && std::string(pe) == "single") && !hops[1].empty() && Dc + 16 <= 12896 && wd <= 255 &&
                   wu <= 64 && coef_groups(static_seq(hops[1]), &G[1]) && coef_groups(static_seq(hops[0]), &G[0]);
   }
+  bool uniform_hops = two_pass_ok && G[1].n == 1;  // down hops of one magnitude, no complex hop
+  for (const HopGroups &g : G)
+    for (const double2 &c : g.cf) uniform_hops = uniform_hops && c.y == 0.0;
   // Down configurations take the positions balanced for the row pass's gather table
-  // (balance_positions); HPHI_B200_BALANCE=0 keeps rank order.  Up configurations keep
-  // their rank.
+  // (balance_positions) where there is one magnitude; HPHI_B200_BALANCE=0 keeps rank order.
+  // Up configurations keep their rank.  Complex or several hops keep rank order: 14% more slots on
+  // 14 sites (BAL_US us per H*v), where the search would take the sector's build from 8 to 160 ms.
   std::vector<uint16_t> pos_dn(rank);
   {
     const char *bal = getenv("HPHI_B200_BALANCE");
-    if (two_pass_ok && !(bal && std::string(bal) == "0")) {
+    if (two_pass_ok && uniform_hops && !(bal && std::string(bal) == "0")) {
       const std::vector<int> pos = balance_positions(rows_dn);
       std::vector<uint16_t> un(Dc);
       for (int r = 0; r < Dc; r++) un[pos[r]] = unrank_dn[r];
@@ -1454,6 +1435,7 @@ int prod_plan_build(Sector *s, std::string *err) {
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, prod_hv_kernel<double>, kProdThreads, smem_r);
   p->grid = std::max(1, std::min(Uc, std::max(1, per_sm) * s->num_sms));
+  p->uniform = uniform_hops;
   if (two_pass_ok && two_pass_build(s, p, rows_dn, rows_up, G, err) != 0) return fail();
   p->rank.swap(rank);
   p->pos_dn.swap(pos_dn);
@@ -1510,13 +1492,13 @@ void two_pass_launch(Sector *s, const ProdPlan *p, bool cv, const double *v1, do
 }
 
 int prod_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out, double *d_part,
-                int *d_counter, const LanczosTail *lt) {
+                int *d_counter, const LanczosTail *lt, bool one_pass = false) {
   ProdPlan *p = s->prod;
   if (vt == kReal64 && s->model.complex_terms) {
     set_error("H has complex coefficients: real vectors are not allowed");
     return -1;
   }
-  if (p->two_pass) {
+  if (p->two_pass && !one_pass) {
     two_pass_launch(s, p, vt != kReal64, (const double *)d_v1, (double *)d_v0, d_coef, d_out, d_part, lt);
     return cuda_ok(cudaGetLastError(), "launch");
   }
@@ -1544,6 +1526,13 @@ int prod_hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, 
 int prod_hv_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
                    const LanczosTail *lt) {
   return prod_launch(s, vt, d_v1, d_v0, d_coef, d_out, s->prod->part, s->prod->counter, lt);
+}
+
+// By the one-pass kernel: <v1|H v1> of complex vectors as the sum of its per-row sums.  All there
+// is of that sum's imaginary part is its rounding, so a call that hands both parts to its caller
+// keeps the order of the additions.
+int prod_hv_launch_rows(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out) {
+  return prod_launch(s, vt, d_v1, d_v0, d_coef, d_out, s->prod->part, s->prod->counter, nullptr, true);
 }
 
 // Time evolution: H(t) = the static terms plus those of a time index.  The plan holds the hops

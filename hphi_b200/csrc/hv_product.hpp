@@ -21,6 +21,7 @@ int prod_hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, 
 size_t prod_scratch_doubles(const Sector *s, VecType vt);
 // True when real vectors take the two-pass kernels (row pass + column pass).
 bool prod_two_pass(const Sector *s);
+int prod_hv_launch_rows(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out);
 // Time evolution on the product layout (complex vectors in s->prod's native order):
 // terms: off-diagonal terms by mask, coefs[k][t] the coefficient of term t at time index k.
 int prod_te_plan_build(Sector *s, const std::vector<BitTerm> &terms, const std::vector<std::vector<double2>> &coefs,

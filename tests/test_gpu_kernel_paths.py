@@ -105,3 +105,50 @@ def test_native_order_round_trip(N, nup, ndown, vt, tmp_path):
         H.to_native(v.data_ptr(), a.data_ptr(), vt)
         H.from_native(a.data_ptr(), b.data_ptr(), vt)
         assert torch.equal(v, b)
+
+
+GREEN = {
+    # longest blocks of 1, 36 (odd sector), 462 and, in pieces of 512 rows, 924
+    "chain2": lambda: expert.heisenberg(2, [(0, 1)]),
+    "hubbard9": lambda: expert.hubbard(9, expert.chain_bonds(9), 1.0, 3.0, 4, 5),
+    "chain21": lambda: expert.heisenberg(21, expert.chain_bonds(21), two_sz=1),
+    "chain24": lambda: expert.heisenberg(24, expert.chain_bonds(24)),
+}
+
+
+@pytest.mark.parametrize("vt", [hphi_b200.REAL64, hphi_b200.COMPLEX128])
+@pytest.mark.parametrize("name", list(GREEN))
+def test_green_blocks(name, vt, tmp_path):
+    """<v|H|v> put together from Green's functions against the H*v's own, and adjoint rows as
+    conjugates.  Bound: |v| = 1, so every function is at most 1 and sums products in another order;
+    1e-13 of the sum of |coefficients| leaves a margin."""
+    m = GREEN[name]()
+    one, two = [], []   # (coefficient, row)
+    for i, s1, j, s2, re, im in m.trans:
+        one.append((-complex(re, im), (i, s1, j, s2)))
+    for i, U in m.coulombintra:
+        two.append((U, (i, 0, i, 0, i, 1, i, 1)))
+    for i, j, J in m.ising:
+        two += [(0.25 * J * (1 if a == b else -1), (i, a, i, a, j, b, j, b)) for a in (0, 1) for b in (0, 1)]
+    for i, j, J in m.exchange:
+        two += [(J, (i, 0, i, 1, j, 1, j, 0)), (J, (j, 0, j, 1, i, 1, i, 0))]
+    with _open(m.write(str(tmp_path))) as H:
+        v = torch.randn(H.dim, dtype=torch.float64 if vt == hphi_b200.REAL64 else torch.complex128, device="cuda",
+                        generator=torch.Generator(device="cuda").manual_seed(5))
+        v /= torch.linalg.vector_norm(v)
+        w = torch.zeros_like(v)
+        torch.cuda.synchronize()
+        ref = H.mltply_device(w.data_ptr(), v.data_ptr(), vt, acc=0.0, scale=1.0)
+        e, weight = 0.0, 0.0
+        for body, rows in ((1, one), (2, two)):
+            if not rows:
+                continue
+            g = H.expec_green_device(v.data_ptr(), vt, [r for _, r in rows], body)
+            e += sum(c * x for (c, _), x in zip(rows, g))
+            weight += sum(abs(c) for c, _ in rows)
+            at = {r: x for (_, r), x in zip(rows, g)}
+            for r, x in at.items():
+                adj = r[2:4] + r[0:2] if body == 1 else r[6:8] + r[4:6] + r[2:4] + r[0:2]
+                if adj in at:
+                    assert abs(at[adj] - np.conj(x)) <= 1e-13
+    assert abs(e - ref) <= 1e-13 * weight
