@@ -39,7 +39,7 @@ INFO_FIELDS = ["dim", "nsite", "calc_model", "calc_type", "size_list_2_1", "size
                "n_green_one", "n_green_two"]
 EXPORTED_SYMBOLS = ["hphi_version", "hphi_last_error", "hphi_open_expert", "hphi_close", "hphi_info",
                     "hphi_sz", "hphi_diagonalcalc", "hphi_mltply", "hphi_mltply_device", "hphi_lanczos",
-                    "hphi_lanczos_eigenvector", "hphi_tpq", "hphi_tem", "hphi_run", "hphi_inspect_terms",
+                    "hphi_lanczos_eigenvector", "hphi_tpq", "hphi_tpq_vectors", "hphi_tem", "hphi_run", "hphi_inspect_terms",
                     "hphi_lanczos_tridiagonal", "hphi_mltply_device_async", "hphi_stream",
                     "hphi_synchronize", "hphi_to_native", "hphi_from_native", "hphi_mltply_device_noalloc",
                     "hphi_lanczos_steps", "hphi_batch_create", "hphi_batch_lanczos", "hphi_batch_tuning",
@@ -94,6 +94,7 @@ def load_library() -> ctypes.CDLL:
     lib.hphi_lanczos.argtypes = [P, pd, ctypes.c_char_p, pd, I]
     lib.hphi_lanczos_eigenvector.argtypes = [P, pd]
     lib.hphi_tpq.argtypes = [P, pd, ctypes.c_char_p, pd, I]
+    lib.hphi_tpq_vectors.argtypes = [P, ctypes.POINTER(pd), ctypes.c_char_p, pd, I]
     lib.hphi_tem.argtypes = [P, pd, ctypes.c_char_p, pd, I]
     lib.hphi_run.argtypes = [P, ctypes.c_char_p]
     lib.hphi_spectrum.argtypes = [P, pd, ctypes.c_char_p, pd, I]
@@ -397,13 +398,14 @@ class Hamiltonian:
                     nresult: Optional[int] = None) -> np.ndarray:
         n = nresult or self.info["lanczos_max"]
         res = np.zeros(n)
-        buf = None
+        ptrs = None
         if v_init is not None:
-            buf = np.ascontiguousarray(np.stack([_as_hphi_vector(v, self.dim) for v in v_init]))
-            if buf.shape[0] < self.info["num_ave"]:
+            vecs = [_as_hphi_vector(v, self.dim) for v in v_init]
+            if len(vecs) < self.info["num_ave"]:
                 raise ValueError("need one start vector per TPQ sample (NumAve)")
-        _check(load_library().hphi_tpq(self._h, None if buf is None else _dptr(buf.view(np.float64)),
-                                       None if output_dir is None else os.fsencode(output_dir), _dptr(res), n))
+            ptrs = (ctypes.POINTER(ctypes.c_double) * len(vecs))(*[_dptr(v.view(np.float64)) for v in vecs])
+        _check(load_library().hphi_tpq_vectors(self._h, ptrs, None if output_dir is None else os.fsencode(output_dir),
+                                               _dptr(res), n))
         return res
 
     def calc_by_tem(self, v_init: Optional[np.ndarray] = None, output_dir: Optional[str] = None,

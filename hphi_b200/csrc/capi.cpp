@@ -528,6 +528,14 @@ int hphi_lanczos_eigenvector(hphi_handle *h, double *v) {
 
 int hphi_tpq(hphi_handle *h, const double *v_init, const char *output_dir, double *result, int nresult) {
   CHECK_HANDLE(h);
+  std::vector<const double *> v;
+  for (int i = 0; v_init && i < h->sector->model.num_ave; i++)
+    v.push_back(v_init + 2 * (size_t)(h->sector->dim + 1) * i);
+  return hphi_tpq_vectors(h, v_init ? v.data() : nullptr, output_dir, result, nresult);
+}
+
+int hphi_tpq_vectors(hphi_handle *h, const double *const *v_init, const char *output_dir, double *result, int nresult) {
+  CHECK_HANDLE(h);
   Sector *s = h->sector;
   const VecType vt = default_vec_type(*s);
   const std::string out = output_dir ? output_dir : "output";
@@ -571,9 +579,9 @@ int hphi_tpq(hphi_handle *h, const double *v_init, const char *output_dir, doubl
   auto run_pending = [&]() -> int {
     if (pending.empty()) return 0;
     std::vector<const double *> hv;
-    for (size_t b = 0; b < pending.size(); b++) hv.push_back(starts[b].empty() ? v_init + stride * pending[b] : starts[b].data());
+    for (size_t b = 0; b < pending.size(); b++) hv.push_back(starts[b].empty() ? v_init[pending[b]] : starts[b].data());
     std::vector<TpqResult> rr;
-    if (tpq_run_samples(s, vt, hv, pending, out, &rr, opt, block_ok && pending.size() > 1) != 0) return -1;
+    if (tpq_run_samples(s, vt, hv, pending, out, &rr, opt, hv_block_applies(s, vt)) != 0) return -1;
     for (size_t b = 0; b < pending.size(); b++)
       if (opt.keep_vector && save(pending[b], rr[b]) != 0) return -1;
     r = std::move(rr.back());

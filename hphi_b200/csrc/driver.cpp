@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <array>
 #include <cmath>
+#include <complex>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -33,6 +34,7 @@
 #include "batch.hpp"
 #include "driver.hpp"
 #include "engine.hpp"
+#include "hv_product.hpp"
 
 namespace hphi {
 
@@ -158,6 +160,48 @@ int cuda_ok(cudaError_t e, const char *what) {
 }
 
 #define RET(x) do { if ((x) != 0) return -1; } while (0)
+
+// Device memory of one driver call.  Mapping and unmapping the vectors cost a short run more than
+// its steps (four 14 MB vectors: 2 of 8 ms), so up to kWorkspaceKeep bytes stay with the sector
+// and the next call carves its vectors from them; what does not fit is allocated and freed by
+// the call, as is everything of a call inside another one on the same handle.
+constexpr size_t kWorkspaceKeep = (size_t)64 << 20;
+class Workspace {
+ public:
+  // bytes: what the call is going to take, each piece rounded up to 256
+  Workspace(Sector *s, size_t bytes) : s_(s), mine_(!s->ws_busy.exchange(true)) {
+    if (!mine_) return;
+    if (bytes <= s->ws_bytes || bytes > kWorkspaceKeep) return;
+    cudaFree(s->ws);
+    s->ws = nullptr;
+    s->ws_bytes = 0;
+    if (cudaMalloc(&s->ws, bytes) == cudaSuccess) s->ws_bytes = bytes;
+    else cudaGetLastError();
+  }
+  ~Workspace() {
+    for (void *p : own_) cudaFree(p);
+    if (mine_) s_->ws_busy = false;
+  }
+  Workspace(const Workspace &) = delete;
+  Workspace &operator=(const Workspace &) = delete;
+  static size_t round(size_t bytes) { return (bytes + 255) / 256 * 256; }
+  int get(void **p, size_t bytes, const char *what) {
+    if (mine_ && s_->ws && at_ + round(bytes) <= s_->ws_bytes) {
+      *p = (char *)s_->ws + at_;
+      at_ += round(bytes);
+      return 0;
+    }
+    RET(cuda_ok(cudaMalloc(p, bytes), what));
+    own_.push_back(*p);
+    return 0;
+  }
+
+ private:
+  Sector *s_;
+  bool mine_;
+  size_t at_ = 0;
+  std::vector<void *> own_;
+};
 
 }  // namespace
 
@@ -375,10 +419,8 @@ int lanczos_run(Sector *s, VecType vt, const double *h_init, const LanczosOption
   const int64_t dim = s->dim;
   const size_t esz = (vt == kReal64) ? sizeof(double) : sizeof(cplx);
   RET(cuda_ok(cudaSetDevice(s->device), "cudaSetDevice"));
-  DevBuf P, Q, V0, ST, AL, BE;
-  RET(cuda_ok(cudaMalloc(&P.p, esz * dim), "alloc P"));
-  RET(cuda_ok(cudaMalloc(&Q.p, esz * dim), "alloc Q"));
-  RET(cuda_ok(cudaMalloc(&ST.p, sizeof(double) * 32), "alloc scalars"));  // slots used: [0, 29)
+  struct { void *p = nullptr; } P, Q, ST, AL, BE;
+  DevBuf V0;
   const bool fixed = opt.fixed_steps > 0;
   const LanczosRestart *rs = opt.resume;
   const int n0 = rs ? rs->steps : 0;  // steps already done (restart)
@@ -390,8 +432,13 @@ int lanczos_run(Sector *s, VecType vt, const double *h_init, const LanczosOption
     return -1;
   }
   if (!fixed && dim < m.lanczos_target) max_steps = (int)dim;
-  RET(cuda_ok(cudaMalloc(&AL.p, sizeof(double) * (max_steps + 2)), "alloc alpha"));
-  RET(cuda_ok(cudaMalloc(&BE.p, sizeof(double) * (max_steps + 2)), "alloc beta"));
+  const size_t nab = sizeof(double) * (size_t)(max_steps + 2);
+  Workspace ws(s, 2 * Workspace::round(esz * dim) + Workspace::round(sizeof(double) * 32) + 2 * Workspace::round(nab));
+  RET(ws.get(&P.p, esz * dim, "alloc P"));
+  RET(ws.get(&Q.p, esz * dim, "alloc Q"));
+  RET(ws.get(&ST.p, sizeof(double) * 32, "alloc scalars"));  // slots used: [0, 29)
+  RET(ws.get(&AL.p, nab, "alloc alpha"));
+  RET(ws.get(&BE.p, nab, "alloc beta"));
   // start vector: HPhi order on the host (or hashed on the device) -> native order on the device
   if (opt.hashed_start) {
     RET(vec_fill_hashed(s, vt, opt.hashed_seed, P.p));
@@ -567,6 +614,7 @@ int lanczos_run(Sector *s, VecType vt, const double *h_init, const LanczosOption
   res->alpha.assign(alpha.begin() + 1, alpha.begin() + 1 + itr);
   res->beta.assign(beta.begin() + 1, beta.begin() + 1 + itr);
   res->energies.clear();
+  if (fixed && !want_vec && res->converged) return 0;  // a fixed number of steps: the caller takes its eigenvalues from alpha and beta
   const int nev = std::min(itr, std::max(m.nvec, m.lanczos_target + 1));
   for (int q = 0; q < nev && q < itr; q++) res->energies.push_back(tridiag_eigenvalue(res->alpha.data(), res->beta.data(), itr, q));
   if (!res->converged) {
@@ -818,7 +866,7 @@ int write_lanczos_outputs(const Sector &s, const LanczosResult &r, const std::st
 int tpq_run(Sector *s, VecType vt, const double *h_init, int rand_i, const std::string &outdir, TpqResult *res,
             const TpqOptions &opt) {
   std::vector<TpqResult> r(1);
-  const int rc = tpq_run_samples(s, vt, {h_init}, {rand_i}, outdir, &r, opt, false);
+  const int rc = tpq_run_samples(s, vt, {h_init}, {rand_i}, outdir, &r, opt, hv_block_applies(s, vt));
   *res = std::move(r[0]);
   return rc;
 }
@@ -841,17 +889,22 @@ int tpq_run_samples(Sector *s, VecType vt, const std::vector<const double *> &h_
   res->assign(nb, TpqResult());
   RET(cuda_ok(cudaSetDevice(s->device), "cudaSetDevice"));
   constexpr int kSlots = 32;  // per-sample scalar slots (coefficients, sums)
-  DevBuf V, H, ST, PART;
-  RET(cuda_ok(cudaMalloc(&V.p, esz * dim * nb), "alloc V"));
-  RET(cuda_ok(cudaMalloc(&H.p, esz * dim * nb), "alloc H"));
-  RET(cuda_ok(cudaMalloc(&ST.p, sizeof(double) * kSlots * nb), "alloc scalars"));
-  if (block) RET(cuda_ok(cudaMalloc(&PART.p, sizeof(double) * 2 * nb * (size_t)s->red_blocks), "alloc partials"));
+  struct { void *p = nullptr; } V, H, ST, PART;
+  const size_t nst = sizeof(double) * kSlots * nb, npart = sizeof(double) * 3 * nb * (size_t)s->red_blocks;
+  Workspace ws(s, (m.calc_type == kcTPQ ? 5 : 2) * Workspace::round(esz * dim * nb) + Workspace::round(nst) +
+                      Workspace::round(npart));
+  RET(ws.get(&V.p, esz * dim * nb, "alloc V"));
+  RET(ws.get(&H.p, esz * dim * nb, "alloc H"));
+  RET(ws.get(&ST.p, nst, "alloc scalars"));
+  RET(ws.get(&PART.p, npart, "alloc partials"));
   auto vec = [&](void *base, int b) { return (void *)((char *)base + esz * dim * b); };
   auto slot = [&](int b) { return (double *)ST.p + kSlots * b; };
   // h_init[b] is the un-normalised start vector of sample b; its norm is global_1st_norm.
+  // Real vectors are staged in the other samples' still empty places of H.
   for (int b = 0; b < nb; b++) {
-    RET(vec_from_host_c128(s, vt, h_init[b], vec(H.p, b)));
-    RET(to_native(s, vt, vec(H.p, b), vec(V.p, b)));
+    void *at = vec(H.p, 0), *tmp = nb >= 3 ? vec(H.p, 1) : nullptr;
+    RET(vec_from_host_c128(s, vt, h_init[b], at, tmp));
+    RET(to_native(s, vt, at, vec(V.p, b)));
     RET(vec_norm2(s, vt, vec(V.p, b), slot(b)));
   }
   std::vector<double> host(kSlots * nb);
@@ -863,10 +916,11 @@ int tpq_run_samples(Sector *s, VecType vt, const std::vector<const double *> &h_
   RET(read_slots());
   const bool resumed = opt.resume_step > 0;
   // global_1st_norm is only set by MakeIniVec, so a continued run prints 0 (its initial value)
-  std::vector<double> first_norm(nb), sv(nb);  // V_b holds the current vector times 1/sv[b]
+  std::vector<double> first_norm(nb), sv(nb), norm2(nb);  // V_b holds the current vector times 1/sv[b]
   for (int b = 0; b < nb; b++) {
     first_norm[b] = resumed ? 0.0 : std::sqrt(host[kSlots * b]);
     sv[b] = 1.0 / std::sqrt(host[kSlots * b]);
+    norm2[b] = host[kSlots * b];
   }
   RET(ensure_dir(outdir));
   std::vector<FILE *> fss(nb, nullptr), fnorm(nb, nullptr), fflct(nb, nullptr);
@@ -898,33 +952,54 @@ int tpq_run_samples(Sector *s, VecType vt, const std::vector<const double *> &h_
     }
   }
   // H applied to every sample: dst_b = acc_b dst_b + scale_b H src_b with (acc, scale) in slot
-  // c0 and <src_b|H src_b> into slot c0 + 2 of each sample
+  // c0 of each sample (slots c0 + 2, c0 + 3 are scratch)
   auto apply_h = [&](void *src, void *dst, int c0) -> int {
     if (block)
-      return hv_block_native(s, vt, nb, dim, src, dst, slot(0) + c0, kSlots, slot(0) + c0 + 2, kSlots,
-                             (double *)PART.p);
+      return hv_block_native(s, vt, nb, dim, src, dst, slot(0) + c0, kSlots);
     for (int b = 0; b < nb; b++) RET(hv_native(s, vt, vec(src, b), vec(dst, b), slot(b) + c0, slot(b) + c0 + 2, false));
     return 0;
   };
   // expec_energy_flct on every sample's current vector sv*V: observables, H = H*(sv V), E, var.
+  // N and Sz are the same for every configuration of a fixed-Sz spin sector (and D is zero), so
+  // there the observables are those numbers times |sv V|^2 and need no pass of their own.
   std::vector<std::array<double, 6>> ob(nb);
-  std::vector<double> E(nb, 0.0), var(nb, 0.0);
+  std::vector<double> E(nb, 0.0), var(nb, 0.0), gnorm(nb, 0.0), inv_temp(nb, 0.0);
+  const bool fixed_obs = m.is_spin() && !m.is_gc();
+  const int fixed_2sz = m.general_spin ? m.total_2sz : 2 * m.ne - m.nsite;
+  bool swept = false;  // the coefficients and norms come from the sweep just launched
   auto expec = [&]() -> int {
     for (int b = 0; b < nb; b++) {
-      RET(native_observables(s, vt, vec(V.p, b), slot(b) + 16));
+      if (!fixed_obs) RET(native_observables(s, vt, vec(V.p, b), slot(b) + 16));
+      if (swept) continue;
       const double coef[2] = {0.0, sv[b]};
       RET(cuda_ok(cudaMemcpyAsync(slot(b) + 4, coef, sizeof(coef), cudaMemcpyHostToDevice, s->stream), "coef"));
     }
     RET(apply_h(V.p, H.p, 4));
-    for (int b = 0; b < nb; b++) RET(vec_norm2(s, vt, vec(H.p, b), slot(b) + 8));
+    if (hv_block_applies(s, vt)) {
+      RET(vec_tpq_energy(s, vt, nb, V.p, H.p, slot(0), kSlots, (double *)PART.p));
+    } else {
+      for (int b = 0; b < nb; b++) RET(vec_norm2(s, vt, vec(H.p, b), slot(b) + 8));
+    }
     RET(read_slots());
     for (int b = 0; b < nb; b++) {
       const double *h = host.data() + kSlots * b;
+      if (swept) {
+        norm2[b] = h[10];
+        gnorm[b] = std::sqrt(h[10]);
+        sv[b] = 1.0 / gnorm[b];
+      }
       const double w2 = sv[b] * sv[b];
-      for (int k = 0; k < 6; k++) ob[b][k] = h[16 + k] * w2;
-      E[b] = h[6] * sv[b] * sv[b];
+      if (fixed_obs) {
+        const double w = norm2[b] * w2, N = (double)m.nsite, Sz = 0.5 * (double)fixed_2sz;
+        ob[b] = {0.0, 0.0, w * N, w * N * N, w * Sz, w * Sz * Sz};
+      } else {
+        for (int k = 0; k < 6; k++) ob[b][k] = h[16 + k] * w2;
+      }
+      // without the block product the H*v's own <V|H V> (slots 6, 7) is unscaled
+      E[b] = hv_block_applies(s, vt) ? h[6] * sv[b] : h[6] * sv[b] * sv[b];
       var[b] = h[8];
     }
+    swept = false;
     return 0;
   };
   auto write_lines = [&](int b, double inv_temp, double gnorm, int step, bool flct) {
@@ -934,16 +1009,14 @@ int tpq_run_samples(Sector *s, VecType vt, const std::vector<const double *> &h_
       fprintf(fflct[b], "%.16lf %.16lf %.16lf %.16lf %.16lf %.16lf %.16lf %d\n", inv_temp, ob[b][2], ob[b][3],
               ob[b][0], ob[b][1], ob[b][4], ob[b][5], step);
   };
-  std::vector<double> gnorm(nb, 0.0), inv_temp(nb, 0.0);
   auto multiply = [&]() -> int {
-    // v = L*v - H v / Ns with v = sv V: V <- (L sv) V - (1/Ns) H, then normalise lazily.
-    for (int b = 0; b < nb; b++) RET(vec_tpq_sweep(s, vt, L * sv[b], 1.0 / Ns, vec(V.p, b), vec(H.p, b), slot(b) + 10));
-    RET(read_slots());
-    for (int b = 0; b < nb; b++) {
-      gnorm[b] = std::sqrt(host[kSlots * b + 10]);
-      sv[b] = 1.0 / gnorm[b];
-    }
-    return 0;
+    // v = L*v - H v / Ns with v = sv V: V <- (L sv) V - (1/Ns) H, then normalise lazily: the sweep
+    // leaves |V|^2 and the coefficients (0, 1/|V|) of the next H*v on the device, read by expec.
+    TpqCoef c{};
+    for (int b = 0; b < nb; b++) c.cv[b] = L * sv[b];
+    c.ch = 1.0 / Ns;
+    swept = true;
+    return vec_tpq_sweep(s, vt, nb, c, V.p, H.p, slot(0), kSlots, (double *)PART.p);
   };
   // Green's functions of the normalised state sv*V at step 0 and at every ExpecInterval-th
   // step from 2 on (src/CalcByTPQ.c:170-179, 261-271), files %s_cisajs_set%dstep%d.dat
@@ -968,11 +1041,11 @@ int tpq_run_samples(Sector *s, VecType vt, const std::vector<const double *> &h_
   const bool canonical = m.calc_type == kcTPQ;
   const int expand = m.expand_coef > 0 ? m.expand_coef : 10;
   const double dtau = 1.0 / L;
-  DevBuf CA, CT, CU;
+  struct { void *p = nullptr; } CA, CT, CU;
   if (canonical) {
-    RET(cuda_ok(cudaMalloc(&CA.p, esz * dim * nb), "alloc cTPQ sum"));
-    RET(cuda_ok(cudaMalloc(&CT.p, esz * dim * nb), "alloc cTPQ term"));
-    RET(cuda_ok(cudaMalloc(&CU.p, esz * dim * nb), "alloc cTPQ term"));
+    RET(ws.get(&CA.p, esz * dim * nb, "alloc cTPQ sum"));
+    RET(ws.get(&CT.p, esz * dim * nb, "alloc cTPQ term"));
+    RET(ws.get(&CU.p, esz * dim * nb, "alloc cTPQ term"));
   }
   auto ctpq_multiply = [&]() -> int {
     // x = sv V and h = H x (expec left H x in H): sum = x + a h + sum_c a^c/c! H^c x;
@@ -999,6 +1072,7 @@ int tpq_run_samples(Sector *s, VecType vt, const std::vector<const double *> &h_
     for (int b = 0; b < nb; b++) {
       gnorm[b] = std::sqrt(host[kSlots * b + 30]);
       sv[b] = 1.0 / gnorm[b];
+      norm2[b] = host[kSlots * b + 30];
     }
     std::swap(V.p, CA.p);
     return 0;
@@ -1085,14 +1159,44 @@ int te_run(Sector *s, const double *h_init, int step_initial, const std::string 
     return -1;
   }
   RET(cuda_ok(cudaSetDevice(s->device), "cudaSetDevice"));
-  // The off-diagonal terms of all time indices by their masks (the union), one split-term plan
-  // for the union, and per index its coefficient table and its generic terms (back to back);
-  // the diagonal terms of each index back to back.
+  // Product layout where the two-pass kernels take H(t): the static hops and every index's by
+  // their masks, with one coefficient per index.  Diagonal terms of an index keep the general path.
+  bool te_diag = false;
+  for (const auto &v : m.te_diag) te_diag = te_diag || !v.empty();
+  if (s->prod && !s->te_prod_tried && !te_diag) {
+    std::vector<BitTerm> uni;
+    std::map<std::tuple<uint64_t, uint64_t, uint64_t, uint64_t>, size_t> where;
+    std::vector<std::vector<double2>> coefs(m.te_time.size());
+    auto add = [&](std::vector<double2> *c, const BitTerm &t) {
+      const auto it = where.emplace(std::make_tuple(t.cm, t.cv, t.flip, t.sm), uni.size());
+      if (it.second) {
+        uni.push_back(t);
+        for (auto &v : coefs) v.push_back(make_double2(0.0, 0.0));
+      }
+      (*c)[it.first->second].x += t.re;
+      (*c)[it.first->second].y += t.im;
+    };
+    for (size_t k = 0; k < coefs.size(); k++) {
+      for (const BitTerm &t : m.offdiag) add(&coefs[k], t);
+      for (const BitTerm &t : m.te_offdiag[k]) add(&coefs[k], t);
+    }
+    std::string err;
+    if (prod_te_plan_build(s, uni, coefs, &s->te_prod, &err) != 0) {
+      set_error("time-evolution plan: " + err);
+      return -1;
+    }
+    s->te_prod_tried = true;
+  }
+  const bool nat = s->te_prod != nullptr;
+  // Otherwise HPhi's row order: the static part by the general row kernel, the off-diagonal terms
+  // of all time indices by their masks (the union) in one split-term plan, and per index its
+  // coefficient table and its generic terms (back to back); the diagonal terms of each index
+  // back to back.
   std::vector<BitTerm> uni;
   std::map<std::tuple<uint64_t, uint64_t, uint64_t, uint64_t>, int> where;
   const size_t nidx = m.te_time.size();
   std::vector<std::vector<std::pair<int, BitTerm>>> by_idx(nidx);
-  for (size_t k = 0; k < nidx; k++)
+  for (size_t k = 0; k < nidx && !nat; k++)
     for (const BitTerm &t : m.te_offdiag[k]) {
       const auto key = std::make_tuple(t.cm, t.cv, t.flip, t.sm);
       auto it = where.find(key);
@@ -1138,7 +1242,9 @@ int te_run(Sector *s, const double *h_init, int step_initial, const std::string 
   }
   off_at.push_back(off.size());
   dg_at.push_back(dg.size());
-  DevBuf OFF, DG, CO, P, HP, ACC, U, ST;
+  DevBuf OFF, DG, CO;
+  struct Vec { void *p = nullptr; } P, HP, ACC, U, ST;
+  Workspace ws(s, 4 * Workspace::round(esz * dim) + Workspace::round(sizeof(double) * 32));
   if (plan.lo_ptr) {
     RET(cuda_ok(cudaMalloc(&CO.p, sizeof(double) * coefs.size()), "alloc coefficient tables"));
     RET(cuda_ok(cudaMemcpyAsync(CO.p, coefs.data(), sizeof(double) * coefs.size(), cudaMemcpyHostToDevice,
@@ -1154,19 +1260,30 @@ int te_run(Sector *s, const double *h_init, int step_initial, const std::string 
     RET(cuda_ok(cudaMemcpyAsync(DG.p, dg.data(), sizeof(DiagTerm) * dg.size(), cudaMemcpyHostToDevice, s->stream),
                 "upload terms"));
   }
-  for (DevBuf *b : {&P, &HP, &ACC, &U}) RET(cuda_ok(cudaMalloc(&b->p, esz * dim), "alloc vector"));
-  RET(cuda_ok(cudaMalloc(&ST.p, sizeof(double) * 32), "alloc scalars"));
+  for (Vec *b : {&P, &HP, &ACC, &U}) RET(ws.get(&b->p, esz * dim, "alloc vector"));
+  RET(ws.get(&ST.p, sizeof(double) * 32, "alloc scalars"));
   double *st = (double *)ST.p;
   const double c01[2] = {0.0, 1.0};
   RET(cuda_ok(cudaMemcpyAsync(st, c01, sizeof(c01), cudaMemcpyHostToDevice, s->stream), "coef"));
-  // y = H(step) x: the static part (general row kernel) plus the step's terms
-  auto apply_h = [&](int step, const void *x, void *y) -> int {
+  // y = H(step) x: the static part (general row kernel) plus the step's terms; with sum also
+  // sum += c y
+  auto apply_h = [&](int step, const void *x, void *y, void *sum, std::complex<double> c) -> int {
+    if (nat) return prod_te_launch(s, s->te_prod, step, x, y, st, st + 2, sum, c.real(), c.imag());
     RET(hv_launch(s, vt, x, y, st, st + 2));
-    return te_terms_apply(s, plan, (const double *)CO.p + (plan.lo_ptr ? step * ncoef : 0),
-                          (const BitTerm *)OFF.p + off_at[step], (int)(off_at[step + 1] - off_at[step]),
-                          (const DiagTerm *)DG.p + dg_at[step], (int)(dg_at[step + 1] - dg_at[step]), x, y);
+    RET(te_terms_apply(s, plan, (const double *)CO.p + (plan.lo_ptr ? step * ncoef : 0),
+                       (const BitTerm *)OFF.p + off_at[step], (int)(off_at[step + 1] - off_at[step]),
+                       (const DiagTerm *)DG.p + dg_at[step], (int)(dg_at[step + 1] - dg_at[step]), x, y));
+    return sum ? vec_caxpy(s, c.real(), c.imag(), y, sum) : 0;
   };
-  RET(vec_from_host_c128(s, vt, h_init, P.p));
+  // the vectors stay in native order on the product layout; hphi() gives the state in HPhi's
+  RET(vec_from_host_c128(s, vt, h_init, nat ? U.p : P.p));
+  if (nat) RET(to_native(s, vt, U.p, P.p));
+  auto hphi = [&](void **v) -> int {
+    *v = P.p;
+    if (!nat) return 0;
+    *v = U.p;
+    return from_native(s, vt, P.p, U.p);
+  };
   // the reference's v0 (H psi of the previous step) is zero before the first step
   RET(cuda_ok(cudaMemsetAsync(HP.p, 0, esz * dim, s->stream), "zero"));
   RET(ensure_dir(outdir));
@@ -1193,7 +1310,9 @@ int te_run(Sector *s, const double *h_init, int step_initial, const std::string 
   auto write_state = [&](int step, int label) -> int {
     // <head>_eigenvec_<label>_rank_0.dat: int step, long dim, complex128[dim + 1]
     host.assign(2 * (dim + 1), 0.0);
-    RET(vec_to_host_c128(s, vt, P.p, host.data()));
+    void *v = nullptr;
+    RET(hphi(&v));
+    RET(vec_to_host_c128(s, vt, v, host.data()));
     char name[256];
     snprintf(name, sizeof(name), "%s_eigenvec_%d_rank_%d.dat", m.data_head.c_str(), label, 0);
     FILE *f = fopen(join(outdir, name).c_str(), "wb");
@@ -1222,8 +1341,7 @@ int te_run(Sector *s, const double *h_init, int step_initial, const std::string 
       void *t = HP.p, *u = U.p;
       for (int k = 2; k <= m.expand_coef; k++) {
         coef *= mi * dt / (double)k;
-        RET(apply_h(step, t, u));
-        RET(vec_caxpy(s, coef.real(), coef.imag(), u, ACC.p));
+        RET(apply_h(step, t, u, ACC.p, coef));
         std::swap(t, u);
       }
       std::swap(P.p, ACC.p);
@@ -1235,8 +1353,8 @@ int te_run(Sector *s, const double *h_init, int step_initial, const std::string 
     const double gnorm = std::sqrt(n2);
     RET(vec_scale(s, vt, 1.0 / gnorm, P.p));
     // expec_energy_flct: observables of psi, H psi with this step's terms, E, var
-    RET(vec_diag_observables(s, vt, P.p, st + 16));
-    RET(apply_h(step, P.p, HP.p));
+    RET(nat ? native_observables(s, vt, P.p, st + 16) : vec_diag_observables(s, vt, P.p, st + 16));
+    RET(apply_h(step, P.p, HP.p, nullptr, 0.0));
     RET(vec_dot(s, vt, P.p, HP.p, st + 6));
     RET(vec_norm2(s, vt, HP.p, st + 8));
     double sc[4], ob[6];
@@ -1256,7 +1374,9 @@ int te_run(Sector *s, const double *h_init, int step_initial, const std::string 
     res->norm.push_back(gnorm);
     if (green && m.expec_interval > 0 && step % m.expec_interval == 0) {
       GreenValues g;
-      RET(model_green(s, vt, P.p, 1.0, &g));
+      void *v = nullptr;
+      RET(hphi(&v));
+      RET(model_green(s, vt, v, 1.0, &g));
       char suffix[64];
       snprintf(suffix, sizeof(suffix), "_step%d", step);
       RET(write_green_files(m, g, outdir, suffix));

@@ -8,6 +8,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -82,12 +83,20 @@ struct Sector {
   unsigned *d_done = nullptr;      // kHvBlockMax counters of finished blocks (grid_sum), zero between launches;
                                    // in the last d_scal slots
   int red_blocks = 0;
+  // Device memory the drivers' calls share (Workspace, driver.cpp): kept between calls up to
+  // kWorkspaceKeep bytes, freed with the sector.
+  void *ws = nullptr;
+  size_t ws_bytes = 0;
+  std::atomic<bool> ws_busy{false};  // a call has the workspace; calls inside or beside it allocate their own
   int num_sms = 0;
   // Optional specialised plan (canonical Hubbard).  When present, the drivers keep
   // vectors in the plan's native order; see hv_native / to_native.
   HubPlan *hub = nullptr;
   // Product-layout plan (canonical Hubbard); preferred over the block plan when both apply.
   ProdPlan *prod = nullptr;
+  // Product-layout plan of the time-dependent H (time evolution), built on the first run.
+  ProdPlan *te_prod = nullptr;
+  bool te_prod_tried = false;
   // Row-block plan (spin models, HPhi order): row pass + column pass over the blocks of
   // rows that share an upper half (hv_rowblock.cu).
   RowBlockPlan *rb = nullptr;
@@ -136,13 +145,12 @@ int hv_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double 
 // exact per-block permutation of it).  hv_native runs the fastest kernel on native
 // vectors; to_native / from_native convert (they copy when the orders coincide).
 bool has_native_order(const Sector *s);
-// Block H*V over nb <= kHvBlockMax vectors at d_v1 + b * stride (general kernel path only,
-// hv_block_applies): v0_b = acc_b * v0_b + scale_b * H v1_b with (acc_b, scale_b) at
-// d_coef + b * cstride and <v1_b|H v1_b> at d_out + b * ostride; d_part holds
-// 2 * nb * red_blocks doubles.
+// Block H*V over nb <= kHvBlockMax vectors at d_v1 + b * stride (sectors kept in HPhi's order
+// without a row-block plan, hv_block_applies): v0_b = acc_b * v0_b + scale_b * H v1_b with
+// (acc_b, scale_b) at d_coef + b * cstride.
 bool hv_block_applies(const Sector *s, VecType vt);
 int hv_block_native(Sector *s, VecType vt, int nb, int64_t stride, const void *d_v1, void *d_v0,
-                    const double *d_coef, int cstride, double *d_out, int ostride, double *d_part);
+                    const double *d_coef, int cstride);
 int hv_native(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
               bool acc_read = true, const LanczosTail *lt = nullptr);
 int to_native(Sector *s, VecType vt, const void *d_hphi, void *d_native);
@@ -178,7 +186,15 @@ int lanczos_scalars(Sector *s, int phase, int k, double *st, double *alpha, doub
 // p = p - a_sq*q; vg += c_over_b * p  (eigenvector replay)
 int vec_replay_sweep(Sector *s, VecType vt, double a_sq, double c_over_b, void *p, const void *q, void *vg);
 // v = cv*v - ch*h and d_out[0] = |v|^2 (TPQ step before normalisation)
-int vec_tpq_sweep(Sector *s, VecType vt, double cv, double ch, void *v, const void *h, double *d_out);
+// TPQ, nb <= kHvBlockMax samples side by side (sample b's vectors at b * dim, its scalars at
+// slots + b * nslot).  Sweep (before normalisation): v_b = cv_b v_b - ch h_b, then
+// slots[10] = |v_b|^2 and slots[4, 5] = (0, 1 / |v_b|), the coefficients of the H*v of the
+// normalised state; energies: slots[6, 7] = <v_b|h_b>, slots[8] = |h_b|^2.  Each sample's sums
+// are the same for any nb.  d_part: 3 * nb * red_blocks doubles.
+struct TpqCoef { double cv[kHvBlockMax]; double ch; };
+int vec_tpq_sweep(Sector *s, VecType vt, int nb, const TpqCoef &c, void *v, const void *h, double *slots, int nslot,
+                  double *d_part);
+int vec_tpq_energy(Sector *s, VecType vt, int nb, const void *v, const void *h, double *slots, int nslot, double *d_part);
 
 // CG sweep (eigenvector refinement): x += a*p; r -= a*(hp + shift*p); d_out[0] = |r|^2.
 int vec_cg_sweep(Sector *s, VecType vt, double a, double shift, const void *p, const void *hp, void *x, void *r,
@@ -211,7 +227,8 @@ int vec_join_c128(Sector *s, const double *d_re, const double *d_im, void *d_c);
 int vec_add_c128(Sector *s, cudaStream_t st, int64_t n, void *d_y, const void *d_x);
 
 // Copies between HPhi's 1-based complex128 host layout and a device vector.
-int vec_from_host_c128(Sector *s, VecType vt, const double *h_v_1based, void *d_v);
+// tmp: dim complex128 of device memory for real vectors (nullptr: allocated by the call).
+int vec_from_host_c128(Sector *s, VecType vt, const double *h_v_1based, void *d_v, void *tmp = nullptr);
 int vec_to_host_c128(Sector *s, VecType vt, const void *d_v, double *h_v_1based);
 
 void set_error(const std::string &msg);

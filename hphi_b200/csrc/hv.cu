@@ -91,11 +91,10 @@ void launch_general(Sector *s, const T *v1, T *v0, const double *coef, const Sum
 }
 
 // B vectors at once (independent samples of one sector, vector b at v + b * stride): the
-// configuration, diagonal, split-plan entries, list lookups and signs of a row are worked out
-// once and applied to all B, which is where the general kernel spends its memory traffic.
-// Per vector the arithmetic and its order are the general kernel's, so every output equals a
-// separate launch bit for bit.  Coefficients (acc, scale) of vector b at coef + b * cstride;
-// partial sums of <v1_b|H v1_b> in part[(2B) * block + 2b (+1)].
+// configuration, diagonal, split-plan entries, list lookups and signs of a row are worked out once
+// and applied to all B.  Per vector the arithmetic and its order are the general kernel's, so every
+// output equals a separate launch bit for bit.  Coefficients (acc, scale) of vector b at coef + b *
+// cstride.  No sums: the callers' next sweep over the vectors has them.
 template <typename T, int B>
 struct Blk {
   T v[B];
@@ -121,7 +120,7 @@ __global__ void __launch_bounds__(kHvThreads) hv_block_kernel(
     int64_t dim, int64_t stride, const uint64_t *__restrict__ list_1, const uint32_t *__restrict__ l21,
     const uint32_t *__restrict__ l22, int lo_bits, uint64_t lo_mask, SplitView split,
     const BitTerm *__restrict__ gterms, int nterms, const double *__restrict__ diag, const T *__restrict__ v1,
-    T *__restrict__ v0, const double *__restrict__ coef, int cstride, double *__restrict__ part) {
+    T *__restrict__ v0, const double *__restrict__ coef, int cstride) {
   extern __shared__ BitTerm sterms[];
   const BitTerm *terms = gterms;
   if (SMEM) {
@@ -129,9 +128,6 @@ __global__ void __launch_bounds__(kHvThreads) hv_block_kernel(
     __syncthreads();
     terms = sterms;
   }
-  double pr[2 * B];
-#pragma unroll
-  for (int q = 0; q < 2 * B; q++) pr[q] = 0.0;
   auto load = [&](int64_t j) {
     Blk<T, B> z;
 #pragma unroll
@@ -187,42 +183,16 @@ __global__ void __launch_bounds__(kHvThreads) hv_block_kernel(
     }
 #pragma unroll
     for (int q = 0; q < B; q++) {
-      pr[2 * q] += VT<T>::conj_mul_re(x.v[q], y.v[q]);
-      pr[2 * q + 1] += VT<T>::conj_mul_im(x.v[q], y.v[q]);
       const double acc = coef[q * cstride], scale = coef[q * cstride + 1];
       const T yq = VT<T>::scale(scale, y.v[q]);
       T *o = v0 + q * stride + r;
       *o = (acc == 0.0) ? yq : VT<T>::add(VT<T>::scale(acc, *o), yq);
     }
   }
-  block_sum<2 * B>(pr);
-  if (threadIdx.x == 0)
-#pragma unroll
-    for (int q = 0; q < 2 * B; q++) part[2 * B * blockIdx.x + q] = pr[q];
-}
-
-// out[q * ostride + (0, 1)] = sum over blocks of part[(2B) * block + 2q (+1)]
-template <int B>
-__global__ void finalize_block_partials_kernel(const double *__restrict__ part, int n, double *__restrict__ out,
-                                               int ostride) {
-  double v[2 * B];
-#pragma unroll
-  for (int k = 0; k < 2 * B; k++) v[k] = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x)
-#pragma unroll
-    for (int k = 0; k < 2 * B; k++) v[k] += part[i * 2 * B + k];
-  block_sum<2 * B>(v);
-  if (threadIdx.x == 0)
-#pragma unroll
-    for (int q = 0; q < B; q++) {
-      out[q * ostride] = v[2 * q];
-      out[q * ostride + 1] = v[2 * q + 1];
-    }
 }
 
 template <typename T, bool GC, int B>
-void launch_block(Sector *s, int64_t stride, const T *v1, T *v0, const double *coef, int cstride, double *out,
-                  int ostride, double *part) {
+void launch_block(Sector *s, int64_t stride, const T *v1, T *v0, const double *coef, int cstride) {
   const int grid = s->red_blocks;
   const uint64_t lo_mask = s->ihfbit - 1;
   const SplitView sv = split_view(s->split);
@@ -230,27 +200,25 @@ void launch_block(Sector *s, int64_t stride, const T *v1, T *v0, const double *c
     const size_t smem = sizeof(BitTerm) * (size_t)s->split.ngen;
     hv_block_kernel<T, GC, true, B><<<grid, kHvThreads, smem, s->stream>>>(
         s->dim, stride, s->d_list_1, s->d_list_2_1, s->d_list_2_2, s->lo_bits, lo_mask, sv, s->split.gen,
-        s->split.ngen, s->d_diag, v1, v0, coef, cstride, part);
+        s->split.ngen, s->d_diag, v1, v0, coef, cstride);
   } else {
     hv_block_kernel<T, GC, false, B><<<grid, kHvThreads, 0, s->stream>>>(
         s->dim, stride, s->d_list_1, s->d_list_2_1, s->d_list_2_2, s->lo_bits, lo_mask, sv, s->split.gen,
-        s->split.ngen, s->d_diag, v1, v0, coef, cstride, part);
+        s->split.ngen, s->d_diag, v1, v0, coef, cstride);
   }
-  finalize_block_partials_kernel<B><<<1, 256, 0, s->stream>>>(part, grid, out, ostride);
 }
 
 template <typename T, bool GC>
-void launch_block_n(Sector *s, int nb, int64_t stride, const T *v1, T *v0, const double *coef, int cstride,
-                    double *out, int ostride, double *part) {
+void launch_block_n(Sector *s, int nb, int64_t stride, const T *v1, T *v0, const double *coef, int cstride) {
   switch (nb) {
-    case 1: launch_block<T, GC, 1>(s, stride, v1, v0, coef, cstride, out, ostride, part); break;
-    case 2: launch_block<T, GC, 2>(s, stride, v1, v0, coef, cstride, out, ostride, part); break;
-    case 3: launch_block<T, GC, 3>(s, stride, v1, v0, coef, cstride, out, ostride, part); break;
-    case 4: launch_block<T, GC, 4>(s, stride, v1, v0, coef, cstride, out, ostride, part); break;
-    case 5: launch_block<T, GC, 5>(s, stride, v1, v0, coef, cstride, out, ostride, part); break;
-    case 6: launch_block<T, GC, 6>(s, stride, v1, v0, coef, cstride, out, ostride, part); break;
-    case 7: launch_block<T, GC, 7>(s, stride, v1, v0, coef, cstride, out, ostride, part); break;
-    default: launch_block<T, GC, 8>(s, stride, v1, v0, coef, cstride, out, ostride, part); break;
+    case 1: launch_block<T, GC, 1>(s, stride, v1, v0, coef, cstride); break;
+    case 2: launch_block<T, GC, 2>(s, stride, v1, v0, coef, cstride); break;
+    case 3: launch_block<T, GC, 3>(s, stride, v1, v0, coef, cstride); break;
+    case 4: launch_block<T, GC, 4>(s, stride, v1, v0, coef, cstride); break;
+    case 5: launch_block<T, GC, 5>(s, stride, v1, v0, coef, cstride); break;
+    case 6: launch_block<T, GC, 6>(s, stride, v1, v0, coef, cstride); break;
+    case 7: launch_block<T, GC, 7>(s, stride, v1, v0, coef, cstride); break;
+    default: launch_block<T, GC, 8>(s, stride, v1, v0, coef, cstride); break;
   }
 }
 
@@ -261,21 +229,17 @@ bool hv_block_applies(const Sector *s, VecType vt) {
 }
 
 int hv_block_native(Sector *s, VecType vt, int nb, int64_t stride, const void *d_v1, void *d_v0,
-                    const double *d_coef, int cstride, double *d_out, int ostride, double *d_part) {
+                    const double *d_coef, int cstride) {
   if (nb < 1 || nb > kHvBlockMax || !hv_block_applies(s, vt)) {
-    set_error("hv_block_native: block products need the general kernel and 1..8 vectors");
+    set_error("hv_block_native: block products need HPhi's row order and 1..8 vectors");
     return -1;
   }
   if (vt == kReal64) {
-    if (s->gc) launch_block_n<double, true>(s, nb, stride, (const double *)d_v1, (double *)d_v0, d_coef, cstride,
-                                            d_out, ostride, d_part);
-    else launch_block_n<double, false>(s, nb, stride, (const double *)d_v1, (double *)d_v0, d_coef, cstride,
-                                       d_out, ostride, d_part);
+    if (s->gc) launch_block_n<double, true>(s, nb, stride, (const double *)d_v1, (double *)d_v0, d_coef, cstride);
+    else launch_block_n<double, false>(s, nb, stride, (const double *)d_v1, (double *)d_v0, d_coef, cstride);
   } else {
-    if (s->gc) launch_block_n<cplx, true>(s, nb, stride, (const cplx *)d_v1, (cplx *)d_v0, d_coef, cstride, d_out,
-                                          ostride, d_part);
-    else launch_block_n<cplx, false>(s, nb, stride, (const cplx *)d_v1, (cplx *)d_v0, d_coef, cstride, d_out,
-                                     ostride, d_part);
+    if (s->gc) launch_block_n<cplx, true>(s, nb, stride, (const cplx *)d_v1, (cplx *)d_v0, d_coef, cstride);
+    else launch_block_n<cplx, false>(s, nb, stride, (const cplx *)d_v1, (cplx *)d_v0, d_coef, cstride);
   }
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {

@@ -734,11 +734,12 @@ void sector_free(Sector *s) {
   cudaSetDevice(s->device);
   if (s->stream) cudaStreamSynchronize(s->stream);
   cudaFree(s->d_list_1); cudaFree(s->d_list_2_1); cudaFree(s->d_list_2_2); cudaFree(s->d_diag);
-  cudaFree(s->d_terms); cudaFree(s->d_dterms); cudaFree(s->d_red); cudaFree(s->d_scal);
+  cudaFree(s->d_terms); cudaFree(s->d_dterms); cudaFree(s->d_red); cudaFree(s->d_scal); cudaFree(s->ws);
   cudaFree(s->split.lo_ptr); cudaFree(s->split.lo_ent); cudaFree(s->split.hi_ptr); cudaFree(s->split.hi_ent);
   cudaFree(s->split.coef); cudaFree(s->split.gen); cudaFree(s->d_pieces); cudaFree(s->d_low);
   hub_plan_free(s->hub);
   prod_plan_free(s->prod);
+  prod_plan_free(s->te_prod);
   rb_plan_free(s->rb);
   if (s->stream) cudaStreamDestroy(s->stream);
   delete s;

@@ -183,7 +183,7 @@ int vec_diag_observables(Sector *s, VecType vt, const void *x, double *out) {
   return check_launch("vec_diag_observables");
 }
 
-int vec_from_host_c128(Sector *s, VecType vt, const double *h, void *d) {
+int vec_from_host_c128(Sector *s, VecType vt, const double *h, void *d, void *space) {
   const size_t bytes = sizeof(cplx) * (size_t)s->dim;
   if (vt == kComplex128) {
     if (cudaMemcpyAsync(d, h + 2, bytes, cudaMemcpyHostToDevice, s->stream) != cudaSuccess) {
@@ -192,11 +192,14 @@ int vec_from_host_c128(Sector *s, VecType vt, const double *h, void *d) {
     }
     return 0;
   }
-  cplx *tmp = nullptr;
-  if (cudaMallocAsync(&tmp, bytes, s->stream) != cudaSuccess) { set_error("vec_from_host_c128: out of memory"); return -1; }
+  cplx *tmp = (cplx *)space;
+  if (!tmp && cudaMallocAsync(&tmp, bytes, s->stream) != cudaSuccess) {
+    set_error("vec_from_host_c128: out of memory");
+    return -1;
+  }
   cudaMemcpyAsync(tmp, h + 2, bytes, cudaMemcpyHostToDevice, s->stream);
   real_from_c128_kernel<<<s->red_blocks, kThreads, 0, s->stream>>>(s->dim, tmp, (double *)d);
-  cudaFreeAsync(tmp, s->stream);
+  if (!space) cudaFreeAsync(tmp, s->stream);
   return check_launch("vec_from_host_c128");
 }
 
@@ -242,18 +245,52 @@ __global__ void replay_sweep_kernel(int64_t n, double a_sq, double c_over_b, T *
   }
 }
 
-// TPQ sweep (src/Multiply.c:42-68 with the normalisation deferred):
-// w = (L*sv)*v - (sh/Ns)*h written into v, |w|^2 into part.
+// One sample of a TPQ block: blockIdx.y picks its vectors, records, counter and slots.
+__device__ __forceinline__ SumOut tpq_sum(double *part, unsigned *done, double *slots, int nslot, int nv) {
+  const int b = blockIdx.y;
+  return SumOut{part + (size_t)b * gridDim.x * nv, 0, (int)gridDim.x, done + b, slots + (size_t)b * nslot, -1, {}};
+}
+
+// TPQ sweep (src/Multiply.c:42-68 with the normalisation deferred): w = (L*sv)*v - (1/Ns)*h
+// written into v, |w|^2 and the coefficients of the next H*v.
 template <typename T>
-__global__ void tpq_sweep_kernel(int64_t n, double cv, double ch, T *__restrict__ v, const T *__restrict__ h,
-                                 SumOut so) {
+__global__ void tpq_sweep_kernel(int64_t n, TpqCoef c, T *__restrict__ v, const T *__restrict__ h, double *part,
+                                 unsigned *done, double *slots, int nslot) {
+  const double cv = c.cv[blockIdx.y], ch = c.ch;
+  v += blockIdx.y * n;
+  h += blockIdx.y * n;
   double acc[1] = {0.0};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const T w = VT<T>::sub(VT<T>::scale(cv, v[i]), VT<T>::scale(ch, h[i]));
     v[i] = w;
     acc[0] += VT<T>::abs2(w);
   }
-  grid_sum<1>(acc, so);
+  const SumOut so = tpq_sum(part, done, slots, nslot, 1);
+  grid_sum<1>(acc, so, [&](const double(&s)[1]) {
+    so.out[10] = s[0];
+    so.out[4] = 0.0;
+    so.out[5] = 1.0 / sqrt(s[0]);
+  });
+}
+
+template <typename T>
+__global__ void tpq_energy_kernel(int64_t n, const T *__restrict__ v, const T *__restrict__ h, double *part,
+                                  unsigned *done, double *slots, int nslot) {
+  v += blockIdx.y * n;
+  h += blockIdx.y * n;
+  double acc[3] = {0.0, 0.0, 0.0};
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const T x = v[i], y = h[i];
+    acc[0] += VT<T>::conj_mul_re(x, y);
+    acc[1] += VT<T>::conj_mul_im(x, y);
+    acc[2] += VT<T>::abs2(y);
+  }
+  const SumOut so = tpq_sum(part, done, slots, nslot, 3);
+  grid_sum<3>(acc, so, [&](const double(&s)[3]) {
+    so.out[6] = s[0];
+    so.out[7] = s[1];
+    so.out[8] = s[2];
+  });
 }
 
 // CG sweep of the eigenvector refinement (src/CG_EigenVector.c:143-185) with the shifted
@@ -322,15 +359,27 @@ int vec_replay_sweep(Sector *s, VecType vt, double a_sq, double c_over_b, void *
   return check_launch("vec_replay_sweep");
 }
 
-int vec_tpq_sweep(Sector *s, VecType vt, double cv, double ch, void *v, const void *h, double *out) {
-  const SumOut so = sum_out(s->d_red, 0, s->red_blocks, s->d_done, out);
+int vec_tpq_sweep(Sector *s, VecType vt, int nb, const TpqCoef &c, void *v, const void *h, double *slots, int nslot,
+                  double *part) {
+  const dim3 grid(s->red_blocks, nb);
   if (vt == kReal64)
-    tpq_sweep_kernel<double><<<s->red_blocks, kThreads, 0, s->stream>>>(s->dim, cv, ch, (double *)v,
-                                                                        (const double *)h, so);
+    tpq_sweep_kernel<double><<<grid, kThreads, 0, s->stream>>>(s->dim, c, (double *)v, (const double *)h, part, s->d_done,
+                                                               slots, nslot);
   else
-    tpq_sweep_kernel<cplx><<<s->red_blocks, kThreads, 0, s->stream>>>(s->dim, cv, ch, (cplx *)v, (const cplx *)h,
-                                                                      so);
+    tpq_sweep_kernel<cplx><<<grid, kThreads, 0, s->stream>>>(s->dim, c, (cplx *)v, (const cplx *)h, part, s->d_done, slots,
+                                                             nslot);
   return check_launch("vec_tpq_sweep");
+}
+
+int vec_tpq_energy(Sector *s, VecType vt, int nb, const void *v, const void *h, double *slots, int nslot, double *part) {
+  const dim3 grid(s->red_blocks, nb);
+  if (vt == kReal64)
+    tpq_energy_kernel<double><<<grid, kThreads, 0, s->stream>>>(s->dim, (const double *)v, (const double *)h, part,
+                                                                s->d_done, slots, nslot);
+  else
+    tpq_energy_kernel<cplx><<<grid, kThreads, 0, s->stream>>>(s->dim, (const cplx *)v, (const cplx *)h, part, s->d_done,
+                                                              slots, nslot);
+  return check_launch("vec_tpq_energy");
 }
 
 }  // namespace hphi

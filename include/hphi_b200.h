@@ -220,6 +220,9 @@ int hphi_lanczos_eigenvector(hphi_handle *h, double *v);
  */
 int hphi_tpq(hphi_handle *h, const double *v_init, const char *output_dir, double *result, int nresult);
 
+/* hphi_tpq with one pointer per sample (NumAve of them) instead of one contiguous array. */
+int hphi_tpq_vectors(hphi_handle *h, const double *const *v_init, const char *output_dir, double *result, int nresult);
+
 /*
  * Real-time evolution (CalcType 4) under H(t) = H + the TEOneBody / TETwoBody terms of each
  * time index.  Per step: psi <- sum_{k<=ExpandCoef} (-i dt H)^k / k! psi, normalised (the

@@ -152,3 +152,47 @@ def test_green_blocks(name, vt, tmp_path):
                 if adj in at:
                     assert abs(at[adj] - np.conj(x)) <= 1e-13
     assert abs(e - ref) <= 1e-13 * weight
+
+
+@pytest.mark.parametrize("static, values", [(False, 1), (True, 1), (True, 5), (False, 12)])
+def test_time_evolution_product_layout(static, values, tmp_path):
+    """Energies, and files, of a run on the product layout against the general path (HPhi's order).
+    static: the hops stay in H and the pulse adds to them; values: amplitudes of the pulse over the
+    bonds (12 is past the coefficient groups, so that run stays on the general path).  Bound: 8
+    steps of order 10 multiply rounding errors by e^(|H| dt) < 2 each; 1e-12 of the energies' scale."""
+    N, steps = 8, 8
+    m = _hubbard(N, 4, 3)
+    m.calc_type, m.lanczos_max, m.input_eigenvec, m.expand_coef = "TimeEvolution", steps, 1, 10
+    m.spectrum_vec, m.output_eigenvec, m.output_interval = "zvo_eigenvec_0", 1, steps - 1
+    m.greenone = [(0, 0, 1, 0), (2, 1, 2, 1)]
+    m.expec_interval = 3
+    hops = list(m.trans)
+    for k in range(steps):
+        rows = []
+        for b, (i, s1, j, s2, re, im) in enumerate(hops):
+            a = 0.3 * np.sin(2.0 * k * 0.02) * (1.0 + 0.1 * ((b // 4) % values)) * (1 if (j - i) % N == 1 else -1)
+            t = complex(re, im) * np.exp(1j * a) - (complex(re, im) if static else 0.0)
+            rows.append((i, s1, j, s2, float(t.real), float(t.imag)))
+        m.te_onebody.append((0.02 * k, rows))
+    if not static:
+        m.trans = []
+    path = m.write(str(tmp_path))
+    out = []
+    for general in (False, True):
+        with _open(path, general=general) as H:
+            rng = np.random.default_rng(4)
+            v = np.zeros(H.dim + 1, dtype=np.complex128)
+            v[1:] = rng.standard_normal(H.dim) + 1j * rng.standard_normal(H.dim)
+            v /= np.linalg.norm(v)
+            d = str(tmp_path / f"out{general}")
+            e = [H.calc_by_tem(v_init=v, output_dir=d) for _ in range(2)]
+            assert np.array_equal(e[0], e[1])
+            with open(os.path.join(d, "zvo_eigenvec_0_rank_0.dat"), "rb") as f:
+                state = np.frombuffer(f.read()[12:], dtype=np.complex128)
+            files = [np.loadtxt(os.path.join(d, n)) for n in ("Flct.dat", "SS.dat", "zvo_cisajs_step3.dat")]
+            out.append((e[0], state[1:], files))
+    (ea, sa, fa), (eg, sg, fg) = out
+    assert np.max(np.abs(ea - eg)) <= 1e-12 * np.max(np.abs(eg))
+    assert np.max(np.abs(sa - sg)) <= 1e-12 * np.max(np.abs(sg))
+    for x, y in zip(fa, fg):
+        np.testing.assert_allclose(x, y, rtol=0, atol=2e-10)
