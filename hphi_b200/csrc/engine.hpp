@@ -20,6 +20,7 @@ namespace hphi {
 struct HubPlan;
 struct ProdPlan;
 struct RowBlockPlan;
+struct BlockPlan;
 
 // Real or complex double scalar for host/device code.
 struct cplx { double x, y; };
@@ -100,6 +101,9 @@ struct Sector {
   // Row-block plan (spin models, HPhi order): row pass + column pass over the blocks of
   // rows that share an upper half (hv_rowblock.cu).
   RowBlockPlan *rb = nullptr;
+  // Block plan (canonical sectors in HPhi's order without one of the plans above): one pass over
+  // the blocks of rows that share an upper half (hv_blocks.cu).
+  BlockPlan *bk = nullptr;
   SplitPlan split;
   SectorBlock *d_pieces = nullptr;  // sector_pieces
   uint32_t *d_low = nullptr;

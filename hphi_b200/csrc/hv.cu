@@ -15,6 +15,7 @@
 
 #include "device_util.cuh"
 #include "engine.hpp"
+#include "hv_blocks.hpp"
 #include "hv_hubbard.hpp"
 #include "hv_product.hpp"
 #include "hv_rowblock.hpp"
@@ -255,10 +256,8 @@ int hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const
     set_error("H has complex coefficients: real vectors are not allowed");
     return -1;
   }
-  if (rb_applies(s, vt)) {
-    if (rb_hv_launch_scratch(s, vt, d_v1, d_v0, d_coef, d_out, d_part) != 0) return -1;
-    return lt ? lanczos_scalars(s, 0, lt->k, lt->st, lt->alpha, lt->beta) : 0;
-  }
+  if (rb_applies(s, vt)) return rb_hv_launch_scratch(s, vt, d_v1, d_v0, d_coef, d_out, d_part, lt);
+  if (bk_applies(s)) return bk_hv_launch(s, vt, d_v1, d_v0, d_coef, d_out, d_part, lt);
   const SumOut so = sum_out(d_part, 0, s->red_blocks, s->d_done, d_out, 0, lt);
   if (vt == kReal64) {
     if (s->gc) launch_general<double, true>(s, (const double *)d_v1, (double *)d_v0, d_coef, so);
@@ -277,17 +276,15 @@ int hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const
 
 int hv_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
               const LanczosTail *lt) {
-  if (rb_applies(s, vt)) {
-    if (rb_hv_launch(s, vt, d_v1, d_v0, d_coef, d_out) != 0) return -1;
-    return lt ? lanczos_scalars(s, 0, lt->k, lt->st, lt->alpha, lt->beta) : 0;
-  }
-  return hv_launch_scratch(s, vt, d_v1, d_v0, d_coef, d_out, s->d_red, lt);
+  double *part = rb_applies(s, vt) ? rb_part(s) : s->d_red;
+  return hv_launch_scratch(s, vt, d_v1, d_v0, d_coef, d_out, part, lt);
 }
 
 size_t hv_scratch_doubles(const Sector *s, VecType vt) {
   if (s->prod) return prod_scratch_doubles(s, vt);
   if (s->hub) return hub_scratch_doubles(s);
   if (rb_applies(s, vt)) return rb_scratch_doubles(s);
+  if (bk_applies(s)) return bk_scratch_doubles(s);
   return 2 * (size_t)s->red_blocks;
 }
 

@@ -1,0 +1,746 @@
+// Block kernel: one-pass H*v for canonical sectors in HPhi's row order (Spin, general spin,
+// Kondo, HubbardNConserved), whose vectors fit in L2 or which have no row-block plan.
+//
+// HPhi's rows come in blocks that share the upper half of the configuration (sector_blocks); the
+// blocks whose lower halves are the same, in the same order, form a class.  Of a term's masks
+//   in the lower half:  the term moves a row within its block, the same way in every block of the
+//                       class: a gather table per class, decoded once for all blocks of a task;
+//   in the upper half:  it moves a whole block, position for position: one row shift per block;
+//   in both:            it acts on the blocks whose upper half matches; its source position
+//                       follows from the lower half (a table per class and flipped bit).
+// A task is P planes of one class: P blocks of a real vector, or the real and imaginary parts of
+// P / 2 blocks of a complex one.  The planes are staged in shared memory, where the lower-half
+// terms are edge-coloured gathers (build_gather_table: no bank conflicts, 16-bit entries); upper
+// and crossing terms are listed per block when the plan is made (source block and coefficient)
+// and read v1 in (nearly) consecutive pieces from L2.  The general kernel (hv.cu) spends three
+// scattered L1 requests per matrix element (entry, coefficient, source) and is bound by them;
+// here an element is one shared-memory word or one coalesced load.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <array>
+#include <cmath>
+#include <cstdint>
+#include <map>
+#include <string>
+#include <vector>
+
+#include "device_util.cuh"
+#include "engine.hpp"
+#include "hv_blocks.hpp"
+#include "hv_product.hpp"
+#include "tma.cuh"
+
+namespace hphi {
+namespace {
+
+constexpr int kBkGroups = 8;      // lower-half coefficients, up to sign
+constexpr int kBkCross = 64;      // crossing terms
+constexpr int kBkList = 96;       // upper or crossing terms acting on one block
+constexpr uint32_t kBkNone = 0x7FFFu;
+
+struct BkClass {
+  int n, nblk, boff, uoff;                // rows of a block, blocks, first block in b_*, first lower half
+  int gat, sets;                          // gather table (16-byte units), sets of 8 slots per warp of 32 positions
+  int head;                               // per warp: slots of each group (8 bits each)
+};
+
+// A term on a block: the first row of its source block, the table of source positions (crossing
+// terms; positions keep their number under an upper-half term), and the coefficient, signs of the
+// upper half included.
+struct BkRec {
+  uint32_t row, tab;
+  double re;
+};
+
+struct BkArgs {
+  int ncls, ng, nlist;     // nlist: room for a block's list (both kinds, whole steps)
+  const BkClass *cls;
+  const uint32_t *b_row0;  // per block, by class: its first row
+  const uint2 *b_list;     // its first record, and numbers of upper (low half) and crossing terms
+  const BkRec *rec;
+  const double *rec_im;    // imaginary parts of the records' coefficients (nullptr: none)
+  const uint4 *gat;
+  const uint2 *head;
+  const double2 *cf;       // [ng]
+  const uint16_t *tab;     // source position | sign << 15 of each position, kBkNone: not matched
+};
+
+// Shapes by the longest block (planes of `stride` words: a block and 16 zero words) and, where a
+// sector has long and short ones, by the length its rows see.  Two planes share the table entries;
+// a thread takes Q positions, which share the addresses and coefficients of the listed terms, and
+// has U terms per block and position in flight.  Small CTAs, several per SM: a task is staging, then
+// gathers, then loads from L2, and only other CTAs fill the waits between them; five of 128
+// threads with 95 registers, since the address arithmetic of the listed terms wants them (24-site
+// J1-J2 chain, blocks of 924 rows, us per H*v: eight CTAs with 64 registers 107, six with 80: 89,
+// five with 95: 78; four planes and 256 threads 137; the general kernel 146).
+template <int ID> struct BkShape;
+template <> struct BkShape<0> { static constexpr int stride = 96, P = 2, Q = 1, U = 4, threads = 96, ctas = 6; };
+template <> struct BkShape<1> { static constexpr int stride = 288, P = 2, Q = 2, U = 2, threads = 128, ctas = 5; };
+template <> struct BkShape<2> { static constexpr int stride = 960, P = 2, Q = 2, U = 2, threads = 64, ctas = 10; };
+template <> struct BkShape<3> { static constexpr int stride = 960, P = 2, Q = 2, U = 2, threads = 128, ctas = 5; };
+template <> struct BkShape<4> { static constexpr int stride = 1744, P = 2, Q = 2, U = 2, threads = 256, ctas = 2; };
+template <> struct BkShape<5> { static constexpr int stride = 3456, P = 2, Q = 2, U = 2, threads = 256, ctas = 2; };
+template <> struct BkShape<6> { static constexpr int stride = 6560, P = 2, Q = 2, U = 2, threads = 512, ctas = 1; };
+template <> struct BkShape<7> { static constexpr int stride = 12896, P = 2, Q = 2, U = 2, threads = 1024, ctas = 1; };
+constexpr int kBkShapes = 8;
+constexpr int kBkWaves = 2;   // tasks per resident CTA that long blocks are shared out to
+constexpr int kBkLong = 320;  // mean block length from which 128 threads share a task of 960-word planes
+
+template <typename T> struct BkVal;
+template <> struct BkVal<double> {
+  static constexpr int W = 1;
+  static __device__ __forceinline__ double ld(const double *p) { return __ldg(p); }
+  static __device__ __forceinline__ double get(const double *pl, int stride) { return pl[0]; }
+};
+template <> struct BkVal<cplx> {
+  static constexpr int W = 2;
+  static __device__ __forceinline__ cplx ld(const cplx *p) {
+    const double2 z = __ldg(reinterpret_cast<const double2 *>(p));
+    return cplx{z.x, z.y};
+  }
+  static __device__ __forceinline__ cplx get(const double *pl, int stride) { return cplx{pl[0], pl[stride]}; }
+};
+
+// A task: its class, two blocks (the second ~0: none, and with complex vectors), and the positions
+// it computes (first | last + 1 << 16, multiples of 32): long blocks are shared by several tasks.
+struct BkTask {
+  uint32_t cls, b0, b1, span;
+};
+
+// IM: some listed coefficient has an imaginary part (complex vectors only).
+template <int ID, typename T, bool IM>
+__global__ void __launch_bounds__(BkShape<ID>::threads, BkShape<ID>::ctas)
+bk_kernel(BkArgs a, const BkTask *__restrict__ tasks, int ntask, const double *__restrict__ diag,
+          const T *__restrict__ v1, T *__restrict__ v0, const double *__restrict__ coef, SumOut so) {
+  // launched while the kernel before it ends (launch_chained): everything below waits for that one
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+  const double acc = coef[0], scale = coef[1];
+  using S = BkShape<ID>;
+  constexpr int STRIDE = S::stride, P = S::P, Q = S::Q, NT = S::threads;
+  constexpr int W = BkVal<T>::W, R = P / W;  // R blocks per task
+  constexpr uint32_t U = S::U;               // listed terms in flight per block and position
+  extern __shared__ __align__(16) double planes[];
+  BkRec *s_rec = reinterpret_cast<BkRec *>(planes + P * STRIDE);   // [R][nlist]
+  double *s_im = reinterpret_cast<double *>(s_rec + R * a.nlist);  // [R][nlist] (IM)
+  __shared__ double2 s_c[kBkGroups];
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid < a.ng) s_c[tid] = a.cf[tid];
+  double pr[2] = {0.0, 0.0};
+  for (int t = blockIdx.x; t < ntask; t += gridDim.x) {
+    // block r of the task: its first row, lists and vector (planes past the last repeat it)
+    uint32_t row0[R], nh[R], nx[R], hmin = ~0u, hmax = 0, xmax = 0;
+    const uint4 tk = __ldg(reinterpret_cast<const uint4 *>(tasks) + t);
+    const int nr = (R == 2 && tk.z != ~0u) ? 2 : 1;
+    uint32_t blk[R];
+    blk[0] = tk.y;
+    if (R == 2) blk[R - 1] = nr == 2 ? tk.z : tk.y;
+    const BkClass C = a.cls[tk.x];
+    const int n = C.n, npad = (int)(tk.w >> 16), end = min(n, npad);  // npad: whole warps
+    __syncthreads();  // the previous task's planes and lists are no longer read
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      row0[r] = __ldg(a.b_row0 + blk[r]);
+      const uint2 li = __ldg(a.b_list + blk[r]);
+      nh[r] = li.y & 0xFFFFu;
+      nx[r] = li.y >> 16;
+      hmin = min(hmin, nh[r]);
+      hmax = max(hmax, nh[r]);
+      xmax = max(xmax, nx[r]);
+      if constexpr (W == 1) {
+        const uint32_t to = smem_u32(planes + r * STRIDE);
+        for (int i = tid; i < n; i += NT)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(to + 8 * i), "l"(v1 + row0[r] + i) : "memory");
+      } else {
+        for (int i = tid; i < n; i += NT) {
+          const cplx z = BkVal<T>::ld(v1 + row0[r] + i);
+          planes[2 * r * STRIDE + i] = z.x;
+          planes[(2 * r + 1) * STRIDE + i] = z.y;
+        }
+      }
+      for (int k = tid; k < (int)(nh[r] + nx[r]); k += NT) {
+        *(reinterpret_cast<uint4 *>(s_rec + r * a.nlist) + k) = __ldg(reinterpret_cast<const uint4 *>(a.rec + li.x) + k);
+        if (IM) s_im[r * a.nlist + k] = __ldg(a.rec_im + li.x + k);
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    for (int k = tid; k < 16 * P; k += NT) planes[(k >> 4) * STRIDE + n + (k & 15)] = 0.0;  // the empty slots' words
+    const uint2 *headp = a.head + C.head;
+    const uint4 *gatp = a.gat + C.gat + lane;
+    const uint16_t *tabp = a.tab;
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    const char *rb = reinterpret_cast<const char *>(planes);
+    // A position's loads (slots, diagonal, old v0, the first upper-half terms) are issued before
+    // the gathers, and later ones several at a time: waits for L2 are what this loop is made of.
+    for (int p0 = (int)(tk.w & 0xFFFFu) + tid; p0 < npad; p0 += Q * NT) {
+      int p[Q];
+      bool in[Q];
+      uint2 head[Q];
+      uint4 e4[Q];
+      double dg[Q][R], y[Q][P];
+      T old[Q][R], z[U][R][Q];
+#pragma unroll
+      for (int q = 0; q < Q; q++) {
+        p[q] = p0 + q * NT;
+        in[q] = p[q] < end;
+        head[q] = make_uint2(0u, 0u);
+        e4[q] = make_uint4(0u, 0u, 0u, 0u);
+        if (p[q] < npad) {  // the same for the warp
+          head[q] = __ldg(headp + (p[q] >> 5));
+          e4[q] = __ldg(gatp + (int64_t)(p[q] >> 5) * C.sets * 32);
+        }
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          dg[q][r] = 0.0;
+          old[q][r] = VT<T>::zero();
+          if (in[q]) {
+            dg[q][r] = __ldg(diag + row0[r] + p[q]);
+            if (acc != 0.0) old[q][r] = v0[(int64_t)row0[r] + p[q]];
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < P; k++) y[q][k] = 0.0;
+      }
+      // the loads of terms e .. e + U; TAIL: some may be past a block's list
+      auto hi_load = [&](uint32_t e, bool tail) {
+#pragma unroll
+        for (uint32_t u = 0; u < U; u++)
+#pragma unroll
+          for (int r = 0; r < R; r++) {
+            if (tail && e + u >= nh[r]) continue;
+            const T *at = v1 + (s_rec[r * a.nlist + e + u].row + (uint32_t)p0);
+#pragma unroll
+            for (int q = 0; q < Q; q++)
+              if (in[q]) z[u][r][q] = BkVal<T>::ld(at + q * NT);
+          }
+      };
+      auto add = [&](int q, int r, double cr, double ci, const T &x) {
+        if constexpr (W == 2) {
+          y[q][2 * r] = fma(cr, x.x, y[q][2 * r]);
+          y[q][2 * r + 1] = fma(cr, x.y, y[q][2 * r + 1]);
+          if (IM) {
+            y[q][2 * r] = fma(-ci, x.y, y[q][2 * r]);
+            y[q][2 * r + 1] = fma(ci, x.x, y[q][2 * r + 1]);
+          }
+        } else {
+          y[q][r] = fma(cr, x, y[q][r]);
+        }
+      };
+      auto im_of = [&](int r, uint32_t e) { return IM ? s_im[r * a.nlist + e] : 0.0; };
+      auto hi_add = [&](uint32_t e, bool tail) {
+#pragma unroll
+        for (uint32_t u = 0; u < U; u++)
+#pragma unroll
+          for (int r = 0; r < R; r++) {
+            if (tail && e + u >= nh[r]) continue;
+            const double c = s_rec[r * a.nlist + e + u].re, ci = im_of(r, e + u);
+#pragma unroll
+            for (int q = 0; q < Q; q++)
+              if (in[q]) add(q, r, c, ci, z[u][r][q]);
+          }
+      };
+      const bool tail0 = U > hmin;
+      hi_load(0, tail0);
+#pragma unroll
+      for (int q = 0; q < Q; q++) {
+        if (p[q] >= npad) break;
+        const uint4 *gp = gatp + (int64_t)(p[q] >> 5) * C.sets * 32;
+        uint4 e = e4[q];
+        for (int k = 0; k < a.ng; k++) {
+          const int ns = (int)(((k < 4 ? head[q].x : head[q].y) >> (8 * (k & 3))) & 255u);
+          double s[P];
+#pragma unroll
+          for (int c = 0; c < P; c++) s[c] = 0.0;
+          auto gather2 = [&](uint32_t h) {  // two entries: word | sign << 15, the sign as a factor +-1
+            const double *x0 = reinterpret_cast<const double *>(rb + ((h << 3) & 0x3FFF8u));
+            const double *x1 = reinterpret_cast<const double *>(rb + ((h >> 13) & 0x3FFF8u));
+            const double f0 = __hiloint2double((int)(((h << 16) & 0x80000000u) | 0x3FF00000u), 0);
+            const double f1 = __hiloint2double((int)((h & 0x80000000u) | 0x3FF00000u), 0);
+#pragma unroll
+            for (int c = 0; c < P; c++) s[c] = fma(f0, x0[c * STRIDE], s[c]);
+#pragma unroll
+            for (int c = 0; c < P; c++) s[c] = fma(f1, x1[c * STRIDE], s[c]);
+          };
+          for (int j = 0; j < ns; j += 8) {
+            const uint4 w = e;
+            gp += 32;
+            e = __ldg(gp);  // the next set (one past a warp's last is allocated)
+            gather2(w.x);
+            gather2(w.y);
+            if (j + 4 < ns) {
+              gather2(w.z);
+              gather2(w.w);
+            }
+          }
+          const double2 c = s_c[k];
+#pragma unroll
+          for (int r = 0; r < R; r++) {
+            if constexpr (W == 2) {
+              y[q][2 * r] += c.x * s[2 * r] - c.y * s[2 * r + 1];
+              y[q][2 * r + 1] += c.x * s[2 * r + 1] + c.y * s[2 * r];
+            } else {
+              y[q][r] = fma(c.x, s[r], y[q][r]);
+            }
+          }
+        }
+      }
+      // upper-half terms: the task's blocks side by side
+      hi_add(0, tail0);
+      uint32_t e = U;
+      for (; e + U <= hmin; e += U) {
+        hi_load(e, false);
+        hi_add(e, false);
+      }
+      for (; e < hmax; e += U) {
+        hi_load(e, true);
+        hi_add(e, true);
+      }
+      // crossing terms: the source positions from the table, then the elements
+      for (uint32_t i = 0; i < xmax; i += U) {
+        uint32_t tb[U][R][Q];
+#pragma unroll
+        for (uint32_t u = 0; u < U; u++)
+#pragma unroll
+          for (int r = 0; r < R; r++) {
+            const uint16_t *at = tabp + s_rec[r * a.nlist + nh[r] + i + u].tab + p0;
+#pragma unroll
+            for (int q = 0; q < Q; q++) tb[u][r][q] = (i + u < nx[r] && in[q]) ? __ldg(at + q * NT) : kBkNone;
+          }
+#pragma unroll
+        for (uint32_t u = 0; u < U; u++)
+#pragma unroll
+          for (int r = 0; r < R; r++) {
+            const T *at = v1 + s_rec[r * a.nlist + nh[r] + i + u].row;
+#pragma unroll
+            for (int q = 0; q < Q; q++)
+              if ((tb[u][r][q] & 0x7FFFu) != kBkNone) z[u][r][q] = BkVal<T>::ld(at + (tb[u][r][q] & 0x7FFFu));
+          }
+#pragma unroll
+        for (uint32_t u = 0; u < U; u++)
+#pragma unroll
+          for (int r = 0; r < R; r++) {
+            const double c = s_rec[r * a.nlist + nh[r] + i + u].re, ci = im_of(r, nh[r] + i + u);
+#pragma unroll
+            for (int q = 0; q < Q; q++)
+              if ((tb[u][r][q] & 0x7FFFu) != kBkNone) {
+                const int sg = (int)((tb[u][r][q] & 0x8000u) << 16);
+                add(q, r, __hiloint2double(__double2hiint(c) ^ sg, __double2loint(c)),
+                    __hiloint2double(__double2hiint(ci) ^ sg, __double2loint(ci)), z[u][r][q]);
+              }
+          }
+      }
+#pragma unroll
+      for (int q = 0; q < Q; q++)
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          if (!in[q] || r >= nr) continue;
+          const T x = BkVal<T>::get(planes + W * r * STRIDE + p[q], STRIDE);
+          T yy;
+          if constexpr (W == 2) yy = cplx{y[q][2 * r], y[q][2 * r + 1]};
+          else yy = y[q][r];
+          yy = VT<T>::add(yy, VT<T>::scale(dg[q][r], x));
+          pr[0] += VT<T>::conj_mul_re(x, yy);
+          pr[1] += VT<T>::conj_mul_im(x, yy);
+          const T ys = VT<T>::scale(scale, yy);
+          v0[(int64_t)row0[r] + p[q]] = (acc == 0.0) ? ys : VT<T>::add(VT<T>::scale(acc, old[q][r]), ys);
+        }
+    }
+  }
+  if (so.done) {
+    grid_sum<2>(pr, so);
+  } else {  // the column pass sums these records with its own
+    block_sum<2>(pr);
+    if (tid == 0) {
+      so.part[2 * blockIdx.x] = pr[0];
+      so.part[2 * blockIdx.x + 1] = pr[1];
+    }
+  }
+}
+
+}  // namespace
+
+struct BlockPlan {
+  BkArgs args{};
+  std::vector<void *> allocs;
+  int shape = 0;               // BkShape
+  int ntask[2] = {0, 0};       // real, complex vectors
+  const BkTask *tasks[2] = {nullptr, nullptr};
+  bool two_pass = false;       // lower-half and crossing terms only: the row-block plan's row pass
+  bool im = false;             // complex coefficients in the lists
+  size_t smem[2] = {0, 0};
+  int grid[2] = {0, 0};        // resident CTAs
+};
+
+void bk_plan_free(BlockPlan *p) {
+  if (!p) return;
+  for (void *q : p->allocs) cudaFree(q);
+  delete p;
+}
+
+namespace {
+
+template <typename V>
+int bk_upload(BlockPlan *p, const std::vector<V> &h, const V **d, std::string *err) {
+  void *q = nullptr;
+  const size_t bytes = std::max<size_t>(16, sizeof(V) * h.size());
+  if (cudaMalloc(&q, bytes) != cudaSuccess) {
+    *err = "block plan: device allocation failed";
+    return -1;
+  }
+  p->allocs.push_back(q);
+  if (!h.empty() && cudaMemcpy(q, h.data(), sizeof(V) * h.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+    *err = "block plan: copy failed";
+    return -1;
+  }
+  *d = (const V *)q;
+  return 0;
+}
+
+template <typename F>
+void with_bk_shape(int id, F f) {
+  switch (id) {
+    case 0: f(std::integral_constant<int, 0>{}); break;
+    case 1: f(std::integral_constant<int, 1>{}); break;
+    case 2: f(std::integral_constant<int, 2>{}); break;
+    case 3: f(std::integral_constant<int, 3>{}); break;
+    case 4: f(std::integral_constant<int, 4>{}); break;
+    case 5: f(std::integral_constant<int, 5>{}); break;
+    case 6: f(std::integral_constant<int, 6>{}); break;
+    default: f(std::integral_constant<int, 7>{}); break;
+  }
+}
+
+}  // namespace
+
+// Leaves s->bk null where the plan does not apply (no lists, too many or complex-valued groups of
+// terms, blocks longer than shared memory): the general kernel remains.
+int bk_plan_build(Sector *s, bool two_pass, std::string *err) {
+  s->bk = nullptr;
+  const Model &m = s->model;
+  if (s->gc || !s->d_list_1 || s->lo_bits > 20 || s->hi_bits > 20 || m.offdiag.empty()) return 0;
+  const uint64_t lo_mask = s->ihfbit - 1;
+  std::vector<SectorBlock> blk;
+  std::vector<uint32_t> low;  // lower halves by class
+  if (sector_blocks(s, &blk, &low, err) != 0) return -1;
+  uint32_t max_n = 0;
+  for (const SectorBlock &b : blk) max_n = std::max(max_n, b.n);
+  if (max_n + 16 > 12896) return 0;
+  // classes, longest blocks first; block lists by class; each lower half's class and position
+  std::map<uint32_t, std::vector<int>> by_low;
+  for (size_t b = 0; b < blk.size(); b++) by_low[blk[b].low0].push_back((int)b);
+  std::vector<uint32_t> order_c;
+  for (const auto &kv : by_low) order_c.push_back(kv.first);
+  std::stable_sort(order_c.begin(), order_c.end(),
+                   [&](uint32_t x, uint32_t y) { return blk[by_low[x][0]].n > blk[by_low[y][0]].n; });
+  std::vector<int> cls_of(s->ihfbit, -1), pos_of(s->ihfbit, -1);
+  std::vector<BkClass> cls;
+  std::vector<uint32_t> b_ib, b_row0;
+  for (size_t c = 0; c < order_c.size(); c++) {
+    const std::vector<int> &bl = by_low[order_c[c]];
+    BkClass k{};
+    k.n = (int)blk[bl[0]].n;
+    k.nblk = (int)bl.size();
+    k.boff = (int)b_ib.size();
+    k.uoff = (int)order_c[c];
+    for (int p = 0; p < k.n; p++) {
+      const uint32_t ia = low[k.uoff + p];
+      if (cls_of[ia] >= 0) return 0;  // classes that share lower halves: not this layout
+      cls_of[ia] = (int)c;
+      pos_of[ia] = p;
+    }
+    for (int b : bl) {
+      b_ib.push_back(blk[b].ib);
+      b_row0.push_back(blk[b].row0);
+    }
+    cls.push_back(k);
+  }
+  // lower-half terms by coefficient up to sign
+  struct LoTerm {
+    const BitTerm *t;
+    int group;
+    bool neg;
+  };
+  std::vector<LoTerm> lo;
+  std::vector<double2> cf;
+  for (const BitTerm &t : m.offdiag) {
+    if (((t.cm | t.flip | t.sm) & ~lo_mask) != 0) continue;
+    int g = 0;
+    bool neg = false;
+    for (; g < (int)cf.size(); g++) {
+      if (t.re == cf[g].x && t.im == cf[g].y) break;
+      if (t.re == -cf[g].x && t.im == -cf[g].y) { neg = true; break; }
+    }
+    if (g == (int)cf.size()) {
+      if (g == kBkGroups) return 0;
+      cf.push_back(make_double2(t.re, t.im));
+    }
+    lo.push_back(LoTerm{&t, g, neg});
+  }
+  std::vector<uint4> gat;
+  std::vector<uint2> head;
+  const int ng = (int)cf.size();
+  for (size_t c = 0; c < cls.size(); c++) {
+    BkClass &k = cls[c];
+    std::vector<std::vector<std::vector<uint32_t>>> tab(ng, std::vector<std::vector<uint32_t>>(k.n));
+    for (int p = 0; p < k.n; p++) {
+      const uint32_t ia = low[k.uoff + p];
+      for (const LoTerm &t : lo) {
+        if ((ia & t.t->cm) != t.t->cv) continue;
+        const uint32_t src = ia ^ (uint32_t)t.t->flip;
+        if (cls_of[src] < 0) continue;  // list_2_1 == 0: outside the sector
+        if (cls_of[src] != (int)c) return 0;
+        const bool neg = ((__builtin_popcountll((uint64_t)ia & t.t->sm) & 1) != 0) != t.neg;
+        tab[t.group][p].push_back((uint32_t)pos_of[src] | (neg ? 0x10000u : 0u));
+        if (tab[t.group][p].size() > 255) return 0;
+      }
+    }
+    // one table per class: a warp's sets, group after group, at a fixed stride (with one set past
+    // the last, read ahead), so that the first set's address does not wait for the slot counts
+    const int nw = (k.n + 31) / 32;
+    std::vector<std::vector<uint32_t>> t(ng);
+    std::vector<std::vector<uint8_t>> ws(ng);
+    std::vector<int> gs(ng, 1);
+    k.sets = 1;
+    for (int g = 0; g < ng; g++) build_gather_table(tab[g], k.n, &t[g], &ws[g], &gs[g]);
+    for (int w = 0; w < nw; w++) {
+      int n = 1;
+      for (int g = 0; g < ng; g++) n += (ws[g][w] + 7) / 8;
+      k.sets = std::max(k.sets, n);
+    }
+    k.gat = (int)gat.size();
+    k.head = (int)head.size();
+    gat.resize(gat.size() + (size_t)nw * k.sets * 32, make_uint4(0, 0, 0, 0));
+    for (int w = 0; w < nw; w++) {
+      size_t at = (size_t)k.gat + (size_t)w * k.sets * 32;
+      uint64_t cnt = 0;
+      for (int g = 0; g < ng; g++) {
+        cnt |= (uint64_t)ws[g][w] << (8 * g);
+        const uint32_t *src = &t[g][(size_t)w * gs[g] * 128];
+        for (int i = 0; i < (ws[g][w] + 7) / 8 * 32; i++, at++)
+          gat[at] = make_uint4(src[4 * i], src[4 * i + 1], src[4 * i + 2], src[4 * i + 3]);
+      }
+      head.push_back(make_uint2((uint32_t)cnt, (uint32_t)(cnt >> 32)));
+    }
+  }
+  // per block the upper-half and crossing terms that act on it; a crossing term's lower-half
+  // pattern (condition, flip, sign) is a table of source positions per class
+  std::vector<uint32_t> l22(s->sdim);
+  if (cudaMemcpy(l22.data(), s->d_list_2_2, sizeof(uint32_t) * l22.size(), cudaMemcpyDeviceToHost) != cudaSuccess) {
+    *err = "block plan: list copy failed";
+    return -1;
+  }
+  struct HiTerm {
+    const BitTerm *t;
+    int pat;  // lower-half pattern, -1: upper-half term
+  };
+  std::vector<HiTerm> hi;
+  std::vector<std::array<uint32_t, 4>> pats;
+  for (const BitTerm &t : m.offdiag) {
+    if (((t.cm | t.flip | t.sm) & ~lo_mask) == 0) continue;  // lower half
+    HiTerm h{&t, -1};
+    if (((t.cm | t.flip | t.sm) & lo_mask) != 0) {
+      const std::array<uint32_t, 4> pt{(uint32_t)(t.cm & lo_mask), (uint32_t)(t.cv & lo_mask), (uint32_t)(t.flip & lo_mask),
+                                       (uint32_t)(t.sm & lo_mask)};
+      h.pat = (int)(std::find(pats.begin(), pats.end(), pt) - pats.begin());
+      if (h.pat == (int)pats.size()) pats.push_back(pt);
+    }
+    hi.push_back(h);
+  }
+  if (pats.size() > 4 * (size_t)kBkCross) return 0;
+  std::vector<uint16_t> tab;
+  std::vector<uint32_t> tab_at(cls.size() * std::max<size_t>(1, pats.size()), 0);
+  for (size_t c = 0; c < cls.size(); c++)
+    for (size_t q = 0; q < pats.size(); q++) {
+      tab_at[c * pats.size() + q] = (uint32_t)tab.size();
+      int to = -1;  // the class the pattern leads to: one for all its positions
+      for (int p = 0; p < cls[c].n; p++) {
+        const uint32_t ia = low[cls[c].uoff + p], src = ia ^ pats[q][2];
+        uint16_t v = (uint16_t)kBkNone;
+        if ((ia & pats[q][0]) == pats[q][1] && cls_of[src] >= 0) {
+          if (to < 0) to = cls_of[src];
+          if (cls_of[src] != to) return 0;
+          v = (uint16_t)((uint32_t)pos_of[src] | ((__builtin_popcount(ia & pats[q][3]) & 1) ? 0x8000u : 0u));
+        }
+        tab.push_back(v);
+      }
+    }
+  std::vector<int> class_of_block(s->sdim, -1);
+  for (size_t c = 0; c < cls.size(); c++)
+    for (int b = 0; b < cls[c].nblk; b++) class_of_block[b_ib[cls[c].boff + b]] = (int)c;
+  std::vector<uint2> b_list(b_ib.size());
+  std::vector<uint64_t> ib_sorted(b_ib.size());
+  std::vector<BkRec> rec;
+  std::vector<double> rec_im;
+  bool im = false;
+  uint32_t nlist = 1;
+  for (size_t c = 0; c < cls.size(); c++) {
+    std::vector<std::pair<uint64_t, int>> order;  // blocks of equal list lengths side by side
+    std::vector<std::vector<BkRec>> recs(cls[c].nblk);
+    std::vector<std::vector<double>> ims(cls[c].nblk);
+    std::vector<uint32_t> nhb(cls[c].nblk);
+    for (int b = 0; b < cls[c].nblk; b++) {
+      const uint64_t ib = b_ib[cls[c].boff + b], cfg = ib << s->lo_bits;
+      for (int cross = 0; cross < 2; cross++) {
+        for (const HiTerm &h : hi) {
+          if ((h.pat >= 0) != (cross == 1) || (two_pass && !cross)) continue;
+          if ((cfg & h.t->cm) != (h.t->cv & ~lo_mask)) continue;
+          const uint64_t to = (cfg ^ h.t->flip) >> s->lo_bits;
+          if (l22[to] == 0) continue;
+          const bool neg = __builtin_popcountll(cfg & h.t->sm) & 1;
+          if (cross == 0 && class_of_block[to] != (int)c) return 0;  // a moved block keeps its lower halves
+          if (cross == 1) {  // the source positions are those of the class the pattern leads to
+            const uint32_t at = tab_at[c * pats.size() + h.pat];
+            int any = -1;
+            for (int p = 0; p < cls[c].n && any < 0; p++)
+              if ((tab[at + p] & 0x7FFFu) != kBkNone) any = cls_of[low[cls[c].uoff + p] ^ pats[h.pat][2]];
+            if (any < 0) continue;  // no row of the class matches
+            if (class_of_block[to] != any) return 0;
+          }
+          recs[b].push_back(BkRec{l22[to] - 1u, cross ? tab_at[c * pats.size() + h.pat] : 0u, neg ? -h.t->re : h.t->re});
+          ims[b].push_back(neg ? -h.t->im : h.t->im);
+          im = im || h.t->im != 0.0;
+        }
+        if (cross == 0) nhb[b] = (uint32_t)recs[b].size();
+      }
+      if (recs[b].size() > (size_t)kBkList) return 0;
+      nlist = std::max(nlist, (uint32_t)recs[b].size());
+      order.push_back({((uint64_t)nhb[b] << 32) | recs[b].size(), b});
+    }
+    std::stable_sort(order.begin(), order.end());
+    std::vector<uint32_t> r0(cls[c].nblk);
+    for (int b = 0; b < cls[c].nblk; b++) {
+      r0[b] = b_row0[cls[c].boff + order[b].second];
+      ib_sorted[cls[c].boff + b] = b_ib[cls[c].boff + order[b].second];
+    }
+    for (int b = 0; b < cls[c].nblk; b++) {
+      const int o = order[b].second;
+      b_row0[cls[c].boff + b] = r0[b];
+      b_list[cls[c].boff + b] = make_uint2((uint32_t)rec.size(), nhb[o] | ((uint32_t)(recs[o].size() - nhb[o]) << 16));
+      rec.insert(rec.end(), recs[o].begin(), recs[o].end());
+      rec_im.insert(rec_im.end(), ims[o].begin(), ims[o].end());
+    }
+    if (rec.size() > (1u << 26)) return 0;
+  }
+  BlockPlan *p = new BlockPlan();
+  BkArgs &a = p->args;
+  a.ncls = (int)cls.size();
+  a.ng = ng;
+  a.nlist = (int)nlist + 4;  // the last step of four may start inside a list
+  p->im = im;
+  p->two_pass = two_pass;
+  double mean = 0.0;  // block length a row sees on average
+  for (const SectorBlock &b : blk) mean += (double)b.n * b.n / (double)s->dim;
+  for (int id = kBkShapes - 1; id >= 0; id--)
+    with_bk_shape(id, [&](auto st) {
+      if ((int)max_n + 16 <= BkShape<decltype(st)::value>::stride && !(id == 2 && mean >= kBkLong)) p->shape = id;
+    });
+  auto fail = [&]() { bk_plan_free(p); return -1; };
+  if (bk_upload(p, cls, &a.cls, err) || bk_upload(p, b_row0, &a.b_row0, err) || bk_upload(p, b_list, &a.b_list, err) ||
+      bk_upload(p, rec, &a.rec, err) || bk_upload(p, gat, &a.gat, err) || bk_upload(p, head, &a.head, err) ||
+      bk_upload(p, cf, &a.cf, err) || bk_upload(p, tab, &a.tab, err) || (im && bk_upload(p, rec_im, &a.rec_im, err)))
+    return fail();
+  bool fits = true;
+  with_bk_shape(p->shape, [&](auto st) {
+    using S = BkShape<decltype(st)::value>;
+    for (int cv = 0; cv < 2; cv++) {
+      const int R = S::P / (cv ? 2 : 1);
+      constexpr int ST = decltype(st)::value;
+      p->smem[cv] = sizeof(double) * (size_t)S::P * S::stride + (sizeof(BkRec) + (im ? sizeof(double) : 0)) * a.nlist * (size_t)R;
+      const void *f = !cv ? (const void *)bk_kernel<ST, double, false>
+                          : im ? (const void *)bk_kernel<ST, cplx, true> : (const void *)bk_kernel<ST, cplx, false>;
+      int per_sm = 0;
+      if (p->smem[cv] > 227 * 1024 || raise_smem_limit(f, p->smem[cv]) != cudaSuccess ||
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, S::threads, p->smem[cv]) != cudaSuccess || per_sm < 1)
+        fits = false;
+      p->grid[cv] = std::max(1, std::min(per_sm, 10)) * s->num_sms;
+    }
+  });
+  cudaGetLastError();
+  if (!fits) {
+    bk_plan_free(p);
+    return 0;
+  }
+  // Pairs of blocks of one class (complex vectors: single blocks).  Where v1 exceeds
+  // L2 (two_pass), blocks whose upper halves differ only in bits that crossing terms flip read
+  // each other's rows, so they come together and a group's source blocks are read while in L2;
+  // else class by class, the longest first.
+  uint64_t xhi = 0;
+  for (const HiTerm &h : hi)
+    if (h.pat >= 0) xhi |= h.t->flip >> s->lo_bits;
+  struct Blk {
+    uint64_t group;
+    uint32_t cls, b;
+  };
+  std::vector<Blk> all;
+  for (size_t c = 0; c < cls.size(); c++)
+    for (int b = 0; b < cls[c].nblk; b++)
+      all.push_back(Blk{two_pass ? ib_sorted[cls[c].boff + b] & ~xhi : 0, (uint32_t)c, (uint32_t)(cls[c].boff + b)});
+  std::stable_sort(all.begin(), all.end(), [](const Blk &x, const Blk &y) {
+    return x.group != y.group ? x.group < y.group : x.cls < y.cls;
+  });
+  // Whole blocks, unless they are fewer than kBkWaves tasks per resident CTA: then at most that
+  // share of the rows each, but no less than one turn of the threads (8-site Kondo chain, a step:
+  // 36.4 us with whole blocks, 33.8 shared out.  Where there are more tasks the second staging of
+  // a block costs more than the even end gives: 24-site J1-J2 chain, 2.8 tasks per CTA, 105 us
+  // whole and 113 in halves).
+  for (int cv = 0; cv < 2; cv++) {
+    std::vector<BkTask> tk;
+    int64_t total = 0;
+    for (const Blk &b : all) total += cls[b.cls].n;
+    int turn = 0;
+    with_bk_shape(p->shape, [&](auto st) { turn = BkShape<decltype(st)::value>::Q * BkShape<decltype(st)::value>::threads; });
+    const int64_t want = (int64_t)kBkWaves * p->grid[cv];
+    const int whole = (int)(cv ? all.size() : (all.size() + 1) / 2);
+    const int share = whole >= want ? 1 << 15 : (int)std::max<int64_t>(turn, (cv ? total : total / 2) / want);
+    for (size_t q = 0; q < all.size();) {
+      const bool two = !cv && q + 1 < all.size() && all[q + 1].cls == all[q].cls && all[q + 1].group == all[q].group;
+      const int nw = (cls[all[q].cls].n + 31) / 32, parts = std::min(nw, (32 * nw + share - 1) / share);
+      for (int k = 0; k < parts; k++)
+        tk.push_back(BkTask{all[q].cls, all[q].b, two ? all[q + 1].b : ~0u,
+                            (uint32_t)(32 * (nw * k / parts)) | ((uint32_t)(32 * (nw * (k + 1) / parts)) << 16)});
+      q += two ? 2 : 1;
+    }
+    p->ntask[cv] = (int)tk.size();
+    if (bk_upload(p, tk, &p->tasks[cv], err)) return fail();
+  }
+  s->bk = p;
+  return 0;
+}
+
+bool bk_applies(const Sector *s) { return s->bk && !s->bk->two_pass; }
+bool bk_row_pass(const Sector *s) { return s->bk && s->bk->two_pass; }
+
+int bk_grid(const Sector *s, VecType vt) {
+  const int cv = vt == kReal64 ? 0 : 1;
+  return std::max(1, std::min(s->bk->grid[cv], s->bk->ntask[cv]));
+}
+
+size_t bk_scratch_doubles(const Sector *s) { return 2 * (size_t)std::max(s->bk->grid[0], s->bk->grid[1]); }
+
+int bk_hv_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out, double *d_part,
+                 const LanczosTail *lt) {
+  const BlockPlan *p = s->bk;
+  const int cv = vt == kReal64 ? 0 : 1, grid = bk_grid(s, vt);
+  // no output: the records are left for a later launch
+  const SumOut so = sum_out(d_part, 0, grid, d_out ? s->d_done : nullptr, d_out, 0, lt);
+  with_bk_shape(p->shape, [&](auto st) {
+    constexpr int ST = decltype(st)::value;
+#define HPHI_BK(T, IM)                                                                \
+  launch_chained(bk_kernel<ST, T, IM>, grid, BkShape<ST>::threads, p->smem[cv], s->stream, p->args, p->tasks[cv], \
+                 p->ntask[cv], (const double *)s->d_diag, (const T *)d_v1, (T *)d_v0, d_coef, so)
+    if (!cv) HPHI_BK(double, false);
+    else if (p->im) HPHI_BK(cplx, true);
+    else HPHI_BK(cplx, false);
+#undef HPHI_BK
+  });
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    set_error(std::string("block kernel: launch failed: ") + cudaGetErrorString(e));
+    return -1;
+  }
+  return 0;
+}
+
+}  // namespace hphi

@@ -23,15 +23,8 @@
 // Both passes keep per-CTA partial sums of <v1|H v1> (static work assignment, so results are
 // reproducible); the vectors stay in HPhi's order.
 //
-// Fast row pass (canonical Spin, real vectors, every lower-half term of one magnitude, e.g.
-// the Heisenberg exchange): the lower-half operator depends only on the block's class (the
-// popcount of its lower halves), so each class gets the edge-coloured gather table of the
-// Hubbard row pass (hv_product.cu: 16-bit entries position | sign << 15, every 8-byte gather
-// of a half-warp on its own shared-memory bank pair); a CTA of 1024 threads stages two blocks
-// of one class at once and every table entry serves both.  The crossing terms whose
-// upper-half condition the block meets are listed once per block; each then walks its source
-// block in increasing order (a flip of one lower-half bit keeps the order of the positions),
-// through a per-class table of source positions.
+// Canonical Spin: the row pass is the block kernel's (hv_blocks.cu) with the crossing terms and
+// without the upper-half ones; the row pass here takes what that plan does not.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -43,6 +36,7 @@
 
 #include "device_util.cuh"
 #include "engine.hpp"
+#include "hv_blocks.hpp"
 #include "hv_product.hpp"
 #include "hv_rowblock.hpp"
 #include "split.cuh"
@@ -186,7 +180,7 @@ __device__ __forceinline__ void rb_upper_terms(const SplitView &sv, uint32_t ib,
 template <typename T, bool GC, int P>
 __global__ void __launch_bounds__(kColThreads) rb_col_kernel(RBArgs p, const int64_t *__restrict__ cl_task, SplitView sv,
                                                             const T *__restrict__ v1, T *__restrict__ v0,
-                                                            const double *__restrict__ coef, double *__restrict__ part) {
+                                                            const double *__restrict__ coef, SumOut so) {
   constexpr int CH = 32 * P;
   const int lane = threadIdx.x & 31;
   const int64_t warp = (int64_t)((blockIdx.x * (unsigned)kColThreads + threadIdx.x) >> 5);
@@ -225,226 +219,7 @@ __global__ void __launch_bounds__(kColThreads) rb_col_kernel(RBArgs p, const int
         v0[r[q]] = VT<T>::add(v0[r[q]], VT<T>::scale(scale, h[q]));
       }
   }
-  block_sum<2>(pr);
-  if (threadIdx.x == 0) {
-    part[2 * blockIdx.x] = pr[0];
-    part[2 * blockIdx.x + 1] = pr[1];
-  }
-}
-
-constexpr int kSpinThreads = 1024;
-constexpr int kSpinRow2 = 103168;   // shared-memory offset of the second block (>= (12880 + 16) * 8)
-constexpr int kSpinGenMax = 64;     // crossing terms of the fast row pass
-
-struct SpinRowArgs {
-  int ntask;
-  const int64_t *t_start;   // [2 * ntask] first rows of the two blocks (second -1: one block)
-  const uint32_t *t_ib;     // [2 * ntask] their upper halves
-  const int *t_cls;         // [ntask] class
-  const int *c_n;           // per class: positions (block size)
-  const int *c_groups;      // slot groups per warp in the class's table
-  const int *c_uoff;        // offset of the class's lower halves in unrank
-  const int64_t *c_gat;     // offset of the class's table in gat (16-byte units)
-  const int *c_ws;          // offset of the class's slot counts in wslots
-  const uint4 *gat;
-  const uint8_t *wslots;
-  const uint32_t *unrank;
-  double t_lo;              // magnitude of every lower-half term
-  int lo_bits;
-  uint64_t lo_mask;
-  const uint16_t *xt;       // per class and lower site j: position of ia ^ (1 << j) in its class
-  const int64_t *c_xt;      // per class: offset of its [lo_bits][n] part of xt
-  const int8_t *g_xbit;     // per crossing term: its single lower-half flip bit (-1: several)
-};
-
-__device__ __forceinline__ double rb_flip(double x, uint32_t sg) {
-  return __hiloint2double(__double2hiint(x) ^ (int)sg, __double2loint(x));
-}
-
-// A crossing term that acts on rows of a staged block, prepared once per block: it acts on
-// the row of lower half ia iff (ia & cm) == cv; the source row is src + xt[xt_off + position]
-// (one lower-half flip bit) or src + list_2_1[ia ^ flo] - 2; its coefficient is c times
-// (-1)^popcount(ia & sm).
-struct XRec {
-  int64_t src, xt_off;   // xt_off < 0: the source position comes from list_2_1
-  double c;
-  uint32_t cm, cv, sm, flo;
-};
-
-// Fast row pass: v0 = acc * v0 + scale * (diagonal + lower-half + crossing terms) v1 for two
-// blocks of one class at a time; part[blockIdx] = sum of v1 . (...) v1 over the CTA's blocks.
-// The gathers of the lower-half terms come first (one sweep over the columns); the crossing
-// terms follow term by term over the thread's columns (their fields read once per term), each
-// adding into the v0 element the thread has just written.
-__global__ void __launch_bounds__(kSpinThreads, 1) spin_row_kernel(SpinRowArgs a, const BitTerm *__restrict__ gterms,
-                                                                  int ngen, const uint32_t *__restrict__ l21,
-                                                                  const uint32_t *__restrict__ l22,
-                                                                  const double *__restrict__ diag,
-                                                                  const double *__restrict__ v1,
-                                                                  double *__restrict__ v0,
-                                                                  const double *__restrict__ coef,
-                                                                  double *__restrict__ part) {
-  extern __shared__ __align__(128) double srows[];  // block 0 at 0, block 1 at kSpinRow2
-  double *row1 = srows + kSpinRow2 / 8;
-  __shared__ XRec s_x[2][kSpinGenMax];
-  __shared__ int s_nact[2];
-  const double acc = coef[0], scale = coef[1];
-  const int tid = threadIdx.x, lane = tid & 31;
-  const uint32_t sm0 = smem_u32(srows), sm1 = sm0 + kSpinRow2;
-  const char *rb = reinterpret_cast<const char *>(srows);
-  const uint64_t hi_mask = ~a.lo_mask;
-  double pr = 0.0;
-  for (int t = blockIdx.x; t < a.ntask; t += gridDim.x) {
-    const int cls = a.t_cls[t];
-    const int n = a.c_n[cls], npad = (n + 31) & ~31, groups = a.c_groups[cls];
-    const int64_t s0 = a.t_start[2 * t], s1r = a.t_start[2 * t + 1];
-    const bool two = s1r >= 0;
-    const int64_t s1 = two ? s1r : s0;
-    const uint64_t hi0 = (uint64_t)a.t_ib[2 * t] << a.lo_bits;
-    const uint64_t hi1 = two ? ((uint64_t)a.t_ib[2 * t + 1] << a.lo_bits) : hi0;
-    __syncthreads();  // the previous blocks and term lists are no longer read
-    for (int i = tid; i < n; i += kSpinThreads) {
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sm0 + 8 * i), "l"(v1 + s0 + i) : "memory");
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sm1 + 8 * i), "l"(v1 + s1 + i) : "memory");
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-    if (tid < 16) {  // zero words after each block (one per bank pair): the empty slots read them
-      srows[n + tid] = 0.0;
-      row1[n + tid] = 0.0;
-    }
-    if (tid < 64) {  // crossing terms whose upper-half condition block w meets (warp w)
-      const int w = tid >> 5;
-      const uint64_t hi = w ? hi1 : hi0;
-      int m = 0;
-      for (int k0 = 0; k0 < ngen; k0 += 32) {
-        const int k = k0 + lane;
-        bool on = false;
-        XRec x{};
-        if (k < ngen) {
-          const BitTerm t = gterms[k];
-          on = (hi & t.cm) == (t.cv & hi_mask);
-          if (on) {
-            const uint32_t b1 = __ldg(l22 + ((hi ^ t.flip) >> a.lo_bits));
-            on = b1 != 0u;
-            const int xb = a.g_xbit[k];
-            x.src = (int64_t)b1 - 1;
-            x.xt_off = (xb >= 0) ? a.c_xt[cls] + (int64_t)xb * n : -1;
-            x.c = (__popcll(hi & t.sm) & 1) ? -t.re : t.re;
-            x.cm = (uint32_t)(t.cm & a.lo_mask);
-            x.cv = (uint32_t)(t.cv & a.lo_mask);
-            x.sm = (uint32_t)(t.sm & a.lo_mask);
-            x.flo = (uint32_t)(t.flip & a.lo_mask);
-          }
-        }
-        const unsigned bal = __ballot_sync(0xFFFFFFFFu, on);
-        if (on) s_x[w][m + __popc(bal & ((1u << lane) - 1u))] = x;
-        m += __popc(bal);
-      }
-      if (lane == 0) s_nact[w] = m;
-    }
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
-    __syncthreads();
-    const uint4 *gk = a.gat + a.c_gat[cls];
-    const uint8_t *wk = a.wslots + a.c_ws[cls];
-    for (int p = tid; p < npad; p += kSpinThreads) {
-      const int w = p >> 5, ns = wk[w];
-      const uint4 *gp = gk + ((int64_t)w * groups) * 32 + lane;
-      const int pc = (p < n) ? p : n - 1;
-      const double d0 = __ldg(diag + s0 + pc), d1 = __ldg(diag + s1 + pc);
-      const double y0old = (acc != 0.0) ? __ldcs(v0 + s0 + pc) : 0.0;
-      const double y1old = (acc != 0.0 && two) ? __ldcs(v0 + s1 + pc) : 0.0;
-      double g0 = 0.0, g1 = 0.0;
-      auto gather2 = [&](uint32_t r) {
-        const uint32_t o0 = (r << 3) & 0x3FFF8u, o1 = (r >> 13) & 0x3FFF8u;
-        const uint32_t sg0 = r << 16;
-        const double *x0 = reinterpret_cast<const double *>(rb + o0);
-        const double *x1 = reinterpret_cast<const double *>(rb + o1);
-        g0 += rb_flip(x0[0], sg0 & 0x80000000u);
-        g1 += rb_flip(x0[kSpinRow2 / 8], sg0 & 0x80000000u);
-        g0 += rb_flip(x1[0], r & 0x80000000u);
-        g1 += rb_flip(x1[kSpinRow2 / 8], r & 0x80000000u);
-      };
-      for (int g = 0; 8 * g < ns; g++) {
-        const uint4 e = __ldg(gp + g * 32);
-        gather2(e.x);
-        if (8 * g + 2 < ns) gather2(e.y);
-        if (8 * g + 4 < ns) gather2(e.z);
-        if (8 * g + 6 < ns) gather2(e.w);
-      }
-      if (p < n) {
-        const double x0 = srows[p];
-        const double y0 = d0 * x0 + a.t_lo * g0;
-        v0[s0 + p] = (acc == 0.0) ? scale * y0 : acc * y0old + scale * y0;
-        pr += x0 * y0;
-        if (two) {
-          const double x1 = row1[p];
-          const double y1 = d1 * x1 + a.t_lo * g1;
-          v0[s1 + p] = (acc == 0.0) ? scale * y1 : acc * y1old + scale * y1;
-          pr += x1 * y1;
-        }
-      }
-    }
-    // crossing terms: four of the thread's columns at a time, the block's terms one by one with
-    // every load of a term issued before its first use, one update of each v0 element
-    const uint32_t *un = a.unrank + a.c_uoff[cls];
-    constexpr int U = 4;
-    for (int w = 0; w < (two ? 2 : 1); w++) {
-      const int64_t sw = w ? s1 : s0;
-      const double *xw = w ? row1 : srows;
-      const int nact = s_nact[w];
-      if (nact == 0) continue;
-      for (int p0 = tid; p0 < n; p0 += U * kSpinThreads) {
-        uint32_t ia[U];
-        double hx[U];
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-          const int p = p0 + u * kSpinThreads;
-          ia[u] = (p < n) ? __ldg(un + p) : 0u;
-          hx[u] = 0.0;
-        }
-        for (int i = 0; i < nact; i++) {
-          const XRec x = s_x[w][i];
-          bool on[U];
-          int64_t j[U];
-#pragma unroll
-          for (int u = 0; u < U; u++) {
-            const int p = p0 + u * kSpinThreads;
-            on[u] = (p < n) && (ia[u] & x.cm) == x.cv;
-            j[u] = x.src;
-            if (on[u]) {
-              if (x.xt_off >= 0) {
-                j[u] += __ldg(a.xt + x.xt_off + p);
-              } else {
-                const uint32_t a1 = __ldg(l21 + (ia[u] ^ x.flo));
-                on[u] = a1 != 0u;
-                j[u] += (int64_t)a1 - 2;
-              }
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < U; u++)
-            if (on[u]) {
-              const double vv = __ldg(v1 + j[u]);
-              hx[u] += (__popc(ia[u] & x.sm) & 1) ? -x.c * vv : x.c * vv;
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-          const int p = p0 + u * kSpinThreads;
-          if (p < n && hx[u] != 0.0) {
-            v0[sw + p] += scale * hx[u];
-            pr += xw[p] * hx[u];
-          }
-        }
-      }
-    }
-  }
-  double v[2] = {pr, 0.0};
-  block_sum<2>(v);
-  if (tid == 0) {
-    part[2 * blockIdx.x] = v[0];
-    part[2 * blockIdx.x + 1] = 0.0;
-  }
+  grid_sum<2>(pr, so);
 }
 
 uint64_t binom_rb(int n, int k) {
@@ -463,10 +238,7 @@ struct RowBlockPlan {
   size_t smem_row[2] = {0, 0};
   int grid_col = 0;
   const int64_t *cl_task[2] = {nullptr, nullptr};  // column-pass task offsets per class: 128 / 64 positions
-  SpinRowArgs fast{};           // fast row pass (real vectors), when grid_fast > 0
-  int grid_fast = 0;
-  size_t smem_fast = 0;
-  double *part = nullptr;       // 2 * (max(grid_row, grid_fast) + grid_col) doubles
+  double *part = nullptr;       // 2 * (row pass CTAs + grid_col) doubles
 };
 
 void rb_plan_free(RowBlockPlan *p) {
@@ -616,140 +388,6 @@ int rb_plan_build(Sector *s, std::string *err) {
       rb_upload(p, cb_start, &a.cb_start, err) || rb_upload(p, cb_n, &a.cb_n, err) ||
       rb_upload(p, cb_key, &a.cb_key, err))
     return fail();
-  // fast row pass: canonical Spin, every lower-half term real and of one magnitude
-  if (!gc && s->split.ngen <= kSpinGenMax && !std::getenv("HPHI_B200_RB_SIMPLE")) {
-    const uint64_t lo_mask = s->ihfbit - 1;
-    const int L = s->lo_bits;
-    std::vector<const BitTerm *> lo_terms;
-    for (const BitTerm &t : m.offdiag)
-      if (((t.cm | t.flip | t.sm) & ~lo_mask) == 0) lo_terms.push_back(&t);
-    double tlo = -1.0;
-    bool ok = !lo_terms.empty();
-    for (const BitTerm *t : lo_terms) {
-      if (t->im != 0.0 || t->re == 0.0) ok = false;
-      if (tlo < 0.0) tlo = std::fabs(t->re);
-      else if (std::fabs(t->re) != tlo) ok = false;
-    }
-    for (int n : blk_n) ok = ok && (n + 16 <= kSpinRow2 / 8);
-    if (ok) {
-      std::vector<int> pos_of(1u << L, 0);
-      std::vector<std::vector<uint32_t>> by_pop(L + 1);
-      for (uint32_t ia = 0; ia < (1u << L); ia++) {
-        pos_of[ia] = (int)by_pop[__builtin_popcount(ia)].size();
-        by_pop[__builtin_popcount(ia)].push_back(ia);
-      }
-      std::vector<int> c_n(L + 1, 0), c_groups(L + 1, 1), c_uoff(L + 1, 0), c_ws(L + 1, 0);
-      std::vector<int64_t> c_gat(L + 1, 0);
-      std::vector<uint4> gat_all;
-      std::vector<uint8_t> ws_all;
-      std::vector<char> used(L + 1, 0);
-      for (int k : blk_key) used[k] = 1;
-      int key_off = 0;
-      for (int k = 0; k <= L && ok; k++) {
-        c_uoff[k] = key_off;
-        key_off += (int)by_pop[k].size();
-        if (!used[k]) continue;
-        const int n = (int)by_pop[k].size();
-        std::vector<std::vector<uint32_t>> rows(n);
-        for (int q = 0; q < n && ok; q++) {
-          const uint32_t ia = by_pop[k][q];
-          for (const BitTerm *t : lo_terms) {
-            if ((ia & t->cm) != t->cv) continue;
-            const uint32_t src = ia ^ (uint32_t)t->flip;
-            if (__builtin_popcount(src) != k) { ok = false; break; }
-            const bool neg = (t->re < 0.0) != ((__builtin_popcountll((uint64_t)ia & t->sm) & 1) != 0);
-            rows[q].push_back((uint32_t)pos_of[src] | (neg ? 0x10000u : 0u));
-          }
-          if (rows[q].size() > 255) ok = false;
-        }
-        if (!ok) break;
-        std::vector<uint32_t> g;
-        std::vector<uint8_t> ws;
-        int groups = 1;
-        build_gather_table(rows, n, &g, &ws, &groups);
-        c_n[k] = n;
-        c_groups[k] = groups;
-        c_gat[k] = (int64_t)gat_all.size();
-        c_ws[k] = (int)ws_all.size();
-        for (size_t i = 0; i + 3 < g.size(); i += 4) gat_all.push_back(make_uint4(g[i], g[i + 1], g[i + 2], g[i + 3]));
-        ws_all.insert(ws_all.end(), ws.begin(), ws.end());
-      }
-      if (ok) {
-        // tasks: pairs of blocks of one class.  Blocks whose upper halves differ only in bits
-        // that crossing terms flip read each other's rows, so they are grouped (by the other
-        // upper bits) and a group's tasks run together: the source blocks of the crossing terms
-        // are then read while they are in L2.
-        std::vector<BitTerm> gen_h0(s->split.ngen);
-        if (s->split.ngen &&
-            cudaMemcpy(gen_h0.data(), s->split.gen, sizeof(BitTerm) * gen_h0.size(), cudaMemcpyDeviceToHost) != cudaSuccess) {
-          *err = "row-block plan: term copy failed";
-          return fail();
-        }
-        uint64_t xhi = 0;
-        for (const BitTerm &t : gen_h0) xhi |= t.flip >> L;
-        std::vector<int> order_b(nblk);
-        for (int i = 0; i < nblk; i++) order_b[i] = i;
-        std::stable_sort(order_b.begin(), order_b.end(), [&](int x, int y) {
-          const uint64_t gx = blk_ib[x] & ~xhi, gy = blk_ib[y] & ~xhi;
-          if (gx != gy) return gx < gy;
-          if (blk_key[x] != blk_key[y]) return blk_key[x] < blk_key[y];
-          return blk_ib[x] < blk_ib[y];
-        });
-        std::vector<int64_t> t_start;
-        std::vector<uint32_t> t_ib;
-        std::vector<int> t_cls;
-        for (size_t i = 0; i < order_b.size();) {
-          const int b0 = order_b[i];
-          const bool two = i + 1 < order_b.size() && blk_key[order_b[i + 1]] == blk_key[b0] &&
-                           (blk_ib[order_b[i + 1]] & ~xhi) == (blk_ib[b0] & ~xhi);
-          const int b1 = two ? order_b[i + 1] : b0;
-          t_start.push_back(blk_start[b0]);
-          t_start.push_back(two ? blk_start[b1] : -1);
-          t_ib.push_back(blk_ib[b0]);
-          t_ib.push_back(blk_ib[b1]);
-          t_cls.push_back(blk_key[b0]);
-          i += two ? 2 : 1;
-        }
-        // crossing terms: single lower-half flip bit -> per class and site position tables
-        std::vector<BitTerm> gen_h(s->split.ngen);
-        if (s->split.ngen &&
-            cudaMemcpy(gen_h.data(), s->split.gen, sizeof(BitTerm) * gen_h.size(), cudaMemcpyDeviceToHost) != cudaSuccess) {
-          *err = "row-block plan: term copy failed";
-          return fail();
-        }
-        std::vector<int8_t> g_xbit(std::max<size_t>(1, gen_h.size()), -1);
-        for (size_t q = 0; q < gen_h.size(); q++) {
-          const uint64_t fl = gen_h[q].flip & lo_mask;
-          if (fl && (fl & (fl - 1)) == 0) g_xbit[q] = (int8_t)__builtin_ctzll(fl);
-        }
-        std::vector<int64_t> c_xt(L + 1, 0);
-        std::vector<uint16_t> xt;
-        for (int k = 0; k <= L; k++) {
-          if (!used[k]) continue;
-          c_xt[k] = (int64_t)xt.size();
-          for (int j = 0; j < L; j++)
-            for (uint32_t ia : by_pop[k]) xt.push_back((uint16_t)pos_of[ia ^ (1u << j)]);
-        }
-        SpinRowArgs &f = p->fast;
-        if (rb_upload(p, g_xbit, &f.g_xbit, err) || rb_upload(p, c_xt, &f.c_xt, err) || rb_upload(p, xt, &f.xt, err))
-          return fail();
-        f.ntask = (int)t_cls.size();
-        f.t_lo = tlo;
-        f.lo_bits = L;
-        f.lo_mask = lo_mask;
-        f.unrank = a.unrank;
-        if (rb_upload(p, t_start, &f.t_start, err) || rb_upload(p, t_ib, &f.t_ib, err) ||
-            rb_upload(p, t_cls, &f.t_cls, err) || rb_upload(p, c_n, &f.c_n, err) ||
-            rb_upload(p, c_groups, &f.c_groups, err) || rb_upload(p, c_uoff, &f.c_uoff, err) ||
-            rb_upload(p, c_gat, &f.c_gat, err) || rb_upload(p, c_ws, &f.c_ws, err) ||
-            rb_upload(p, gat_all, &f.gat, err) || rb_upload(p, ws_all, &f.wslots, err))
-          return fail();
-        p->smem_fast = 2 * (size_t)kSpinRow2;
-        if (raise_smem_limit((const void *)spin_row_kernel, p->smem_fast) == cudaSuccess)
-          p->grid_fast = std::max(1, std::min(f.ntask, s->num_sms));
-      }
-    }
-  }
   const size_t tbytes = sizeof(BitTerm) * (size_t)s->split.ngen;
   const size_t need[2] = {tbytes + sizeof(double) * (size_t)max_n, tbytes + sizeof(cplx) * (size_t)max_n};
   for (int vt = 0; vt < 2; vt++) {
@@ -770,7 +408,7 @@ int rb_plan_build(Sector *s, std::string *err) {
     p->smem_row[vt] = need[vt];
     p->grid_row[vt] = std::max(1, std::min(nblk, per_sm * s->num_sms));
   }
-  if (p->grid_row[0] == 0 && p->grid_row[1] == 0) {
+  if (gc && p->grid_row[0] == 0 && p->grid_row[1] == 0) {
     rb_plan_free(p);
     return 0;
   }
@@ -779,7 +417,8 @@ int rb_plan_build(Sector *s, std::string *err) {
                                                                 : (const void *)rb_col_kernel<cplx, false, 2>,
                                                 kColThreads, 0);
   p->grid_col = std::max(1, std::max(1, col_per_sm) * s->num_sms);
-  const int rows_max = std::max(std::max(p->grid_row[0], p->grid_row[1]), p->grid_fast);
+  // the block kernel's row pass, where it takes over, has at most ten CTAs per SM
+  const int rows_max = std::max(std::max(p->grid_row[0], p->grid_row[1]), gc ? 0 : 10 * s->num_sms);
   if (cudaMalloc(&p->part, sizeof(double) * 2 * (size_t)(rows_max + p->grid_col)) != cudaSuccess) {
     *err = "row-block plan: device allocation failed";
     return fail();
@@ -791,29 +430,32 @@ int rb_plan_build(Sector *s, std::string *err) {
 }
 
 bool rb_applies(const Sector *s, VecType vt) {
-  return s->rb && (s->rb->grid_row[vt == kReal64 ? 0 : 1] > 0 || (vt == kReal64 && s->rb->grid_fast > 0));
+  return s->rb && (s->rb->grid_row[vt == kReal64 ? 0 : 1] > 0 || bk_row_pass(s));
+}
+
+static int rb_row_grid(const Sector *s, VecType vt) {
+  return bk_row_pass(s) ? bk_grid(s, vt) : s->rb->grid_row[vt == kReal64 ? 0 : 1];
 }
 
 size_t rb_scratch_doubles(const Sector *s) {
-  const RowBlockPlan *p = s->rb;
-  return 2 * (size_t)(std::max(std::max(p->grid_row[0], p->grid_row[1]), p->grid_fast) + p->grid_col);
+  return 2 * (size_t)(std::max(rb_row_grid(s, kReal64), rb_row_grid(s, kComplex128)) + s->rb->grid_col);
 }
 
 int rb_hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
-                         double *d_part) {
+                         double *d_part, const LanczosTail *lt) {
   RowBlockPlan *p = s->rb;
   const int iv = (vt == kReal64) ? 0 : 1;
-  const bool fast = (vt == kReal64) && p->grid_fast > 0;
-  const int gr = fast ? p->grid_fast : p->grid_row[iv], gcol = p->grid_col;
+  const int gr = rb_row_grid(s, vt), gcol = p->grid_col;
   const SplitView sv = split_view(s->split);
-  double *pc = d_part + 2 * (size_t)gr;
-  if (fast) {
-    spin_row_kernel<<<gr, kSpinThreads, p->smem_fast, s->stream>>>(p->fast, s->split.gen, s->split.ngen,
-                                                                   s->d_list_2_1, s->d_list_2_2, s->d_diag,
-                                                                   (const double *)d_v1, (double *)d_v0, d_coef, d_part);
-    rb_col_kernel<double, false, 4><<<gcol, kColThreads, 0, s->stream>>>(p->args, p->cl_task[0], sv,
-                                                                         (const double *)d_v1, (double *)d_v0, d_coef, pc);
-    finalize_partials_kernel<2><<<1, 256, 0, s->stream>>>(d_part, gr + gcol, d_out);
+  const SumOut so = sum_out(d_part, gr, gr + gcol, s->d_done, d_out, 0, lt);
+  if (bk_row_pass(s)) {
+    if (bk_hv_launch(s, vt, d_v1, d_v0, d_coef, nullptr, d_part, nullptr) != 0) return -1;
+    if (vt == kReal64)
+      rb_col_kernel<double, false, 4><<<gcol, kColThreads, 0, s->stream>>>(p->args, p->cl_task[0], sv,
+                                                                           (const double *)d_v1, (double *)d_v0, d_coef, so);
+    else
+      rb_col_kernel<cplx, false, 2><<<gcol, kColThreads, 0, s->stream>>>(p->args, p->cl_task[1], sv, (const cplx *)d_v1,
+                                                                         (cplx *)d_v0, d_coef, so);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
       set_error(std::string("row-block kernels: launch failed: ") + cudaGetErrorString(e));
@@ -827,7 +469,7 @@ int rb_hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, co
         p->args, sv, s->split.gen, s->split.ngen, s->d_list_2_1, s->d_list_2_2, s->d_diag, (const T *)d_v1, (T *)d_v0, \
         d_coef, d_part);                                                                                             \
     rb_col_kernel<T, GC, P><<<gcol, kColThreads, 0, s->stream>>>(p->args, p->cl_task[P == 4 ? 0 : 1], sv,              \
-                                                              (const T *)d_v1, (T *)d_v0, d_coef, pc);                \
+                                                              (const T *)d_v1, (T *)d_v0, d_coef, so);                \
   } while (0)
   if (vt == kReal64) {
     if (s->gc) HPHI_RB_LAUNCH(double, true, 4);
@@ -837,7 +479,6 @@ int rb_hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, co
     else HPHI_RB_LAUNCH(cplx, false, 2);
   }
 #undef HPHI_RB_LAUNCH
-  finalize_partials_kernel<2><<<1, 256, 0, s->stream>>>(d_part, gr + gcol, d_out);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error(std::string("row-block kernels: launch failed: ") + cudaGetErrorString(e));
@@ -846,8 +487,6 @@ int rb_hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, co
   return 0;
 }
 
-int rb_hv_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out) {
-  return rb_hv_launch_scratch(s, vt, d_v1, d_v0, d_coef, d_out, s->rb->part);
-}
+double *rb_part(const Sector *s) { return s->rb->part; }
 
 }  // namespace hphi

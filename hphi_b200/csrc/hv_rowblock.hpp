@@ -15,9 +15,9 @@ void rb_plan_free(RowBlockPlan *p);
 bool rb_applies(const Sector *s, VecType vt);
 // H*v in HPhi's order (as hv_launch); the _scratch form takes rb_scratch_doubles(s) doubles
 // of partial sums from the caller.
-int rb_hv_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out);
+double *rb_part(const Sector *s);  // the plan's own partial-sum records
 int rb_hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
-                         double *d_part);
+                         double *d_part, const LanczosTail *lt);
 size_t rb_scratch_doubles(const Sector *s);
 
 }  // namespace hphi

@@ -22,6 +22,7 @@
 
 #include "engine.hpp"
 #include "hv_hubbard.hpp"
+#include "hv_blocks.hpp"
 #include "hv_rowblock.hpp"
 #include "hv_product.hpp"
 #include "split.cuh"
@@ -725,6 +726,11 @@ int sector_build(const Model &m, int device, Sector **out, std::string *err, boo
       (kname == "rowblock" || s->dim >= (1ll << 24))) {
     if (rb_plan_build(s, err) != 0) return -1;
   }
+  // The block kernel takes whole H*v of the sectors without another plan, and the row pass of the
+  // row-block plan (HPHI_B200_RB_SIMPLE keeps that plan's generic row pass).
+  if (specialise && kname != "general" && !s->prod && !s->hub && !(s->rb && getenv("HPHI_B200_RB_SIMPLE"))) {
+    if (bk_plan_build(s, s->rb != nullptr, err) != 0) return -1;
+  }
   *out = s;
   return 0;
 }
@@ -741,6 +747,7 @@ void sector_free(Sector *s) {
   prod_plan_free(s->prod);
   prod_plan_free(s->te_prod);
   rb_plan_free(s->rb);
+  bk_plan_free(s->bk);
   if (s->stream) cudaStreamDestroy(s->stream);
   delete s;
 }

@@ -56,6 +56,63 @@ def _compare(m, tmp_path, vts=(hphi_b200.REAL64, hphi_b200.COMPLEX128)):
         Hg.close()
 
 
+def _dm_chain(L, two_sz):
+    """Complex exchange: InterAll J/2 (e^{ia} S+S- + h.c.) beside the Ising part."""
+    m = expert.heisenberg(L, expert.chain_bonds(L), two_sz=two_sz)
+    m.exchange = []
+    for i, j in expert.chain_bonds(L):
+        m.interall += [(i, 0, i, 1, j, 1, j, 0, 0.4, 0.3), (j, 0, j, 1, i, 1, i, 0, 0.4, -0.3)]
+    return m
+
+
+def _couplings(L, n):
+    """A chain whose exchange couplings take n different values."""
+    b = expert.chain_bonds(L) + expert.chain_bonds(L, 2)
+    return expert.heisenberg(L, b, [1.0 + 0.1 * (k % n) for k in range(len(b))], two_sz=L % 2)
+
+
+def _nconserved(L, ne):
+    m = expert.hubbard(L, expert.chain_bonds(L), 1.0, 3.0, 1, 1)
+    m.ncond, m.two_sz = ne, None
+    for i in range(L):
+        m.trans += [(i, 0, (i + 1) % L, 1, 0.3, 0.0), ((i + 1) % L, 1, i, 0, 0.3, 0.0)]
+    return m
+
+
+BLOCK = {
+    # longest blocks of 1, 3, 6, 70, 252, 924, 1716, 3432, 6435 and 12870 rows: every plane shape
+    "chain2": lambda: expert.heisenberg(2, [(0, 1)]),
+    "chain3": lambda: expert.heisenberg(3, expert.chain_bonds(3), two_sz=1),
+    "chain5": lambda: expert.heisenberg(5, expert.chain_bonds(5), two_sz=-1),
+    "chain16": lambda: expert.heisenberg(16, expert.chain_bonds(16)),
+    "j1j2_19": lambda: expert.heisenberg(19, expert.chain_bonds(19) + expert.chain_bonds(19, 2), two_sz=1),
+    "square4x6": lambda: expert.heisenberg(24, expert.square_bonds(4, 6)),
+    "chain26_few": lambda: expert.heisenberg(26, expert.chain_bonds(26), two_sz=-12),
+    "chain28_few": lambda: expert.heisenberg(28, expert.chain_bonds(28), two_sz=-14),
+    "chain30_few": lambda: expert.heisenberg(30, expert.chain_bonds(30), two_sz=-16),
+    "chain32_few": lambda: expert.heisenberg(32, expert.chain_bonds(32), two_sz=-16),
+    "groups8": lambda: _couplings(12, 8),
+    "groups9": lambda: _couplings(12, 9),     # more than a plan holds: the general kernel
+    "kondo4": lambda: expert.kondo_chain(4, 1.0, 1.5, U=2.0),
+    "kondo7_odd": lambda: expert.kondo_chain(6, 1.0, 0.7, ncond=5, two_sz=1),
+    # few blocks, longer than one turn of a CTA's threads: shared out over several tasks
+    "kondo8": lambda: expert.kondo_chain(8, 1.0, 1.5),
+    "spin1_14": lambda: expert.general_heisenberg([2] * 14, expert.chain_bonds(14), 1.0, two_sz=0),
+    "spin1": lambda: expert.general_heisenberg([2] * 7, expert.chain_bonds(7), 1.0, D=0.3),
+    "mixed_spins": lambda: expert.general_heisenberg([1, 2, 3, 1, 2, 3], expert.chain_bonds(6), 0.8, two_sz=2),
+    "nconserved": lambda: _nconserved(6, 5),
+}
+
+
+@pytest.mark.parametrize("name", list(BLOCK))
+def test_block_kernel(name, tmp_path):
+    assert _compare(BLOCK[name](), tmp_path) == 0
+
+
+def test_block_kernel_complex_coefficients(tmp_path):
+    _compare(_dm_chain(14, 0), tmp_path, vts=(hphi_b200.COMPLEX128,))
+
+
 def _hubbard(N, nup, ndown, phases=0, anisotropic=0):
     """Ring of N sites; `phases` hops carry their own phase, `anisotropic` their own amplitude."""
     m = expert.hubbard(N, [], 1.0, 4.0, nup, ndown)
