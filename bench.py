@@ -780,7 +780,7 @@ def main():
                     1: ("hv_hub_pass", "hv_hub_pass<double,0> + hv_hub_pass<double,1> + finalize per step"),
                     4: ("spin_rowblock", "bk_kernel (row pass) + rb_col_kernel<double,0,4> (column pass) per step; "
                                          "achieved = B_alg / time of both")}.get(
-        kind, ("hv_row_order", "bk_kernel or hv_general_kernel"))
+        kind, ("hv_row_order", "bk_kernel, gc_tile_kernel or hv_general_kernel"))
     vt = hphi_b200.REAL64
     gen = torch.Generator(device="cuda").manual_seed(1234 + rank)
     v1 = torch.rand(dim, dtype=torch.float64, device="cuda", generator=gen) - 0.5

@@ -21,6 +21,7 @@ struct HubPlan;
 struct ProdPlan;
 struct RowBlockPlan;
 struct BlockPlan;
+struct GcPlan;
 
 // Real or complex double scalar for host/device code.
 struct cplx { double x, y; };
@@ -104,6 +105,9 @@ struct Sector {
   // Block plan (canonical sectors in HPhi's order without one of the plans above): one pass over
   // the blocks of rows that share an upper half (hv_blocks.cu).
   BlockPlan *bk = nullptr;
+  // Tile plan (grand-canonical sectors whose rows are configurations): passes over tiles of rows
+  // that agree in most bits (hv_gc.cu).
+  GcPlan *gcp = nullptr;
   SplitPlan split;
   SectorBlock *d_pieces = nullptr;  // sector_pieces
   uint32_t *d_low = nullptr;

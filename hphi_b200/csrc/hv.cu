@@ -16,6 +16,7 @@
 #include "device_util.cuh"
 #include "engine.hpp"
 #include "hv_blocks.hpp"
+#include "hv_gc.hpp"
 #include "hv_hubbard.hpp"
 #include "hv_product.hpp"
 #include "hv_rowblock.hpp"
@@ -226,7 +227,7 @@ void launch_block_n(Sector *s, int nb, int64_t stride, const T *v1, T *v0, const
 }  // namespace
 
 bool hv_block_applies(const Sector *s, VecType vt) {
-  return !s->prod && !s->hub && !rb_applies(s, vt) && !(vt == kReal64 && s->model.complex_terms);
+  return !s->prod && !s->hub && !rb_applies(s, vt) && !gc_applies(s, vt) && !(vt == kReal64 && s->model.complex_terms);
 }
 
 int hv_block_native(Sector *s, VecType vt, int nb, int64_t stride, const void *d_v1, void *d_v0,
@@ -256,6 +257,7 @@ int hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const
     set_error("H has complex coefficients: real vectors are not allowed");
     return -1;
   }
+  if (gc_applies(s, vt)) return gc_hv_launch(s, vt, d_v1, d_v0, d_coef, d_out, d_part, lt);
   if (rb_applies(s, vt)) return rb_hv_launch_scratch(s, vt, d_v1, d_v0, d_coef, d_out, d_part, lt);
   if (bk_applies(s)) return bk_hv_launch(s, vt, d_v1, d_v0, d_coef, d_out, d_part, lt);
   const SumOut so = sum_out(d_part, 0, s->red_blocks, s->d_done, d_out, 0, lt);
@@ -276,13 +278,14 @@ int hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const
 
 int hv_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
               const LanczosTail *lt) {
-  double *part = rb_applies(s, vt) ? rb_part(s) : s->d_red;
+  double *part = gc_applies(s, vt) ? gc_part(s) : rb_applies(s, vt) ? rb_part(s) : s->d_red;
   return hv_launch_scratch(s, vt, d_v1, d_v0, d_coef, d_out, part, lt);
 }
 
 size_t hv_scratch_doubles(const Sector *s, VecType vt) {
   if (s->prod) return prod_scratch_doubles(s, vt);
   if (s->hub) return hub_scratch_doubles(s);
+  if (gc_applies(s, vt)) return gc_scratch_doubles(s, vt);
   if (rb_applies(s, vt)) return rb_scratch_doubles(s);
   if (bk_applies(s)) return bk_scratch_doubles(s);
   return 2 * (size_t)s->red_blocks;

@@ -1,0 +1,476 @@
+// Tile kernel: H*v of grand-canonical sectors whose rows are their configurations (SpinGC,
+// HubbardGC), src/mltplySpin.c:450-703 and src/mltplyHubbard.c:150-330 in gather form.
+//
+// A term maps row r to row r ^ flip.  A pass picks K of the n bits (the lowest ones always among
+// them, so that rows of a tile come in whole 64-byte pieces) and works on tiles: the 2^K rows
+// that agree in the other bits, staged in shared memory.  Every term whose flip and condition
+// lie in the pass's bits stays inside a tile, where its source is the word at q ^ f: a
+// permutation of the lanes' words, without bank conflicts and without any table.  A few passes
+// (3 or 4 for the 24-site Kitaev-Heisenberg honeycomb) cover all terms; each reads v1 once and
+// updates v0 once.  The row-block passes this replaces test every term of every row one by one
+// (four bit patterns per bond) and gather the crossing ones from memory.
+//
+// Terms are merged to groups of one flip, one sign mask and at most two condition bits; a
+// group's coefficient is picked by those bits.  Bound by memory for few terms per pass, by
+// instruction issue for many (about 6 instructions per group and element).  24-site
+// Kitaev-Heisenberg honeycomb, complex: 4 passes of 201 us, where the row and column passes of
+// the row-block plan took 973 + 369.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <array>
+#include <cmath>
+#include <cstdint>
+#include <map>
+#include <string>
+#include <type_traits>
+#include <vector>
+
+#include "device_util.cuh"
+#include "engine.hpp"
+#include "hv_gc.hpp"
+#include "tma.cuh"
+
+namespace hphi {
+namespace {
+
+constexpr int kTidBits = 9, kGcThreads = 1 << kTidBits;
+constexpr int kGcPasses = 12;     // more passes than this cost more than the general kernels
+constexpr int kGcGroups = 24;     // groups of one pass
+// 64 KB of shared memory per tile, two CTAs per SM: one stages while the other computes
+template <typename T> struct GcTile;
+template <> struct GcTile<double> { static constexpr int K = 13, low = 3; };
+template <> struct GcTile<cplx> { static constexpr int K = 12, low = 2; };
+
+// A group in tile coordinates.  Position q of a tile is thread q % kGcThreads, element q /
+// kGcThreads.  Source q ^ f; coefficient c[bit i of q + 2 * bit j of q]; sign (-1)^popcount(q & sm)
+// times that of the tile's other bits, (-1)^popcount(base & smo).  The element's share of the
+// condition and the sign is worked out here, one bit per element, so that the kernel tests
+// constants: `at` is 0 where both condition bits are the thread's, 1 where j is the element's,
+// 2 where both are.
+struct GcGroup {
+  uint32_t ft, sm;         // flip and sign masks among the thread's bits
+  int fe;                  // flip among the elements
+  int i, j, at;
+  uint32_t bi, bj, sgn;    // per element: condition bits i and j, sign
+  uint32_t any_sign;
+  uint64_t smo;
+  double re[4];
+};
+
+struct GcPass {
+  int ngroup, first, last;   // first: applies acc and the diagonal; last: sums all passes' records
+  int nouter;
+  const uint32_t *dep;       // [2^(K - low)] the tile's bits above the lowest ones, in place
+  uint8_t outer[32];         // bit positions of the other bits, increasing
+  GcGroup g[kGcGroups];      // kernel parameters: uniform operands
+  double im[kGcGroups][4];   // imaginary parts of the coefficients
+};
+
+__device__ __forceinline__ void gc_fma(double &y, double c, double x) { y = fma(c, x, y); }
+__device__ __forceinline__ void gc_fma(cplx &y, double c, const cplx &x) {
+  y.x = fma(c, x.x, y.x);
+  y.y = fma(c, x.y, y.y);
+}
+__device__ __forceinline__ void gc_fma_i(double &, double, const double &) {}
+__device__ __forceinline__ void gc_fma_i(cplx &y, double ci, const cplx &x) {
+  y.x = fma(-ci, x.y, y.x);
+  y.y = fma(ci, x.x, y.y);
+}
+__device__ __forceinline__ double gc_lds(const double *p) { return *p; }
+__device__ __forceinline__ cplx gc_lds(const cplx *p) {
+  const double2 z = *reinterpret_cast<const double2 *>(p);
+  return cplx{z.x, z.y};
+}
+
+// IM: some coefficient has an imaginary part (complex vectors only).
+template <typename T, bool IM>
+__global__ void __launch_bounds__(kGcThreads, 2) gc_tile_kernel(const __grid_constant__ GcPass ps, int64_t ntile,
+                                                                const double *__restrict__ diag,
+                                                                const T *__restrict__ v1, T *__restrict__ v0,
+                                                                const double *__restrict__ coef, SumOut so) {
+  constexpr int K = GcTile<T>::K, LOW = GcTile<T>::low, M = (1 << K) / kGcThreads;
+  constexpr int H = M < 4 ? M : 4;  // elements per thread and sweep over the groups (registers)
+  extern __shared__ __align__(16) unsigned char gc_smem[];
+  T *x = reinterpret_cast<T *>(gc_smem);
+  const double acc = ps.first ? coef[0] : 1.0, scale = coef[1];
+  const int tid = threadIdx.x;
+  __shared__ uint32_t s_dep[1 << (K - LOW)];
+  for (int k = tid; k < (1 << (K - LOW)); k += kGcThreads) s_dep[k] = __ldg(ps.dep + k);
+  auto dep = [&](int m) {  // the thread's m-th row within a tile
+    const int q = tid + m * kGcThreads;
+    return s_dep[q >> LOW] | (uint32_t)(q & ((1 << LOW) - 1));
+  };
+  auto base_of = [&](int64_t t) {
+    uint64_t base = 0;
+    for (int b = 0; b < ps.nouter; b++) base |= (uint64_t)((t >> b) & 1) << ps.outer[b];
+    return base;
+  };
+  double pr[2] = {0.0, 0.0};
+  for (int64_t t = blockIdx.x; t < ntile; t += gridDim.x) {
+    const uint64_t base = base_of(t);
+    __syncthreads();  // the previous tile is no longer read (and s_dep is there)
+    const uint32_t dst = smem_u32(x);
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+      if constexpr (sizeof(T) == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 16 * (tid + m * kGcThreads)),
+                     "l"(v1 + (base | dep(m)))
+                     : "memory");
+      else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst + 8 * (tid + m * kGcThreads)),
+                     "l"(v1 + (base | dep(m)))
+                     : "memory");
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int m0 = 0; m0 < M; m0 += H) {
+      T y[H], old[H];
+      uint32_t row[H];
+#pragma unroll
+      for (int m = 0; m < H; m++) {  // the old v0 and the diagonal arrive during the sweep
+        row[m] = dep(m0 + m);
+        old[m] = VT<T>::zero();
+        if (acc != 0.0) old[m] = v0[base | row[m]];
+        y[m] = VT<T>::zero();
+      }
+      if (ps.first) {
+#pragma unroll
+        for (int m = 0; m < H; m++)
+          y[m] = VT<T>::scale(__ldg(diag + (base | row[m])), gc_lds(x + tid + (m0 + m) * kGcThreads));
+      }
+      for (int k = 0; k < ps.ngroup; k++) {
+        const GcGroup &g = ps.g[k];
+        const T *xs = x + (tid ^ (int)g.ft);
+        // y += coefficient * source of the sweep's elements, coefficient(element) by kind of group
+        auto sweep = [&](auto coefficient, auto imag) {
+#pragma unroll
+          for (int m = 0; m < H; m++) {
+            const double cc = coefficient(m0 + m);
+            const T z = gc_lds(xs + ((m0 + m) ^ g.fe) * kGcThreads);
+            if (decltype(imag)::value) gc_fma_i(y[m], cc, z);
+            else gc_fma(y[m], cc, z);
+          }
+        };
+        auto flip = [](double c, uint32_t sg) { return __hiloint2double(__double2hiint(c) ^ (int)sg, __double2loint(c)); };
+        auto part = [&](const double(&c)[4], auto imag) {
+          const bool bi = (tid >> g.i) & 1;  // read where bit i is the thread's
+          if (g.any_sign) {
+            const uint32_t sg = ((uint32_t)__popc((uint32_t)tid & g.sm) + (uint32_t)__popcll(base & g.smo)) << 31;
+            auto sign = [&](int qe) { return sg ^ ((g.sgn >> qe) << 31); };
+            if (g.at == 0) {
+              const double c0 = ((tid >> g.j) & 1) ? (bi ? c[3] : c[2]) : (bi ? c[1] : c[0]);
+              sweep([&](int qe) { return flip(c0, sign(qe)); }, imag);
+            } else if (g.at == 1) {
+              const double c0 = bi ? c[1] : c[0], c1 = bi ? c[3] : c[2];
+              sweep([&](int qe) { return flip(((g.bj >> qe) & 1u) ? c1 : c0, sign(qe)); }, imag);
+            } else {
+              sweep([&](int qe) { return flip(c[((g.bi >> qe) & 1u) | (((g.bj >> qe) & 1u) << 1)], sign(qe)); }, imag);
+            }
+          } else if (g.at == 0) {
+            const double c0 = ((tid >> g.j) & 1) ? (bi ? c[3] : c[2]) : (bi ? c[1] : c[0]);
+            sweep([&](int) { return c0; }, imag);
+          } else if (g.at == 1) {
+            const double c0 = bi ? c[1] : c[0], c1 = bi ? c[3] : c[2];
+            sweep([&](int qe) { return ((g.bj >> qe) & 1u) ? c1 : c0; }, imag);
+          } else {
+            sweep([&](int qe) { return c[((g.bi >> qe) & 1u) | (((g.bj >> qe) & 1u) << 1)]; }, imag);
+          }
+        };
+        part(g.re, std::false_type{});
+        if (IM) part(ps.im[k], std::true_type{});
+      }
+#pragma unroll
+      for (int m = 0; m < H; m++) {
+        const T xq = gc_lds(x + tid + (m0 + m) * kGcThreads);
+        pr[0] += VT<T>::conj_mul_re(xq, y[m]);
+        pr[1] += VT<T>::conj_mul_im(xq, y[m]);
+        const T ys = VT<T>::scale(scale, y[m]);
+        v0[base | row[m]] = (acc == 0.0) ? ys : VT<T>::add(VT<T>::scale(acc, old[m]), ys);
+      }
+    }
+  }
+  if (ps.last) {
+    grid_sum<2>(pr, so);
+  } else {
+    block_sum<2>(pr);
+    if (tid == 0) {
+      so.part[2 * (so.rec0 + blockIdx.x)] = pr[0];
+      so.part[2 * (so.rec0 + blockIdx.x) + 1] = pr[1];
+    }
+  }
+}
+
+}  // namespace
+
+struct GcPlan {
+  std::vector<void *> allocs;
+  std::vector<GcPass> pass[2];   // real, complex vectors
+  bool im = false;
+  int grid[2] = {0, 0};
+  int64_t ntile[2] = {0, 0};
+  double *part = nullptr;
+};
+
+void gc_plan_free(GcPlan *p) {
+  if (!p) return;
+  for (void *q : p->allocs) cudaFree(q);
+  delete p;
+}
+
+namespace {
+
+// A group in the configuration's bits.
+struct Raw {
+  uint64_t flip, sm;
+  int i, j;  // condition bits (equal: one bit)
+  std::array<double, 4> re{}, im{};
+};
+
+// One term into its group; false when it has more than two condition bits.
+bool merge_term(const BitTerm &t, std::vector<Raw> *raw) {
+  const uint64_t bits = t.cm;
+  const int n = __builtin_popcountll(bits);
+  if (n > 2 || t.flip == 0) return false;
+  // sign bits inside the condition have fixed values: they go into the coefficient
+  const double sg = (__builtin_popcountll(t.cv & t.sm & bits) & 1) ? -1.0 : 1.0;
+  const uint64_t sm = t.sm & ~bits;
+  int i, j;
+  if (n == 0) i = j = __builtin_ctzll(t.flip);
+  else {
+    i = __builtin_ctzll(bits);
+    j = 63 - __builtin_clzll(bits);
+  }
+  Raw *r = nullptr;
+  for (Raw &x : *raw)
+    if (x.flip == t.flip && x.sm == sm && x.i == i && x.j == j) r = &x;
+  if (!r) {
+    raw->push_back(Raw{t.flip, sm, i, j, {}, {}});
+    r = &raw->back();
+  }
+  for (int k = 0; k < 4; k++) {
+    const int bi = k & 1, bj = k >> 1;
+    if (i == j && bi != bj) continue;  // never read
+    if (n > 0 && (((t.cv >> i) & 1) != (uint64_t)bi || ((t.cv >> j) & 1) != (uint64_t)bj)) continue;
+    r->re[k] += sg * t.re;
+    r->im[k] += sg * t.im;
+  }
+  return true;
+}
+
+// Bit sets of K bits (the `low` lowest always among them) that cover every group's flip and
+// condition bits: greedily the set that takes most groups, grown group by group.
+std::vector<uint64_t> cover_passes(const std::vector<Raw> &raw, int n, int K, int low) {
+  auto need = [&](const Raw &r) { return r.flip | (1ull << r.i) | (1ull << r.j); };
+  const uint64_t base = (1ull << low) - 1;
+  std::vector<char> done(raw.size(), 0);
+  std::vector<uint64_t> sets;
+  for (;;) {
+    uint64_t best = 0;
+    int best_n = 0;
+    for (size_t s = 0; s < raw.size(); s++) {
+      if (done[s] || __builtin_popcountll(base | need(raw[s])) > K) continue;
+      uint64_t set = base | need(raw[s]);
+      for (;;) {  // the group that adds the fewest bits, then the one that shares most with others
+        int pick = -1, cost = 99, gain = -1;
+        for (size_t q = 0; q < raw.size(); q++) {
+          const uint64_t add = need(raw[q]) & ~set;
+          if (done[q] || add == 0) continue;
+          const int c = __builtin_popcountll(add);
+          if (__builtin_popcountll(set) + c > K) continue;
+          int g = 0;
+          for (size_t r = 0; r < raw.size(); r++) g += !done[r] && (need(raw[r]) & ~(set | add)) == 0;
+          if (g - 2 * c > gain - 2 * cost || pick < 0) { pick = (int)q; cost = c; gain = g; }
+        }
+        if (pick < 0) break;
+        set |= need(raw[pick]);
+      }
+      int covered = 0;
+      for (size_t r = 0; r < raw.size(); r++) covered += !done[r] && (need(raw[r]) & ~set) == 0;
+      if (covered > best_n) { best_n = covered; best = set; }
+    }
+    if (best_n == 0) break;
+    for (int b = 0; b < n && __builtin_popcountll(best) < K; b++) best |= 1ull << b;  // fill up with low bits
+    sets.push_back(best);
+    for (size_t r = 0; r < raw.size(); r++)
+      if ((need(raw[r]) & ~best) == 0) done[r] = 1;
+  }
+  for (char d : done)
+    if (!d) return {};
+  return sets;
+}
+
+uint64_t extract_bits(uint64_t x, uint64_t set) {  // bits of x at the places of set, packed
+  uint64_t r = 0;
+  int k = 0;
+  for (int b = 0; b < 64; b++)
+    if ((set >> b) & 1) r |= ((x >> b) & 1) << k++;
+  return r;
+}
+
+template <typename V>
+int gc_upload(GcPlan *p, const std::vector<V> &h, const V **d, std::string *err) {
+  void *q = nullptr;
+  if (cudaMalloc(&q, std::max<size_t>(16, sizeof(V) * h.size())) != cudaSuccess ||
+      cudaMemcpy(q, h.data(), sizeof(V) * h.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+    cudaFree(q);
+    *err = "grand-canonical plan: upload failed";
+    return -1;
+  }
+  p->allocs.push_back(q);
+  *d = (const V *)q;
+  return 0;
+}
+
+// Passes of one vector type; leaves p->pass[vt] empty where the plan does not apply.
+template <typename T>
+int build_passes(Sector *s, GcPlan *p, const std::vector<Raw> &raw, int vt, std::string *err) {
+  constexpr int K = GcTile<T>::K, low = GcTile<T>::low;
+  const int n = s->model.nbits;
+  std::vector<uint64_t> sets = raw.empty() ? std::vector<uint64_t>{(1ull << K) - 1} : cover_passes(raw, n, K, low);
+  if (sets.empty() || sets.size() > (size_t)kGcPasses) return 0;
+  // a group that several passes could take goes to the one with fewest, the least movable groups first
+  std::vector<int> owner(raw.size(), -1), load(sets.size(), 0);
+  std::vector<std::pair<int, size_t>> order;
+  auto fits = [&](size_t q, size_t a) {
+    return ((raw[q].flip | (1ull << raw[q].i) | (1ull << raw[q].j)) & ~sets[a]) == 0;
+  };
+  for (size_t q = 0; q < raw.size(); q++) {
+    int n_fit = 0;
+    for (size_t a = 0; a < sets.size(); a++) n_fit += fits(q, a);
+    order.push_back({n_fit, q});
+  }
+  std::sort(order.begin(), order.end());
+  for (const auto &o : order) {
+    for (size_t a = 0; a < sets.size(); a++)
+      if (fits(o.second, a) && (owner[o.second] < 0 || load[a] < load[owner[o.second]])) owner[o.second] = (int)a;
+    load[owner[o.second]]++;
+  }
+  std::vector<GcPass> passes;
+  for (size_t a = 0; a < sets.size(); a++) {
+    const uint64_t set = sets[a];
+    constexpr int M = (1 << K) / kGcThreads;
+    GcPass ps{};
+    for (size_t q = 0; q < raw.size(); q++) {
+      const Raw &r = raw[q];
+      if (owner[q] != (int)a) continue;
+      if (ps.ngroup == kGcGroups) return 0;
+      GcGroup &g = ps.g[ps.ngroup];
+      const uint32_t f = (uint32_t)extract_bits(r.flip, set), sm = (uint32_t)extract_bits(r.sm, set);
+      g.ft = f % kGcThreads;
+      g.fe = (int)(f / kGcThreads);
+      g.sm = sm % kGcThreads;
+      g.smo = r.sm & ~set;
+      g.any_sign = r.sm != 0;
+      g.i = __builtin_popcountll(set & ((1ull << r.i) - 1));
+      g.j = __builtin_popcountll(set & ((1ull << r.j) - 1));
+      g.at = g.j < kTidBits ? 0 : g.i < kTidBits ? 1 : 2;
+      for (int m = 0; m < M; m++) {
+        const uint32_t qm = (uint32_t)m * kGcThreads;
+        if (g.i >= kTidBits) g.bi |= ((qm >> g.i) & 1u) << m;
+        if (g.j >= kTidBits) g.bj |= ((qm >> g.j) & 1u) << m;
+        g.sgn |= ((uint32_t)__builtin_popcount(qm & sm) & 1u) << m;
+      }
+      for (int k = 0; k < 4; k++) {
+        g.re[k] = r.re[k];
+        ps.im[ps.ngroup][k] = r.im[k];
+      }
+      ps.ngroup++;
+    }
+    std::vector<uint32_t> dep(1u << (K - low));
+    std::vector<int> in;
+    for (int b = 0; b < n; b++) {
+      if (!((set >> b) & 1)) ps.outer[ps.nouter++] = (uint8_t)b;
+      else if (b >= low) in.push_back(b);
+    }
+    for (uint32_t q = 0; q < dep.size(); q++)
+      for (size_t k = 0; k < in.size(); k++) dep[q] |= ((q >> k) & 1u) << in[k];
+    ps.first = a == 0;
+    ps.last = a + 1 == sets.size();
+    if (gc_upload(p, dep, &ps.dep, err)) return -1;
+    passes.push_back(ps);
+  }
+  const size_t smem = sizeof(T) << K;
+  int per_sm = 0;
+  const void *f[2] = {(const void *)gc_tile_kernel<T, false>, (const void *)gc_tile_kernel<T, true>};
+  const bool im = p->im && sizeof(T) == 16;
+  if (raise_smem_limit(f[im], smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f[im], kGcThreads, smem) != cudaSuccess || per_sm < 1) {
+    cudaGetLastError();
+    return 0;
+  }
+  p->ntile[vt] = 1ll << (n - K);
+  p->grid[vt] = (int)std::min<int64_t>(p->ntile[vt], (int64_t)per_sm * s->num_sms);
+  p->pass[vt] = passes;
+  return 0;
+}
+
+}  // namespace
+
+int gc_plan_build(Sector *s, std::string *err) {
+  s->gcp = nullptr;
+  const Model &m = s->model;
+  // rows within a tile are 32-bit numbers; below 2^18 rows there are too few tiles for the SMs
+  if (!s->gc || m.general_spin || m.nbits > 32 || m.nbits < 18) return 0;
+  std::vector<Raw> raw;
+  for (const BitTerm &t : m.offdiag)
+    if (!merge_term(t, &raw)) return 0;
+  GcPlan *p = new GcPlan();
+  for (const Raw &r : raw)
+    for (double x : r.im) p->im = p->im || x != 0.0;
+  if ((!m.complex_terms && build_passes<double>(s, p, raw, 0, err) != 0) || build_passes<cplx>(s, p, raw, 1, err) != 0) {
+    gc_plan_free(p);
+    return -1;
+  }
+  if (p->pass[0].empty() && p->pass[1].empty()) {
+    gc_plan_free(p);
+    return 0;
+  }
+  s->gcp = p;
+  const size_t nd = std::max(gc_scratch_doubles(s, kReal64), gc_scratch_doubles(s, kComplex128));
+  if (cudaMalloc(&p->part, sizeof(double) * std::max<size_t>(2, nd)) != cudaSuccess) {
+    *err = "grand-canonical plan: device allocation failed";
+    gc_plan_free(p);
+    s->gcp = nullptr;
+    return -1;
+  }
+  p->allocs.push_back(p->part);
+  return 0;
+}
+
+bool gc_applies(const Sector *s, VecType vt) { return s->gcp && !s->gcp->pass[vt == kReal64 ? 0 : 1].empty(); }
+
+size_t gc_scratch_doubles(const Sector *s, VecType vt) {
+  const int v = vt == kReal64 ? 0 : 1;
+  return 2 * s->gcp->pass[v].size() * (size_t)s->gcp->grid[v];
+}
+
+double *gc_part(const Sector *s) { return s->gcp->part; }
+
+int gc_hv_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
+                 double *d_part, const LanczosTail *lt) {
+  const GcPlan *p = s->gcp;
+  const int v = vt == kReal64 ? 0 : 1, grid = p->grid[v];
+  for (size_t a = 0; a < p->pass[v].size(); a++) {
+    const SumOut so = sum_out(d_part, (int)a * grid, (int)p->pass[v].size() * grid, s->d_done, d_out, 0, lt);
+    if (v == 0)
+      gc_tile_kernel<double, false><<<grid, kGcThreads, sizeof(double) << GcTile<double>::K, s->stream>>>(
+          p->pass[v][a], p->ntile[v], s->d_diag, (const double *)d_v1, (double *)d_v0, d_coef, so);
+    else if (p->im)
+      gc_tile_kernel<cplx, true><<<grid, kGcThreads, sizeof(cplx) << GcTile<cplx>::K, s->stream>>>(
+          p->pass[v][a], p->ntile[v], s->d_diag, (const cplx *)d_v1, (cplx *)d_v0, d_coef, so);
+    else
+      gc_tile_kernel<cplx, false><<<grid, kGcThreads, sizeof(cplx) << GcTile<cplx>::K, s->stream>>>(
+          p->pass[v][a], p->ntile[v], s->d_diag, (const cplx *)d_v1, (cplx *)d_v0, d_coef, so);
+  }
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    set_error(std::string("grand-canonical kernel: launch failed: ") + cudaGetErrorString(e));
+    return -1;
+  }
+  return 0;
+}
+
+}  // namespace hphi

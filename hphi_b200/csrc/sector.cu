@@ -23,6 +23,7 @@
 #include "engine.hpp"
 #include "hv_hubbard.hpp"
 #include "hv_blocks.hpp"
+#include "hv_gc.hpp"
 #include "hv_rowblock.hpp"
 #include "hv_product.hpp"
 #include "split.cuh"
@@ -722,7 +723,12 @@ int sector_build(const Model &m, int device, Sector **out, std::string *err, boo
   // Row-block plan (spin sectors): from 2^24 rows up, where the vectors no longer stay in L2
   // and the general kernel's scattered gathers go to memory (below that the general kernel is
   // faster); HPHI_B200_KERNEL=rowblock builds it at any size.
-  if (specialise && kname != "general" && !s->prod && !s->hub &&
+  // The tile plan takes the grand-canonical sectors from 2^18 rows.
+  if (specialise && kname != "general" && kname != "rowblock") {
+    if (gc_plan_build(s, err) != 0) return -1;
+  }
+  const bool tiled = s->gcp && gc_applies(s, kComplex128) && (m.complex_terms || gc_applies(s, kReal64));
+  if (specialise && kname != "general" && !s->prod && !s->hub && !tiled &&
       (kname == "rowblock" || s->dim >= (1ll << 24))) {
     if (rb_plan_build(s, err) != 0) return -1;
   }
@@ -748,6 +754,7 @@ void sector_free(Sector *s) {
   prod_plan_free(s->te_prod);
   rb_plan_free(s->rb);
   bk_plan_free(s->bk);
+  gc_plan_free(s->gcp);
   if (s->stream) cudaStreamDestroy(s->stream);
   delete s;
 }

@@ -113,6 +113,53 @@ def test_block_kernel_complex_coefficients(tmp_path):
     _compare(_dm_chain(14, 0), tmp_path, vts=(hphi_b200.COMPLEX128,))
 
 
+def _spin_gc(n, field, seed=3):
+    m = expert.kitaev_heisenberg(3, n // 6, -1.0, 0.3) if n % 6 == 0 else None
+    if m is None:
+        m = expert.heisenberg(n, expert.chain_bonds(n), 0.9)
+        m.model, m.two_sz = "SpinGC", None
+    rng = np.random.default_rng(seed)
+    for i in range(n if field else 0):   # h.S with complex off-diagonal parts
+        h = complex(rng.normal(), rng.normal()) if field == "complex" else complex(rng.normal(), 0.0)
+        m.trans += [(i, 0, i, 1, h.real, h.imag), (i, 1, i, 0, h.real, -h.imag), (i, 0, i, 0, 0.1 * i, 0.0)]
+    return m
+
+
+def _hubbard_gc(L, complex_t=False, four_body=False):
+    m = expert.hubbard(L, expert.chain_bonds(L), 1.0, 4.0, 1, 1)
+    m.model, m.ncond, m.two_sz = "HubbardGC", None, None
+    if complex_t:
+        m.trans = []
+        for i, j in expert.chain_bonds(L):
+            for s in (0, 1):
+                m.trans += [(i, s, j, s, 0.8, 0.3), (j, s, i, s, 0.8, -0.3)]
+    m.trans += [(i, 0, i, 1, 0.2, 0.0) for i in range(L)] + [(i, 1, i, 0, 0.2, 0.0) for i in range(L)]
+    if four_body:   # condition on four bits: not a tile group
+        m.pairhop = [(0, 3, 0.5)]
+    return m
+
+
+GC = {
+    "kitaev18": lambda: _spin_gc(18, None),            # the smallest sector with tiles
+    "kitaev18_field": lambda: _spin_gc(18, "real"),
+    "chain17": lambda: _spin_gc(17, "real"),           # below it
+    "chain19": lambda: _spin_gc(19, "real"),
+    "hubbard9": lambda: _hubbard_gc(9),                # signs over bits inside and outside a tile
+    "hubbard10": lambda: _hubbard_gc(10),
+    "hubbard9_four_body": lambda: _hubbard_gc(9, four_body=True),
+}
+
+
+@pytest.mark.parametrize("name", list(GC))
+def test_tile_kernel(name, tmp_path):
+    _compare(GC[name](), tmp_path)
+
+
+@pytest.mark.parametrize("m", [lambda: _spin_gc(18, "complex"), lambda: _hubbard_gc(9, complex_t=True)])
+def test_tile_kernel_complex_coefficients(m, tmp_path):
+    _compare(m(), tmp_path, vts=(hphi_b200.COMPLEX128,))
+
+
 def _hubbard(N, nup, ndown, phases=0, anisotropic=0):
     """Ring of N sites; `phases` hops carry their own phase, `anisotropic` their own amplitude."""
     m = expert.hubbard(N, [], 1.0, 4.0, nup, ndown)
