@@ -41,6 +41,7 @@
 #include <cstdint>
 #include <cstdlib>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "device_util.cuh"
@@ -666,6 +667,7 @@ template <> __device__ __forceinline__ cplx signed_v<cplx>(const cplx &x, uint32
 
 constexpr int kPermThreads = 256;
 constexpr int kPermBatch = 4;    // elements in flight per thread
+constexpr int kPermShort = 32;   // mean rows per HPhi block below which a thread takes a row
 
 // HPhi order -> native: a CTA per up configuration u.  HPhi's row of (u, d) is
 // list_2_1[lower half] + list_2_2[upper half] - 3; with u fixed each term depends on the downs
@@ -739,6 +741,24 @@ __global__ void __launch_bounds__(kPermThreads) prod_from_native_kernel(int N, i
         if (a < n) out[(int64_t)w.y + a] = signed_v<T>(v[q], par[q]);
       }
     }
+  }
+}
+
+// Either direction, a thread per HPhi row: sectors whose HPhi blocks are shorter than a warp
+// (kPermShort), where the kernels above leave most of their lanes idle (15 sites with 3 + 3
+// electrons, complex, blocks of 21 rows: a whole hphi_mltply_device 114 -> 73 us).
+template <typename T, bool TO_NATIVE>
+__global__ void __launch_bounds__(kPermThreads) prod_permute_rows_kernel(int64_t dim, int Dc,
+                                                                         const uint64_t *__restrict__ list_1,
+                                                                         const uint16_t *__restrict__ rank,
+                                                                         const uint16_t *__restrict__ pos_dn,
+                                                                         const T *__restrict__ in, T *__restrict__ out) {
+  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < dim; r += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t c = (uint32_t)__ldg(list_1 + r);  // 2 N <= 32 bits
+    const uint32_t u = compress_even(c), d = compress_even(c >> 1);
+    const int64_t pos = (int64_t)__ldg(rank + u) * Dc + __ldg(pos_dn + d);
+    if (TO_NATIVE) out[pos] = signed_v<T>(ldg_v<T>(in + r), species_parity16(u, d));
+    else out[r] = signed_v<T>(ldg_v<T>(in + pos), species_parity16(u, d));
   }
 }
 
@@ -1597,6 +1617,19 @@ int prod_te_launch(Sector *s, const ProdPlan *te, int index, const void *d_v1, v
 int prod_permute(Sector *s, VecType vt, const void *in, void *out, bool to_native) {
   const ProdPlan *p = s->prod;
   const ProdArgs &a = p->args;
+  if (s->dim < (int64_t)kPermShort * p->nperm) {
+    const unsigned nb = (unsigned)std::min<int64_t>((s->dim + kPermThreads - 1) / kPermThreads, (int64_t)s->num_sms * 16);
+    auto rows = [&](auto *x, auto *y) {
+      using T = std::remove_reference_t<decltype(*y)>;
+      if (to_native)
+        prod_permute_rows_kernel<T, true><<<nb, kPermThreads, 0, s->stream>>>(s->dim, a.Dc, s->d_list_1, a.rank, a.pos_dn, x, y);
+      else
+        prod_permute_rows_kernel<T, false><<<nb, kPermThreads, 0, s->stream>>>(s->dim, a.Dc, s->d_list_1, a.rank, a.pos_dn, x, y);
+    };
+    if (vt == kReal64) rows((const double *)in, (double *)out);
+    else rows((const cplx *)in, (cplx *)out);
+    return cuda_ok(cudaGetLastError(), "permute");
+  }
   if (to_native) {
     const unsigned nb = (unsigned)std::min(a.Uc, s->num_sms * 8);
     if (vt == kReal64)
