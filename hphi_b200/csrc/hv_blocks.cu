@@ -25,36 +25,22 @@
 #include <string>
 #include <vector>
 
+#include "block_tables.hpp"
 #include "device_util.cuh"
 #include "engine.hpp"
 #include "hv_blocks.hpp"
-#include "hv_product.hpp"
 #include "tma.cuh"
 
 namespace hphi {
 namespace {
 
-constexpr int kBkGroups = 8;      // lower-half coefficients, up to sign
-constexpr int kBkCross = 64;      // crossing terms
-constexpr int kBkList = 96;       // upper or crossing terms acting on one block
-constexpr uint32_t kBkNone = 0x7FFFu;
-
-struct BkClass {
-  int n, nblk, boff, uoff;                // rows of a block, blocks, first block in b_*, first lower half
-  int gat, sets;                          // gather table (16-byte units), sets of 8 slots per warp of 32 positions
-  int head;                               // per warp: slots of each group (8 bits each)
-};
-
-// A term on a block: the first row of its source block, the table of source positions (crossing
-// terms; positions keep their number under an upper-half term), and the coefficient, signs of the
-// upper half included.
-struct BkRec {
-  uint32_t row, tab;
-  double re;
+template <int ID> struct BkShape {
+  static constexpr int stride = kBkShapeDefs[ID].stride, P = kBkShapeDefs[ID].P, Q = kBkShapeDefs[ID].Q,
+                       U = kBkShapeDefs[ID].U, threads = kBkShapeDefs[ID].threads, ctas = kBkShapeDefs[ID].ctas;
 };
 
 struct BkArgs {
-  int ncls, ng, nlist;     // nlist: room for a block's list (both kinds, whole steps)
+  int ncls, ng, nlist;     // nlist: BlockTables
   const BkClass *cls;
   const uint32_t *b_row0;  // per block, by class: its first row
   const uint2 *b_list;     // its first record, and numbers of upper (low half) and crossing terms
@@ -65,27 +51,6 @@ struct BkArgs {
   const double2 *cf;       // [ng]
   const uint16_t *tab;     // source position | sign << 15 of each position, kBkNone: not matched
 };
-
-// Shapes by the longest block (planes of `stride` words: a block and 16 zero words) and, where a
-// sector has long and short ones, by the length its rows see.  Two planes share the table entries;
-// a thread takes Q positions, which share the addresses and coefficients of the listed terms, and
-// has U terms per block and position in flight.  Small CTAs, several per SM: a task is staging, then
-// gathers, then loads from L2, and only other CTAs fill the waits between them; five of 128
-// threads with 95 registers, since the address arithmetic of the listed terms wants them (24-site
-// J1-J2 chain, blocks of 924 rows, us per H*v: eight CTAs with 64 registers 107, six with 80: 89,
-// five with 95: 78; four planes and 256 threads 137; the general kernel 146).
-template <int ID> struct BkShape;
-template <> struct BkShape<0> { static constexpr int stride = 96, P = 2, Q = 1, U = 4, threads = 96, ctas = 6; };
-template <> struct BkShape<1> { static constexpr int stride = 288, P = 2, Q = 2, U = 2, threads = 128, ctas = 5; };
-template <> struct BkShape<2> { static constexpr int stride = 960, P = 2, Q = 2, U = 2, threads = 64, ctas = 10; };
-template <> struct BkShape<3> { static constexpr int stride = 960, P = 2, Q = 2, U = 2, threads = 128, ctas = 5; };
-template <> struct BkShape<4> { static constexpr int stride = 1744, P = 2, Q = 2, U = 2, threads = 256, ctas = 2; };
-template <> struct BkShape<5> { static constexpr int stride = 3456, P = 2, Q = 2, U = 2, threads = 256, ctas = 2; };
-template <> struct BkShape<6> { static constexpr int stride = 6560, P = 2, Q = 2, U = 2, threads = 512, ctas = 1; };
-template <> struct BkShape<7> { static constexpr int stride = 12896, P = 2, Q = 2, U = 2, threads = 1024, ctas = 1; };
-constexpr int kBkShapes = 8;
-constexpr int kBkWaves = 2;   // tasks per resident CTA that long blocks are shared out to
-constexpr int kBkLong = 320;  // mean block length from which 128 threads share a task of 960-word planes
 
 template <typename T> struct BkVal;
 template <> struct BkVal<double> {
@@ -100,12 +65,6 @@ template <> struct BkVal<cplx> {
     return cplx{z.x, z.y};
   }
   static __device__ __forceinline__ cplx get(const double *pl, int stride) { return cplx{pl[0], pl[stride]}; }
-};
-
-// A task: its class, two blocks (the second ~0: none, and with complex vectors), and the positions
-// it computes (first | last + 1 << 16, multiples of 32): long blocks are shared by several tasks.
-struct BkTask {
-  uint32_t cls, b0, b1, span;
 };
 
 // IM: some listed coefficient has an imaginary part (complex vectors only).
@@ -414,232 +373,31 @@ void with_bk_shape(int id, F f) {
 
 }  // namespace
 
-// Leaves s->bk null where the plan does not apply (no lists, too many or complex-valued groups of
-// terms, blocks longer than shared memory): the general kernel remains.
+// Leaves s->bk null where the plan does not apply (block_tables): the general kernel remains.
 int bk_plan_build(Sector *s, bool two_pass, std::string *err) {
   s->bk = nullptr;
-  const Model &m = s->model;
-  if (s->gc || !s->d_list_1 || s->lo_bits > 20 || s->hi_bits > 20 || m.offdiag.empty()) return 0;
-  const uint64_t lo_mask = s->ihfbit - 1;
+  if (s->gc || !s->d_list_1 || s->lo_bits > 20 || s->hi_bits > 20 || s->model.offdiag.empty()) return 0;
   std::vector<SectorBlock> blk;
-  std::vector<uint32_t> low;  // lower halves by class
+  std::vector<uint32_t> low, l22(s->sdim);
   if (sector_blocks(s, &blk, &low, err) != 0) return -1;
-  uint32_t max_n = 0;
-  for (const SectorBlock &b : blk) max_n = std::max(max_n, b.n);
-  if (max_n + 16 > 12896) return 0;
-  // classes, longest blocks first; block lists by class; each lower half's class and position
-  std::map<uint32_t, std::vector<int>> by_low;
-  for (size_t b = 0; b < blk.size(); b++) by_low[blk[b].low0].push_back((int)b);
-  std::vector<uint32_t> order_c;
-  for (const auto &kv : by_low) order_c.push_back(kv.first);
-  std::stable_sort(order_c.begin(), order_c.end(),
-                   [&](uint32_t x, uint32_t y) { return blk[by_low[x][0]].n > blk[by_low[y][0]].n; });
-  std::vector<int> cls_of(s->ihfbit, -1), pos_of(s->ihfbit, -1);
-  std::vector<BkClass> cls;
-  std::vector<uint32_t> b_ib, b_row0;
-  for (size_t c = 0; c < order_c.size(); c++) {
-    const std::vector<int> &bl = by_low[order_c[c]];
-    BkClass k{};
-    k.n = (int)blk[bl[0]].n;
-    k.nblk = (int)bl.size();
-    k.boff = (int)b_ib.size();
-    k.uoff = (int)order_c[c];
-    for (int p = 0; p < k.n; p++) {
-      const uint32_t ia = low[k.uoff + p];
-      if (cls_of[ia] >= 0) return 0;  // classes that share lower halves: not this layout
-      cls_of[ia] = (int)c;
-      pos_of[ia] = p;
-    }
-    for (int b : bl) {
-      b_ib.push_back(blk[b].ib);
-      b_row0.push_back(blk[b].row0);
-    }
-    cls.push_back(k);
-  }
-  // lower-half terms by coefficient up to sign
-  struct LoTerm {
-    const BitTerm *t;
-    int group;
-    bool neg;
-  };
-  std::vector<LoTerm> lo;
-  std::vector<double2> cf;
-  for (const BitTerm &t : m.offdiag) {
-    if (((t.cm | t.flip | t.sm) & ~lo_mask) != 0) continue;
-    int g = 0;
-    bool neg = false;
-    for (; g < (int)cf.size(); g++) {
-      if (t.re == cf[g].x && t.im == cf[g].y) break;
-      if (t.re == -cf[g].x && t.im == -cf[g].y) { neg = true; break; }
-    }
-    if (g == (int)cf.size()) {
-      if (g == kBkGroups) return 0;
-      cf.push_back(make_double2(t.re, t.im));
-    }
-    lo.push_back(LoTerm{&t, g, neg});
-  }
-  std::vector<uint4> gat;
-  std::vector<uint2> head;
-  const int ng = (int)cf.size();
-  for (size_t c = 0; c < cls.size(); c++) {
-    BkClass &k = cls[c];
-    std::vector<std::vector<std::vector<uint32_t>>> tab(ng, std::vector<std::vector<uint32_t>>(k.n));
-    for (int p = 0; p < k.n; p++) {
-      const uint32_t ia = low[k.uoff + p];
-      for (const LoTerm &t : lo) {
-        if ((ia & t.t->cm) != t.t->cv) continue;
-        const uint32_t src = ia ^ (uint32_t)t.t->flip;
-        if (cls_of[src] < 0) continue;  // list_2_1 == 0: outside the sector
-        if (cls_of[src] != (int)c) return 0;
-        const bool neg = ((__builtin_popcountll((uint64_t)ia & t.t->sm) & 1) != 0) != t.neg;
-        tab[t.group][p].push_back((uint32_t)pos_of[src] | (neg ? 0x10000u : 0u));
-        if (tab[t.group][p].size() > 255) return 0;
-      }
-    }
-    // one table per class: a warp's sets, group after group, at a fixed stride (with one set past
-    // the last, read ahead), so that the first set's address does not wait for the slot counts
-    const int nw = (k.n + 31) / 32;
-    std::vector<std::vector<uint32_t>> t(ng);
-    std::vector<std::vector<uint8_t>> ws(ng);
-    std::vector<int> gs(ng, 1);
-    k.sets = 1;
-    for (int g = 0; g < ng; g++) build_gather_table(tab[g], k.n, &t[g], &ws[g], &gs[g]);
-    for (int w = 0; w < nw; w++) {
-      int n = 1;
-      for (int g = 0; g < ng; g++) n += (ws[g][w] + 7) / 8;
-      k.sets = std::max(k.sets, n);
-    }
-    k.gat = (int)gat.size();
-    k.head = (int)head.size();
-    gat.resize(gat.size() + (size_t)nw * k.sets * 32, make_uint4(0, 0, 0, 0));
-    for (int w = 0; w < nw; w++) {
-      size_t at = (size_t)k.gat + (size_t)w * k.sets * 32;
-      uint64_t cnt = 0;
-      for (int g = 0; g < ng; g++) {
-        cnt |= (uint64_t)ws[g][w] << (8 * g);
-        const uint32_t *src = &t[g][(size_t)w * gs[g] * 128];
-        for (int i = 0; i < (ws[g][w] + 7) / 8 * 32; i++, at++)
-          gat[at] = make_uint4(src[4 * i], src[4 * i + 1], src[4 * i + 2], src[4 * i + 3]);
-      }
-      head.push_back(make_uint2((uint32_t)cnt, (uint32_t)(cnt >> 32)));
-    }
-  }
-  // per block the upper-half and crossing terms that act on it; a crossing term's lower-half
-  // pattern (condition, flip, sign) is a table of source positions per class
-  std::vector<uint32_t> l22(s->sdim);
   if (cudaMemcpy(l22.data(), s->d_list_2_2, sizeof(uint32_t) * l22.size(), cudaMemcpyDeviceToHost) != cudaSuccess) {
     *err = "block plan: list copy failed";
     return -1;
   }
-  struct HiTerm {
-    const BitTerm *t;
-    int pat;  // lower-half pattern, -1: upper-half term
-  };
-  std::vector<HiTerm> hi;
-  std::vector<std::array<uint32_t, 4>> pats;
-  for (const BitTerm &t : m.offdiag) {
-    if (((t.cm | t.flip | t.sm) & ~lo_mask) == 0) continue;  // lower half
-    HiTerm h{&t, -1};
-    if (((t.cm | t.flip | t.sm) & lo_mask) != 0) {
-      const std::array<uint32_t, 4> pt{(uint32_t)(t.cm & lo_mask), (uint32_t)(t.cv & lo_mask), (uint32_t)(t.flip & lo_mask),
-                                       (uint32_t)(t.sm & lo_mask)};
-      h.pat = (int)(std::find(pats.begin(), pats.end(), pt) - pats.begin());
-      if (h.pat == (int)pats.size()) pats.push_back(pt);
-    }
-    hi.push_back(h);
-  }
-  if (pats.size() > 4 * (size_t)kBkCross) return 0;
-  std::vector<uint16_t> tab;
-  std::vector<uint32_t> tab_at(cls.size() * std::max<size_t>(1, pats.size()), 0);
-  for (size_t c = 0; c < cls.size(); c++)
-    for (size_t q = 0; q < pats.size(); q++) {
-      tab_at[c * pats.size() + q] = (uint32_t)tab.size();
-      int to = -1;  // the class the pattern leads to: one for all its positions
-      for (int p = 0; p < cls[c].n; p++) {
-        const uint32_t ia = low[cls[c].uoff + p], src = ia ^ pats[q][2];
-        uint16_t v = (uint16_t)kBkNone;
-        if ((ia & pats[q][0]) == pats[q][1] && cls_of[src] >= 0) {
-          if (to < 0) to = cls_of[src];
-          if (cls_of[src] != to) return 0;
-          v = (uint16_t)((uint32_t)pos_of[src] | ((__builtin_popcount(ia & pats[q][3]) & 1) ? 0x8000u : 0u));
-        }
-        tab.push_back(v);
-      }
-    }
-  std::vector<int> class_of_block(s->sdim, -1);
-  for (size_t c = 0; c < cls.size(); c++)
-    for (int b = 0; b < cls[c].nblk; b++) class_of_block[b_ib[cls[c].boff + b]] = (int)c;
-  std::vector<uint2> b_list(b_ib.size());
-  std::vector<uint64_t> ib_sorted(b_ib.size());
-  std::vector<BkRec> rec;
-  std::vector<double> rec_im;
-  bool im = false;
-  uint32_t nlist = 1;
-  for (size_t c = 0; c < cls.size(); c++) {
-    std::vector<std::pair<uint64_t, int>> order;  // blocks of equal list lengths side by side
-    std::vector<std::vector<BkRec>> recs(cls[c].nblk);
-    std::vector<std::vector<double>> ims(cls[c].nblk);
-    std::vector<uint32_t> nhb(cls[c].nblk);
-    for (int b = 0; b < cls[c].nblk; b++) {
-      const uint64_t ib = b_ib[cls[c].boff + b], cfg = ib << s->lo_bits;
-      for (int cross = 0; cross < 2; cross++) {
-        for (const HiTerm &h : hi) {
-          if ((h.pat >= 0) != (cross == 1) || (two_pass && !cross)) continue;
-          if ((cfg & h.t->cm) != (h.t->cv & ~lo_mask)) continue;
-          const uint64_t to = (cfg ^ h.t->flip) >> s->lo_bits;
-          if (l22[to] == 0) continue;
-          const bool neg = __builtin_popcountll(cfg & h.t->sm) & 1;
-          if (cross == 0 && class_of_block[to] != (int)c) return 0;  // a moved block keeps its lower halves
-          if (cross == 1) {  // the source positions are those of the class the pattern leads to
-            const uint32_t at = tab_at[c * pats.size() + h.pat];
-            int any = -1;
-            for (int p = 0; p < cls[c].n && any < 0; p++)
-              if ((tab[at + p] & 0x7FFFu) != kBkNone) any = cls_of[low[cls[c].uoff + p] ^ pats[h.pat][2]];
-            if (any < 0) continue;  // no row of the class matches
-            if (class_of_block[to] != any) return 0;
-          }
-          recs[b].push_back(BkRec{l22[to] - 1u, cross ? tab_at[c * pats.size() + h.pat] : 0u, neg ? -h.t->re : h.t->re});
-          ims[b].push_back(neg ? -h.t->im : h.t->im);
-          im = im || h.t->im != 0.0;
-        }
-        if (cross == 0) nhb[b] = (uint32_t)recs[b].size();
-      }
-      if (recs[b].size() > (size_t)kBkList) return 0;
-      nlist = std::max(nlist, (uint32_t)recs[b].size());
-      order.push_back({((uint64_t)nhb[b] << 32) | recs[b].size(), b});
-    }
-    std::stable_sort(order.begin(), order.end());
-    std::vector<uint32_t> r0(cls[c].nblk);
-    for (int b = 0; b < cls[c].nblk; b++) {
-      r0[b] = b_row0[cls[c].boff + order[b].second];
-      ib_sorted[cls[c].boff + b] = b_ib[cls[c].boff + order[b].second];
-    }
-    for (int b = 0; b < cls[c].nblk; b++) {
-      const int o = order[b].second;
-      b_row0[cls[c].boff + b] = r0[b];
-      b_list[cls[c].boff + b] = make_uint2((uint32_t)rec.size(), nhb[o] | ((uint32_t)(recs[o].size() - nhb[o]) << 16));
-      rec.insert(rec.end(), recs[o].begin(), recs[o].end());
-      rec_im.insert(rec_im.end(), ims[o].begin(), ims[o].end());
-    }
-    if (rec.size() > (1u << 26)) return 0;
-  }
+  BlockTables t;
+  if (!block_tables(s->model.offdiag, s->lo_bits, l22, blk, low, s->dim, two_pass, &t)) return 0;
   BlockPlan *p = new BlockPlan();
   BkArgs &a = p->args;
-  a.ncls = (int)cls.size();
-  a.ng = ng;
-  a.nlist = (int)nlist + 4;  // the last step of four may start inside a list
-  p->im = im;
+  a.ncls = (int)t.cls.size();
+  a.ng = (int)t.cf.size();
+  a.nlist = t.nlist;
+  p->im = t.im;
   p->two_pass = two_pass;
-  double mean = 0.0;  // block length a row sees on average
-  for (const SectorBlock &b : blk) mean += (double)b.n * b.n / (double)s->dim;
-  for (int id = kBkShapes - 1; id >= 0; id--)
-    with_bk_shape(id, [&](auto st) {
-      if ((int)max_n + 16 <= BkShape<decltype(st)::value>::stride && !(id == 2 && mean >= kBkLong)) p->shape = id;
-    });
+  p->shape = t.shape;
   auto fail = [&]() { bk_plan_free(p); return -1; };
-  if (bk_upload(p, cls, &a.cls, err) || bk_upload(p, b_row0, &a.b_row0, err) || bk_upload(p, b_list, &a.b_list, err) ||
-      bk_upload(p, rec, &a.rec, err) || bk_upload(p, gat, &a.gat, err) || bk_upload(p, head, &a.head, err) ||
-      bk_upload(p, cf, &a.cf, err) || bk_upload(p, tab, &a.tab, err) || (im && bk_upload(p, rec_im, &a.rec_im, err)))
+  if (bk_upload(p, t.cls, &a.cls, err) || bk_upload(p, t.b_row0, &a.b_row0, err) || bk_upload(p, t.b_list, &a.b_list, err) ||
+      bk_upload(p, t.rec, &a.rec, err) || bk_upload(p, t.gat, &a.gat, err) || bk_upload(p, t.head, &a.head, err) ||
+      bk_upload(p, t.cf, &a.cf, err) || bk_upload(p, t.tab, &a.tab, err) || (t.im && bk_upload(p, t.rec_im, &a.rec_im, err)))
     return fail();
   bool fits = true;
   with_bk_shape(p->shape, [&](auto st) {
@@ -647,9 +405,9 @@ int bk_plan_build(Sector *s, bool two_pass, std::string *err) {
     for (int cv = 0; cv < 2; cv++) {
       const int R = S::P / (cv ? 2 : 1);
       constexpr int ST = decltype(st)::value;
-      p->smem[cv] = sizeof(double) * (size_t)S::P * S::stride + (sizeof(BkRec) + (im ? sizeof(double) : 0)) * a.nlist * (size_t)R;
+      p->smem[cv] = sizeof(double) * (size_t)S::P * S::stride + (sizeof(BkRec) + (t.im ? sizeof(double) : 0)) * a.nlist * (size_t)R;
       const void *f = !cv ? (const void *)bk_kernel<ST, double, false>
-                          : im ? (const void *)bk_kernel<ST, cplx, true> : (const void *)bk_kernel<ST, cplx, false>;
+                          : t.im ? (const void *)bk_kernel<ST, cplx, true> : (const void *)bk_kernel<ST, cplx, false>;
       int per_sm = 0;
       if (p->smem[cv] > 227 * 1024 || raise_smem_limit(f, p->smem[cv]) != cudaSuccess ||
           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, S::threads, p->smem[cv]) != cudaSuccess || per_sm < 1)
@@ -662,46 +420,8 @@ int bk_plan_build(Sector *s, bool two_pass, std::string *err) {
     bk_plan_free(p);
     return 0;
   }
-  // Pairs of blocks of one class (complex vectors: single blocks).  Where v1 exceeds
-  // L2 (two_pass), blocks whose upper halves differ only in bits that crossing terms flip read
-  // each other's rows, so they come together and a group's source blocks are read while in L2;
-  // else class by class, the longest first.
-  uint64_t xhi = 0;
-  for (const HiTerm &h : hi)
-    if (h.pat >= 0) xhi |= h.t->flip >> s->lo_bits;
-  struct Blk {
-    uint64_t group;
-    uint32_t cls, b;
-  };
-  std::vector<Blk> all;
-  for (size_t c = 0; c < cls.size(); c++)
-    for (int b = 0; b < cls[c].nblk; b++)
-      all.push_back(Blk{two_pass ? ib_sorted[cls[c].boff + b] & ~xhi : 0, (uint32_t)c, (uint32_t)(cls[c].boff + b)});
-  std::stable_sort(all.begin(), all.end(), [](const Blk &x, const Blk &y) {
-    return x.group != y.group ? x.group < y.group : x.cls < y.cls;
-  });
-  // Whole blocks, unless they are fewer than kBkWaves tasks per resident CTA: then at most that
-  // share of the rows each, but no less than one turn of the threads (8-site Kondo chain, a step:
-  // 36.4 us with whole blocks, 33.8 shared out.  Where there are more tasks the second staging of
-  // a block costs more than the even end gives: 24-site J1-J2 chain, 2.8 tasks per CTA, 105 us
-  // whole and 113 in halves).
   for (int cv = 0; cv < 2; cv++) {
-    std::vector<BkTask> tk;
-    int64_t total = 0;
-    for (const Blk &b : all) total += cls[b.cls].n;
-    int turn = 0;
-    with_bk_shape(p->shape, [&](auto st) { turn = BkShape<decltype(st)::value>::Q * BkShape<decltype(st)::value>::threads; });
-    const int64_t want = (int64_t)kBkWaves * p->grid[cv];
-    const int whole = (int)(cv ? all.size() : (all.size() + 1) / 2);
-    const int share = whole >= want ? 1 << 15 : (int)std::max<int64_t>(turn, (cv ? total : total / 2) / want);
-    for (size_t q = 0; q < all.size();) {
-      const bool two = !cv && q + 1 < all.size() && all[q + 1].cls == all[q].cls && all[q + 1].group == all[q].group;
-      const int nw = (cls[all[q].cls].n + 31) / 32, parts = std::min(nw, (32 * nw + share - 1) / share);
-      for (int k = 0; k < parts; k++)
-        tk.push_back(BkTask{all[q].cls, all[q].b, two ? all[q + 1].b : ~0u,
-                            (uint32_t)(32 * (nw * k / parts)) | ((uint32_t)(32 * (nw * (k + 1) / parts)) << 16)});
-      q += two ? 2 : 1;
-    }
+    const std::vector<BkTask> tk = block_tasks(t, cv != 0, p->grid[cv]);
     p->ntask[cv] = (int)tk.size();
     if (bk_upload(p, tk, &p->tasks[cv], err)) return fail();
   }
