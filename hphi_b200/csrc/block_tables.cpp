@@ -92,7 +92,8 @@ bool block_tables(const std::vector<BitTerm> &terms, int lo_bits, const std::vec
     std::vector<std::vector<uint8_t>> ws(ng);
     std::vector<int> gs(ng, 1);
     k.sets = 1;
-    for (int g = 0; g < ng; g++) build_gather_table(tab[g], k.n, &t[g], &ws[g], &gs[g]);
+    for (int g = 0; g < ng; g++)
+      if (!build_gather_table(tab[g], k.n, &t[g], &ws[g], &gs[g])) return false;
     for (int w = 0; w < nw; w++) {
       int n = 1;
       for (int g = 0; g < ng; g++) n += (ws[g][w] + 7) / 8;

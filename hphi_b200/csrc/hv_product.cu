@@ -890,7 +890,7 @@ uint64_t spread_species(uint32_t x, int s, int N) {
 // Dc .. Dc+15, one per bank pair).  Stored packed: per warp and group of 8 slots, each lane's
 // 8 entries (16 bits: word | sign << 15) are one 16-byte load.
 void build_gather(const std::vector<std::vector<uint32_t>> &rows_dn, const std::vector<SpeciesHop> &hops, int Dc,
-                  int npad, std::vector<uint32_t> *gat, std::vector<uint8_t> *wslots, int *nslots, int *groups) {
+                  int npad, std::vector<uint32_t> *gat, std::vector<int> *wslots, int *nslots, int *groups) {
   const int nwarp = npad / 32;
   auto zero_word = [&](int bank) { return (uint32_t)(Dc + (((bank - Dc) % 16) + 16) % 16); };
   std::vector<std::vector<uint32_t>> lane_slots(npad);  // per column: entry of each slot of its half
@@ -960,7 +960,7 @@ void build_gather(const std::vector<std::vector<uint32_t>> &rows_dn, const std::
       }
       wmax = std::max(wmax, D);
     }
-    (*wslots)[w] = (uint8_t)wmax;
+    (*wslots)[w] = wmax;
     *nslots = std::max(*nslots, wmax);
   }
   // packed: per warp and slot group g, 32 lanes x 8 entries of 16 bits (word | sign << 15)
@@ -1074,12 +1074,15 @@ std::vector<int> balance_positions(const std::vector<std::vector<uint32_t>> &row
 
 }  // namespace
 
-void build_gather_table(const std::vector<std::vector<uint32_t>> &rows, int n, std::vector<uint32_t> *gat,
+bool build_gather_table(const std::vector<std::vector<uint32_t>> &rows, int n, std::vector<uint32_t> *gat,
                         std::vector<uint8_t> *wslots, int *groups) {
   // entries carry their sign directly: one hop of coefficient +1, sign bit = (entry >> 16) & 1
   const std::vector<SpeciesHop> unit{SpeciesHop{0, 0, 1.0, 0.0}};
   int nslots = 0;
-  build_gather(rows, unit, n, (n + 31) / 32 * 32, gat, wslots, &nslots, groups);
+  std::vector<int> slots;
+  build_gather(rows, unit, n, (n + 31) / 32 * 32, gat, &slots, &nslots, groups);
+  wslots->assign(slots.begin(), slots.end());
+  return nslots <= 255;
 }
 
 // The species (0 up, 1 down) and hop of a term that moves one electron; false for any other.
@@ -1150,7 +1153,7 @@ static void with_row_kernel(int stride, bool cplx_v, bool onsite, F f) {
 }
 
 // Tables and launch shapes of the two-pass kernels.  rows_*: per configuration its hops as
-// source | (2 * hop + sign) << 16.
+// source | (2 * hop + sign) << 16.  Leaves p->two_pass false where a gather table does not apply.
 static int two_pass_build(Sector *s, ProdPlan *p, const std::vector<std::vector<uint32_t>> &rows_dn,
                           const std::vector<std::vector<uint32_t>> &rows_up, const HopGroups (&G)[2], std::string *err) {
   const int Uc = p->args.Uc, Dc = p->args.Dc;
@@ -1168,7 +1171,7 @@ static int two_pass_build(Sector *s, ProdPlan *p, const std::vector<std::vector<
         const uint32_t h = (e >> 16) >> 1, sign = (e >> 16) & 1u;
         if (G[1].gid[h] == g) rows[r].push_back((e & 0xFFFFu) | ((sign ^ (G[1].gsign[h] < 0 ? 1u : 0u)) << 16));
       }
-    build_gather_table(rows, Dc, &tabs[g], &slots[g], &gsets[g]);
+    if (!build_gather_table(rows, Dc, &tabs[g], &slots[g], &gsets[g])) return 0;
   }
   std::vector<uint4> gat, whead(nw);
   for (int w = 0; w < nw; w++) {
@@ -1590,9 +1593,10 @@ int prod_te_plan_build(Sector *s, const std::vector<BitTerm> &terms, const std::
   if (wd > 255 || wu > 64) return 0;
   ProdPlan *p = new ProdPlan();
   p->args = base->args;
-  if (two_pass_build(s, p, rows_dn, rows_up, G, err) != 0) {
+  const int rc = two_pass_build(s, p, rows_dn, rows_up, G, err);
+  if (rc != 0 || !p->two_pass) {
     prod_plan_free(p);
-    return -1;
+    return rc;
   }
   *out = p;
   return 0;

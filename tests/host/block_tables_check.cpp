@@ -1,5 +1,5 @@
 // Checks the block kernel's host tables (block_tables.hpp) of one model against its terms, without
-// a device: argv[1] is a namelist.def of a canonical model of at most 24 bits.  Every index the
+// a device: argv[1] is a namelist.def of a canonical model of at most 24 bits, or "crowded".  Every index the
 // kernel would form is compared with the room it has, and H*v put together from the tables, the
 // way the kernel does it, with H*v from the terms.  Prints what the tables are like; the exit
 // status is 1, with a message, when something is wrong.
@@ -21,38 +21,11 @@ static void fail(const char *what, long a = 0, long b = 0) {
   exit(1);
 }
 
-int main(int argc, char **argv) {
-  Model m;
-  std::string err;
-  if (argc < 2 || read_expert(argv[1], &m, &err) != 0) fail(err.c_str());
-  const int lo_bits = (m.nbits + 1) / 2, hi_bits = m.nbits - lo_bits;
-  const uint64_t lo_mask = (1ull << lo_bits) - 1, even = 0x5555555555555555ull;
-  auto in_sector = [&](uint64_t c) {
-    if (m.calc_model == kHubbard)
-      return __builtin_popcountll(c & even) == m.nup && __builtin_popcountll(c & ~even) == m.ndown;
-    return __builtin_popcountll(c) == m.ne;
-  };
-  // HPhi's rows: by upper half, then lower half
-  std::vector<uint64_t> list_1;
-  std::vector<uint32_t> l22(1ull << hi_bits, 0), low;
-  std::vector<SectorBlock> blk;
-  std::map<std::vector<uint32_t>, uint32_t> cls;
-  std::vector<int64_t> row_of(1ull << m.nbits, -1);
-  for (uint64_t ib = 0; ib < (1ull << hi_bits); ib++) {
-    std::vector<uint32_t> mine;
-    const uint32_t row0 = (uint32_t)list_1.size();
-    for (uint64_t ia = 0; ia <= lo_mask; ia++)
-      if (in_sector(ib << lo_bits | ia)) {
-        mine.push_back((uint32_t)ia);
-        row_of[ib << lo_bits | ia] = (int64_t)list_1.size();
-        list_1.push_back(ib << lo_bits | ia);
-      }
-    if (mine.empty()) continue;
-    l22[ib] = row0 + 1;
-    const auto it = cls.emplace(mine, (uint32_t)low.size());
-    if (it.second) low.insert(low.end(), mine.begin(), mine.end());
-    blk.push_back(SectorBlock{(uint32_t)ib, row0, it.first->second, (uint32_t)mine.size()});
-  }
+// The tables of these terms; row_of: row of a configuration, -1 outside the sector.
+static void check(const std::vector<BitTerm> &terms, int lo_bits, const std::vector<uint32_t> &l22,
+                  const std::vector<SectorBlock> &blk, const std::vector<uint32_t> &low,
+                  const std::vector<uint64_t> &list_1, const std::vector<int64_t> &row_of) {
+  const uint64_t lo_mask = (1ull << lo_bits) - 1;
   const int64_t dim = (int64_t)list_1.size();
   std::mt19937_64 rng(5);
   std::normal_distribution<double> gauss;
@@ -60,7 +33,7 @@ int main(int argc, char **argv) {
   for (Z &x : v) x = Z(gauss(rng), gauss(rng));
   for (int two_pass = 0; two_pass < 2; two_pass++) {
     BlockTables t;
-    if (!block_tables(m.offdiag, lo_bits, l22, blk, low, dim, two_pass != 0, &t)) {
+    if (!block_tables(terms, lo_bits, l22, blk, low, dim, two_pass != 0, &t)) {
       printf("no plan ");
       continue;
     }
@@ -137,7 +110,7 @@ int main(int argc, char **argv) {
             }
           }
           const uint64_t cfg = list_1[t.b_row0[b] + p];
-          for (const BitTerm &q : m.offdiag) {
+          for (const BitTerm &q : terms) {
             if (two_pass && ((q.cm | q.flip | q.sm) & lo_mask) == 0) continue;
             if ((cfg & q.cm) != q.cv || row_of[cfg ^ q.flip] < 0) continue;
             want += ((__builtin_popcountll(cfg & q.sm) & 1) ? -1.0 : 1.0) * Z(q.re, q.im) * v[row_of[cfg ^ q.flip]];
@@ -151,6 +124,63 @@ int main(int argc, char **argv) {
     if (worst > 1e-13 * std::max(1.0, big)) fail("H*v differs");
     printf("shape %d longest list %d room %d ", t.shape, longest, t.nlist);
   }
+}
+
+// One block of 512 rows whose first 16 rows read the same 20 words each, all on one of the 16 bank
+// pairs: 320 entries that no two slots of a half-warp can share.
+static void crowded() {
+  std::vector<BitTerm> terms;
+  for (uint64_t r = 0; r < 16; r++)
+    for (uint64_t k = 0; k < 20; k++) terms.push_back(BitTerm{511, r, r ^ (32 + 16 * k), 0, 1.0, 0.0});
+  std::vector<uint32_t> low;
+  std::vector<uint64_t> list_1;
+  std::vector<int64_t> row_of(1024, -1);
+  for (uint32_t ia = 0; ia < 512; ia++) {
+    low.push_back(ia);
+    list_1.push_back(ia);
+    row_of[ia] = ia;
+  }
+  check(terms, 9, {1, 0}, {SectorBlock{0, 0, 0, 512}}, low, list_1, row_of);
+}
+
+int main(int argc, char **argv) {
+  if (argc == 2 && std::string(argv[1]) == "crowded") {
+    crowded();
+    printf("\n");
+    return 0;
+  }
+  Model m;
+  std::string err;
+  if (argc < 2 || read_expert(argv[1], &m, &err) != 0) fail(err.c_str());
+  const int lo_bits = (m.nbits + 1) / 2, hi_bits = m.nbits - lo_bits;
+  const uint64_t lo_mask = (1ull << lo_bits) - 1, even = 0x5555555555555555ull;
+  auto in_sector = [&](uint64_t c) {
+    if (m.calc_model == kHubbard)
+      return __builtin_popcountll(c & even) == m.nup && __builtin_popcountll(c & ~even) == m.ndown;
+    return __builtin_popcountll(c) == m.ne;
+  };
+  // HPhi's rows: by upper half, then lower half
+  std::vector<uint64_t> list_1;
+  std::vector<uint32_t> l22(1ull << hi_bits, 0), low;
+  std::vector<SectorBlock> blk;
+  std::map<std::vector<uint32_t>, uint32_t> cls;
+  std::vector<int64_t> row_of(1ull << m.nbits, -1);
+  for (uint64_t ib = 0; ib < (1ull << hi_bits); ib++) {
+    std::vector<uint32_t> mine;
+    const uint32_t row0 = (uint32_t)list_1.size();
+    for (uint64_t ia = 0; ia <= lo_mask; ia++)
+      if (in_sector(ib << lo_bits | ia)) {
+        mine.push_back((uint32_t)ia);
+        row_of[ib << lo_bits | ia] = (int64_t)list_1.size();
+        list_1.push_back(ib << lo_bits | ia);
+      }
+    if (mine.empty()) continue;
+    l22[ib] = row0 + 1;
+    const auto it = cls.emplace(mine, (uint32_t)low.size());
+    if (it.second) low.insert(low.end(), mine.begin(), mine.end());
+    blk.push_back(SectorBlock{(uint32_t)ib, row0, it.first->second, (uint32_t)mine.size()});
+  }
+  check(m.offdiag, lo_bits, l22, blk, low, list_1, row_of);
   printf("\n");
   return 0;
 }

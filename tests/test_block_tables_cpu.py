@@ -83,3 +83,9 @@ def test_block_tables(name, checker, tmp_path):
     assert r.returncode == 0, r.stdout + r.stderr
     if not name.startswith("random"):
         assert "shape" in r.stdout  # the plan applies
+
+
+def test_crowded_bank(checker):
+    """More entries on one bank pair than a packed slot count holds: the plan must not lose any."""
+    r = subprocess.run([checker, "crowded"], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
