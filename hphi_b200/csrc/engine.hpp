@@ -149,6 +149,14 @@ void sector_free(Sector *s);
 int hv_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
               const LanczosTail *lt = nullptr);
 
+// Complex vectors come at multiples of 8 bytes, the type's alignment; kernels that move whole
+// elements need multiples of 16, and a vector at another address takes the kernel that does not.
+inline bool whole_elements(VecType vt, const void *v) { return vt == kReal64 || (uintptr_t)v % 16 == 0; }
+
+// The kernels of an H*v in HPhi's row order from the vector v1.
+enum HvRoute : int { kRouteGeneral = 0, kRouteBlock, kRouteRowBlock, kRouteTile };
+HvRoute hv_route(const Sector *s, VecType vt, const void *d_v1);
+
 // Native vector order: HPhi order unless a specialised plan defines its own (then an
 // exact per-block permutation of it).  hv_native runs the fastest kernel on native
 // vectors; to_native / from_native convert (they copy when the orders coincide).

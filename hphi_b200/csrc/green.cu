@@ -261,7 +261,8 @@ struct GreenSpace {
 template <typename T>
 int green_batches(Sector *s, const T *d_v, const std::vector<GreenTerm> &nz, std::vector<double> *out) {
   constexpr int W = GreenWidth<T>::w, NB = kGreenAcc / W;
-  const bool blocks = !s->gc && s->lo_bits <= 31 && s->hi_bits <= 31;
+  // the block kernels read whole complex elements; a vector at another address takes the row kernel
+  const bool blocks = !s->gc && s->lo_bits <= 31 && s->hi_bits <= 31 && whole_elements(W == 2 ? kComplex128 : kReal64, d_v);
   std::string err;
   if (blocks && sector_pieces(s, &err) != 0) {
     set_error("Green's functions: " + err);

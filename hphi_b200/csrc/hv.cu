@@ -13,6 +13,8 @@
 // conj(v1[r]) * (H v1)[r].
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "device_util.cuh"
 #include "engine.hpp"
 #include "hv_blocks.hpp"
@@ -251,15 +253,26 @@ int hv_block_native(Sector *s, VecType vt, int nb, int64_t stride, const void *d
   return 0;
 }
 
+HvRoute hv_route(const Sector *s, VecType vt, const void *d_v1) {
+  const bool whole = whole_elements(vt, d_v1);
+  if (whole && gc_applies(s, vt)) return kRouteTile;
+  if (rb_applies(s, vt) && (whole || rb_own_rows(s, vt))) return kRouteRowBlock;
+  if (whole && bk_applies(s)) return kRouteBlock;
+  return kRouteGeneral;
+}
+
 int hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
                       double *d_part, const LanczosTail *lt) {
   if (vt == kReal64 && s->model.complex_terms) {
     set_error("H has complex coefficients: real vectors are not allowed");
     return -1;
   }
-  if (gc_applies(s, vt)) return gc_hv_launch(s, vt, d_v1, d_v0, d_coef, d_out, d_part, lt);
-  if (rb_applies(s, vt)) return rb_hv_launch_scratch(s, vt, d_v1, d_v0, d_coef, d_out, d_part, lt);
-  if (bk_applies(s)) return bk_hv_launch(s, vt, d_v1, d_v0, d_coef, d_out, d_part, lt);
+  switch (hv_route(s, vt, d_v1)) {
+    case kRouteTile: return gc_hv_launch(s, vt, d_v1, d_v0, d_coef, d_out, d_part, lt);
+    case kRouteRowBlock: return rb_hv_launch_scratch(s, vt, d_v1, d_v0, d_coef, d_out, d_part, lt);
+    case kRouteBlock: return bk_hv_launch(s, vt, d_v1, d_v0, d_coef, d_out, d_part, lt);
+    case kRouteGeneral: break;
+  }
   const SumOut so = sum_out(d_part, 0, s->red_blocks, s->d_done, d_out, 0, lt);
   if (vt == kReal64) {
     if (s->gc) launch_general<double, true>(s, (const double *)d_v1, (double *)d_v0, d_coef, so);
@@ -278,17 +291,19 @@ int hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const
 
 int hv_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
               const LanczosTail *lt) {
-  double *part = gc_applies(s, vt) ? gc_part(s) : rb_applies(s, vt) ? rb_part(s) : s->d_red;
+  const HvRoute route = hv_route(s, vt, d_v1);
+  double *part = route == kRouteTile ? gc_part(s) : route == kRouteRowBlock ? rb_part(s) : s->d_red;
   return hv_launch_scratch(s, vt, d_v1, d_v0, d_coef, d_out, part, lt);
 }
 
 size_t hv_scratch_doubles(const Sector *s, VecType vt) {
   if (s->prod) return prod_scratch_doubles(s, vt);
   if (s->hub) return hub_scratch_doubles(s);
-  if (gc_applies(s, vt)) return gc_scratch_doubles(s, vt);
-  if (rb_applies(s, vt)) return rb_scratch_doubles(s);
-  if (bk_applies(s)) return bk_scratch_doubles(s);
-  return 2 * (size_t)s->red_blocks;
+  size_t n = 2 * (size_t)s->red_blocks;  // the general kernel, which an unaligned vector takes
+  if (gc_applies(s, vt)) n = std::max(n, gc_scratch_doubles(s, vt));
+  if (rb_applies(s, vt)) n = std::max(n, rb_scratch_doubles(s));
+  if (bk_applies(s)) n = std::max(n, bk_scratch_doubles(s));
+  return n;
 }
 
 int hv_native_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,

@@ -747,7 +747,8 @@ __global__ void __launch_bounds__(kPermThreads) prod_from_native_kernel(int N, i
 // Either direction, a thread per HPhi row: sectors whose HPhi blocks are shorter than a warp
 // (kPermShort), where the kernels above leave most of their lanes idle (15 sites with 3 + 3
 // electrons, complex, blocks of 21 rows: a whole hphi_mltply_device 114 -> 73 us).
-template <typename T, bool TO_NATIVE>
+// Also any vector whose complex elements are not at multiples of 16 bytes (WHOLE false).
+template <typename T, bool TO_NATIVE, bool WHOLE>
 __global__ void __launch_bounds__(kPermThreads) prod_permute_rows_kernel(int64_t dim, int Dc,
                                                                          const uint64_t *__restrict__ list_1,
                                                                          const uint16_t *__restrict__ rank,
@@ -757,8 +758,11 @@ __global__ void __launch_bounds__(kPermThreads) prod_permute_rows_kernel(int64_t
     const uint32_t c = (uint32_t)__ldg(list_1 + r);  // 2 N <= 32 bits
     const uint32_t u = compress_even(c), d = compress_even(c >> 1);
     const int64_t pos = (int64_t)__ldg(rank + u) * Dc + __ldg(pos_dn + d);
-    if (TO_NATIVE) out[pos] = signed_v<T>(ldg_v<T>(in + r), species_parity16(u, d));
-    else out[r] = signed_v<T>(ldg_v<T>(in + pos), species_parity16(u, d));
+    const T *from = in + (TO_NATIVE ? r : pos);
+    T v;
+    if constexpr (WHOLE) v = ldg_v<T>(from);
+    else v = *from;
+    out[TO_NATIVE ? pos : r] = signed_v<T>(v, species_parity16(u, d));
   }
 }
 
@@ -1522,6 +1526,13 @@ int prod_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const doubl
     set_error("H has complex coefficients: real vectors are not allowed");
     return -1;
   }
+  if (!whole_elements(vt, d_v1) || !whole_elements(vt, d_v0)) {
+    if (p->args.wu > 0) {  // the source rows of up hops are read in whole elements
+      set_error("complex vectors in native order must start at a multiple of 16 bytes");
+      return -1;
+    }
+    one_pass = true;
+  }
   if (p->two_pass && !one_pass) {
     two_pass_launch(s, p, vt != kReal64, (const double *)d_v1, (double *)d_v0, d_coef, d_out, d_part, lt);
     return cuda_ok(cudaGetLastError(), "launch");
@@ -1540,7 +1551,8 @@ int prod_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const doubl
 
 int prod_hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
                            double *d_part, int *d_counter) {
-  if (!s->prod->two_pass && cudaMemsetAsync(d_counter, 0, 2 * sizeof(int), s->stream) != cudaSuccess) {
+  const bool one_pass = !s->prod->two_pass || !whole_elements(vt, d_v1) || !whole_elements(vt, d_v0);
+  if (one_pass && cudaMemsetAsync(d_counter, 0, 2 * sizeof(int), s->stream) != cudaSuccess) {
     set_error("product kernel: clearing the row counter failed");
     return -1;
   }
@@ -1621,17 +1633,20 @@ int prod_te_launch(Sector *s, const ProdPlan *te, int index, const void *d_v1, v
 int prod_permute(Sector *s, VecType vt, const void *in, void *out, bool to_native) {
   const ProdPlan *p = s->prod;
   const ProdArgs &a = p->args;
-  if (s->dim < (int64_t)kPermShort * p->nperm) {
+  const bool whole = whole_elements(vt, in);
+  if (s->dim < (int64_t)kPermShort * p->nperm || !whole) {
     const unsigned nb = (unsigned)std::min<int64_t>((s->dim + kPermThreads - 1) / kPermThreads, (int64_t)s->num_sms * 16);
-    auto rows = [&](auto *x, auto *y) {
+    auto rows = [&](auto *x, auto *y, auto w) {
       using T = std::remove_reference_t<decltype(*y)>;
+      constexpr bool W = decltype(w)::value;
       if (to_native)
-        prod_permute_rows_kernel<T, true><<<nb, kPermThreads, 0, s->stream>>>(s->dim, a.Dc, s->d_list_1, a.rank, a.pos_dn, x, y);
+        prod_permute_rows_kernel<T, true, W><<<nb, kPermThreads, 0, s->stream>>>(s->dim, a.Dc, s->d_list_1, a.rank, a.pos_dn, x, y);
       else
-        prod_permute_rows_kernel<T, false><<<nb, kPermThreads, 0, s->stream>>>(s->dim, a.Dc, s->d_list_1, a.rank, a.pos_dn, x, y);
+        prod_permute_rows_kernel<T, false, W><<<nb, kPermThreads, 0, s->stream>>>(s->dim, a.Dc, s->d_list_1, a.rank, a.pos_dn, x, y);
     };
-    if (vt == kReal64) rows((const double *)in, (double *)out);
-    else rows((const cplx *)in, (cplx *)out);
+    if (vt == kReal64) rows((const double *)in, (double *)out, std::true_type{});
+    else if (whole) rows((const cplx *)in, (cplx *)out, std::true_type{});
+    else rows((const cplx *)in, (cplx *)out, std::false_type{});
     return cuda_ok(cudaGetLastError(), "permute");
   }
   if (to_native) {

@@ -429,26 +429,24 @@ int rb_plan_build(Sector *s, std::string *err) {
   return 0;
 }
 
-bool rb_applies(const Sector *s, VecType vt) {
-  return s->rb && (s->rb->grid_row[vt == kReal64 ? 0 : 1] > 0 || bk_row_pass(s));
-}
-
-static int rb_row_grid(const Sector *s, VecType vt) {
-  return bk_row_pass(s) ? bk_grid(s, vt) : s->rb->grid_row[vt == kReal64 ? 0 : 1];
-}
+bool rb_own_rows(const Sector *s, VecType vt) { return s->rb && s->rb->grid_row[vt == kReal64 ? 0 : 1] > 0; }
+bool rb_applies(const Sector *s, VecType vt) { return s->rb && (rb_own_rows(s, vt) || bk_row_pass(s)); }
 
 size_t rb_scratch_doubles(const Sector *s) {
-  return 2 * (size_t)(std::max(rb_row_grid(s, kReal64), rb_row_grid(s, kComplex128)) + s->rb->grid_col);
+  int rows = std::max(s->rb->grid_row[0], s->rb->grid_row[1]);
+  if (bk_row_pass(s)) rows = std::max({rows, bk_grid(s, kReal64), bk_grid(s, kComplex128)});
+  return 2 * (size_t)(rows + s->rb->grid_col);
 }
 
 int rb_hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
                          double *d_part, const LanczosTail *lt) {
   RowBlockPlan *p = s->rb;
   const int iv = (vt == kReal64) ? 0 : 1;
-  const int gr = rb_row_grid(s, vt), gcol = p->grid_col;
+  const bool block_rows = bk_row_pass(s) && whole_elements(vt, d_v1);
+  const int gr = block_rows ? bk_grid(s, vt) : p->grid_row[iv], gcol = p->grid_col;
   const SplitView sv = split_view(s->split);
   const SumOut so = sum_out(d_part, gr, gr + gcol, s->d_done, d_out, 0, lt);
-  if (bk_row_pass(s)) {
+  if (block_rows) {
     if (bk_hv_launch(s, vt, d_v1, d_v0, d_coef, nullptr, d_part, nullptr) != 0) return -1;
     if (vt == kReal64)
       rb_col_kernel<double, false, 4><<<gcol, kColThreads, 0, s->stream>>>(p->args, p->cl_task[0], sv,

@@ -12,6 +12,8 @@ struct RowBlockPlan;
 int rb_plan_build(Sector *s, std::string *err);
 void rb_plan_free(RowBlockPlan *p);
 // True when vectors of type vt take the row-block kernels (the block fits in shared memory).
+// The plan has row kernels of its own for these vectors (the block kernel takes their place otherwise).
+bool rb_own_rows(const Sector *s, VecType vt);
 bool rb_applies(const Sector *s, VecType vt);
 // H*v in HPhi's order (as hv_launch); the _scratch form takes rb_scratch_doubles(s) doubles
 // of partial sums from the caller.

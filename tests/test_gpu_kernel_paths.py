@@ -300,3 +300,79 @@ def test_time_evolution_product_layout(static, values, tmp_path):
     assert np.max(np.abs(sa - sg)) <= 1e-12 * np.max(np.abs(sg))
     for x, y in zip(fa, fg):
         np.testing.assert_allclose(x, y, rtol=0, atol=2e-10)
+
+
+def _odd_copy(x):
+    """x in memory that starts 8 bytes past a multiple of 16, as complex128 allows; (data pointer, view
+    of the doubles, the buffer)."""
+    buf = torch.zeros(2 * x.numel() + 2, dtype=torch.float64, device="cuda")
+    at = 1 if buf.data_ptr() % 16 == 0 else 0
+    view = buf[at:at + 2 * x.numel()]
+    view.copy_(torch.view_as_real(x).reshape(-1))
+    return view.data_ptr(), view, buf
+
+
+ODD = {
+    "block": (lambda: expert.heisenberg(16, expert.chain_bonds(16)), None),
+    "row_block": (lambda: expert.heisenberg(16, expert.chain_bonds(16)), "rowblock"),
+    "tiles": (lambda: _spin_gc(20, "real"), None),
+    "product": (lambda: _hubbard(10, 5, 4), None),
+    "product_no_up_hops": (lambda: _hubbard(6, 6, 3), None),
+    "product_short_blocks": (lambda: _hubbard(9, 2, 2), None),
+}
+
+
+@pytest.mark.parametrize("name", list(ODD))
+def test_complex_vectors_at_8_byte_boundaries(name, tmp_path, monkeypatch):
+    """Every call that takes device vectors, with complex vectors at 8 mod 16 bytes (the type's own
+    alignment): the results of the same call on vectors at 16 (bound of _compare; copies bit for bit)."""
+    make, kernel = ODD[name]
+    if kernel:
+        monkeypatch.setenv("HPHI_B200_KERNEL", kernel)
+    C = hphi_b200.COMPLEX128
+    with hphi_b200.Hamiltonian(make().write(str(tmp_path))) as H:
+        g = torch.Generator(device="cuda").manual_seed(3)
+        v1, w = (torch.randn(H.dim, dtype=torch.complex128, device="cuda", generator=g) for _ in range(2))
+        p1, _, keep = _odd_copy(v1)
+        coef = torch.tensor([0.5, -2.0], dtype=torch.float64, device="cuda")
+        pr = torch.zeros(2, 2, dtype=torch.float64, device="cuda")
+
+        def close(view, ref, pa, pb):
+            big = ref.abs().max().item()
+            assert (torch.view_as_complex(view.clone().reshape(-1, 2)) - ref).abs().max().item() <= 1e-13 * big
+            n = torch.linalg.vector_norm(v1).item() * torch.linalg.vector_norm(ref).item()
+            assert abs(pa - pb) <= 1e-13 * n
+
+        ref = w.clone()
+        p0, o0, keep0 = _odd_copy(w)
+        torch.cuda.synchronize()
+        a = H.mltply_device(ref.data_ptr(), v1.data_ptr(), C, acc=0.5, scale=-2.0)
+        b = H.mltply_device(p0, p1, C, acc=0.5, scale=-2.0)
+        close(o0, ref, a, b)
+        for native in (H.to_native, H.from_native):
+            x = torch.zeros_like(v1)
+            px, ox, keepx = _odd_copy(x)
+            torch.cuda.synchronize()
+            native(v1.data_ptr(), x.data_ptr(), C)
+            native(p1, px, C)
+            assert torch.equal(torch.view_as_real(x).reshape(-1), ox)
+        # vectors in native order
+        ref = w.clone()
+        p0, o0, keep0 = _odd_copy(w)
+        pn, on, keepn = _odd_copy(w)
+        torch.cuda.synchronize()
+        H.mltply_device_async(ref.data_ptr(), v1.data_ptr(), C, coef.data_ptr(), pr[0].data_ptr())
+        if name.startswith("product") and name != "product_no_up_hops":   # refused, not read past the alignment
+            for call in (lambda: H.mltply_device_async(p0, p1, C, coef.data_ptr(), pr[1].data_ptr()),
+                         lambda: H.mltply_device_noalloc(pn, p1, C, acc=0.5, scale=-2.0)):
+                with pytest.raises(hphi_b200.HPhiError, match="multiple of 16"):
+                    call()
+        else:
+            H.mltply_device_async(p0, p1, C, coef.data_ptr(), pr[1].data_ptr())
+            H.synchronize()
+            close(o0, ref, complex(*pr[0].tolist()), complex(*pr[1].tolist()))
+            close(on, ref, complex(*pr[0].tolist()), H.mltply_device_noalloc(pn, p1, C, acc=0.5, scale=-2.0))
+        rows = [(0, 0, 0, 0), (0, 0, 1, 0), (1, 0, 0, 0)] if H.info["calc_model"] in (0, 3) else [(0, 0, 0, 0), (1, 1, 1, 1)]
+        a = H.expec_green_device(v1.data_ptr(), C, rows, 1)
+        b = H.expec_green_device(p1, C, rows, 1)
+        assert np.max(np.abs(a - b)) <= 1e-13 * np.sum(np.abs(v1.cpu().numpy()) ** 2)
