@@ -83,6 +83,28 @@ __device__ __forceinline__ cplx gc_lds(const cplx *p) {
   return cplx{z.x, z.y};
 }
 
+// y of one element (position q of the tile) without the patterns that no term matches.  The kernel
+// multiplies their sources by 0 (passing them by in its sweep took the 24-site Kitaev-Heisenberg
+// honeycomb, complex, from 769 to 932 us; this way it is 782), which must not spread an infinity to rows that H does not
+// couple to it: a non-finite y shows in the products with x that a sweep sums anyway, and the sweep's
+// elements are then left out there and worked out here.
+template <typename T, bool IM>
+__device__ __forceinline__ T gc_element(const GcPass &ps, const T *x, uint64_t base, int q, double diag) {
+  const int tid = q % kGcThreads, qe = q / kGcThreads;
+  T y = ps.first ? VT<T>::scale(diag, x[q]) : VT<T>::zero();
+#pragma unroll 1
+  for (int k = 0; k < ps.ngroup; k++) {
+    const GcGroup &g = ps.g[k];
+    const int c = ((q >> g.i) & 1) | (((q >> g.j) & 1) << 1);
+    const uint32_t sg = (uint32_t)__popc((uint32_t)tid & g.sm) + (uint32_t)__popcll(base & g.smo) + (g.sgn >> qe);
+    const double re = g.re[c], im = IM ? ps.im[k][c] : 0.0;
+    const T z = x[(tid ^ (int)g.ft) + ((qe ^ g.fe) * kGcThreads)];
+    if (re != 0.0) gc_fma(y, sg & 1u ? -re : re, z);
+    if (im != 0.0) gc_fma_i(y, sg & 1u ? -im : im, z);
+  }
+  return y;
+}
+
 // IM: some coefficient has an imaginary part (complex vectors only).
 template <typename T, bool IM>
 __global__ void __launch_bounds__(kGcThreads, 2) gc_tile_kernel(const __grid_constant__ GcPass ps, int64_t ntile,
@@ -125,6 +147,7 @@ __global__ void __launch_bounds__(kGcThreads, 2) gc_tile_kernel(const __grid_con
     asm volatile("cp.async.commit_group;\n" ::: "memory");
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
+    uint32_t again = 0;  // elements whose products with x are not finite: gc_element
 #pragma unroll
     for (int m0 = 0; m0 < M; m0 += H) {
       T y[H], old[H];
@@ -182,14 +205,34 @@ __global__ void __launch_bounds__(kGcThreads, 2) gc_tile_kernel(const __grid_con
         part(g.re, std::false_type{});
         if (IM) part(ps.im[k], std::true_type{});
       }
+      double d[2] = {0.0, 0.0};
 #pragma unroll
       for (int m = 0; m < H; m++) {
         const T xq = gc_lds(x + tid + (m0 + m) * kGcThreads);
-        pr[0] += VT<T>::conj_mul_re(xq, y[m]);
-        pr[1] += VT<T>::conj_mul_im(xq, y[m]);
+        d[0] += VT<T>::conj_mul_re(xq, y[m]);
+        d[1] += VT<T>::conj_mul_im(xq, y[m]);
+      }
+      if (!isfinite(d[0])) {
+        again |= ((1u << H) - 1) << m0;
+        continue;
+      }
+      pr[0] += d[0];
+      pr[1] += d[1];
+#pragma unroll
+      for (int m = 0; m < H; m++) {
         const T ys = VT<T>::scale(scale, y[m]);
         v0[base | row[m]] = (acc == 0.0) ? ys : VT<T>::add(VT<T>::scale(acc, old[m]), ys);
       }
+    }
+#pragma unroll 1
+    for (; again; again &= again - 1) {
+      const int q = tid + (__ffs((int)again) - 1) * kGcThreads;
+      const int64_t r = (int64_t)(base | dep(q / kGcThreads));
+      const T xq = gc_lds(x + q), y = gc_element<T, IM>(ps, x, base, q, ps.first ? __ldg(diag + r) : 0.0);
+      pr[0] += VT<T>::conj_mul_re(xq, y);
+      pr[1] += VT<T>::conj_mul_im(xq, y);
+      const T ys = VT<T>::scale(scale, y);
+      v0[r] = (acc == 0.0) ? ys : VT<T>::add(VT<T>::scale(acc, v0[r]), ys);
     }
   }
   if (ps.last) {

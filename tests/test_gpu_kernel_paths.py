@@ -376,3 +376,48 @@ def test_complex_vectors_at_8_byte_boundaries(name, tmp_path, monkeypatch):
         a = H.expec_green_device(v1.data_ptr(), C, rows, 1)
         b = H.expec_green_device(p1, C, rows, 1)
         assert np.max(np.abs(a - b)) <= 1e-13 * np.sum(np.abs(v1.cpu().numpy()) ** 2)
+
+
+NONFINITE = {
+    "tiles": lambda: _spin_gc(20, "real"),
+    "tiles_kitaev": lambda: expert.kitaev_heisenberg(5, 2, -1.0, 0.3),
+    "tiles_signs": lambda: _hubbard_gc(10),
+    "block": lambda: expert.heisenberg(16, expert.chain_bonds(16)),
+    "block_complex": lambda: _dm_chain(14, 0),
+    "product": lambda: _hubbard(10, 5, 4),
+    "product_complex": lambda: _hubbard(10, 5, 4, phases=3),
+}
+
+
+@pytest.mark.parametrize("vt", [hphi_b200.REAL64, hphi_b200.COMPLEX128])
+@pytest.mark.parametrize("name", list(NONFINITE))
+def test_non_finite_elements_reach_their_neighbours_only(name, vt, tmp_path):
+    """An infinity in v1 changes the rows that H couples to it and no other: elsewhere H v1 is that of
+    the vector with a zero in its place, exactly (the terms of those rows are the same)."""
+    if vt == hphi_b200.REAL64 and name.endswith("complex"):
+        pytest.skip("complex H")
+    dt = torch.float64 if vt == hphi_b200.REAL64 else torch.complex128
+    path = NONFINITE[name]().write(str(tmp_path))
+    with _open(path) as H, _open(path, general=True) as Hg:
+        v = torch.randn(H.dim, dtype=dt, device="cuda", generator=torch.Generator(device="cuda").manual_seed(11))
+        at = H.dim // 3
+        probe = torch.zeros_like(v)
+        probe[at] = 1.0
+        out = {}
+        for key, vec, h in (("near", probe, Hg), ("zero", v.clone(), H), ("inf", v.clone(), H)):
+            if key != "near":
+                vec[at] = 0.0 if key == "zero" else float("inf")
+            out[key] = torch.zeros_like(v)
+            torch.cuda.synchronize()
+            coef = torch.tensor([0.0, 1.0], dtype=torch.float64, device="cuda")
+            pr = torch.zeros(2, dtype=torch.float64, device="cuda")
+            a, b = torch.zeros_like(v), torch.zeros_like(v)
+            torch.cuda.synchronize()
+            h.to_native(vec.data_ptr(), a.data_ptr(), vt)
+            h.mltply_device_async(b.data_ptr(), a.data_ptr(), vt, coef.data_ptr(), pr.data_ptr())
+            h.from_native(b.data_ptr(), out[key].data_ptr(), vt)
+        far = out["near"] == 0
+        far[at] = False
+        assert 0 < int((~far).sum()) < H.dim
+        assert torch.equal(out["inf"][far], out["zero"][far])
+        assert not torch.isfinite(torch.view_as_real(out["inf"]) if dt == torch.complex128 else out["inf"]).all()
