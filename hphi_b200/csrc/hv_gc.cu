@@ -37,6 +37,12 @@ namespace {
 constexpr int kTidBits = 9, kGcThreads = 1 << kTidBits;
 constexpr int kGcPasses = 12;     // more passes than this cost more than the general kernels
 constexpr int kGcGroups = 24;     // groups of one pass
+// Smallest sectors, in bits.  A tile is a CTA's task, and below 64 to 128 of them too few of the 148
+// SMs work; real vectors with fermion signs have the longest sweep per byte and wait for the sector to
+// leave L2.  H*v in us, tiles against the kernel without them (the general one, the row-block
+// plan at 24 bits): chains with a field, complex 18 bits 33 / 31, 19: 35 / 53; real 19: 44 / 30, 20: 46 /
+// 52; Hubbard rings, complex 18: 30 / 25, 20: 48 / 68; real 20: 43 / 38, 22: 143 / 130, 24: 512 / 620.
+constexpr int kGcBitsComplex = 19, kGcBitsReal = 20, kGcBitsSigned = 24;
 // 64 KB of shared memory per tile, two CTAs per SM: one stages while the other computes
 template <typename T> struct GcTile;
 template <> struct GcTile<double> { static constexpr int K = 13, low = 3; };
@@ -455,15 +461,18 @@ int build_passes(Sector *s, GcPlan *p, const std::vector<Raw> &raw, int vt, std:
 int gc_plan_build(Sector *s, std::string *err) {
   s->gcp = nullptr;
   const Model &m = s->model;
-  // rows within a tile are 32-bit numbers; below 2^18 rows there are too few tiles for the SMs
-  if (!s->gc || m.general_spin || m.nbits > 32 || m.nbits < 18) return 0;
+  // rows within a tile are 32-bit numbers
+  if (!s->gc || m.general_spin || m.nbits > 32 || m.nbits < kGcBitsComplex) return 0;
   std::vector<Raw> raw;
   for (const BitTerm &t : m.offdiag)
     if (!merge_term(t, &raw)) return 0;
   GcPlan *p = new GcPlan();
   for (const Raw &r : raw)
     for (double x : r.im) p->im = p->im || x != 0.0;
-  if ((!m.complex_terms && build_passes<double>(s, p, raw, 0, err) != 0) || build_passes<cplx>(s, p, raw, 1, err) != 0) {
+  bool signs = false;
+  for (const Raw &r : raw) signs = signs || r.sm != 0;
+  const bool real = !m.complex_terms && m.nbits >= (signs ? kGcBitsSigned : kGcBitsReal);
+  if ((real && build_passes<double>(s, p, raw, 0, err) != 0) || build_passes<cplx>(s, p, raw, 1, err) != 0) {
     gc_plan_free(p);
     return -1;
   }

@@ -723,7 +723,7 @@ int sector_build(const Model &m, int device, Sector **out, std::string *err, boo
   // Row-block plan (spin sectors): from 2^24 rows up, where the vectors no longer stay in L2
   // and the general kernel's scattered gathers go to memory (below that the general kernel is
   // faster); HPHI_B200_KERNEL=rowblock builds it at any size.
-  // The tile plan takes the grand-canonical sectors from 2^18 rows.
+  // The tile plan takes the grand-canonical sectors from the sizes of hv_gc.cu.
   if (specialise && kname != "general" && kname != "rowblock") {
     if (gc_plan_build(s, err) != 0) return -1;
   }
