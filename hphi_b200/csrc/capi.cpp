@@ -565,14 +565,14 @@ int hphi_tpq_vectors(hphi_handle *h, const double *const *v_init, const char *ou
     return 0;
   };
   // The samples of the reference's loop (src/CalcByTPQ.c:76) run in blocks of up to
-  // kHvBlockMax in lockstep, sharing each H application (one block H*V), where the sector's
-  // H*v is the general kernel; a sample continued from a stored state runs alone.
+  // kHvBlockMax in lockstep, sharing each H application (one block H*V), where tpq_lockstep says
+  // so; a sample continued from a stored state runs alone.
   // HPHI_B200_TPQ_BLOCK: 0 runs the samples one after another, N in 2..8 caps the block size
   // (default 8).
   const char *blk_env = std::getenv("HPHI_B200_TPQ_BLOCK");
   int block_cap = kHvBlockMax;
   if (blk_env && *blk_env) block_cap = std::max(0, std::min(kHvBlockMax, std::atoi(blk_env)));
-  const bool block_ok = hv_block_applies(s, vt) && block_cap > 1;
+  const bool lockstep = tpq_lockstep(s, vt), block_ok = lockstep && block_cap > 1;
   const int block_max = block_ok ? block_cap : 1;
   std::vector<std::vector<double>> starts;
   std::vector<int> pending;
@@ -581,7 +581,7 @@ int hphi_tpq_vectors(hphi_handle *h, const double *const *v_init, const char *ou
     std::vector<const double *> hv;
     for (size_t b = 0; b < pending.size(); b++) hv.push_back(starts[b].empty() ? v_init[pending[b]] : starts[b].data());
     std::vector<TpqResult> rr;
-    if (tpq_run_samples(s, vt, hv, pending, out, &rr, opt, hv_block_applies(s, vt)) != 0) return -1;
+    if (tpq_run_samples(s, vt, hv, pending, out, &rr, opt, lockstep) != 0) return -1;
     for (size_t b = 0; b < pending.size(); b++)
       if (opt.keep_vector && save(pending[b], rr[b]) != 0) return -1;
     r = std::move(rr.back());

@@ -866,7 +866,7 @@ int write_lanczos_outputs(const Sector &s, const LanczosResult &r, const std::st
 int tpq_run(Sector *s, VecType vt, const double *h_init, int rand_i, const std::string &outdir, TpqResult *res,
             const TpqOptions &opt) {
   std::vector<TpqResult> r(1);
-  const int rc = tpq_run_samples(s, vt, {h_init}, {rand_i}, outdir, &r, opt, hv_block_applies(s, vt));
+  const int rc = tpq_run_samples(s, vt, {h_init}, {rand_i}, outdir, &r, opt, tpq_lockstep(s, vt));
   *res = std::move(r[0]);
   return rc;
 }
@@ -975,7 +975,7 @@ int tpq_run_samples(Sector *s, VecType vt, const std::vector<const double *> &h_
       RET(cuda_ok(cudaMemcpyAsync(slot(b) + 4, coef, sizeof(coef), cudaMemcpyHostToDevice, s->stream), "coef"));
     }
     RET(apply_h(V.p, H.p, 4));
-    if (hv_block_applies(s, vt)) {
+    if (block) {
       RET(vec_tpq_energy(s, vt, nb, V.p, H.p, slot(0), kSlots, (double *)PART.p));
     } else {
       for (int b = 0; b < nb; b++) RET(vec_norm2(s, vt, vec(H.p, b), slot(b) + 8));
@@ -996,7 +996,7 @@ int tpq_run_samples(Sector *s, VecType vt, const std::vector<const double *> &h_
         for (int k = 0; k < 6; k++) ob[b][k] = h[16 + k] * w2;
       }
       // without the block product the H*v's own <V|H V> (slots 6, 7) is unscaled
-      E[b] = hv_block_applies(s, vt) ? h[6] * sv[b] : h[6] * sv[b] * sv[b];
+      E[b] = block ? h[6] * sv[b] : h[6] * sv[b] * sv[b];
       var[b] = h[8];
     }
     swept = false;

@@ -165,6 +165,13 @@ bool has_native_order(const Sector *s);
 // without a row-block plan, hv_block_applies): v0_b = acc_b * v0_b + scale_b * H v1_b with
 // (acc_b, scale_b) at d_coef + b * cstride.
 bool hv_block_applies(const Sector *s, VecType vt);
+// The samples of a TPQ run take their H*v as block products (general kernel's arithmetic, shared
+// lookups) rather than one by one by the sector's own kernel: a sector's decision, whatever the
+// block size, so that a sample's results do not depend on it.  One sample alone has nothing to
+// share.  Tiles lose to sharing while the vectors stay in L2 (60 steps, real, ms: 20-site chain with a
+// field, 4 samples 32 by tiles and 22 in lockstep, 8: 66 and 39; 22 sites, 8: 171 and 120) and
+// win from 2^24 rows (24-site Kitaev-Heisenberg, 4 samples: 257 and 279 real, 353 and 444 complex).
+bool tpq_lockstep(const Sector *s, VecType vt);
 int hv_block_native(Sector *s, VecType vt, int nb, int64_t stride, const void *d_v1, void *d_v0,
                     const double *d_coef, int cstride);
 int hv_native(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,

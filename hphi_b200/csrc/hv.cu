@@ -229,7 +229,14 @@ void launch_block_n(Sector *s, int nb, int64_t stride, const T *v1, T *v0, const
 }  // namespace
 
 bool hv_block_applies(const Sector *s, VecType vt) {
-  return !s->prod && !s->hub && !rb_applies(s, vt) && !gc_applies(s, vt) && !(vt == kReal64 && s->model.complex_terms);
+  return !s->prod && !s->hub && !rb_applies(s, vt) && !(vt == kReal64 && s->model.complex_terms);
+}
+
+bool tpq_lockstep(const Sector *s, VecType vt) {
+  if (!hv_block_applies(s, vt)) return false;
+  const bool tiles = gc_applies(s, vt);
+  if (s->model.num_ave == 1 && (tiles || bk_applies(s))) return false;
+  return !tiles || s->dim < ((int64_t)1 << 24);
 }
 
 int hv_block_native(Sector *s, VecType vt, int nb, int64_t stride, const void *d_v1, void *d_v0,

@@ -53,3 +53,48 @@ def test_block_samples_equal_serial_samples(name, tmp_path, monkeypatch):
         assert files == sorted(os.listdir(outs[mode]))
         for f in files:
             assert (outs["0"] / f).read_text() == (outs[mode] / f).read_text(), (mode, f)
+
+
+def _larger(kind):
+    if kind == "chain14":
+        m = expert.heisenberg(14, expert.chain_bonds(14), calc_type="TPQ", lanczos_max=12, large_value=3.0)
+    else:   # a sector whose single H*v goes by tiles
+        m = expert.kitaev_heisenberg(5, 2, 1.0, 0.3, calc_type="TPQ", lanczos_max=12, large_value=3.0)
+    m.initial_vec_type = 1
+    return m
+
+
+@pytest.mark.parametrize("num_ave", [1, 3])
+@pytest.mark.parametrize("kind", ["chain14", "kitaev5x2"])
+def test_samples_of_planned_sectors(kind, num_ave, tmp_path, monkeypatch):
+    """Sectors with a plan for single products: the same files whatever the block size, the contiguous
+    start array (hphi_tpq) and one pointer per sample give the same numbers, and one sample alone and the
+    general kernel agree (bound: 12 steps of order 10 multiply rounding by at most 2 each; 1e-11 of L)."""
+    import ctypes
+
+    import numpy as np
+    m = _larger(kind)
+    m.num_ave = num_ave
+    path = m.write(str(tmp_path / "in"))
+    rng = np.random.default_rng(2)
+    runs = {}
+    for mode in ("0", "8", "contiguous", "general"):
+        monkeypatch.setenv("HPHI_B200_TPQ_BLOCK", mode if mode in "08" else "8")
+        if mode == "general":
+            monkeypatch.setenv("HPHI_B200_KERNEL", "general")
+        o = str(tmp_path / f"out{mode}")
+        with hphi_b200.Hamiltonian(path) as H:
+            if not runs:
+                starts = np.zeros((num_ave, H.dim + 1), dtype=np.complex128)
+                starts[:, 1:] = rng.standard_normal((num_ave, H.dim))
+            if mode == "contiguous":
+                e = np.zeros(H.info["lanczos_max"])
+                ptr = starts.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
+                out = e.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
+                assert hphi_b200.load_library().hphi_tpq(H.handle, ptr, os.fsencode(o), out, e.size) == 0
+            else:
+                e = H.calc_by_tpq(v_init=list(starts), output_dir=o)
+        runs[mode] = (e, {f: open(os.path.join(o, f)).read() for f in sorted(os.listdir(o))})
+    for mode in ("8", "contiguous"):
+        assert np.array_equal(runs[mode][0], runs["0"][0]) and runs[mode][1] == runs["0"][1]
+    assert np.max(np.abs(runs["general"][0] - runs["0"][0])) <= 1e-11 * 3.0 * m.nsite
