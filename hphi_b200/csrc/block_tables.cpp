@@ -2,9 +2,11 @@
 
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <map>
 
-#include "hv_product.hpp"
+#include "gather_table.hpp"
+#include "host_parallel.hpp"
 
 namespace hphi {
 
@@ -48,98 +50,55 @@ bool block_tables(const std::vector<BitTerm> &terms, int lo_bits, const std::vec
   // lower-half terms by coefficient up to sign
   struct LoTerm {
     const BitTerm *t;
-    int group;
     bool neg;
   };
-  std::vector<LoTerm> lo;
+  std::vector<std::vector<LoTerm>> lo;  // by group
   std::vector<double2> &cf = T.cf;
-  for (const BitTerm &t : terms) {
-    if (((t.cm | t.flip | t.sm) & ~lo_mask) != 0) continue;
-    int g = 0;
-    bool neg = false;
-    for (; g < (int)cf.size(); g++) {
-      if (t.re == cf[g].x && t.im == cf[g].y) break;
-      if (t.re == -cf[g].x && t.im == -cf[g].y) { neg = true; break; }
-    }
-    if (g == (int)cf.size()) {
-      if (g == kBkGroups) return false;
-      cf.push_back(make_double2(t.re, t.im));
-    }
-    lo.push_back(LoTerm{&t, g, neg});
-  }
-  std::vector<uint4> &gat = T.gat;
-  std::vector<uint2> &head = T.head;
-  const int ng = (int)cf.size();
-  for (size_t c = 0; c < cls.size(); c++) {
-    BkClass &k = cls[c];
-    std::vector<std::vector<std::vector<uint32_t>>> tab(ng, std::vector<std::vector<uint32_t>>(k.n));
-    for (int p = 0; p < k.n; p++) {
-      const uint32_t ia = low[k.uoff + p];
-      for (const LoTerm &t : lo) {
-        if ((ia & t.t->cm) != t.t->cv) continue;
-        const uint32_t src = ia ^ (uint32_t)t.t->flip;
-        if (cls_of[src] < 0) continue;  // list_2_1 == 0: outside the sector
-        if (cls_of[src] != (int)c) return false;
-        const bool neg = ((__builtin_popcountll((uint64_t)ia & t.t->sm) & 1) != 0) != t.neg;
-        tab[t.group][p].push_back((uint32_t)pos_of[src] | (neg ? 0x10000u : 0u));
-        if (tab[t.group][p].size() > 255) return false;
-      }
-    }
-    // one table per class: a warp's sets, group after group, at a fixed stride (with one set past
-    // the last, read ahead), so that the first set's address does not wait for the slot counts
-    const int nw = (k.n + 31) / 32;
-    std::vector<std::vector<uint32_t>> t(ng);
-    std::vector<std::vector<uint8_t>> ws(ng);
-    std::vector<int> gs(ng, 1);
-    k.sets = 1;
-    for (int g = 0; g < ng; g++)
-      if (!build_gather_table(tab[g], k.n, &t[g], &ws[g], &gs[g])) return false;
-    for (int w = 0; w < nw; w++) {
-      int n = 1;
-      for (int g = 0; g < ng; g++) n += (ws[g][w] + 7) / 8;
-      k.sets = std::max(k.sets, n);
-    }
-    k.gat = (int)gat.size();
-    k.head = (int)head.size();
-    gat.resize(gat.size() + (size_t)nw * k.sets * 32, make_uint4(0, 0, 0, 0));
-    for (int w = 0; w < nw; w++) {
-      size_t at = (size_t)k.gat + (size_t)w * k.sets * 32;
-      uint64_t cnt = 0;
-      for (int g = 0; g < ng; g++) {
-        cnt |= (uint64_t)ws[g][w] << (8 * g);
-        const uint32_t *src = &t[g][(size_t)w * gs[g] * 128];
-        for (int i = 0; i < (ws[g][w] + 7) / 8 * 32; i++, at++)
-          gat[at] = make_uint4(src[4 * i], src[4 * i + 1], src[4 * i + 2], src[4 * i + 3]);
-      }
-      head.push_back(make_uint2((uint32_t)cnt, (uint32_t)(cnt >> 32)));
-    }
-  }
-  // per block the upper-half and crossing terms that act on it; a crossing term's lower-half
-  // pattern (condition, flip, sign) is a table of source positions per class
+  // upper-half and crossing terms, in bits of the upper half; a crossing term's lower-half pattern
+  // (condition, flip, sign) is a table of source positions per class
   struct HiTerm {
-    const BitTerm *t;
+    uint32_t cm, cv, flip, sm;
     int pat;  // lower-half pattern, -1: upper-half term
+    double re, im;
   };
   std::vector<HiTerm> hi;
   std::vector<std::array<uint32_t, 4>> pats;
   for (const BitTerm &t : terms) {
-    if (((t.cm | t.flip | t.sm) & ~lo_mask) == 0) continue;  // lower half
-    HiTerm h{&t, -1};
-    if (((t.cm | t.flip | t.sm) & lo_mask) != 0) {
+    const uint64_t all = t.cm | t.flip | t.sm;
+    if ((all & ~lo_mask) == 0) {
+      size_t g = 0;
+      bool neg = false;
+      for (; g < cf.size(); g++) {
+        if (t.re == cf[g].x && t.im == cf[g].y) break;
+        if (t.re == -cf[g].x && t.im == -cf[g].y) { neg = true; break; }
+      }
+      if (g == cf.size()) {
+        if (g == (size_t)kBkGroups) return false;
+        cf.push_back(make_double2(t.re, t.im));
+        lo.emplace_back();
+      }
+      lo[g].push_back(LoTerm{&t, neg});
+      continue;
+    }
+    HiTerm h{(uint32_t)(t.cm >> lo_bits), (uint32_t)(t.cv >> lo_bits), (uint32_t)(t.flip >> lo_bits),
+             (uint32_t)(t.sm >> lo_bits), -1, t.re, t.im};
+    if ((all & lo_mask) != 0) {
       const std::array<uint32_t, 4> pt{(uint32_t)(t.cm & lo_mask), (uint32_t)(t.cv & lo_mask), (uint32_t)(t.flip & lo_mask),
                                        (uint32_t)(t.sm & lo_mask)};
       h.pat = (int)(std::find(pats.begin(), pats.end(), pt) - pats.begin());
       if (h.pat == (int)pats.size()) pats.push_back(pt);
+      if (pats.size() > 4 * (size_t)kBkCross) return false;
     }
     hi.push_back(h);
   }
-  if (pats.size() > 4 * (size_t)kBkCross) return false;
+  const size_t np = pats.size();
   std::vector<uint16_t> &tab = T.tab;
-  std::vector<uint32_t> tab_at(cls.size() * std::max<size_t>(1, pats.size()), 0);
+  std::vector<uint32_t> tab_at(cls.size() * std::max<size_t>(1, np), 0);
+  std::vector<int> tab_to(tab_at.size(), -1);  // the class the pattern leads to: one for all its positions
   for (size_t c = 0; c < cls.size(); c++)
-    for (size_t q = 0; q < pats.size(); q++) {
-      tab_at[c * pats.size() + q] = (uint32_t)tab.size();
-      int to = -1;  // the class the pattern leads to: one for all its positions
+    for (size_t q = 0; q < np; q++) {
+      tab_at[c * np + q] = (uint32_t)tab.size();
+      int &to = tab_to[c * np + q];
       for (int p = 0; p < cls[c].n; p++) {
         const uint32_t ia = low[cls[c].uoff + p], src = ia ^ pats[q][2];
         uint16_t v = (uint16_t)kBkNone;
@@ -151,6 +110,7 @@ bool block_tables(const std::vector<BitTerm> &terms, int lo_bits, const std::vec
         tab.push_back(v);
       }
     }
+  // per block the upper-half and crossing terms that act on it
   std::vector<int> class_of_block(l22.size(), -1);
   for (size_t c = 0; c < cls.size(); c++)
     for (int b = 0; b < cls[c].nblk; b++) class_of_block[b_ib[cls[c].boff + b]] = (int)c;
@@ -159,53 +119,150 @@ bool block_tables(const std::vector<BitTerm> &terms, int lo_bits, const std::vec
   std::vector<uint64_t> ib_sorted(b_ib.size());
   std::vector<BkRec> &rec = T.rec;
   std::vector<double> &rec_im = T.rec_im;
-  bool &im = T.im;
-  for (size_t c = 0; c < cls.size(); c++) {
-    std::vector<std::pair<uint64_t, int>> order;  // blocks of equal list lengths side by side
-    std::vector<std::vector<BkRec>> recs(cls[c].nblk);
-    std::vector<std::vector<double>> ims(cls[c].nblk);
-    std::vector<uint32_t> nhb(cls[c].nblk);
-    for (int b = 0; b < cls[c].nblk; b++) {
-      const uint64_t ib = b_ib[cls[c].boff + b], cfg = ib << lo_bits;
-      for (int cross = 0; cross < 2; cross++) {
-        for (const HiTerm &h : hi) {
-          if ((h.pat >= 0) != (cross == 1) || (two_pass && !cross)) continue;
-          if ((cfg & h.t->cm) != (h.t->cv & ~lo_mask)) continue;
-          const uint64_t to = (cfg ^ h.t->flip) >> lo_bits;
-          if (l22[to] == 0) continue;
-          const bool neg = __builtin_popcountll(cfg & h.t->sm) & 1;
-          if (cross == 0 && class_of_block[to] != (int)c) return false;  // a moved block keeps its lower halves
-          if (cross == 1) {  // the source positions are those of the class the pattern leads to
-            const uint32_t at = tab_at[c * pats.size() + h.pat];
-            int any = -1;
-            for (int p = 0; p < cls[c].n && any < 0; p++)
-              if ((tab[at + p] & 0x7FFFu) != kBkNone) any = cls_of[low[cls[c].uoff + p] ^ pats[h.pat][2]];
-            if (any < 0) continue;  // no row of the class matches
-            if (class_of_block[to] != any) return false;
-          }
-          recs[b].push_back(BkRec{l22[to] - 1u, cross ? tab_at[c * pats.size() + h.pat] : 0u, neg ? -h.t->re : h.t->re});
-          ims[b].push_back(neg ? -h.t->im : h.t->im);
-          im = im || h.t->im != 0.0;
-        }
-        if (cross == 0) nhb[b] = (uint32_t)recs[b].size();
+  for (const HiTerm &h : hi) T.im = T.im || (h.im != 0.0 && !(two_pass && h.pat < 0));
+  std::stable_sort(hi.begin(), hi.end(), [](const HiTerm &x, const HiTerm &y) { return (x.pat >= 0) < (y.pat >= 0); });
+  const size_t n_up = std::find_if(hi.begin(), hi.end(), [](const HiTerm &h) { return h.pat >= 0; }) - hi.begin();
+  struct List {  // a block's records, upper-half terms first
+    const BkRec *rec;
+    const double *im;
+    uint32_t nh, nx;
+  };
+  constexpr int kRun = 64;  // blocks of a piece
+  struct Run {
+    std::vector<BkRec> rec;
+    std::vector<double> im;
+  };
+  std::vector<Run> runs((b_ib.size() + kRun - 1) / kRun);
+  std::vector<List> lists(b_ib.size());
+  const int ng = (int)cf.size();
+  struct Warp {
+    int cls, warp;
+    std::vector<std::vector<uint16_t>> code;  // by group
+    std::vector<int> slots;
+  };
+  std::vector<Warp> warps;
+  for (size_t c = 0; c < cls.size(); c++)
+    for (int w = 0; w < (cls[c].n + 31) / 32; w++) warps.push_back(Warp{(int)c, w, {}, {}});
+  std::atomic<bool> fits{true};
+  auto list_run = [&](size_t u) {
+    Run &r = runs[u];
+    r.rec.reserve((size_t)kRun * std::min<size_t>(hi.size(), kBkList));
+    const size_t q0 = (size_t)u * kRun, q1 = std::min(b_ib.size(), q0 + kRun);
+    for (size_t q = q0; q < q1 && fits; q++) {
+      const uint32_t ib = b_ib[q];
+      const int c = class_of_block[ib];
+      List &l = lists[q];
+      l.nh = l.nx = 0;
+      for (size_t k = two_pass ? n_up : 0; k < hi.size(); k++) {
+        const HiTerm &h = hi[k];
+        if ((ib & h.cm) != h.cv) continue;
+        const uint32_t to = ib ^ h.flip;
+        if (l22[to] == 0) continue;
+        const bool cross = h.pat >= 0;
+        const int lead = cross ? tab_to[c * np + h.pat] : c;  // a moved block keeps its lower halves
+        if (lead < 0) continue;                               // no row of the class matches
+        if (class_of_block[to] != lead) fits = false;
+        const bool neg = h.sm && (__builtin_popcount(ib & h.sm) & 1);
+        r.rec.push_back(BkRec{l22[to] - 1u, cross ? tab_at[c * np + h.pat] : 0u, neg ? -h.re : h.re});
+        if (T.im) r.im.push_back(neg ? -h.im : h.im);
+        (cross ? l.nx : l.nh)++;
       }
-      if (recs[b].size() > (size_t)kBkList) return false;
-      order.push_back({((uint64_t)nhb[b] << 32) | recs[b].size(), b});
+      if (l.nh + l.nx > (uint32_t)kBkList) fits = false;
     }
-    std::stable_sort(order.begin(), order.end());
-    std::vector<uint32_t> r0(cls[c].nblk);
-    for (int b = 0; b < cls[c].nblk; b++) {
-      r0[b] = b_row0[cls[c].boff + order[b].second];
-      ib_sorted[cls[c].boff + b] = b_ib[cls[c].boff + order[b].second];
+    size_t at = 0;  // the run's vectors do not move any more
+    for (size_t q = q0; q < q1; at += lists[q].nh + lists[q].nx, q++) {
+      lists[q].rec = r.rec.data() + at;
+      lists[q].im = T.im ? r.im.data() + at : nullptr;
     }
-    for (int b = 0; b < cls[c].nblk; b++) {
-      const int o = order[b].second;
-      b_row0[cls[c].boff + b] = r0[b];
-      b_list[cls[c].boff + b] = make_uint2((uint32_t)rec.size(), nhb[o] | ((uint32_t)(recs[o].size() - nhb[o]) << 16));
-      rec.insert(rec.end(), recs[o].begin(), recs[o].end());
-      rec_im.insert(rec_im.end(), ims[o].begin(), ims[o].end());
+  };
+  auto gather = [&](Warp &w) {
+    std::vector<uint32_t> ptr, ent;
+    const BkClass &k = cls[w.cls];
+    w.code.resize(ng);
+    for (int g = 0; g < ng; g++) {
+      ptr.assign(1, 0);
+      ent.clear();
+      for (int p = 32 * w.warp; p < 32 * (w.warp + 1); p++) {
+        const uint32_t ia = p < k.n ? low[k.uoff + p] : 0;
+        for (const LoTerm &t : lo[g]) {
+          if (p >= k.n || (ia & t.t->cm) != t.t->cv) continue;
+          const uint32_t src = ia ^ (uint32_t)t.t->flip;
+          if (cls_of[src] < 0) continue;  // list_2_1 == 0: outside the sector
+          if (cls_of[src] != w.cls) fits = false;
+          const bool neg = (t.t->sm && (__builtin_popcount(ia & (uint32_t)t.t->sm) & 1)) != t.neg;
+          ent.push_back((uint32_t)pos_of[src] | (neg ? 0x10000u : 0u));
+        }
+        ptr.push_back((uint32_t)ent.size());
+      }
+      w.slots.push_back(gather_warp(ptr.data(), ent.data(), k.n, &w.code[g]));
     }
-    if (rec.size() > (1u << 26)) return false;
+  };
+  // lists first: their limits decline without the gather tables.  ~10 ns per block and term, 100
+  // per gather entry (about half the terms act on a row)
+  size_t n_lo = 0;
+  for (const auto &g : lo) n_lo += g.size();
+  host_parallel((int64_t)(runs.size() + warps.size()), 0.01 * (double)(b_ib.size() * hi.size()) + 1.5 * (double)(warps.size() * n_lo),
+                [&](int64_t k) {
+                  if (!fits) return;
+                  if (k < (int64_t)runs.size()) list_run((size_t)k);
+                  else gather(warps[k - runs.size()]);
+                });
+  if (!fits) return false;
+  size_t total = 0;
+  for (const Run &r : runs) total += r.rec.size();
+  if (total > (1u << 26)) return false;
+  rec.reserve(total);
+  std::vector<uint32_t> r0;
+  std::vector<std::pair<uint64_t, int>> order;
+  for (const BkClass &k : cls) {
+    order.clear();
+    for (int b = 0; b < k.nblk; b++) {
+      const List &l = lists[k.boff + b];
+      order.push_back({((uint64_t)l.nh << 32) | (l.nh + l.nx), b});
+    }
+    std::stable_sort(order.begin(), order.end());  // blocks of equal list lengths side by side
+    r0.resize(k.nblk);
+    for (int b = 0; b < k.nblk; b++) {
+      r0[b] = b_row0[k.boff + order[b].second];
+      ib_sorted[k.boff + b] = b_ib[k.boff + order[b].second];
+    }
+    for (int b = 0; b < k.nblk; b++) {
+      const List &l = lists[k.boff + order[b].second];
+      b_row0[k.boff + b] = r0[b];
+      b_list[k.boff + b] = make_uint2((uint32_t)rec.size(), l.nh | (l.nx << 16));
+      rec.insert(rec.end(), l.rec, l.rec + l.nh + l.nx);
+      if (T.im) rec_im.insert(rec_im.end(), l.im, l.im + l.nh + l.nx);
+    }
+  }
+  // one table per class: a warp's sets, group after group, at a fixed stride (with one set past
+  // the last, read ahead), so that the first set's address does not wait for the slot counts
+  std::vector<uint4> &gat = T.gat;
+  std::vector<uint2> &head = T.head;
+  for (const Warp &w : warps) {
+    int n = 1;
+    for (int ns : w.slots) {
+      if (ns > 255) return false;  // counts are packed in 8 bits
+      n += (ns + 7) / 8;
+    }
+    cls[w.cls].sets = std::max(cls[w.cls].sets, n);
+  }
+  for (const Warp &w : warps) {
+    BkClass &k = cls[w.cls];
+    if (w.warp == 0) {
+      k.gat = (int)gat.size();
+      k.head = (int)head.size();
+    }
+    uint64_t cnt = 0;
+    for (int g = 0; g < ng; g++) {
+      cnt |= (uint64_t)w.slots[g] << (8 * g);
+      for (int j = 0; j < w.slots[g]; j += 8)
+        for (int lane = 0; lane < 32; lane++) {
+          const GatherSet s = gather_set(w.code[g], j, lane);
+          gat.push_back(make_uint4(s.w[0], s.w[1], s.w[2], s.w[3]));
+        }
+    }
+    gat.resize((size_t)k.gat + (size_t)(w.warp + 1) * k.sets * 32, make_uint4(0, 0, 0, 0));
+    head.push_back(make_uint2((uint32_t)cnt, (uint32_t)(cnt >> 32)));
   }
   double mean = 0.0;  // block length a row sees on average
   for (const SectorBlock &b : blk) mean += (double)b.n * b.n / (double)dim;
@@ -217,7 +274,7 @@ bool block_tables(const std::vector<BitTerm> &terms, int lo_bits, const std::vec
   // else class by class, the longest first.
   uint64_t xhi = 0;
   for (const HiTerm &h : hi)
-    if (h.pat >= 0) xhi |= h.t->flip >> lo_bits;
+    if (h.pat >= 0) xhi |= h.flip;
   for (size_t c = 0; c < cls.size(); c++)
     for (int b = 0; b < cls[c].nblk; b++)
       T.order.push_back({two_pass ? ib_sorted[cls[c].boff + b] & ~xhi : 0, (uint32_t)c, (uint32_t)(cls[c].boff + b)});

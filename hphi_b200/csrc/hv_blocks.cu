@@ -10,7 +10,7 @@
 //                       follows from the lower half (a table per class and flipped bit).
 // A task is P planes of one class: P blocks of a real vector, or the real and imaginary parts of
 // P / 2 blocks of a complex one.  The planes are staged in shared memory, where the lower-half
-// terms are edge-coloured gathers (build_gather_table: no bank conflicts, 16-bit entries); upper
+// terms are edge-coloured gathers (gather_warp: no bank conflicts, 16-bit entries); upper
 // and crossing terms are listed per block when the plan is made (source block and coefficient)
 // and read v1 in (nearly) consecutive pieces from L2.  The general kernel (hv.cu) spends three
 // scattered L1 requests per matrix element (entry, coefficient, source) and is bound by them;
@@ -29,6 +29,7 @@
 #include "device_util.cuh"
 #include "engine.hpp"
 #include "hv_blocks.hpp"
+#include "plan_upload.hpp"
 #include "tma.cuh"
 
 namespace hphi {
@@ -340,23 +341,6 @@ void bk_plan_free(BlockPlan *p) {
 
 namespace {
 
-template <typename V>
-int bk_upload(BlockPlan *p, const std::vector<V> &h, const V **d, std::string *err) {
-  void *q = nullptr;
-  const size_t bytes = std::max<size_t>(16, sizeof(V) * h.size());
-  if (cudaMalloc(&q, bytes) != cudaSuccess) {
-    *err = "block plan: device allocation failed";
-    return -1;
-  }
-  p->allocs.push_back(q);
-  if (!h.empty() && cudaMemcpy(q, h.data(), sizeof(V) * h.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
-    *err = "block plan: copy failed";
-    return -1;
-  }
-  *d = (const V *)q;
-  return 0;
-}
-
 template <typename F>
 void with_bk_shape(int id, F f) {
   switch (id) {
@@ -394,11 +378,6 @@ int bk_plan_build(Sector *s, bool two_pass, std::string *err) {
   p->im = t.im;
   p->two_pass = two_pass;
   p->shape = t.shape;
-  auto fail = [&]() { bk_plan_free(p); return -1; };
-  if (bk_upload(p, t.cls, &a.cls, err) || bk_upload(p, t.b_row0, &a.b_row0, err) || bk_upload(p, t.b_list, &a.b_list, err) ||
-      bk_upload(p, t.rec, &a.rec, err) || bk_upload(p, t.gat, &a.gat, err) || bk_upload(p, t.head, &a.head, err) ||
-      bk_upload(p, t.cf, &a.cf, err) || bk_upload(p, t.tab, &a.tab, err) || (t.im && bk_upload(p, t.rec_im, &a.rec_im, err)))
-    return fail();
   bool fits = true;
   with_bk_shape(p->shape, [&](auto st) {
     using S = BkShape<decltype(st)::value>;
@@ -420,10 +399,26 @@ int bk_plan_build(Sector *s, bool two_pass, std::string *err) {
     bk_plan_free(p);
     return 0;
   }
+  PlanUpload up;
+  up.add(t.cls, &a.cls);
+  up.add(t.b_row0, &a.b_row0);
+  up.add(t.b_list, &a.b_list);
+  up.add(t.rec, &a.rec);
+  up.add(t.gat, &a.gat);
+  up.add(t.head, &a.head);
+  up.add(t.cf, &a.cf);
+  up.add(t.tab, &a.tab);
+  if (t.im) up.add(t.rec_im, &a.rec_im);
+  std::vector<BkTask> tk[2];
   for (int cv = 0; cv < 2; cv++) {
-    const std::vector<BkTask> tk = block_tasks(t, cv != 0, p->grid[cv]);
-    p->ntask[cv] = (int)tk.size();
-    if (bk_upload(p, tk, &p->tasks[cv], err)) return fail();
+    tk[cv] = block_tasks(t, cv != 0, p->grid[cv]);
+    p->ntask[cv] = (int)tk[cv].size();
+    up.add(tk[cv], &p->tasks[cv]);
+  }
+  if (up.run(&p->allocs) != 0) {
+    *err = "block plan: device allocation or copy failed";
+    bk_plan_free(p);
+    return -1;
   }
   s->bk = p;
   return 0;

@@ -46,6 +46,8 @@
 
 #include "device_util.cuh"
 #include "engine.hpp"
+#include "gather_table.hpp"
+#include "host_parallel.hpp"
 #include "hv_product.hpp"
 #include "tma.cuh"
 
@@ -639,7 +641,7 @@ __device__ __forceinline__ uint32_t species_parity16(uint32_t u, uint32_t d) {
   d ^= d << 8;
   return (uint32_t)__popc(u & (d << 1)) & 1u;
 }
-__device__ __forceinline__ uint32_t compress_even(uint32_t x) {  // bit 2i -> bit i
+__host__ __device__ __forceinline__ uint32_t compress_even(uint32_t x) {  // bit 2i -> bit i
   x &= 0x55555555u;
   x = (x | (x >> 1)) & 0x33333333u;
   x = (x | (x >> 2)) & 0x0F0F0F0Fu;
@@ -885,113 +887,10 @@ uint64_t spread_species(uint32_t x, int s, int N) {
   return c;
 }
 
-// Gather table of the row pass.  Column p belongs to warp p / 32 and half-warp (p / 16) % 2;
-// the entries of the 16 columns of a half-warp form a bipartite multigraph between lanes and
-// shared-memory bank pairs (source word mod 16).  A proper edge colouring with Delta colours
-// (Delta = its largest degree; Konig's theorem, built by swapping alternating paths) gives
-// slots in which every lane and every bank pair carries at most one entry.  Lanes left
-// without an entry in a slot read a zero word of a bank pair that slot leaves free (words
-// Dc .. Dc+15, one per bank pair).  Stored packed: per warp and group of 8 slots, each lane's
-// 8 entries (16 bits: word | sign << 15) are one 16-byte load.
-void build_gather(const std::vector<std::vector<uint32_t>> &rows_dn, const std::vector<SpeciesHop> &hops, int Dc,
-                  int npad, std::vector<uint32_t> *gat, std::vector<int> *wslots, int *nslots, int *groups) {
-  const int nwarp = npad / 32;
-  auto zero_word = [&](int bank) { return (uint32_t)(Dc + (((bank - Dc) % 16) + 16) % 16); };
-  std::vector<std::vector<uint32_t>> lane_slots(npad);  // per column: entry of each slot of its half
-  std::vector<int> el, eb, L, B, colr, path;
-  std::vector<uint32_t> ev;
-  wslots->assign(nwarp, 0);
-  *nslots = 0;
-  for (int w = 0; w < nwarp; w++) {
-    int wmax = 0;
-    for (int hw = 0; hw < 2; hw++) {
-      el.clear();
-      eb.clear();
-      ev.clear();
-      for (int l = 0; l < 16; l++) {
-        const int col = 32 * w + 16 * hw + l;
-        if (col >= Dc) continue;
-        for (uint32_t e : rows_dn[col]) {
-          const uint32_t word = e & 0xFFFFu, h = (e >> 16) >> 1, sign = (e >> 16) & 1u;
-          const bool neg = ((hops[h].re < 0) != (sign != 0));
-          el.push_back(l);
-          eb.push_back((int)(word % 16));
-          ev.push_back((word * 8u) | (neg ? 0x80000000u : 0u));
-        }
-      }
-      int ldeg[16] = {0}, bdeg[16] = {0};
-      for (size_t i = 0; i < el.size(); i++) { ldeg[el[i]]++; bdeg[eb[i]]++; }
-      int D = 0;
-      for (int i = 0; i < 16; i++) D = std::max(D, std::max(ldeg[i], bdeg[i]));
-      L.assign(16 * std::max(D, 1), -1);
-      B.assign(16 * std::max(D, 1), -1);
-      colr.assign(el.size(), -1);
-      for (size_t i = 0; i < el.size(); i++) {
-        const int l = el[i], bk = eb[i];
-        int a = 0, c = 0;
-        while (L[l * D + a] >= 0) a++;
-        while (B[bk * D + c] >= 0) c++;
-        if (B[bk * D + a] >= 0) {
-          // alternating a/c path from bank bk; swapping it frees a at bk
-          path.clear();
-          int node = bk, want = a;
-          bool at_bank = true;
-          for (;;) {
-            const int ed = at_bank ? B[node * D + want] : L[node * D + want];
-            if (ed < 0) break;
-            path.push_back(ed);
-            node = at_bank ? el[ed] : eb[ed];
-            at_bank = !at_bank;
-            want = (want == a) ? c : a;
-          }
-          for (int ed : path) { L[el[ed] * D + colr[ed]] = -1; B[eb[ed] * D + colr[ed]] = -1; }
-          for (int ed : path) colr[ed] = (colr[ed] == a) ? c : a;
-          for (int ed : path) { L[el[ed] * D + colr[ed]] = ed; B[eb[ed] * D + colr[ed]] = ed; }
-        }
-        colr[i] = a;
-        L[l * D + a] = (int)i;
-        B[bk * D + a] = (int)i;
-      }
-      for (int l = 0; l < 16; l++) lane_slots[32 * w + 16 * hw + l].assign(D, 0u);
-      for (int c = 0; c < D; c++) {
-        int f = 0;  // next bank pair that the slot may leave free
-        for (int l = 0; l < 16; l++) {
-          const int ed = L[l * D + c];
-          if (ed < 0)
-            while (B[f * D + c] >= 0) f++;
-          lane_slots[32 * w + 16 * hw + l][c] = (ed >= 0) ? ev[ed] : zero_word(f++) * 8u;
-        }
-      }
-      wmax = std::max(wmax, D);
-    }
-    (*wslots)[w] = wmax;
-    *nslots = std::max(*nslots, wmax);
-  }
-  // packed: per warp and slot group g, 32 lanes x 8 entries of 16 bits (word | sign << 15)
-  *groups = std::max(1, (*nslots + 7) / 8);
-  gat->assign((size_t)nwarp * *groups * 32 * 4, 0u);
-  for (int p = 0; p < npad; p++) {
-    const int w = p / 32, lane = p % 32, l = p % 16;
-    for (int sl = 0; sl < 8 * *groups; sl++) {
-      uint32_t word, neg = 0;
-      if (sl < (int)lane_slots[p].size()) {
-        word = (lane_slots[p][sl] & 0x7FFFFFFFu) / 8u;
-        neg = lane_slots[p][sl] >> 31;
-      } else {
-        word = zero_word(l);
-      }
-      const uint32_t e16 = word | (neg << 15);
-      const size_t q = (((size_t)w * *groups + sl / 8) * 32 + lane) * 4 + (sl % 8) / 2;
-      (*gat)[q] |= (sl % 2) ? (e16 << 16) : e16;
-    }
-  }
-}
-
-
 // Positions of the down configurations for the row pass.  The row pass gives column p to
 // lane p % 32 of warp p / 32, and an 8-byte gather of source column q hits the shared-memory
 // bank pair q % 16; a half-warp's slot count is max(largest lane degree, largest bank-pair
-// load) (the edge colouring of build_gather), so positions decide both.  Start from the
+// load) (the edge colouring of gather_warp), so positions decide both.  Start from the
 // configurations sorted by hop count (equal lane degrees in a half-warp), then swap positions
 // (within a half-warp: a bank change; across half-warps: only between equal hop counts) when
 // that does not raise the summed slot counts of the half-warps it touches.  rows[r]: sources
@@ -1078,17 +977,6 @@ std::vector<int> balance_positions(const std::vector<std::vector<uint32_t>> &row
 
 }  // namespace
 
-bool build_gather_table(const std::vector<std::vector<uint32_t>> &rows, int n, std::vector<uint32_t> *gat,
-                        std::vector<uint8_t> *wslots, int *groups) {
-  // entries carry their sign directly: one hop of coefficient +1, sign bit = (entry >> 16) & 1
-  const std::vector<SpeciesHop> unit{SpeciesHop{0, 0, 1.0, 0.0}};
-  int nslots = 0;
-  std::vector<int> slots;
-  build_gather(rows, unit, n, (n + 31) / 32 * 32, gat, &slots, &nslots, groups);
-  wslots->assign(slots.begin(), slots.end());
-  return nslots <= 255;
-}
-
 // The species (0 up, 1 down) and hop of a term that moves one electron; false for any other.
 static bool species_hop(const BitTerm &t, SpeciesHop *h, int *species) {
   if (__builtin_popcountll(t.flip) != 2 || t.cm != t.flip) return false;
@@ -1165,26 +1053,38 @@ static int two_pass_build(Sector *s, ProdPlan *p, const std::vector<std::vector<
   b.npad = (Dc + 31) / 32 * 32;
   b.ng = G[1].n;
   const int nw = b.npad / 32;
-  std::vector<std::vector<uint32_t>> tabs(b.ng);
-  std::vector<std::vector<uint8_t>> slots(b.ng);
-  std::vector<int> gsets(b.ng);
+  std::vector<std::vector<uint32_t>> ptr(b.ng), ents(b.ng);
   for (int g = 0; g < b.ng; g++) {
-    std::vector<std::vector<uint32_t>> rows(Dc);
-    for (int r = 0; r < Dc; r++)
-      for (uint32_t e : rows_dn[r]) {
+    ptr[g].push_back(0);
+    for (int r = 0; r < b.npad; r++) {
+      for (uint32_t e : r < Dc ? rows_dn[r] : std::vector<uint32_t>()) {
         const uint32_t h = (e >> 16) >> 1, sign = (e >> 16) & 1u;
-        if (G[1].gid[h] == g) rows[r].push_back((e & 0xFFFFu) | ((sign ^ (G[1].gsign[h] < 0 ? 1u : 0u)) << 16));
+        if (G[1].gid[h] == g) ents[g].push_back((e & 0xFFFFu) | ((sign ^ (G[1].gsign[h] < 0 ? 1u : 0u)) << 16));
       }
-    if (!build_gather_table(rows, Dc, &tabs[g], &slots[g], &gsets[g])) return 0;
+      ptr[g].push_back((uint32_t)ents[g].size());
+    }
   }
+  std::vector<std::vector<uint16_t>> code((size_t)nw * b.ng);
+  std::vector<int> slots((size_t)nw * b.ng);
+  size_t n_ent = 0;
+  for (const auto &e : ents) n_ent += e.size();
+  host_parallel(nw, 0.1 * (double)n_ent, [&](int64_t w) {
+    for (int g = 0; g < b.ng; g++)
+      slots[w * b.ng + g] = gather_warp(&ptr[g][32 * w], ents[g].data(), Dc, &code[w * b.ng + g]);
+  });
   std::vector<uint4> gat, whead(nw);
   for (int w = 0; w < nw; w++) {
     uint64_t cnt = 0;
     whead[w].x = (uint32_t)(gat.size() / 32);
     for (int g = 0; g < b.ng; g++) {
-      cnt |= (uint64_t)slots[g][w] << (8 * g);
-      const uint32_t *t = &tabs[g][(size_t)w * gsets[g] * 128];
-      for (int i = 0; i < (slots[g][w] + 7) / 8 * 32; i++) gat.push_back(make_uint4(t[4 * i], t[4 * i + 1], t[4 * i + 2], t[4 * i + 3]));
+      const int ns = slots[(size_t)w * b.ng + g];
+      if (ns > 255) return 0;  // counts are packed in 8 bits
+      cnt |= (uint64_t)ns << (8 * g);
+      for (int j = 0; j < ns; j += 8)
+        for (int lane = 0; lane < 32; lane++) {
+          const GatherSet q = gather_set(code[(size_t)w * b.ng + g], j, lane);
+          gat.push_back(make_uint4(q.w[0], q.w[1], q.w[2], q.w[3]));
+        }
     }
     whead[w].y = (uint32_t)cnt;
     whead[w].z = (uint32_t)(cnt >> 32);
@@ -1261,16 +1161,17 @@ static int perm_tasks_build(Sector *s, ProdPlan *p, std::string *err) {
   if (sector_blocks(s, &blk, &low, err) != 0) return -1;
   // the upper half's even bits are ups when N (the lower half's bits) is even, else downs
   const uint32_t up_bits = (p->args.N % 2 == 0) ? 0x5555u : 0xAAAAu;
-  std::vector<std::pair<uint32_t, uint32_t>> order;  // (upper ups and downs, block)
+  // the blocks at their places (upper ups, upper downs)
+  std::vector<uint32_t> at((size_t)1 << 16, 0u);
   for (size_t b = 0; b < blk.size(); b++) {
-    uint32_t up = 0, dn = 0;
-    for (int i = 0; i < 16; i++)
-      if ((blk[b].ib >> i) & 1u) ((up_bits >> i) & 1u ? up : dn) |= 1u << (i / 2);
-    order.push_back({(up << 8) | dn, (uint32_t)b});
+    const uint32_t x = compress_even(blk[b].ib), y = compress_even(blk[b].ib >> 1);
+    const uint32_t up = up_bits & 1u ? x : y, dn = up_bits & 1u ? y : x;
+    at[(up << 8) | dn] = (uint32_t)b + 1;
   }
-  std::sort(order.begin(), order.end());
-  for (const auto &o : order) {
-    const SectorBlock &b = blk[o.second];
+  tasks.reserve(blk.size() + s->dim / kBlockPiece + 1);
+  for (uint32_t q : at) {
+    if (q == 0) continue;
+    const SectorBlock &b = blk[q - 1];
     for (uint32_t a = 0; a < b.n; a += kBlockPiece)
       tasks.push_back(SectorBlock{b.ib, b.row0 + a, b.low0 + a, std::min<uint32_t>(kBlockPiece, b.n - a)});
   }

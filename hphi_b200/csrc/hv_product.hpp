@@ -31,14 +31,5 @@ int prod_te_launch(Sector *s, const ProdPlan *te, int index, const void *d_v1, v
                    double *d_out, void *d_sum, double c_re, double c_im);
 int prod_permute(Sector *s, VecType vt, const void *in, void *out, bool to_native);
 int prod_observables(Sector *s, VecType vt, const void *v, double *d_out);
-// Edge-coloured gather table of the row pass for n columns (positions): rows[p] lists the
-// sources of column p as (source position | negative << 16).  gat: per warp of 32 columns and
-// group of 8 slots, 32 lanes x 4 words of two 16-bit entries (position | sign << 15);
-// wslots: slots per warp; groups: slot groups per warp in the table.  Empty slots read one of
-// the zero words n .. n + 15 (one per shared-memory bank pair).  A warp takes as many slots as its
-// busiest lane or bank pair has entries; false, and no table, where that is more than the 255 that
-// the callers' packed counts hold.
-bool build_gather_table(const std::vector<std::vector<uint32_t>> &rows, int n, std::vector<uint32_t> *gat,
-                        std::vector<uint8_t> *wslots, int *groups);
 
 }  // namespace hphi
