@@ -45,6 +45,7 @@ struct SplitPlan {
   uint32_t lo_stride = 0;  // lo_ent[slot * lo_stride + lower half]
   HiEnt *hi_ent = nullptr;
   double *coef = nullptr;
+  void *tables = nullptr;  // the allocation of the arrays above
   BitTerm *gen = nullptr;  // terms left to the generic path
   int ngen = 0;
   int64_t n_lo_ent = 0, n_hi_ent = 0;

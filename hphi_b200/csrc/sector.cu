@@ -15,17 +15,20 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <map>
 
 #include "engine.hpp"
+#include "host_parallel.hpp"
 #include "hv_hubbard.hpp"
 #include "hv_blocks.hpp"
 #include "hv_gc.hpp"
 #include "hv_rowblock.hpp"
 #include "hv_product.hpp"
+#include "plan_upload.hpp"
 #include "split.cuh"
 
 namespace hphi {
@@ -249,39 +252,32 @@ int split_plan_for_terms(Sector *s, const std::vector<BitTerm> &T, SplitPlan *pl
   }
   const uint64_t nlo = s->ihfbit, nhi = s->sdim;
   std::vector<uint32_t> lo_ptr(nlo, 0), lo_ent;
-  for (int pass = 0; pass < 2; pass++) {  // count, then fill slot by slot
-    uint32_t most = 0;
-    for (uint64_t ia = 0; ia < nlo; ia++) {
-      uint32_t n = 0;
-      if (!s->gc && l21[ia] == 0) continue;
-      for (size_t i = 0; i < lo_t.size(); i++) {
-        const BitTerm &t = T[lo_t[i]];
-        if ((ia & t.cm) != t.cv) continue;
-        const uint64_t src = ia ^ t.flip;
-        const uint64_t val = s->gc ? src : l21[src];
-        if (!s->gc && val == 0) continue;
-        if (val >= (1ull << kSplitTargetBits)) {
-          *err = "split plan: lower-half value out of range";
-          return -1;
-        }
-        if (pass == 1) {
-          const uint32_t k = coef_at[2 * i + (size_t)(__builtin_popcountll(ia & t.sm) & 1)];
-          lo_ent[(size_t)n * nlo + ia] = (uint32_t)val | (k << kSplitTargetBits);
-        }
-        n++;
-      }
-      lo_ptr[ia] = n;
-      most = std::max(most, n);
-    }
-    if (pass == 0) lo_ent.assign((size_t)most * nlo, 0u);
-  }
-  P.lo_stride = (uint32_t)nlo;
+  std::atomic<bool> in_range{true};
   std::vector<uint32_t> hi_ptr(nhi + 1, 0);
-  std::vector<HiEnt> hi_ent;
-  for (uint64_t ib = 0; ib < nhi; ib++) {
-    hi_ptr[ib] = (uint32_t)hi_ent.size();
-    if (!s->gc && l22[ib] == 0) continue;
+  // pieces of kRun lower or upper halves; a piece's upper-half entries in order
+  constexpr uint64_t kRun = 512;
+  const uint64_t n_lo = (nlo + kRun - 1) / kRun, n_hi = (nhi + kRun - 1) / kRun;
+  std::vector<std::vector<HiEnt>> hi_run(n_hi);
+  auto lower = [&](uint64_t ia, bool fill) {
+    if (!s->gc && l21[ia] == 0) return;
+    uint32_t n = 0;
+    for (size_t i = 0; i < lo_t.size(); i++) {
+      const BitTerm &t = T[lo_t[i]];
+      if ((ia & t.cm) != t.cv) continue;
+      const uint64_t src = ia ^ t.flip;
+      const uint64_t val = s->gc ? src : l21[src];
+      if (!s->gc && val == 0) continue;
+      if (val >= (1ull << kSplitTargetBits)) in_range = false;
+      const uint32_t k = coef_at[2 * i + (size_t)(t.sm ? __builtin_popcountll(ia & t.sm) & 1 : 0)];
+      if (fill) lo_ent[(size_t)n * nlo + ia] = (uint32_t)val | (k << kSplitTargetBits);
+      n++;
+    }
+    lo_ptr[ia] = n;
+  };
+  auto upper = [&](uint64_t ib, std::vector<HiEnt> *out) {
+    if (!s->gc && l22[ib] == 0) return;
     const uint64_t cfg = ib << s->lo_bits;
+    const size_t before = out->size();
     for (size_t i = 0; i < hi_t.size(); i++) {
       const BitTerm &t = T[hi_t[i]];
       if ((cfg & t.cm) != t.cv) continue;
@@ -293,30 +289,63 @@ int split_plan_for_terms(Sector *s, const std::vector<BitTerm> &T, SplitPlan *pl
         if (l22[src] == 0) continue;
         h.delta = (int64_t)l22[src] - (int64_t)l22[ib];
       }
-      h.k = coef_at[2 * (lo_t.size() + i) + (size_t)(__builtin_popcountll(cfg & t.sm) & 1)];
-      hi_ent.push_back(h);
+      h.k = coef_at[2 * (lo_t.size() + i) + (size_t)(t.sm ? __builtin_popcountll(cfg & t.sm) & 1 : 0)];
+      out->push_back(h);
     }
-    if (hi_ent.size() > 0xFFFFFFF0ull) { *err = "split plan: too many entries"; return -1; }
+    hi_ptr[ib + 1] = (uint32_t)(out->size() - before);
+  };
+  // room for a slot per term, cut to those in use below; counted first where that is much
+  size_t most = lo_t.size();
+  if (most * nlo > ((size_t)1 << 22)) {
+    host_parallel((int64_t)n_lo, 0.005 * (double)(nlo * lo_t.size()), [&](int64_t u) {
+      for (uint64_t ia = u * kRun; ia < std::min(nlo, (u + 1) * kRun); ia++) lower(ia, false);
+    });
+    most = *std::max_element(lo_ptr.begin(), lo_ptr.end());
   }
-  hi_ptr[nhi] = (uint32_t)hi_ent.size();
+  lo_ent.resize(most * nlo);
+  host_parallel((int64_t)(n_lo + n_hi), 0.005 * (double)(nlo * lo_t.size() + nhi * hi_t.size()), [&](int64_t q) {
+    const uint64_t u = (uint64_t)q;
+    if (u < n_lo)
+      for (uint64_t ia = u * kRun; ia < std::min(nlo, (u + 1) * kRun); ia++) lower(ia, true);
+    else
+      for (uint64_t ib = (u - n_lo) * kRun; ib < std::min(nhi, (u - n_lo + 1) * kRun); ib++) upper(ib, &hi_run[u - n_lo]);
+  });
+  if (!in_range) {
+    *err = "split plan: lower-half value out of range";
+    return -1;
+  }
+  lo_ent.resize((size_t)*std::max_element(lo_ptr.begin(), lo_ptr.end()) * nlo);
+  P.lo_stride = (uint32_t)nlo;
+  uint64_t n_ent = 0;
+  for (uint64_t ib = 0; ib < nhi; ib++) {
+    n_ent += hi_ptr[ib + 1];
+    hi_ptr[ib + 1] = (uint32_t)n_ent;
+  }
+  if (n_ent > 0xFFFFFFF0ull) { *err = "split plan: too many entries"; return -1; }
+  std::vector<HiEnt> hi_ent;
+  hi_ent.reserve(n_ent);
+  for (const auto &r : hi_run) hi_ent.insert(hi_ent.end(), r.begin(), r.end());
   P.n_lo_ent = (int64_t)lo_ent.size();
   P.n_hi_ent = (int64_t)hi_ent.size();
-  CK(cudaMalloc(&P.lo_ptr, sizeof(uint32_t) * lo_ptr.size()));
-  CK(cudaMalloc(&P.lo_ent, sizeof(uint32_t) * std::max<size_t>(1, lo_ent.size())));
-  CK(cudaMalloc(&P.hi_ptr, sizeof(uint32_t) * hi_ptr.size()));
-  CK(cudaMalloc(&P.hi_ent, sizeof(HiEnt) * std::max<size_t>(1, hi_ent.size())));
-  CK(cudaMalloc(&P.coef, sizeof(double) * coef.size()));
-  CK(cudaMemcpy(P.lo_ptr, lo_ptr.data(), sizeof(uint32_t) * lo_ptr.size(), cudaMemcpyHostToDevice));
-  if (!lo_ent.empty()) CK(cudaMemcpy(P.lo_ent, lo_ent.data(), sizeof(uint32_t) * lo_ent.size(), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(P.hi_ptr, hi_ptr.data(), sizeof(uint32_t) * hi_ptr.size(), cudaMemcpyHostToDevice));
-  if (!hi_ent.empty()) CK(cudaMemcpy(P.hi_ent, hi_ent.data(), sizeof(HiEnt) * hi_ent.size(), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(P.coef, coef.data(), sizeof(double) * coef.size(), cudaMemcpyHostToDevice));
+  PlanUpload up;
+  std::vector<void *> one;
+  up.add(lo_ptr, (const uint32_t **)&P.lo_ptr);
+  up.add(lo_ent, (const uint32_t **)&P.lo_ent);
+  up.add(hi_ptr, (const uint32_t **)&P.hi_ptr);
+  up.add(hi_ent, (const HiEnt **)&P.hi_ent);
+  up.add(coef, (const double **)&P.coef);
+  const int rc = up.run(&one);
+  if (!one.empty()) P.tables = one[0];
+  if (rc != 0) {
+    *err = "split plan: device allocation or copy failed";
+    return -1;
+  }
   return 0;
 }
 
 void split_plan_free(SplitPlan *p) {
-  cudaFree(p->lo_ptr); cudaFree(p->lo_ent); cudaFree(p->hi_ptr); cudaFree(p->hi_ent);
-  cudaFree(p->coef); cudaFree(p->gen);
+  cudaFree(p->tables);
+  cudaFree(p->gen);
   *p = SplitPlan();
 }
 
@@ -357,10 +386,19 @@ int64_t sector_dim(const Model &m) {
 }
 
 namespace {
-__global__ void first_lower_kernel(int n, const uint32_t *__restrict__ start, const uint64_t *__restrict__ list_1,
-                                   uint64_t lo_mask, uint32_t *__restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = (uint32_t)(list_1[start[i]] & lo_mask);
+// out[i] = lower half of row start[i] (lens null), or the lower halves of rows start[i] ..
+// start[i] + lens[i] from out[off[i]] on, a block of threads per i.
+__global__ void lower_halves_kernel(int n, const uint32_t *__restrict__ start, const uint32_t *__restrict__ lens,
+                                    const uint32_t *__restrict__ off, const uint64_t *__restrict__ list_1,
+                                    uint64_t lo_mask, uint32_t *__restrict__ out) {
+  if (!lens) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = (uint32_t)(list_1[start[i]] & lo_mask);
+    return;
+  }
+  for (int i = blockIdx.x; i < n; i += gridDim.x)
+    for (uint32_t k = threadIdx.x; k < lens[i]; k += blockDim.x)
+      out[off[i] + k] = (uint32_t)(list_1[start[i] + k] & lo_mask);
 }
 }  // namespace
 
@@ -374,41 +412,53 @@ int sector_blocks(const Sector *s, std::vector<SectorBlock> *out, std::vector<ui
       ibs.push_back((uint32_t)ib);
       start.push_back(l22[ib] - 1u);
     }
-  // a lower half belongs to one class (list_2_1 gives it one rank), so a block's first one names it
+  // A lower half belongs to one class (list_2_1 gives it one rank), so a block's first one names it.
+  // The classes' halves are as many as there are lower halves at most.
+  if (start.empty()) return 0;
   uint32_t *d = nullptr;
-  std::vector<uint32_t> first(start.size());
-  CK(cudaMalloc(&d, sizeof(uint32_t) * 2 * std::max<size_t>(1, start.size())));
-  cudaError_t e = cudaMemcpy(d, start.data(), sizeof(uint32_t) * start.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && !start.empty()) {
-    first_lower_kernel<<<(unsigned)((start.size() + 255) / 256), 256, 0, s->stream>>>(
-        (int)start.size(), d, s->d_list_1, s->ihfbit - 1, d + start.size());
-    e = cudaMemcpyAsync(first.data(), d + start.size(), sizeof(uint32_t) * start.size(), cudaMemcpyDeviceToHost, s->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
-  }
-  cudaFree(d);
-  CK(e);
-  struct Class {
-    uint32_t n, low0;
+  const size_t nb = start.size();
+  CK(cudaMalloc(&d, sizeof(uint32_t) * (4 * nb + s->ihfbit)));
+  std::vector<uint32_t> first(nb), cs;  // class starts, lengths, offsets, one after another
+  auto rest = [&]() -> int {
+    CK(cudaMemcpyAsync(d, start.data(), sizeof(uint32_t) * nb, cudaMemcpyHostToDevice, s->stream));
+    lower_halves_kernel<<<(unsigned)((nb + 255) / 256), 256, 0, s->stream>>>((int)nb, d, nullptr, nullptr, s->d_list_1,
+                                                                             s->ihfbit - 1, d + nb);
+    CK(cudaMemcpyAsync(first.data(), d + nb, sizeof(uint32_t) * nb, cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
+    struct Class {
+      uint32_t start, n, low0;
+    };
+    std::vector<Class> cls;
+    std::map<uint32_t, size_t> at;  // by first lower half
+    size_t total = 0;
+    for (size_t b = 0; b < nb; b++) {
+      const int64_t n = (b + 1 < nb ? (int64_t)start[b + 1] : s->dim) - (int64_t)start[b];
+      const auto it = at.emplace(first[b], cls.size());
+      if (it.second && n > 0) {
+        cls.push_back(Class{start[b], (uint32_t)n, (uint32_t)total});
+        total += (size_t)n;
+      }
+      if (n <= 0 || cls[it.first->second].n != (uint32_t)n || total > s->ihfbit) {
+        *err = "sector blocks: unexpected layout";
+        return -1;
+      }
+      out->push_back(SectorBlock{ibs[b], start[b], cls[it.first->second].low0, (uint32_t)n});
+    }
+    const size_t nc = cls.size();
+    for (const Class &c : cls) cs.push_back(c.start);
+    for (const Class &c : cls) cs.push_back(c.n);
+    for (const Class &c : cls) cs.push_back(c.low0);
+    low->resize(total);
+    CK(cudaMemcpyAsync(d, cs.data(), sizeof(uint32_t) * cs.size(), cudaMemcpyHostToDevice, s->stream));
+    lower_halves_kernel<<<(unsigned)nc, 256, 0, s->stream>>>((int)nc, d, d + nc, d + 2 * nc, s->d_list_1, s->ihfbit - 1,
+                                                             d + 3 * nc);
+    CK(cudaMemcpyAsync(low->data(), d + 3 * nc, sizeof(uint32_t) * total, cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
+    return 0;
   };
-  std::map<uint32_t, Class> cls;  // by first lower half
-  std::vector<uint64_t> rows;
-  for (size_t b = 0; b < start.size(); b++) {
-    const int64_t end = b + 1 < start.size() ? (int64_t)start[b + 1] : s->dim;
-    const int64_t n = end - (int64_t)start[b];
-    auto it = cls.find(first[b]);
-    if (n > 0 && it == cls.end()) {
-      it = cls.emplace(first[b], Class{(uint32_t)n, (uint32_t)low->size()}).first;
-      rows.resize((size_t)n);
-      CK(cudaMemcpy(rows.data(), s->d_list_1 + start[b], sizeof(uint64_t) * (size_t)n, cudaMemcpyDeviceToHost));
-      for (uint64_t c : rows) low->push_back((uint32_t)(c & (s->ihfbit - 1)));
-    }
-    if (n <= 0 || it->second.n != (uint32_t)n) {
-      *err = "sector blocks: unexpected layout";
-      return -1;
-    }
-    out->push_back(SectorBlock{ibs[b], start[b], it->second.low0, (uint32_t)n});
-  }
-  return 0;
+  const int rc = rest();
+  cudaFree(d);
+  return rc;
 }
 
 int sector_pieces(Sector *s, std::string *err) {
@@ -572,6 +622,7 @@ int sector_build(const Model &m, int device, Sector **out, std::string *err, boo
       members[key].push_back((uint32_t)ia);
     }
     std::vector<uint64_t> l1;
+    l1.reserve((size_t)sector_dim(m));
     uint64_t jb = 0;
     for (uint64_t ib = 0; ib < nh; ib++) {
       if (!admissible(ib, half)) continue;
@@ -640,23 +691,21 @@ int sector_build(const Model &m, int device, Sector **out, std::string *err, boo
       for (int k = 0; k <= n; k++) binom[n * 65 + k] = binom_host(n, k);
     CK(cudaMemcpyToSymbol(c_binom, binom.data(), sizeof(uint64_t) * 65 * 65));
 
-    unsigned char *d_valid;
-    uint64_t *d_cls_off, *d_cls_cnt, *d_cnt, *d_jb, *d_total;
-    uint32_t *d_unrank;
-    int *d_need;
-    CK(cudaMalloc(&d_valid, ncls));
-    CK(cudaMalloc(&d_cls_off, sizeof(uint64_t) * (ncls + 1)));
-    CK(cudaMalloc(&d_cls_cnt, sizeof(uint64_t) * ncls));
-    CK(cudaMalloc(&d_unrank, sizeof(uint32_t) * s->ihfbit));
-    CK(cudaMalloc(&d_cnt, sizeof(uint64_t) * s->sdim));
-    CK(cudaMalloc(&d_jb, sizeof(uint64_t) * s->sdim));
-    CK(cudaMalloc(&d_total, sizeof(uint64_t)));
-    CK(cudaMalloc(&d_need, sizeof(int) * s->sdim));
+    // temporaries in one allocation, 8-byte words first; the class tables in one copy
+    uint64_t *tmp = nullptr;
+    const size_t words = 2 * (size_t)ncls + 2 + 2 * s->sdim;
+    CK(cudaMalloc(&tmp, sizeof(uint64_t) * words + sizeof(uint32_t) * (s->ihfbit + s->sdim) + (size_t)ncls));
+    uint64_t *d_cls_off = tmp, *d_cls_cnt = d_cls_off + ncls + 1, *d_total = d_cls_cnt + ncls, *d_cnt = d_total + 1,
+             *d_jb = d_cnt + s->sdim;
+    uint32_t *d_unrank = reinterpret_cast<uint32_t *>(d_jb + s->sdim);
+    int *d_need = reinterpret_cast<int *>(d_unrank + s->ihfbit);
+    unsigned char *d_valid = reinterpret_cast<unsigned char *>(d_need + s->sdim);
+    std::vector<uint64_t> tables(cls_off);
+    tables.insert(tables.end(), cls_cnt.begin(), cls_cnt.end());
     CK(cudaMalloc(&s->d_list_2_1, sizeof(uint32_t) * s->ihfbit));
     CK(cudaMalloc(&s->d_list_2_2, sizeof(uint32_t) * s->sdim));
     CK(cudaMemcpyAsync(d_valid, valid.data(), ncls, cudaMemcpyHostToDevice, s->stream));
-    CK(cudaMemcpyAsync(d_cls_off, cls_off.data(), sizeof(uint64_t) * (ncls + 1), cudaMemcpyHostToDevice, s->stream));
-    CK(cudaMemcpyAsync(d_cls_cnt, cls_cnt.data(), sizeof(uint64_t) * ncls, cudaMemcpyHostToDevice, s->stream));
+    CK(cudaMemcpyAsync(d_cls_off, tables.data(), sizeof(uint64_t) * tables.size(), cudaMemcpyHostToDevice, s->stream));
     const int T = 256;
     lo_tables_kernel<<<(unsigned)((s->ihfbit + T - 1) / T), T, 0, s->stream>>>(
         s->ihfbit, s->lo_bits, hubbard, Dlo, d_valid, d_cls_off, s->d_list_2_1, d_unrank);
@@ -685,8 +734,7 @@ int sector_build(const Model &m, int device, Sector **out, std::string *err, boo
                                              s->d_list_1);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(s->stream));
-    cudaFree(d_valid); cudaFree(d_cls_off); cudaFree(d_cls_cnt); cudaFree(d_unrank);
-    cudaFree(d_cnt); cudaFree(d_jb); cudaFree(d_total); cudaFree(d_need);
+    cudaFree(tmp);
   }
 
   // a block per 256 rows at most: the 1184-block grids of 8 per SM cost small sectors more in
@@ -747,8 +795,8 @@ void sector_free(Sector *s) {
   if (s->stream) cudaStreamSynchronize(s->stream);
   cudaFree(s->d_list_1); cudaFree(s->d_list_2_1); cudaFree(s->d_list_2_2); cudaFree(s->d_diag);
   cudaFree(s->d_terms); cudaFree(s->d_dterms); cudaFree(s->d_red); cudaFree(s->d_scal); cudaFree(s->ws);
-  cudaFree(s->split.lo_ptr); cudaFree(s->split.lo_ent); cudaFree(s->split.hi_ptr); cudaFree(s->split.hi_ent);
-  cudaFree(s->split.coef); cudaFree(s->split.gen); cudaFree(s->d_pieces); cudaFree(s->d_low);
+  split_plan_free(&s->split);
+  cudaFree(s->d_pieces); cudaFree(s->d_low);
   hub_plan_free(s->hub);
   prod_plan_free(s->prod);
   prod_plan_free(s->te_prod);
