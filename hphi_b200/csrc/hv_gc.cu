@@ -29,6 +29,7 @@
 #include "device_util.cuh"
 #include "engine.hpp"
 #include "hv_gc.hpp"
+#include "plan_upload.hpp"
 #include "tma.cuh"
 
 namespace hphi {
@@ -312,42 +313,47 @@ bool merge_term(const BitTerm &t, std::vector<Raw> *raw) {
 // Bit sets of K bits (the `low` lowest always among them) that cover every group's flip and
 // condition bits: greedily the set that takes most groups, grown group by group.
 std::vector<uint64_t> cover_passes(const std::vector<Raw> &raw, int n, int K, int low) {
-  auto need = [&](const Raw &r) { return r.flip | (1ull << r.i) | (1ull << r.j); };
-  const uint64_t base = (1ull << low) - 1;
-  std::vector<char> done(raw.size(), 0);
+  const uint32_t base = (1u << low) - 1u;
+  std::vector<uint32_t> need;  // of the groups still to cover (n <= 32 bits)
+  for (const Raw &r : raw) need.push_back((uint32_t)(r.flip | (1ull << r.i) | (1ull << r.j)));
+  // groups within a set: the loop that the whole search spends its time in
+  auto within = [&](uint32_t set) {
+    int g = 0;
+    for (uint32_t x : need) g += (x & ~set) == 0;
+    return g;
+  };
   std::vector<uint64_t> sets;
-  for (;;) {
-    uint64_t best = 0;
+  while (!need.empty()) {
+    uint32_t best = 0;
     int best_n = 0;
-    for (size_t s = 0; s < raw.size(); s++) {
-      if (done[s] || __builtin_popcountll(base | need(raw[s])) > K) continue;
-      uint64_t set = base | need(raw[s]);
+    // all seeds of up to 64 groups, 32 of more (the search grows with the cube of the groups)
+    const size_t step = need.size() <= 64 ? 1 : (need.size() + 31) / 32;
+    for (size_t q = 0; q < need.size(); q += step) {
+      uint32_t set = base | need[q];
+      if (__builtin_popcount(set) > K) continue;
       for (;;) {  // the group that adds the fewest bits, then the one that shares most with others
-        int pick = -1, cost = 99, gain = -1;
-        for (size_t q = 0; q < raw.size(); q++) {
-          const uint64_t add = need(raw[q]) & ~set;
-          if (done[q] || add == 0) continue;
-          const int c = __builtin_popcountll(add);
-          if (__builtin_popcountll(set) + c > K) continue;
-          int g = 0;
-          for (size_t r = 0; r < raw.size(); r++) g += !done[r] && (need(raw[r]) & ~(set | add)) == 0;
-          if (g - 2 * c > gain - 2 * cost || pick < 0) { pick = (int)q; cost = c; gain = g; }
+        int cost = 99, gain = -1;
+        uint32_t pick = 0;
+        for (uint32_t x : need) {
+          const uint32_t add = x & ~set;
+          if (add == 0) continue;
+          const int c = __builtin_popcount(add);
+          if (__builtin_popcount(set) + c > K) continue;
+          const int g = within(set | add);
+          if (g - 2 * c > gain - 2 * cost || pick == 0) { pick = add; cost = c; gain = g; }
         }
-        if (pick < 0) break;
-        set |= need(raw[pick]);
+        if (pick == 0) break;
+        set |= pick;
       }
-      int covered = 0;
-      for (size_t r = 0; r < raw.size(); r++) covered += !done[r] && (need(raw[r]) & ~set) == 0;
+      const int covered = within(set);
       if (covered > best_n) { best_n = covered; best = set; }
     }
-    if (best_n == 0) break;
-    for (int b = 0; b < n && __builtin_popcountll(best) < K; b++) best |= 1ull << b;  // fill up with low bits
+    if (best_n == 0) return {};
+    for (int b = 0; b < n && __builtin_popcount(best) < K; b++) best |= 1u << b;  // fill up with low bits
     sets.push_back(best);
-    for (size_t r = 0; r < raw.size(); r++)
-      if ((need(raw[r]) & ~best) == 0) done[r] = 1;
+    if (sets.size() > (size_t)kGcPasses) return {};
+    need.erase(std::remove_if(need.begin(), need.end(), [&](uint32_t x) { return (x & ~best) == 0; }), need.end());
   }
-  for (char d : done)
-    if (!d) return {};
   return sets;
 }
 
@@ -359,27 +365,13 @@ uint64_t extract_bits(uint64_t x, uint64_t set) {  // bits of x at the places of
   return r;
 }
 
-template <typename V>
-int gc_upload(GcPlan *p, const std::vector<V> &h, const V **d, std::string *err) {
-  void *q = nullptr;
-  if (cudaMalloc(&q, std::max<size_t>(16, sizeof(V) * h.size())) != cudaSuccess ||
-      cudaMemcpy(q, h.data(), sizeof(V) * h.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
-    cudaFree(q);
-    *err = "grand-canonical plan: upload failed";
-    return -1;
-  }
-  p->allocs.push_back(q);
-  *d = (const V *)q;
-  return 0;
-}
-
 // Passes of one vector type; leaves p->pass[vt] empty where the plan does not apply.
 template <typename T>
 int build_passes(Sector *s, GcPlan *p, const std::vector<Raw> &raw, int vt, std::string *err) {
   constexpr int K = GcTile<T>::K, low = GcTile<T>::low;
   const int n = s->model.nbits;
   std::vector<uint64_t> sets = raw.empty() ? std::vector<uint64_t>{(1ull << K) - 1} : cover_passes(raw, n, K, low);
-  if (sets.empty() || sets.size() > (size_t)kGcPasses) return 0;
+  if (sets.empty()) return 0;
   // a group that several passes could take goes to the one with fewest, the least movable groups first
   std::vector<int> owner(raw.size(), -1), load(sets.size(), 0);
   std::vector<std::pair<int, size_t>> order;
@@ -397,11 +389,14 @@ int build_passes(Sector *s, GcPlan *p, const std::vector<Raw> &raw, int vt, std:
       if (fits(o.second, a) && (owner[o.second] < 0 || load[a] < load[owner[o.second]])) owner[o.second] = (int)a;
     load[owner[o.second]]++;
   }
-  std::vector<GcPass> passes;
+  std::vector<GcPass> passes(sets.size());
+  std::vector<std::vector<uint32_t>> deps(sets.size());
+  PlanUpload up;
   for (size_t a = 0; a < sets.size(); a++) {
     const uint64_t set = sets[a];
     constexpr int M = (1 << K) / kGcThreads;
-    GcPass ps{};
+    GcPass &ps = passes[a];
+    ps = GcPass{};
     for (size_t q = 0; q < raw.size(); q++) {
       const Raw &r = raw[q];
       if (owner[q] != (int)a) continue;
@@ -428,7 +423,8 @@ int build_passes(Sector *s, GcPlan *p, const std::vector<Raw> &raw, int vt, std:
       }
       ps.ngroup++;
     }
-    std::vector<uint32_t> dep(1u << (K - low));
+    std::vector<uint32_t> &dep = deps[a];
+    dep.resize(1u << (K - low));
     std::vector<int> in;
     for (int b = 0; b < n; b++) {
       if (!((set >> b) & 1)) ps.outer[ps.nouter++] = (uint8_t)b;
@@ -438,8 +434,7 @@ int build_passes(Sector *s, GcPlan *p, const std::vector<Raw> &raw, int vt, std:
       for (size_t k = 0; k < in.size(); k++) dep[q] |= ((q >> k) & 1u) << in[k];
     ps.first = a == 0;
     ps.last = a + 1 == sets.size();
-    if (gc_upload(p, dep, &ps.dep, err)) return -1;
-    passes.push_back(ps);
+    up.add(dep, &ps.dep);
   }
   const size_t smem = sizeof(T) << K;
   int per_sm = 0;
@@ -449,6 +444,10 @@ int build_passes(Sector *s, GcPlan *p, const std::vector<Raw> &raw, int vt, std:
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f[im], kGcThreads, smem) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
     return 0;
+  }
+  if (up.run(&p->allocs) != 0) {
+    *err = "grand-canonical plan: upload failed";
+    return -1;
   }
   p->ntile[vt] = 1ll << (n - K);
   p->grid[vt] = (int)std::min<int64_t>(p->ntile[vt], (int64_t)per_sm * s->num_sms);
@@ -465,7 +464,7 @@ int gc_plan_build(Sector *s, std::string *err) {
   if (!s->gc || m.general_spin || m.nbits > 32 || m.nbits < kGcBitsComplex) return 0;
   std::vector<Raw> raw;
   for (const BitTerm &t : m.offdiag)
-    if (!merge_term(t, &raw)) return 0;
+    if (!merge_term(t, &raw) || raw.size() > (size_t)kGcPasses * kGcGroups) return 0;
   GcPlan *p = new GcPlan();
   for (const Raw &r : raw)
     for (double x : r.im) p->im = p->im || x != 0.0;
