@@ -262,12 +262,11 @@ template <typename T>
 int green_batches(Sector *s, const T *d_v, const std::vector<GreenTerm> &nz, std::vector<double> *out) {
   constexpr int W = GreenWidth<T>::w, NB = kGreenAcc / W;
   // the block kernels read whole complex elements; a vector at another address takes the row kernel
-  const bool blocks = !s->gc && s->lo_bits <= 31 && s->hi_bits <= 31 && whole_elements(W == 2 ? kComplex128 : kReal64, d_v);
+  // (as does a sector whose pieces there is no memory for)
   std::string err;
-  if (blocks && sector_pieces(s, &err) != 0) {
-    set_error("Green's functions: " + err);
-    return -1;
-  }
+  const bool blocks = !s->gc && s->lo_bits <= 31 && s->hi_bits <= 31 &&
+                      whole_elements(W == 2 ? kComplex128 : kReal64, d_v) && sector_pieces(s, &err) == 0;
+  cudaGetLastError();
   const uint64_t lo_mask = s->ihfbit - 1;
   auto halves = [&](const GreenTerm &t) {
     const int b = s->lo_bits;

@@ -357,19 +357,21 @@ void with_bk_shape(int id, F f) {
 
 }  // namespace
 
-// Leaves s->bk null where the plan does not apply (block_tables): the general kernel remains.
-int bk_plan_build(Sector *s, bool two_pass, std::string *err) {
+// Leaves s->bk null where the plan does not apply (block_tables) or there is no memory for it: the
+// general kernel remains.
+void bk_plan_build(Sector *s, bool two_pass) {
   s->bk = nullptr;
-  if (s->gc || !s->d_list_1 || s->lo_bits > 20 || s->hi_bits > 20 || s->model.offdiag.empty()) return 0;
+  if (s->gc || !s->d_list_1 || s->lo_bits > 20 || s->hi_bits > 20 || s->model.offdiag.empty()) return;
   std::vector<SectorBlock> blk;
   std::vector<uint32_t> low, l22(s->sdim);
-  if (sector_blocks(s, &blk, &low, err) != 0) return -1;
-  if (cudaMemcpy(l22.data(), s->d_list_2_2, sizeof(uint32_t) * l22.size(), cudaMemcpyDeviceToHost) != cudaSuccess) {
-    *err = "block plan: list copy failed";
-    return -1;
+  std::string why;
+  if (sector_blocks(s, &blk, &low, &why) != 0 ||
+      cudaMemcpy(l22.data(), s->d_list_2_2, sizeof(uint32_t) * l22.size(), cudaMemcpyDeviceToHost) != cudaSuccess) {
+    cudaGetLastError();
+    return;
   }
   BlockTables t;
-  if (!block_tables(s->model.offdiag, s->lo_bits, l22, blk, low, s->dim, two_pass, &t)) return 0;
+  if (!block_tables(s->model.offdiag, s->lo_bits, l22, blk, low, s->dim, two_pass, &t)) return;
   BlockPlan *p = new BlockPlan();
   BkArgs &a = p->args;
   a.ncls = (int)t.cls.size();
@@ -397,7 +399,7 @@ int bk_plan_build(Sector *s, bool two_pass, std::string *err) {
   cudaGetLastError();
   if (!fits) {
     bk_plan_free(p);
-    return 0;
+    return;
   }
   PlanUpload up;
   up.add(t.cls, &a.cls);
@@ -416,12 +418,11 @@ int bk_plan_build(Sector *s, bool two_pass, std::string *err) {
     up.add(tk[cv], &p->tasks[cv]);
   }
   if (up.run(&p->allocs) != 0) {
-    *err = "block plan: device allocation or copy failed";
+    cudaGetLastError();
     bk_plan_free(p);
-    return -1;
+    return;
   }
   s->bk = p;
-  return 0;
 }
 
 bool bk_applies(const Sector *s) { return s->bk && !s->bk->two_pass; }

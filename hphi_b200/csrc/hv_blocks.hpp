@@ -8,7 +8,7 @@ namespace hphi {
 
 struct BlockPlan;
 // two_pass: the row pass of the row-block plan (lower-half and crossing terms only), else all terms.
-int bk_plan_build(Sector *s, bool two_pass, std::string *err);
+void bk_plan_build(Sector *s, bool two_pass);
 void bk_plan_free(BlockPlan *p);
 bool bk_applies(const Sector *s);   // whole H*v in one launch
 bool bk_row_pass(const Sector *s);  // the row-block plan's row pass

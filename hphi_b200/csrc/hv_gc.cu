@@ -367,11 +367,11 @@ uint64_t extract_bits(uint64_t x, uint64_t set) {  // bits of x at the places of
 
 // Passes of one vector type; leaves p->pass[vt] empty where the plan does not apply.
 template <typename T>
-int build_passes(Sector *s, GcPlan *p, const std::vector<Raw> &raw, int vt, std::string *err) {
+void build_passes(Sector *s, GcPlan *p, const std::vector<Raw> &raw, int vt) {
   constexpr int K = GcTile<T>::K, low = GcTile<T>::low;
   const int n = s->model.nbits;
   std::vector<uint64_t> sets = raw.empty() ? std::vector<uint64_t>{(1ull << K) - 1} : cover_passes(raw, n, K, low);
-  if (sets.empty()) return 0;
+  if (sets.empty()) return;
   // a group that several passes could take goes to the one with fewest, the least movable groups first
   std::vector<int> owner(raw.size(), -1), load(sets.size(), 0);
   std::vector<std::pair<int, size_t>> order;
@@ -400,7 +400,7 @@ int build_passes(Sector *s, GcPlan *p, const std::vector<Raw> &raw, int vt, std:
     for (size_t q = 0; q < raw.size(); q++) {
       const Raw &r = raw[q];
       if (owner[q] != (int)a) continue;
-      if (ps.ngroup == kGcGroups) return 0;
+      if (ps.ngroup == kGcGroups) return;
       GcGroup &g = ps.g[ps.ngroup];
       const uint32_t f = (uint32_t)extract_bits(r.flip, set), sm = (uint32_t)extract_bits(r.sm, set);
       g.ft = f % kGcThreads;
@@ -443,52 +443,49 @@ int build_passes(Sector *s, GcPlan *p, const std::vector<Raw> &raw, int vt, std:
   if (raise_smem_limit(f[im], smem) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f[im], kGcThreads, smem) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
-    return 0;
+    return;
   }
   if (up.run(&p->allocs) != 0) {
-    *err = "grand-canonical plan: upload failed";
-    return -1;
+    cudaGetLastError();
+    return;
   }
   p->ntile[vt] = 1ll << (n - K);
   p->grid[vt] = (int)std::min<int64_t>(p->ntile[vt], (int64_t)per_sm * s->num_sms);
   p->pass[vt] = passes;
-  return 0;
 }
 
 }  // namespace
 
-int gc_plan_build(Sector *s, std::string *err) {
+// Leaves s->gcp null where the plan does not apply or there is no memory for it: the other kernels remain.
+void gc_plan_build(Sector *s) {
   s->gcp = nullptr;
   const Model &m = s->model;
   // rows within a tile are 32-bit numbers
-  if (!s->gc || m.general_spin || m.nbits > 32 || m.nbits < kGcBitsComplex) return 0;
+  if (!s->gc || m.general_spin || m.nbits > 32 || m.nbits < kGcBitsComplex) return;
   std::vector<Raw> raw;
   for (const BitTerm &t : m.offdiag)
-    if (!merge_term(t, &raw) || raw.size() > (size_t)kGcPasses * kGcGroups) return 0;
+    if (!merge_term(t, &raw) || raw.size() > (size_t)kGcPasses * kGcGroups) return;
   GcPlan *p = new GcPlan();
   for (const Raw &r : raw)
     for (double x : r.im) p->im = p->im || x != 0.0;
   bool signs = false;
   for (const Raw &r : raw) signs = signs || r.sm != 0;
   const bool real = !m.complex_terms && m.nbits >= (signs ? kGcBitsSigned : kGcBitsReal);
-  if ((real && build_passes<double>(s, p, raw, 0, err) != 0) || build_passes<cplx>(s, p, raw, 1, err) != 0) {
-    gc_plan_free(p);
-    return -1;
-  }
+  if (real) build_passes<double>(s, p, raw, 0);
+  build_passes<cplx>(s, p, raw, 1);
   if (p->pass[0].empty() && p->pass[1].empty()) {
     gc_plan_free(p);
-    return 0;
+    return;
   }
   s->gcp = p;
   const size_t nd = std::max(gc_scratch_doubles(s, kReal64), gc_scratch_doubles(s, kComplex128));
   if (cudaMalloc(&p->part, sizeof(double) * std::max<size_t>(2, nd)) != cudaSuccess) {
-    *err = "grand-canonical plan: device allocation failed";
+    cudaGetLastError();
     gc_plan_free(p);
     s->gcp = nullptr;
-    return -1;
+    return;
   }
   p->allocs.push_back(p->part);
-  return 0;
 }
 
 bool gc_applies(const Sector *s, VecType vt) { return s->gcp && !s->gcp->pass[vt == kReal64 ? 0 : 1].empty(); }

@@ -7,7 +7,7 @@
 namespace hphi {
 
 struct GcPlan;
-int gc_plan_build(Sector *s, std::string *err);
+void gc_plan_build(Sector *s);
 void gc_plan_free(GcPlan *p);
 bool gc_applies(const Sector *s, VecType vt);
 size_t gc_scratch_doubles(const Sector *s, VecType vt);

@@ -1045,7 +1045,8 @@ static void with_row_kernel(int stride, bool cplx_v, bool onsite, F f) {
 }
 
 // Tables and launch shapes of the two-pass kernels.  rows_*: per configuration its hops as
-// source | (2 * hop + sign) << 16.  Leaves p->two_pass false where a gather table does not apply.
+// source | (2 * hop + sign) << 16.  Leaves p->two_pass false, and the plan as it was, where a gather
+// table does not apply; -1 where there is no memory for the tables.
 static int two_pass_build(Sector *s, ProdPlan *p, const std::vector<std::vector<uint32_t>> &rows_dn,
                           const std::vector<std::vector<uint32_t>> &rows_up, const HopGroups (&G)[2], std::string *err) {
   const int Uc = p->args.Uc, Dc = p->args.Dc;
@@ -1130,27 +1131,22 @@ static int two_pass_build(Sector *s, ProdPlan *p, const std::vector<std::vector<
       const int rows = cv ? S::P / 2 : S::P;
       p->grid_row[cv] = std::max(1, std::min((Uc + rows - 1) / rows, per_sm * s->num_sms));
     });
-    if (rc != 0) {
-      *err = "product plan: row pass does not fit";
-      return -1;
-    }
+    if (rc != 0) return -1;
   }
   int col = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&col, prod_col_kernel<2, true, true, false>, kUpThreads, 0);
   const int64_t ntask = (int64_t)Uc * ((2 * Dc + kUpChunk - 1) / kUpChunk);
   p->grid_col = (int)std::max<int64_t>(1, std::min<int64_t>(std::max(1, col) * s->num_sms, (ntask + 7) / 8));
-  p->two_pass = true;
   const int nrec = std::max(p->grid_row[0], p->grid_row[1]) + p->grid_col;
   if (nrec > Uc || !p->part) {
+    double *part = nullptr;
+    if (cudaMalloc(&part, sizeof(double) * 2 * (size_t)nrec) != cudaSuccess) return -1;
     if (p->part) p->allocs.erase(std::find(p->allocs.begin(), p->allocs.end(), (void *)p->part));
     cudaFree(p->part);
-    p->part = nullptr;
-    if (cudaMalloc(&p->part, sizeof(double) * 2 * (size_t)nrec) != cudaSuccess) {
-      *err = "product plan: device allocation failed";
-      return -1;
-    }
+    p->part = part;
     p->allocs.push_back(p->part);
   }
+  p->two_pass = true;
   return 0;
 }
 
@@ -1175,8 +1171,9 @@ static int perm_tasks_build(Sector *s, ProdPlan *p, std::string *err) {
     for (uint32_t a = 0; a < b.n; a += kBlockPiece)
       tasks.push_back(SectorBlock{b.ib, b.row0 + a, b.low0 + a, std::min<uint32_t>(kBlockPiece, b.n - a)});
   }
+  if (upload(p, tasks, &p->perm, err) || upload(p, low, &p->perm_low, err)) return -1;
   p->nperm = (int)tasks.size();
-  return upload(p, tasks, &p->perm, err) || upload(p, low, &p->perm_low, err) ? -1 : 0;
+  return 0;
 }
 
 int prod_plan_build(Sector *s, std::string *err) {
@@ -1365,12 +1362,13 @@ int prod_plan_build(Sector *s, std::string *err) {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, prod_hv_kernel<double>, kProdThreads, smem_r);
   p->grid = std::max(1, std::min(Uc, std::max(1, per_sm) * s->num_sms));
   p->uniform = uniform_hops;
-  if (two_pass_ok && two_pass_build(s, p, rows_dn, rows_up, G, err) != 0) return fail();
+  // without them the one-pass kernel remains
+  if (two_pass_ok && two_pass_build(s, p, rows_dn, rows_up, G, err) != 0) cudaGetLastError();
   p->rank.swap(rank);
   p->pos_dn.swap(pos_dn);
   p->unrank_up.swap(unrank_up);
   p->unrank_dn.swap(unrank_dn);
-  if (perm_tasks_build(s, p, err) != 0) return fail();
+  if (perm_tasks_build(s, p, err) != 0) cudaGetLastError();  // a thread per row then
   s->prod = p;
   return 0;
 }
@@ -1506,10 +1504,10 @@ int prod_te_plan_build(Sector *s, const std::vector<BitTerm> &terms, const std::
   if (wd > 255 || wu > 64) return 0;
   ProdPlan *p = new ProdPlan();
   p->args = base->args;
-  const int rc = two_pass_build(s, p, rows_dn, rows_up, G, err);
-  if (rc != 0 || !p->two_pass) {
+  if (two_pass_build(s, p, rows_dn, rows_up, G, err) != 0) cudaGetLastError();
+  if (!p->two_pass) {
     prod_plan_free(p);
-    return rc;
+    return 0;
   }
   *out = p;
   return 0;
@@ -1535,7 +1533,7 @@ int prod_permute(Sector *s, VecType vt, const void *in, void *out, bool to_nativ
   const ProdPlan *p = s->prod;
   const ProdArgs &a = p->args;
   const bool whole = whole_elements(vt, in);
-  if (s->dim < (int64_t)kPermShort * p->nperm || !whole) {
+  if (p->nperm == 0 || s->dim < (int64_t)kPermShort * p->nperm || !whole) {
     const unsigned nb = (unsigned)std::min<int64_t>((s->dim + kPermThreads - 1) / kPermThreads, (int64_t)s->num_sms * 16);
     auto rows = [&](auto *x, auto *y, auto w) {
       using T = std::remove_reference_t<decltype(*y)>;

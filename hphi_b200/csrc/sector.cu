@@ -462,7 +462,7 @@ int sector_blocks(const Sector *s, std::vector<SectorBlock> *out, std::vector<ui
 }
 
 int sector_pieces(Sector *s, std::string *err) {
-  if (s->d_pieces) return 0;
+  if (s->npieces > 0) return 0;
   std::vector<SectorBlock> blk, pc;
   std::vector<uint32_t> low;
   if (sector_blocks(s, &blk, &low, err) != 0) return -1;
@@ -471,12 +471,20 @@ int sector_pieces(Sector *s, std::string *err) {
   for (const SectorBlock &b : blk)
     for (uint32_t a = 0; a < b.n; a += kBlockPiece)
       pc.push_back(SectorBlock{b.ib, b.row0 + a, b.low0 + a, std::min<uint32_t>(kBlockPiece, b.n - a)});
-  CK(cudaMalloc(&s->d_low, sizeof(uint32_t) * std::max<size_t>(1, low.size())));
-  CK(cudaMemcpy(s->d_low, low.data(), sizeof(uint32_t) * low.size(), cudaMemcpyHostToDevice));
-  SectorBlock *d = nullptr;
-  CK(cudaMalloc(&d, sizeof(SectorBlock) * std::max<size_t>(1, pc.size())));
-  s->d_pieces = d;
-  CK(cudaMemcpy(d, pc.data(), sizeof(SectorBlock) * pc.size(), cudaMemcpyHostToDevice));
+  PlanUpload up;
+  const SectorBlock *d = nullptr;
+  const uint32_t *d_low = nullptr;
+  std::vector<void *> one;
+  up.add(pc, &d);
+  up.add(low, &d_low);
+  if (up.run(&one) != 0) {
+    cudaGetLastError();
+    if (!one.empty()) cudaFree(one[0]);
+    *err = "sector pieces: device allocation or copy failed";
+    return -1;
+  }
+  s->d_pieces = const_cast<SectorBlock *>(d);  // the allocation's address: freed with the sector
+  s->d_low = const_cast<uint32_t *>(d_low);
   s->npieces = (int)pc.size();
   s->nlow = (int)low.size();
   return 0;
@@ -773,7 +781,7 @@ int sector_build(const Model &m, int device, Sector **out, std::string *err, boo
   // faster); HPHI_B200_KERNEL=rowblock builds it at any size.
   // The tile plan takes the grand-canonical sectors from the sizes of hv_gc.cu.
   if (specialise && kname != "general" && kname != "rowblock") {
-    if (gc_plan_build(s, err) != 0) return -1;
+    gc_plan_build(s);
   }
   const bool tiled = s->gcp && gc_applies(s, kComplex128) && (m.complex_terms || gc_applies(s, kReal64));
   if (specialise && kname != "general" && !s->prod && !s->hub && !tiled &&
@@ -783,7 +791,7 @@ int sector_build(const Model &m, int device, Sector **out, std::string *err, boo
   // The block kernel takes whole H*v of the sectors without another plan, and the row pass of the
   // row-block plan (HPHI_B200_RB_SIMPLE keeps that plan's generic row pass).
   if (specialise && kname != "general" && !s->prod && !s->hub && !(s->rb && getenv("HPHI_B200_RB_SIMPLE"))) {
-    if (bk_plan_build(s, s->rb != nullptr, err) != 0) return -1;
+    bk_plan_build(s, s->rb != nullptr);
   }
   *out = s;
   return 0;
@@ -796,7 +804,7 @@ void sector_free(Sector *s) {
   cudaFree(s->d_list_1); cudaFree(s->d_list_2_1); cudaFree(s->d_list_2_2); cudaFree(s->d_diag);
   cudaFree(s->d_terms); cudaFree(s->d_dterms); cudaFree(s->d_red); cudaFree(s->d_scal); cudaFree(s->ws);
   split_plan_free(&s->split);
-  cudaFree(s->d_pieces); cudaFree(s->d_low);
+  cudaFree(s->d_pieces);
   hub_plan_free(s->hub);
   prod_plan_free(s->prod);
   prod_plan_free(s->te_prod);

@@ -1,5 +1,6 @@
 // Checks the block kernel's host tables (block_tables.hpp) of one model against its terms, without
-// a device: argv[1] is a namelist.def of a canonical model of at most 24 bits, or "crowded".  Every index the
+// a device: argv[1] is a namelist.def of a canonical model of at most 24 bits, or "crowded"; with
+// "no_memory" as argv[2], whether the plans decline without a device.  Every index the
 // kernel would form is compared with the room it has, and H*v put together from the tables, the
 // way the kernel does it, with H*v from the terms.  Prints what the tables are like; the exit
 // status is 1, with a message, when something is wrong.
@@ -12,6 +13,8 @@
 #include <random>
 
 #include "block_tables.hpp"
+#include "hv_blocks.hpp"
+#include "hv_gc.hpp"
 
 using namespace hphi;
 using Z = std::complex<double>;
@@ -143,7 +146,34 @@ static void crowded() {
   check(terms, 9, {1, 0}, {SectorBlock{0, 0, 0, 512}}, low, list_1, row_of);
 }
 
+// A plan that cannot have device memory (there is no device) leaves the sector without one: the caller goes
+// on with the kernels that need none.
+static void no_memory(const char *namelist) {
+  Sector s;
+  std::string err;
+  if (read_expert(namelist, &s.model, &err) != 0) fail(err.c_str());
+  s.num_sms = 148;
+  s.gc = s.model.rows_are_configs();
+  s.lo_bits = (s.model.nbits + 1) / 2;
+  s.hi_bits = s.model.nbits - s.lo_bits;
+  s.ihfbit = 1ull << s.lo_bits;
+  s.sdim = 1ull << s.hi_bits;
+  s.dim = sector_dim(s.model);
+  std::vector<uint64_t> list_1((size_t)s.dim);
+  std::vector<uint32_t> l21(s.ihfbit), l22(s.sdim);
+  s.d_list_1 = list_1.data();
+  s.d_list_2_1 = l21.data();
+  s.d_list_2_2 = l22.data();
+  bk_plan_build(&s, false);
+  gc_plan_build(&s);
+  if (s.bk || s.gcp) fail("a plan without a device");
+}
+
 int main(int argc, char **argv) {
+  if (argc == 3 && std::string(argv[2]) == "no_memory") {
+    no_memory(argv[1]);
+    return 0;
+  }
   if (argc == 2 && std::string(argv[1]) == "crowded") {
     crowded();
     printf("\n");

@@ -89,3 +89,12 @@ def test_crowded_bank(checker):
     """More entries on one bank pair than a packed slot count holds: the plan must not lose any."""
     r = subprocess.run([checker, "crowded"], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("gc", [False, True])
+def test_plans_without_device_memory(gc, checker, tmp_path):
+    """The plans are optional: where the device gives no memory for one, opening the sector goes on."""
+    m = expert.kitaev_heisenberg(5, 2, -1.0, 0.3) if gc else expert.heisenberg(12, expert.chain_bonds(12))
+    r = subprocess.run([checker, m.write(str(tmp_path)), "no_memory"], capture_output=True, text=True,
+                       env={**os.environ, "CUDA_VISIBLE_DEVICES": ""})
+    assert r.returncode == 0, r.stdout + r.stderr
