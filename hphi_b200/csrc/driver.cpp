@@ -164,19 +164,39 @@ int cuda_ok(cudaError_t e, const char *what) {
 // Device memory of one driver call.  Mapping and unmapping the vectors cost a short run more than
 // its steps (four 14 MB vectors: 2 of 8 ms), so up to kWorkspaceKeep bytes stay with the sector
 // and the next call carves its vectors from them; what does not fit is allocated and freed by
-// the call, as is everything of a call inside another one on the same handle.
-constexpr size_t kWorkspaceKeep = (size_t)64 << 20;
+// the call, as is everything of a call inside another one on the same handle.  All sectors
+// together keep kWorkspaceKeepAll at most: a program with hundreds of open handles does not pay
+// for those that are idle.
+constexpr int64_t kWorkspaceKeep = (int64_t)64 << 20, kWorkspaceKeepAll = (int64_t)256 << 20;
+std::atomic<int64_t> g_kept{0};  // bytes kept by all sectors
+}  // namespace
+
+void workspace_free(Sector *s) {
+  cudaFree(s->ws);
+  g_kept -= (int64_t)s->ws_bytes;
+  s->ws = nullptr;
+  s->ws_bytes = 0;
+}
+
+namespace {
+
 class Workspace {
  public:
   // bytes: what the call is going to take, each piece rounded up to 256
   Workspace(Sector *s, size_t bytes) : s_(s), mine_(!s->ws_busy.exchange(true)) {
     if (!mine_) return;
-    if (bytes <= s->ws_bytes || bytes > kWorkspaceKeep) return;
+    if (bytes <= s->ws_bytes || bytes > (size_t)kWorkspaceKeep) return;
+    if (g_kept.fetch_add((int64_t)(bytes - s->ws_bytes)) + (int64_t)(bytes - s->ws_bytes) > kWorkspaceKeepAll) {
+      g_kept -= (int64_t)(bytes - s->ws_bytes);
+      return;
+    }
     cudaFree(s->ws);
     s->ws = nullptr;
-    s->ws_bytes = 0;
-    if (cudaMalloc(&s->ws, bytes) == cudaSuccess) s->ws_bytes = bytes;
-    else cudaGetLastError();
+    s->ws_bytes = bytes;
+    if (cudaMalloc(&s->ws, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      workspace_free(s);
+    }
   }
   ~Workspace() {
     for (void *p : own_) cudaFree(p);

@@ -86,8 +86,8 @@ struct Sector {
   unsigned *d_done = nullptr;      // kHvBlockMax counters of finished blocks (grid_sum), zero between launches;
                                    // in the last d_scal slots
   int red_blocks = 0;
-  // Device memory the drivers' calls share (Workspace, driver.cpp): kept between calls up to
-  // kWorkspaceKeep bytes, freed with the sector.
+  // Device memory the drivers' calls share (Workspace, driver.cpp): kept between calls within its
+  // limits, freed with the sector (workspace_free).
   void *ws = nullptr;
   size_t ws_bytes = 0;
   std::atomic<bool> ws_busy{false};  // a call has the workspace; calls inside or beside it allocate their own
@@ -143,6 +143,7 @@ int sector_build(const Model &m, int device, Sector **out, std::string *err, boo
 // idim_max of the model's sector, computed on the host (src/check.c:51-209).
 int64_t sector_dim(const Model &m);
 void sector_free(Sector *s);
+void workspace_free(Sector *s);
 
 // v0 = acc * v0 + s * (H v1) with (acc, s) = d_coef[0..1] read on the device, and the raw
 // sum_r conj(v1[r]) (H v1)[r] written to d_out[0..1] (re, im).  HPhi's mltply

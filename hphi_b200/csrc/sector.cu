@@ -802,7 +802,8 @@ void sector_free(Sector *s) {
   cudaSetDevice(s->device);
   if (s->stream) cudaStreamSynchronize(s->stream);
   cudaFree(s->d_list_1); cudaFree(s->d_list_2_1); cudaFree(s->d_list_2_2); cudaFree(s->d_diag);
-  cudaFree(s->d_terms); cudaFree(s->d_dterms); cudaFree(s->d_red); cudaFree(s->d_scal); cudaFree(s->ws);
+  cudaFree(s->d_terms); cudaFree(s->d_dterms); cudaFree(s->d_red); cudaFree(s->d_scal);
+  workspace_free(s);
   split_plan_free(&s->split);
   cudaFree(s->d_pieces);
   hub_plan_free(s->hub);
