@@ -127,6 +127,7 @@ bool block_tables(const std::vector<BitTerm> &terms, int lo_bits, const std::vec
     const double *im;
     uint32_t nh, nx;
   };
+  const uint32_t longest = two_pass ? kBkListRows : kBkList;
   constexpr int kRun = 64;  // blocks of a piece
   struct Run {
     std::vector<BkRec> rec;
@@ -146,7 +147,7 @@ bool block_tables(const std::vector<BitTerm> &terms, int lo_bits, const std::vec
   std::atomic<bool> fits{true};
   auto list_run = [&](size_t u) {
     Run &r = runs[u];
-    r.rec.reserve((size_t)kRun * std::min<size_t>(hi.size(), kBkList));
+    r.rec.reserve((size_t)kRun * std::min<size_t>(hi.size(), longest));
     const size_t q0 = (size_t)u * kRun, q1 = std::min(b_ib.size(), q0 + kRun);
     for (size_t q = q0; q < q1 && fits; q++) {
       const uint32_t ib = b_ib[q];
@@ -167,7 +168,7 @@ bool block_tables(const std::vector<BitTerm> &terms, int lo_bits, const std::vec
         if (T.im) r.im.push_back(neg ? -h.im : h.im);
         (cross ? l.nx : l.nh)++;
       }
-      if (l.nh + l.nx > (uint32_t)kBkList) fits = false;
+      if (l.nh + l.nx > longest) fits = false;
     }
     size_t at = 0;  // the run's vectors do not move any more
     for (size_t q = q0; q < q1; at += lists[q].nh + lists[q].nx, q++) {

@@ -10,7 +10,8 @@ namespace hphi {
 
 constexpr int kBkGroups = 8;      // lower-half coefficients, up to sign
 constexpr int kBkCross = 64;      // crossing terms
-constexpr int kBkList = 96;       // upper or crossing terms acting on one block
+constexpr int kBkList = 96;       // upper or crossing terms acting on one block: whole products,
+constexpr int kBkListRows = 256;  // row passes (as many crossing terms as the row-block plan takes)
 constexpr uint32_t kBkNone = 0x7FFFu;
 
 struct BkClass {

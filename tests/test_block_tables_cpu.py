@@ -85,6 +85,14 @@ def test_block_tables(name, checker, tmp_path):
         assert "shape" in r.stdout  # the plan applies
 
 
+def test_many_crossing_terms(checker, tmp_path):
+    """100 bonds between the halves, each acting on every block: too many for whole products, not for the
+    row-block plan's row pass."""
+    m = expert.heisenberg(20, [(i, j) for i in range(10) for j in range(10, 20)], two_sz=-14)
+    r = subprocess.run([checker, m.write(str(tmp_path))], capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.startswith("no plan shape"), r.stdout + r.stderr
+
+
 def test_crowded_bank(checker):
     """More entries on one bank pair than a packed slot count holds: the plan must not lose any."""
     r = subprocess.run([checker, "crowded"], capture_output=True, text=True)
