@@ -400,9 +400,10 @@ def run_green_mode(args):
     cl = clocks.stop()
     t = e0.elapsed_time(e1) / 1e3 / args.steps
     n_rows = len(rows)
-    per_pass = 16                                   # real rows evaluated per pass over the sector
-    passes = (n_rows + per_pass - 1) // per_pass
-    stream_bytes = passes * dim * 16.0              # list_1 + the vector, once per pass
+    # an adjoint pair is one entry; 16 off-diagonal entries, or diagonal patterns (the 16 modes of the
+    # lower half and the empty one), per pass
+    passes_off, passes_diag = 16 * 15 // 16, 2
+    stream_bytes = passes_off * dim * 8.0 + passes_diag * dim * 8.0   # the vector, once per pass
     value = n_rows * dim / t / 1e9
     # checks: densities sum to the electron number, every <n_i s> in [0, 1]
     dens = np.array([g[k] for k in range(n_rows) if rows[k, 0] == rows[k, 2]]).real
@@ -422,12 +423,12 @@ def run_green_mode(args):
                "d2h_bytes_per_step": 16 * n_rows, "ms_per_step": 1e3 * te,
                "max_abs_diff_vs_device": float(np.max(np.abs(ge - g)))}
     peak, peak_src = peak_hbm()
-    traffic = profile_traffic("green_kernel", args.workload)
+    traffic = profile_traffic("green_block_kernel", args.workload)
     roof = {"bound": "hbm", "achieved": stream_bytes / t / 1e9, "peak": peak, "unit": "GB/s",
             "frac": stream_bytes / t / 1e9 / peak, "traffic": traffic, "peak_source": peak_src,
-            "kernel": "green_kernel<double,false> + finalize_partials_kernel<16>, one pass per 16 rows; "
-                      "achieved counts 16 bytes per sector row per pass (list_1 and the vector), traffic is "
-                      "DRAM bytes per green_kernel launch"}
+            "kernel": "green_block_kernel (with green_table_kernel) per 16 off-diagonal entries, green_diag_kernel per 16 "
+                      "diagonal patterns; achieved counts 8 bytes per sector row per pass (the vector), traffic is "
+                      "DRAM bytes per green_block_kernel launch"}
     cpu = None
     if not args.no_cpu_baseline:
         sample = 8
@@ -450,7 +451,7 @@ def run_green_mode(args):
                       "rows_desc": "c+_{i s} c_{j s}, i, j = 0..15, s = 0, 1",
                       "l2": "vectors and list_1 (1.3 GB each) exceed L2; no flush"},
            "checks_ok": bool(ok), "roofline": roof, "cpu_baseline": cpu, "e2e": e2e,
-           "gpu_launches": passes * args.steps, "clocks": cl}
+           "gpu_launches": (2 * passes_off + passes_diag + 1) * args.steps, "clocks": cl}
     print(json.dumps(out))
 
 
@@ -774,13 +775,17 @@ def main():
     dim = H.dim
     H_native = bool(H.info.get("native_order"))
     kind = H.info.get("kernel", 0)
-    kname, kdesc = {3: ("prod_two_pass", "prod_row_kernel (row pass) + prod_col_kernel (column pass) per step; "
-                                         "achieved = B_alg / time of both"),
-                    2: ("prod_hv_kernel", "prod_hv_kernel<double> + finalize_partials_kernel<2> per step"),
-                    1: ("hv_hub_pass", "hv_hub_pass<double,0> + hv_hub_pass<double,1> + finalize per step"),
-                    4: ("spin_rowblock", "bk_kernel (row pass) + rb_col_kernel<double,0,4> (column pass) per step; "
-                                         "achieved = B_alg / time of both")}.get(
-        kind, ("hv_row_order", "bk_kernel, gc_tile_kernel or hv_general_kernel"))
+    plan = H.hv_plan(hphi_b200.REAL64)
+    kname, kdesc = {
+        "two_pass": ("prod_two_pass", "prod_row_kernel (row pass) + prod_col_kernel (column pass) per step; "
+                                      "achieved = B_alg / time of both"),
+        "one_pass": ("prod_hv_kernel", "prod_hv_kernel<double> + finalize_partials_kernel<2> per step"),
+        "hubbard_block": ("hv_hub_pass", "hv_hub_pass<double,0> + hv_hub_pass<double,1> + finalize per step"),
+        "rowblock": ("rowblock", ("bk_kernel" if plan["shape"] else "rb_row_kernel") +
+                     " (row pass) + rb_col_kernel (column pass) per step; achieved = B_alg / time of both"),
+        "block": ("bk_kernel", "bk_kernel per step"),
+        "tile": ("gc_tile_kernel", f"gc_tile_kernel, {plan['launches']} passes per step"),
+        "general": ("hv_general", "hv_general_kernel per step")}[plan["kernel"]]
     vt = hphi_b200.REAL64
     gen = torch.Generator(device="cuda").manual_seed(1234 + rank)
     v1 = torch.rand(dim, dtype=torch.float64, device="cuda", generator=gen) - 0.5
@@ -836,7 +841,7 @@ def main():
         e2e = run_e2e(H, v1, dim, world, dist, args)
     H.close()
     shutil.rmtree(tmp, ignore_errors=True)
-    finish(args, H_native, kind, kname, kdesc, desc, dim, balg, value, t_max, achieved, hphi_order_ms, e2e, clocks,
+    finish(args, H_native, kind, plan["launches"], kname, kdesc, desc, dim, balg, value, t_max, achieved, hphi_order_ms, e2e, clocks,
            world, rank, dist)
 
 
@@ -911,7 +916,7 @@ def run_e2e(H, v1, dim, world, dist, args):
             "ms_per_step": te * 1e3}
 
 
-def finish(args, H_native, kind, kname, kdesc, desc, dim, balg, value, t_max, achieved, hphi_order_ms, e2e, clocks,
+def finish(args, H_native, kind, launches, kname, kdesc, desc, dim, balg, value, t_max, achieved, hphi_order_ms, e2e, clocks,
            world, rank, dist):
     if rank != 0:
         if dist:
@@ -944,7 +949,7 @@ def finish(args, H_native, kind, kname, kdesc, desc, dim, balg, value, t_max, ac
                         "frac": achieved / peak, "peak_kind": peak_kind,
                         "traffic": profile_traffic(kname, args.workload),
                         "kernels": kdesc},
-           "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": {1: 3, 2: 2, 3: 2, 4: 2}.get(kind, 1) * args.steps, "clocks": clocks}
+           "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": launches * args.steps, "clocks": clocks}
     if world == 1 and not args.no_modes:
         out["modes"] = run_modes()
     print(json.dumps(out))

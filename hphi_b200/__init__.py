@@ -37,10 +37,11 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 INFO_FIELDS = ["dim", "nsite", "calc_model", "calc_type", "size_list_2_1", "size_list_2_2", "is_gc",
                "vec_type", "n_offdiag", "n_diag", "lanczos_max", "num_ave", "native_order", "exct", "kernel",
                "n_green_one", "n_green_two"]
+HV_KERNELS = ["general", "block", "rowblock", "tile", "hubbard_block", "one_pass", "two_pass"]
 EXPORTED_SYMBOLS = ["hphi_version", "hphi_last_error", "hphi_open_expert", "hphi_close", "hphi_info",
                     "hphi_sz", "hphi_diagonalcalc", "hphi_mltply", "hphi_mltply_device", "hphi_lanczos",
                     "hphi_lanczos_eigenvector", "hphi_tpq", "hphi_tpq_vectors", "hphi_tem", "hphi_run", "hphi_inspect_terms",
-                    "hphi_lanczos_tridiagonal", "hphi_mltply_device_async", "hphi_stream",
+                    "hphi_lanczos_tridiagonal", "hphi_hv_plan", "hphi_mltply_device_async", "hphi_stream",
                     "hphi_synchronize", "hphi_to_native", "hphi_from_native", "hphi_mltply_device_noalloc",
                     "hphi_lanczos_steps", "hphi_batch_create", "hphi_batch_lanczos", "hphi_batch_tuning",
                     "hphi_batch_free", "hphi_server_create", "hphi_server_submit", "hphi_server_step",
@@ -91,6 +92,7 @@ def load_library() -> ctypes.CDLL:
     lib.hphi_diagonalcalc.argtypes = [P, pd]
     lib.hphi_mltply.argtypes = [P, pd, pd, pd]
     lib.hphi_mltply_device.argtypes = [P, I, VP, VP, D, D, pd]
+    lib.hphi_hv_plan.argtypes = [P, I, ctypes.POINTER(ctypes.c_int64), I]
     lib.hphi_lanczos.argtypes = [P, pd, ctypes.c_char_p, pd, I]
     lib.hphi_lanczos_eigenvector.argtypes = [P, pd]
     lib.hphi_tpq.argtypes = [P, pd, ctypes.c_char_p, pd, I]
@@ -249,6 +251,13 @@ class Hamiltonian:
     @property
     def handle(self) -> ctypes.c_void_p:
         return self._h
+
+    def hv_plan(self, vec_type: int) -> dict:
+        """The kernels of an H*v on vectors of this type (hphi_hv_plan): their name, launches per
+        product, and shape."""
+        v = (ctypes.c_int64 * 3)()
+        _check(load_library().hphi_hv_plan(self._h, vec_type, v, 3))
+        return {"kernel": HV_KERNELS[v[0]], "launches": v[1], "shape": v[2]}
 
     # ------------------------------------------------------------ reference ops
     def sz(self):

@@ -182,6 +182,19 @@ int hphi_info(const hphi_handle *h, int64_t *info, int n) {
   return 0;
 }
 
+int hphi_hv_plan(const hphi_handle *h, int vec_type, int64_t *plan, int n) {
+  CHECK_HANDLE(h);
+  if (vec_type != HPHI_REAL64 && vec_type != HPHI_COMPLEX128) { set_error("bad vec_type"); return -1; }
+  if (vec_type == HPHI_REAL64 && h->sector->model.complex_terms) {
+    set_error("H has complex coefficients: real vectors are not allowed");
+    return -1;
+  }
+  const HvPlan p = hv_plan(h->sector, (VecType)vec_type);
+  const int64_t v[3] = {p.kernel, p.launches, p.shape};
+  for (int i = 0; i < n && i < 3; i++) plan[i] = v[i];
+  return 0;
+}
+
 int hphi_sz(const hphi_handle *h, uint64_t *list_1, uint64_t *list_2_1, uint64_t *list_2_2) {
   CHECK_HANDLE(h);
   const Sector &s = *h->sector;

@@ -158,6 +158,11 @@ inline bool whole_elements(VecType vt, const void *v) { return vt == kReal64 || 
 // The kernels of an H*v in HPhi's row order from the vector v1.
 enum HvRoute : int { kRouteGeneral = 0, kRouteBlock, kRouteRowBlock, kRouteTile };
 HvRoute hv_route(const Sector *s, VecType vt, const void *d_v1);
+// hphi_hv_plan
+struct HvPlan {
+  int kernel, launches, shape;
+};
+HvPlan hv_plan(const Sector *s, VecType vt);
 
 // Native vector order: HPhi order unless a specialised plan defines its own (then an
 // exact per-block permutation of it).  hv_native runs the fastest kernel on native

@@ -15,6 +15,7 @@
 
 #include <algorithm>
 
+#include "../../include/hphi_b200.h"
 #include "device_util.cuh"
 #include "engine.hpp"
 #include "hv_blocks.hpp"
@@ -266,6 +267,21 @@ HvRoute hv_route(const Sector *s, VecType vt, const void *d_v1) {
   if (rb_applies(s, vt) && (whole || rb_own_rows(s, vt))) return kRouteRowBlock;
   if (whole && bk_applies(s)) return kRouteBlock;
   return kRouteGeneral;
+}
+
+HvPlan hv_plan(const Sector *s, VecType vt) {
+  if (s->prod) {
+    const int row = prod_row_words(s);
+    return row ? HvPlan{HPHI_HV_TWO_PASS, 2, row} : HvPlan{HPHI_HV_ONE_PASS, 2, 0};
+  }
+  if (s->hub) return HvPlan{HPHI_HV_HUBBARD_BLOCK, 3, 0};
+  switch (hv_route(s, vt, nullptr)) {
+    case kRouteTile: return HvPlan{HPHI_HV_TILE, gc_passes(s, vt), 0};
+    case kRouteRowBlock: return HvPlan{HPHI_HV_ROWBLOCK, 2, bk_row_pass(s) ? 1 : 0};
+    case kRouteBlock: return HvPlan{HPHI_HV_BLOCK, 1, bk_shape(s)};
+    case kRouteGeneral: break;
+  }
+  return HvPlan{HPHI_HV_GENERAL, 1, 0};
 }
 
 int hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,

@@ -426,6 +426,7 @@ void bk_plan_build(Sector *s, bool two_pass) {
 }
 
 bool bk_applies(const Sector *s) { return s->bk && !s->bk->two_pass; }
+int bk_shape(const Sector *s) { return s->bk->shape; }
 bool bk_row_pass(const Sector *s) { return s->bk && s->bk->two_pass; }
 
 int bk_grid(const Sector *s, VecType vt) {

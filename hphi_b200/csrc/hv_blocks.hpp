@@ -12,6 +12,7 @@ void bk_plan_build(Sector *s, bool two_pass);
 void bk_plan_free(BlockPlan *p);
 bool bk_applies(const Sector *s);   // whole H*v in one launch
 bool bk_row_pass(const Sector *s);  // the row-block plan's row pass
+int bk_shape(const Sector *s);      // kBkShapeDefs
 size_t bk_scratch_doubles(const Sector *s);
 int bk_grid(const Sector *s, VecType vt);  // CTAs (records of partial sums) of a launch
 // v0 = coef[0] * v0 + coef[1] * H v1, sum conj(v1) (H v1) to d_out (and lt); with d_out null the

@@ -490,6 +490,8 @@ void gc_plan_build(Sector *s) {
 
 bool gc_applies(const Sector *s, VecType vt) { return s->gcp && !s->gcp->pass[vt == kReal64 ? 0 : 1].empty(); }
 
+int gc_passes(const Sector *s, VecType vt) { return (int)s->gcp->pass[vt == kReal64 ? 0 : 1].size(); }
+
 size_t gc_scratch_doubles(const Sector *s, VecType vt) {
   const int v = vt == kReal64 ? 0 : 1;
   return 2 * s->gcp->pass[v].size() * (size_t)s->gcp->grid[v];

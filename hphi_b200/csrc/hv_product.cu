@@ -1376,6 +1376,8 @@ int prod_plan_build(Sector *s, std::string *err) {
 // The kernel number that hphi_info reports: 3 for hops of one real magnitude per species.
 bool prod_two_pass(const Sector *s) { return s->prod && s->prod->two_pass && s->prod->uniform; }
 
+int prod_row_words(const Sector *s) { return s->prod->two_pass ? s->prod->stride : 0; }
+
 size_t prod_scratch_doubles(const Sector *s, VecType vt) {
   const ProdPlan *p = s->prod;
   // the two-pass kernels keep one partial sum per CTA of each pass, the one-pass kernel one per

@@ -19,6 +19,8 @@ int prod_hv_launch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const do
 int prod_hv_launch_scratch(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out,
                            double *d_part, int *d_counter);
 size_t prod_scratch_doubles(const Sector *s, VecType vt);
+// Words of a row's plane in the two-pass kernels, 0 where the one-pass kernel runs.
+int prod_row_words(const Sector *s);
 // True when real vectors take the two-pass kernels (row pass + column pass).
 bool prod_two_pass(const Sector *s);
 int prod_hv_launch_rows(Sector *s, VecType vt, const void *d_v1, void *d_v0, const double *d_coef, double *d_out);

@@ -40,7 +40,7 @@ typedef struct hphi_handle hphi_handle;
 #define HPHI_INFO_NUM_AVE 11
 #define HPHI_INFO_NATIVE_ORDER 12 /* 1 if the engine's native vector order differs from HPhi's */
 #define HPHI_INFO_EXCT 13         /* exct: states of LOBPCG / the Lanczos eigenvector index */
-#define HPHI_INFO_KERNEL 14       /* native H*v kernel: 0 general, 1 Hubbard block plan, 2 Hubbard product layout, 3 product layout two-pass (real vectors), 4 spin row-block passes */
+#define HPHI_INFO_KERNEL 14       /* vector layout and plan, as a sector opens: 0 HPhi's rows (which kernel: hphi_hv_plan), 1 Hubbard block plan, 2 Hubbard product layout, 3 the same with hops of one real magnitude, 4 row-block plan */
 #define HPHI_INFO_N_GREEN_ONE 15  /* OneBodyG rows read (NCisAjt) */
 #define HPHI_INFO_N_GREEN_TWO 16  /* TwoBodyG rows read (NCisAjtCkuAlvDC) */
 #define HPHI_INFO_COUNT 17
@@ -92,6 +92,22 @@ void hphi_close(hphi_handle *h);
 int hphi_info(const hphi_handle *h, int64_t *info, int n);
 
 /*
+ * The kernels that an H*v on vectors of type vec_type takes (in native order; vectors whose complex
+ * elements are not at multiples of 16 bytes may take others).  Fills plan[0 .. min(n, 3)):
+ * [0] HPHI_HV_*  [1] kernel launches per product  [2] HPHI_HV_BLOCK: the shape of its planes;
+ * HPHI_HV_TWO_PASS: doubles of a row's plane; HPHI_HV_ROWBLOCK: 1 where the block kernel is its row
+ * pass; else 0.  -1 where H*v refuses the type.  No counterpart in the reference.
+ */
+#define HPHI_HV_GENERAL 0        /* a thread per row, every sector */
+#define HPHI_HV_BLOCK 1          /* blocks of rows in shared memory (canonical sectors) */
+#define HPHI_HV_ROWBLOCK 2       /* row pass and column pass over blocks */
+#define HPHI_HV_TILE 3           /* passes over tiles (grand-canonical sectors) */
+#define HPHI_HV_HUBBARD_BLOCK 4  /* HPHI_B200_KERNEL=block */
+#define HPHI_HV_ONE_PASS 5       /* Hubbard product layout */
+#define HPHI_HV_TWO_PASS 6       /* Hubbard product layout, row pass and column pass */
+int hphi_hv_plan(const hphi_handle *h, int vec_type, int64_t *plan, int n);
+
+/*
  * Copies the sector tables in HPhi's layout: list_1[0 .. dim] (element 0 unused),
  * list_2_1[0 .. SizeOflist_2_1), list_2_2[0 .. SizeOflist_2_2), as filled by
  * sz() (src/sz.c:62-832).  Any pointer may be NULL.  Fails for grand-canonical models,
@@ -113,7 +129,9 @@ int hphi_mltply(hphi_handle *h, double *v0, const double *v1, double *prdct);
 /*
  * Device form of mltply: d_v0 = acc * d_v0 + scale * (H d_v1) on 0-based device vectors
  * of element type vec_type (acc == 0 never reads d_v0), and prdct (host, 2 doubles) =
- * sum conj(d_v1) (H d_v1).  Runs on the handle's stream and waits for it.
+ * sum conj(d_v1) (H d_v1).  Runs on the handle's stream and waits for it.  Device vectors start
+ * at a multiple of 8 bytes, here and below; complex vectors in a native order of its own
+ * (HPHI_INFO_NATIVE_ORDER 1) at a multiple of 16.
  * Replaces: mltply (src/mltply.c:56-132) for callers that keep vectors on the device.
  */
 int hphi_mltply_device(hphi_handle *h, int vec_type, void *d_v0, const void *d_v1, double acc, double scale,

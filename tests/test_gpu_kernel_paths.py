@@ -1,7 +1,8 @@
 """Every H*v path against the general row kernel (HPHI_B200_KERNEL=general, itself pinned to the
 reference by test_gpu_parity) at the sizes where a path can go wrong: the shapes of the row, block
 and tile kernels and one below and above their limits, odd row lengths, one-row sectors,
-coefficient groups up to and past what a plan holds."""
+coefficient groups up to and past what a plan holds.  Each case names the kernel it is there for,
+which the engine has to report (hv_plan, the decision its launches take)."""
 import os
 
 import numpy as np
@@ -27,14 +28,22 @@ def _open(path, general=False):
             os.environ["HPHI_B200_KERNEL"] = saved
 
 
-def _compare(m, tmp_path, vts=(hphi_b200.REAL64, hphi_b200.COMPLEX128)):
-    """v0 = acc v0 + scale H v1 and <v1|H|v1> in HPhi's order, both paths.  Bound: a row sums at most
+def _compare(m, tmp_path, vts=(hphi_b200.REAL64, hphi_b200.COMPLEX128), plan=None):
+    """v0 = acc v0 + scale H v1 and <v1|H|v1>, both paths: mltply_device on vectors in HPhi's order and
+    mltply_device_async between the changes of order, as the drivers' loops run (the product layout has
+    kernels of its own for complex vectors there).  plan: the kernel expected for each vector type.
+    Bound: a row sums at most
     ~200 products in another order, so |difference| <= 200 eps |H| |v| elementwise; 1e-13 of the
     largest element leaves a margin for the sums' size."""
     path = m.write(str(tmp_path))
     Ha, Hg = _open(path), _open(path, general=True)
     try:
         for vt in vts:
+            if plan is not None:
+                got = Ha.hv_plan(vt)
+                want = plan if isinstance(plan, tuple) else (plan, None)
+                assert got["kernel"] == want[0] and want[1] in (None, got["shape"]), got
+            assert Hg.hv_plan(vt)["kernel"] == "general"
             dt = torch.float64 if vt == hphi_b200.REAL64 else torch.complex128
             g = torch.Generator(device="cuda").manual_seed(7)
             v1 = torch.randn(Ha.dim, dtype=dt, device="cuda", generator=g)
@@ -50,6 +59,17 @@ def _compare(m, tmp_path, vts=(hphi_b200.REAL64, hphi_b200.COMPLEX128)):
                 assert (out[0] - out[1]).abs().max().item() <= 1e-13 * big
                 n = torch.linalg.vector_norm(v1).item() * torch.linalg.vector_norm(out[1]).item()
                 assert abs(pr[0] - pr[1]) <= 1e-13 * max(n, abs(pr[1]))
+                a, b, o = (torch.zeros_like(v1) for _ in range(3))
+                coef = torch.tensor([acc, scale], dtype=torch.float64, device="cuda")
+                pa = torch.zeros(2, dtype=torch.float64, device="cuda")
+                w0 = w if acc else torch.full_like(w, float("nan"))
+                torch.cuda.synchronize()
+                Ha.to_native(v1.data_ptr(), a.data_ptr(), vt)
+                Ha.to_native(w0.data_ptr(), b.data_ptr(), vt)
+                Ha.mltply_device_async(b.data_ptr(), a.data_ptr(), vt, coef.data_ptr(), pa.data_ptr())
+                Ha.from_native(b.data_ptr(), o.data_ptr(), vt)
+                assert (o - out[1]).abs().max().item() <= 1e-13 * big
+                assert abs(complex(*pa.tolist()) - pr[1]) <= 1e-13 * max(n, abs(pr[1]))
         return Ha.info["kernel"]
     finally:
         Ha.close()
@@ -66,9 +86,11 @@ def _dm_chain(L, two_sz):
 
 
 def _couplings(L, n):
-    """A chain whose exchange couplings take n different values."""
+    """A chain whose bonds within the lower half take n different couplings."""
     b = expert.chain_bonds(L) + expert.chain_bonds(L, 2)
-    return expert.heisenberg(L, b, [1.0 + 0.1 * (k % n) for k in range(len(b))], two_sz=L % 2)
+    lower = [x for x in b if max(x) < L // 2]
+    assert n <= len(lower)
+    return expert.heisenberg(L, b, [1.0 + 0.1 * (lower.index(x) % n if x in lower else 0) for x in b], two_sz=L % 2)
 
 
 def _nconserved(L, ne):
@@ -79,38 +101,39 @@ def _nconserved(L, ne):
     return m
 
 
-BLOCK = {
+BLOCK = {   # name: (shape of the planes, or the kernel instead of the block kernel; model)
     # longest blocks of 1, 3, 6, 70, 252, 924, 1716, 3432, 6435 and 12870 rows: every plane shape
-    "chain2": lambda: expert.heisenberg(2, [(0, 1)]),
-    "chain3": lambda: expert.heisenberg(3, expert.chain_bonds(3), two_sz=1),
-    "chain5": lambda: expert.heisenberg(5, expert.chain_bonds(5), two_sz=-1),
-    "chain16": lambda: expert.heisenberg(16, expert.chain_bonds(16)),
-    "j1j2_19": lambda: expert.heisenberg(19, expert.chain_bonds(19) + expert.chain_bonds(19, 2), two_sz=1),
-    "square4x6": lambda: expert.heisenberg(24, expert.square_bonds(4, 6)),
-    "chain26_few": lambda: expert.heisenberg(26, expert.chain_bonds(26), two_sz=-12),
-    "chain28_few": lambda: expert.heisenberg(28, expert.chain_bonds(28), two_sz=-14),
-    "chain30_few": lambda: expert.heisenberg(30, expert.chain_bonds(30), two_sz=-16),
-    "chain32_few": lambda: expert.heisenberg(32, expert.chain_bonds(32), two_sz=-16),
-    "groups8": lambda: _couplings(12, 8),
-    "groups9": lambda: _couplings(12, 9),     # more than a plan holds: the general kernel
-    "kondo4": lambda: expert.kondo_chain(4, 1.0, 1.5, U=2.0),
-    "kondo7_odd": lambda: expert.kondo_chain(6, 1.0, 0.7, ncond=5, two_sz=1),
+    "chain2": (0, lambda: expert.heisenberg(2, [(0, 1)])),
+    "chain3": (0, lambda: expert.heisenberg(3, expert.chain_bonds(3), two_sz=1)),
+    "chain5": (0, lambda: expert.heisenberg(5, expert.chain_bonds(5), two_sz=-1)),
+    "chain16": (0, lambda: expert.heisenberg(16, expert.chain_bonds(16))),
+    "j1j2_19": (1, lambda: expert.heisenberg(19, expert.chain_bonds(19) + expert.chain_bonds(19, 2), two_sz=1)),
+    "square4x6": (3, lambda: expert.heisenberg(24, expert.square_bonds(4, 6))),
+    "chain26_few": (4, lambda: expert.heisenberg(26, expert.chain_bonds(26), two_sz=-12)),
+    "chain28_few": (5, lambda: expert.heisenberg(28, expert.chain_bonds(28), two_sz=-14)),
+    "chain30_few": (6, lambda: expert.heisenberg(30, expert.chain_bonds(30), two_sz=-16)),
+    "chain32_few": (7, lambda: expert.heisenberg(32, expert.chain_bonds(32), two_sz=-16)),
+    "groups8": (0, lambda: _couplings(12, 8)),
+    "groups9": ("general", lambda: _couplings(12, 9)),     # more than a plan holds
+    "kondo4": (0, lambda: expert.kondo_chain(4, 1.0, 1.5, U=2.0)),
+    "kondo7_odd": (0, lambda: expert.kondo_chain(6, 1.0, 0.7, ncond=5, two_sz=1)),
     # few blocks, longer than one turn of a CTA's threads: shared out over several tasks
-    "kondo8": lambda: expert.kondo_chain(8, 1.0, 1.5),
-    "spin1_14": lambda: expert.general_heisenberg([2] * 14, expert.chain_bonds(14), 1.0, two_sz=0),
-    "spin1": lambda: expert.general_heisenberg([2] * 7, expert.chain_bonds(7), 1.0, D=0.3),
-    "mixed_spins": lambda: expert.general_heisenberg([1, 2, 3, 1, 2, 3], expert.chain_bonds(6), 0.8, two_sz=2),
-    "nconserved": lambda: _nconserved(6, 5),
+    "kondo8": (2, lambda: expert.kondo_chain(8, 1.0, 1.5)),
+    "spin1_14": (3, lambda: expert.general_heisenberg([2] * 14, expert.chain_bonds(14), 1.0, two_sz=0)),
+    "spin1": (0, lambda: expert.general_heisenberg([2] * 7, expert.chain_bonds(7), 1.0, D=0.3)),
+    "mixed_spins": (0, lambda: expert.general_heisenberg([1, 2, 3, 1, 2, 3], expert.chain_bonds(6), 0.8, two_sz=2)),
+    "nconserved": (0, lambda: _nconserved(6, 5)),
 }
 
 
 @pytest.mark.parametrize("name", list(BLOCK))
 def test_block_kernel(name, tmp_path):
-    assert _compare(BLOCK[name](), tmp_path) == 0
+    want, make = BLOCK[name]
+    assert _compare(make(), tmp_path, plan=want if isinstance(want, str) else ("block", want)) == 0
 
 
 def test_block_kernel_complex_coefficients(tmp_path):
-    _compare(_dm_chain(14, 0), tmp_path, vts=(hphi_b200.COMPLEX128,))
+    _compare(_dm_chain(14, 0), tmp_path, vts=(hphi_b200.COMPLEX128,), plan="block")
 
 
 def _spin_gc(n, field, seed=3):
@@ -139,25 +162,33 @@ def _hubbard_gc(L, complex_t=False, four_body=False):
     return m
 
 
-GC = {
-    "kitaev18": lambda: _spin_gc(18, None),            # the smallest sector with tiles
-    "kitaev18_field": lambda: _spin_gc(18, "real"),
-    "chain17": lambda: _spin_gc(17, "real"),           # below it
-    "chain19": lambda: _spin_gc(19, "real"),
-    "hubbard9": lambda: _hubbard_gc(9),                # signs over bits inside and outside a tile
-    "hubbard10": lambda: _hubbard_gc(10),
-    "hubbard9_four_body": lambda: _hubbard_gc(9, four_body=True),
+GC = {   # name: (kernels of real and complex vectors, model)
+    # below, at and above the sizes from which tiles are taken (2^19 rows complex, 2^20 real, 2^24 real with signs)
+    "chain17": ("general", "general", lambda: _spin_gc(17, "real")),
+    "kitaev18": ("general", "general", lambda: _spin_gc(18, None)),
+    "kitaev18_field": ("general", "general", lambda: _spin_gc(18, "real")),
+    "chain19": ("general", "tile", lambda: _spin_gc(19, "real")),
+    "chain20": ("tile", "tile", lambda: _spin_gc(20, "real")),
+    "kitaev20": ("tile", "tile", lambda: expert.kitaev_heisenberg(5, 2, -1.0, 0.3)),
+    "hubbard9": ("general", "general", lambda: _hubbard_gc(9)),
+    "hubbard10": ("general", "tile", lambda: _hubbard_gc(10)),   # signs over bits inside and outside a tile
+    "hubbard12": ("tile", "tile", lambda: _hubbard_gc(12)),
+    "hubbard9_four_body": ("general", "general", lambda: _hubbard_gc(9, four_body=True)),
+    "hubbard10_four_body": ("general", "general", lambda: _hubbard_gc(10, four_body=True)),
 }
 
 
+@pytest.mark.parametrize("vt", [hphi_b200.REAL64, hphi_b200.COMPLEX128])
 @pytest.mark.parametrize("name", list(GC))
-def test_tile_kernel(name, tmp_path):
-    _compare(GC[name](), tmp_path)
+def test_tile_kernel(name, vt, tmp_path):
+    _compare(GC[name][2](), tmp_path, vts=(vt,), plan=GC[name][vt])
 
 
-@pytest.mark.parametrize("m", [lambda: _spin_gc(18, "complex"), lambda: _hubbard_gc(9, complex_t=True)])
-def test_tile_kernel_complex_coefficients(m, tmp_path):
-    _compare(m(), tmp_path, vts=(hphi_b200.COMPLEX128,))
+@pytest.mark.parametrize("m, plan", [(lambda: _spin_gc(18, "complex"), "general"), (lambda: _spin_gc(20, "complex"), "tile"),
+                                     (lambda: _hubbard_gc(9, complex_t=True), "general"),
+                                     (lambda: _hubbard_gc(10, complex_t=True), "tile")])
+def test_tile_kernel_complex_coefficients(m, plan, tmp_path):
+    _compare(m(), tmp_path, vts=(hphi_b200.COMPLEX128,), plan=plan)
 
 
 def _hubbard(N, nup, ndown, phases=0, anisotropic=0):
@@ -170,31 +201,33 @@ def _hubbard(N, nup, ndown, phases=0, anisotropic=0):
     return m
 
 
-PROD = {
+PROD = {   # name: (words of a row's plane, 0 for the one-pass kernel; model)
     # rows of 924, 1287 (odd), 1716, 3432, 5005 (odd) and 8008 elements: every row shape, both loads
-    "n12": lambda: _hubbard(12, 3, 6),
-    "n13": lambda: _hubbard(13, 2, 5),
-    "n13_6": lambda: _hubbard(13, 3, 6),
-    "n14": lambda: _hubbard(14, 2, 7),
-    "n15": lambda: _hubbard(15, 2, 6),
-    "n16": lambda: _hubbard(16, 2, 6),
-    "n7_odd": lambda: _hubbard(7, 3, 3),
-    "one_row": lambda: _hubbard(6, 6, 3),
-    "one_column": lambda: _hubbard(6, 3, 6),
-    "two_amplitudes": lambda: _hubbard(10, 5, 4, anisotropic=1),
-    "eight_amplitudes": lambda: _hubbard(10, 5, 4, anisotropic=8),
-    "ten_amplitudes": lambda: _hubbard(10, 5, 4, anisotropic=10),   # past the groups: the one-pass kernel
+    "n12": (960, lambda: _hubbard(12, 3, 6)),
+    "n13": (1744, lambda: _hubbard(13, 2, 5)),
+    "n13_6": (1744, lambda: _hubbard(13, 3, 6)),
+    "n14": (3456, lambda: _hubbard(14, 2, 7)),
+    "n15": (6560, lambda: _hubbard(15, 2, 6)),
+    "n16": (12896, lambda: _hubbard(16, 2, 6)),
+    "n7_odd": (960, lambda: _hubbard(7, 3, 3)),
+    "one_row": (960, lambda: _hubbard(6, 6, 3)),
+    "one_column": (960, lambda: _hubbard(6, 3, 6)),
+    "two_amplitudes": (960, lambda: _hubbard(10, 5, 4, anisotropic=1)),
+    "eight_amplitudes": (960, lambda: _hubbard(10, 5, 4, anisotropic=8)),
+    "ten_amplitudes": (0, lambda: _hubbard(10, 5, 4, anisotropic=10)),   # past the groups: the one-pass kernel
 }
 
 
 @pytest.mark.parametrize("name", list(PROD))
 def test_product_layout(name, tmp_path):
-    assert _compare(PROD[name](), tmp_path) in (2, 3)
+    words, make = PROD[name]
+    assert _compare(make(), tmp_path, plan=("two_pass", words) if words else "one_pass") in (2, 3)
 
 
 @pytest.mark.parametrize("phases", [1, 3, 10])
 def test_product_layout_complex_coefficients(phases, tmp_path):
-    _compare(_hubbard(10, 5, 4, phases=phases), tmp_path, vts=(hphi_b200.COMPLEX128,))
+    _compare(_hubbard(10, 5, 4, phases=phases), tmp_path, vts=(hphi_b200.COMPLEX128,),
+             plan="two_pass" if phases < 10 else "one_pass")
 
 
 @pytest.mark.parametrize("N, nup, ndown", [(1, 1, 0), (5, 2, 3), (8, 4, 4), (11, 5, 6), (12, 6, 6)])
@@ -331,6 +364,7 @@ def test_complex_vectors_at_8_byte_boundaries(name, tmp_path, monkeypatch):
         monkeypatch.setenv("HPHI_B200_KERNEL", kernel)
     C = hphi_b200.COMPLEX128
     with hphi_b200.Hamiltonian(make().write(str(tmp_path))) as H:
+        assert H.hv_plan(C)["kernel"] == {"block": "block", "row_block": "rowblock", "tiles": "tile"}.get(name, "two_pass")
         g = torch.Generator(device="cuda").manual_seed(3)
         v1, w = (torch.randn(H.dim, dtype=torch.complex128, device="cuda", generator=g) for _ in range(2))
         p1, _, keep = _odd_copy(v1)

@@ -29,7 +29,7 @@ CASES = {
     "hubbard3x4": (lambda: expert.hubbard(12, expert.square_bonds(3, 4), 1.0, 8.0, 6, 6), False, 1, 3, {}),
     # the half-filled 4x4 sector of the headline workload (dim 165,636,900)
     "hubbard4x4": (lambda: expert.hubbard(16, expert.square_bonds(4, 4), 1.0, 8.0, 8, 8), False, 1, 3, {}),
-    # product-layout plan, complex vectors: the one-pass kernel
+    # product-layout plan, complex vectors and hops: the two-pass kernels
     "hubbard_chain10_complex": (lambda: _complex_hubbard_chain(10), True, 1, 2, {}),
     # block plan of canonical Hubbard sectors (its counter and partial sums live in the array)
     "hubbard3x4_block": (lambda: expert.hubbard(12, expert.square_bonds(3, 4), 1.0, 8.0, 6, 6), False, 1, 1,
@@ -84,8 +84,8 @@ def test_noalloc_matches_async_on_two_calls(name, tmp_path, monkeypatch):
 
 
 def test_noalloc_refuses_sector_beyond_fixed_scratch(tmp_path):
-    """Complex vectors on the product-layout plan keep one partial sum per up-spin row: with
-    11,440 rows (16 sites, 7 up and 1 down electron) that is more than the array holds, so the
+    """Complex vectors on the product-layout plan are counted one partial sum per up-spin row (the
+    one-pass kernel's; the two-pass kernels need fewer): with 11,440 rows (16 sites, 7 up and 1 down electron) that is more than the array holds, so the
     call is refused with an error instead of writing past the array."""
     L = 16
     m = _complex_hubbard_chain(L)
