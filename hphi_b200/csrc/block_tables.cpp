@@ -306,10 +306,10 @@ bool block_pair(const BlockTables &t, size_t q) {
 }
 
 // Whole blocks, unless they are fewer than kBkWaves tasks per resident CTA: then at most that
-// share of the rows each, but no less than one turn of the threads (8-site Kondo chain, a step:
-// 36.4 us with whole blocks, 33.8 shared out.  Where there are more tasks the second staging of
-// a block costs more than the even end gives: 24-site J1-J2 chain, 2.8 tasks per CTA, 105 us
-// whole and 113 in halves).
+// share of the rows each, but no less than one turn of the threads.  us per H*v (real) with whole
+// blocks, shares for 2 tasks per CTA, and for 8: 23-site J1-J2 chain 48.7, 42.6, 44.0; 22 sites 30.9,
+// 28.8, 28.7; 8-site Kondo 32.5, 29.4, 29.4; spin-1 chain of 14 sites 27.1, 24.5, 24.5.  Where there are
+// more blocks the second staging costs more than the even end gives: 24 sites 77.7, 77.7, 81.4.
 std::vector<BkTask> block_tasks(const BlockTables &t, bool cplx, int ctas) {
   std::vector<BkTask> tk;
   int64_t total = 0;

@@ -50,8 +50,15 @@ constexpr BkShapeDef kBkShapeDefs[] = {
     {1744, 2, 2, 2, 256, 2},  {3456, 2, 2, 2, 256, 2},  {6560, 2, 2, 2, 512, 1},   {12896, 2, 2, 2, 1024, 1},
 };
 constexpr int kBkShapes = 8;
-constexpr int kBkWaves = 2;   // tasks per resident CTA that long blocks are shared out to
-constexpr int kBkLong = 320;  // mean block length from which 128 threads share a task of 960-word planes
+// Tasks per resident CTA that long blocks are shared out to (block_tasks).
+constexpr int kBkWaves = 2;
+// Mean block length, as a row sees it, from which 128 threads share a task of 960-word planes
+// (else 64).  us per H*v with 128 and with 64 threads, real | complex, by mean length: 23-site chain
+// 757: 42 / 55 | 65 / 67, 22 sites 395: 29 / 33 | 40 / 46, spin-1 chain of 13 sites 326: 12.6 / 16.1 |
+// 15.6 / 21.2; below, it depends on the sector: 24 sites with 2Sz = -12, 278: 17.2 / 21.4 | 31 / 24,
+// spin-3/2 of 12 sites with 2Sz = 14, 286: 35 / 28 | 38 / 48, 8-site Kondo 234: 28.5 / 29.5 | 38.6 / 41.6,
+// 24 sites with 2Sz = -14, 183: 15.5 / 14.0 | 23.6 / 19.5.
+constexpr int kBkLong = 320;
 
 struct BlockTables {
   std::vector<BkClass> cls;

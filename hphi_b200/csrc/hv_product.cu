@@ -669,7 +669,12 @@ template <> __device__ __forceinline__ cplx signed_v<cplx>(const cplx &x, uint32
 
 constexpr int kPermThreads = 256;
 constexpr int kPermBatch = 4;    // elements in flight per thread
-constexpr int kPermShort = 32;   // mean rows per HPhi block below which a thread takes a row
+// Mean rows per HPhi block (piece) below which a thread takes a row.  us per call, blocks and rows, to
+// native | from native, with the wait of the call in each: 12 sites with 3 + 3 electrons (27 rows) 13.0 /
+// 12.5 | 14.9 / 12.6; 15 with 4 + 4 (115) 19.9 / 18.5 | 24.0 / 18.2; 14 with 5 + 5 (278, 4 M rows) 25.7 / 25.3 |
+// 30.1 / 27.0; 14 half filled (719, 12 M) 57 / 89 | 57 / 64; 4x4 with 6 + 6 (64 M) 233 / 594 | 259 / 274.
+// (Down configurations in rank order; the long blocks' gain is in the change to native order.)
+constexpr int kPermShort = 32;
 
 // HPhi order -> native: a CTA per up configuration u.  HPhi's row of (u, d) is
 // list_2_1[lower half] + list_2_2[upper half] - 3; with u fixed each term depends on the downs

@@ -776,9 +776,9 @@ int sector_build(const Model &m, int device, Sector **out, std::string *err, boo
   if (specialise && kname != "general" && !s->prod) {
     if (hub_plan_build(s, err) != 0) return -1;
   }
-  // Row-block plan (spin sectors): from 2^24 rows up, where the vectors no longer stay in L2
-  // and the general kernel's scattered gathers go to memory (below that the general kernel is
-  // faster); HPHI_B200_KERNEL=rowblock builds it at any size.
+  // Row-block plan (spin sectors, grand-canonical ones without tiles): from 2^24 rows up, where the
+  // vectors no longer stay in L2; below, a canonical sector is one launch of the block kernel.
+  // HPHI_B200_KERNEL=rowblock builds it at any size.
   // The tile plan takes the grand-canonical sectors from the sizes of hv_gc.cu.
   if (specialise && kname != "general" && kname != "rowblock") {
     gc_plan_build(s);
