@@ -198,11 +198,11 @@ bool block_tables(const std::vector<BitTerm> &terms, int lo_bits, const std::vec
       w.slots.push_back(gather_warp(ptr.data(), ent.data(), k.n, &w.code[g]));
     }
   };
-  // lists first: their limits decline without the gather tables.  ~10 ns per block and term, 100
-  // per gather entry (about half the terms act on a row)
+  // lists first: their limits decline without the gather tables.  ~6 ns per block and term, 500 per
+  // warp and lower-half term (up to 32 entries, about half of them there)
   size_t n_lo = 0;
   for (const auto &g : lo) n_lo += g.size();
-  host_parallel((int64_t)(runs.size() + warps.size()), 0.01 * (double)(b_ib.size() * hi.size()) + 1.5 * (double)(warps.size() * n_lo),
+  host_parallel((int64_t)(runs.size() + warps.size()), 0.006 * (double)(b_ib.size() * hi.size()) + 0.5 * (double)(warps.size() * n_lo),
                 [&](int64_t k) {
                   if (!fits) return;
                   if (k < (int64_t)runs.size()) list_run((size_t)k);

@@ -263,10 +263,12 @@ int green_batches(Sector *s, const T *d_v, const std::vector<GreenTerm> &nz, std
   constexpr int W = GreenWidth<T>::w, NB = kGreenAcc / W;
   // the block kernels read whole complex elements; a vector at another address takes the row kernel
   // (as does a sector whose pieces there is no memory for)
+  bool blocks = !s->gc && s->lo_bits <= 31 && s->hi_bits <= 31 && whole_elements(W == 2 ? kComplex128 : kReal64, d_v);
   std::string err;
-  const bool blocks = !s->gc && s->lo_bits <= 31 && s->hi_bits <= 31 &&
-                      whole_elements(W == 2 ? kComplex128 : kReal64, d_v) && sector_pieces(s, &err) == 0;
-  cudaGetLastError();
+  if (blocks && sector_pieces(s, &err) != 0) {
+    cudaGetLastError();
+    blocks = false;
+  }
   const uint64_t lo_mask = s->ihfbit - 1;
   auto halves = [&](const GreenTerm &t) {
     const int b = s->lo_bits;
@@ -306,13 +308,21 @@ int green_batches(Sector *s, const T *d_v, const std::vector<GreenTerm> &nz, std
   // one workspace: upper halves, a pass's table, the entries' sums, a pass's records and pieces' sums
   const size_t nrec = (size_t)grid * kGreenAcc, nout = noff * kGreenAcc + dg.size();
   const size_t ntab = blocks && noff ? (sizeof(uint32_t) * (size_t)NB * s->nlow + 15) / 16 * 2 : 0;
-  // pieces' sums of as many patterns as 128 MB hold, whole passes
-  const size_t nkeep = std::max<size_t>(1, ((size_t)1 << 24) / std::max(1, s->npieces) / kGreenDiag) * kGreenDiag;
-  const size_t nsum = std::min(pats.size(), nkeep) * (size_t)s->npieces, nup = (sizeof(GreenUpper) * upper.size()) / sizeof(double);
+  // pieces' sums of as many patterns as 128 MB hold, whole passes; of one pass where that is too much
+  size_t nkeep = std::max<size_t>(1, ((size_t)1 << 24) / std::max(1, s->npieces) / kGreenDiag) * kGreenDiag;
+  const size_t nup = (sizeof(GreenUpper) * upper.size()) / sizeof(double);
+  auto bytes = [&]() {
+    const size_t nsum = std::min(pats.size(), nkeep) * (size_t)s->npieces;
+    return sizeof(double) * std::max<size_t>(1, nrec + nout + nout % 2 + ntab + nup + nsum);
+  };
   GreenSpace ws;
-  if (cudaMalloc(&ws.p, sizeof(double) * std::max<size_t>(1, nrec + nout + nout % 2 + ntab + nup + nsum)) != cudaSuccess) {
-    set_error("Green's functions: device allocation failed");
-    return -1;
+  if (cudaMalloc(&ws.p, bytes()) != cudaSuccess) {
+    cudaGetLastError();
+    nkeep = kGreenDiag;
+    if (cudaMalloc(&ws.p, bytes()) != cudaSuccess) {
+      set_error("Green's functions: device allocation failed");
+      return -1;
+    }
   }
   GreenUpper *d_up = reinterpret_cast<GreenUpper *>(ws.p);  // 16-byte units first
   uint32_t *d_tab = reinterpret_cast<uint32_t *>(ws.p + nup);

@@ -97,7 +97,7 @@ class Pool {
 void host_parallel(int64_t n, double us, const std::function<void(int64_t)> &f) {
   static Pool pool;
   const int cores = std::max(1, (int)std::thread::hardware_concurrency());
-  const int helpers = (int)std::min<int64_t>({7, cores - 1, n - 1, (int64_t)(us / 100.0)});
+  const int helpers = (int)std::min<int64_t>({7, cores - 1, n - 1, (int64_t)(us / 200.0)});
   if (helpers > 0 && pool.run(n, helpers, f)) return;
   for (int64_t k = 0; k < n; k++) f(k);
 }

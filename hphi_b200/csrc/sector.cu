@@ -297,13 +297,13 @@ int split_plan_for_terms(Sector *s, const std::vector<BitTerm> &T, SplitPlan *pl
   // room for a slot per term, cut to those in use below; counted first where that is much
   size_t most = lo_t.size();
   if (most * nlo > ((size_t)1 << 22)) {
-    host_parallel((int64_t)n_lo, 0.005 * (double)(nlo * lo_t.size()), [&](int64_t u) {
+    host_parallel((int64_t)n_lo, 0.0025 * (double)(nlo * lo_t.size()), [&](int64_t u) {
       for (uint64_t ia = u * kRun; ia < std::min(nlo, (u + 1) * kRun); ia++) lower(ia, false);
     });
     most = *std::max_element(lo_ptr.begin(), lo_ptr.end());
   }
   lo_ent.resize(most * nlo);
-  host_parallel((int64_t)(n_lo + n_hi), 0.005 * (double)(nlo * lo_t.size() + nhi * hi_t.size()), [&](int64_t q) {
+  host_parallel((int64_t)(n_lo + n_hi), 0.0025 * (double)(nlo * lo_t.size() + nhi * hi_t.size()), [&](int64_t q) {
     const uint64_t u = (uint64_t)q;
     if (u < n_lo)
       for (uint64_t ia = u * kRun; ia < std::min(nlo, (u + 1) * kRun); ia++) lower(ia, true);

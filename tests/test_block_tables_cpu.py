@@ -14,7 +14,7 @@ from hphi_b200 import expert
 
 
 @pytest.fixture(scope="session")
-def checker(tmp_path_factory):
+def tables_check(tmp_path_factory):
     lib = hphi_b200.library_path()
     exe = str(tmp_path_factory.mktemp("host") / "block_tables_check")
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
@@ -78,31 +78,31 @@ for _k in range(24):
 
 
 @pytest.mark.parametrize("name", list(MODELS))
-def test_block_tables(name, checker, tmp_path):
-    r = subprocess.run([checker, MODELS[name]().write(str(tmp_path))], capture_output=True, text=True)
+def test_block_tables(name, tables_check, tmp_path):
+    r = subprocess.run([tables_check, MODELS[name]().write(str(tmp_path))], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
     if not name.startswith("random"):
         assert "shape" in r.stdout  # the plan applies
 
 
-def test_many_crossing_terms(checker, tmp_path):
+def test_many_crossing_terms(tables_check, tmp_path):
     """100 bonds between the halves, each acting on every block: too many for whole products, not for the
     row-block plan's row pass."""
     m = expert.heisenberg(20, [(i, j) for i in range(10) for j in range(10, 20)], two_sz=-14)
-    r = subprocess.run([checker, m.write(str(tmp_path))], capture_output=True, text=True)
+    r = subprocess.run([tables_check, m.write(str(tmp_path))], capture_output=True, text=True)
     assert r.returncode == 0 and r.stdout.startswith("no plan shape"), r.stdout + r.stderr
 
 
-def test_crowded_bank(checker):
+def test_crowded_bank(tables_check):
     """More entries on one bank pair than a packed slot count holds: the plan must not lose any."""
-    r = subprocess.run([checker, "crowded"], capture_output=True, text=True)
+    r = subprocess.run([tables_check, "crowded"], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
 
 
 @pytest.mark.parametrize("gc", [False, True])
-def test_plans_without_device_memory(gc, checker, tmp_path):
+def test_plans_without_device_memory(gc, tables_check, tmp_path):
     """The plans are optional: where the device gives no memory for one, opening the sector goes on."""
     m = expert.kitaev_heisenberg(5, 2, -1.0, 0.3) if gc else expert.heisenberg(12, expert.chain_bonds(12))
-    r = subprocess.run([checker, m.write(str(tmp_path)), "no_memory"], capture_output=True, text=True,
+    r = subprocess.run([tables_check, m.write(str(tmp_path)), "no_memory"], capture_output=True, text=True,
                        env={**os.environ, "CUDA_VISIBLE_DEVICES": ""})
     assert r.returncode == 0, r.stdout + r.stderr
